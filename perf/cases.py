@@ -78,7 +78,7 @@ def listed():
         dict(name="mixed_96x4", kind="mixed", shape="96x96x96x96", ranks="16x16x16x16",
              prec="xh", sweeps=30, tol=1e-9, noise=1e-6, decay=0.9, stream="side"),
         # Tensor-core sweeps of an ordinary size, called from the default stream.
-        dict(name="mixed_3way", kind="mixed", shape="128x160x96", ranks="16x8x16", prec="x2",
+        dict(name="mixed_3way", kind="mixed", shape="128x112x96", ranks="16x8x16", prec="x2",
              sweeps=5, tol=0.0, noise=1e-6, decay=0.9, stream="default"),
         # The batch configuration: 4096 tensors.
         dict(name="batched_4096", kind="batched", count=4096, lo=8, hi=64, rlo=2, rhi=8,
@@ -127,8 +127,10 @@ def draw(rng):
                     tol=0.0, noise=1e-4, decay=1.0, stream=stream)
     if kind == "mixed":
         nd = rng.choice([3, 4])
-        side = _log_between(rng, 1e6, 6e7) ** (1.0 / nd)
-        shape = [min(256, max(16, 8 * int(side * rng.uniform(0.8, 1.25) / 8))) for _ in range(nd)]
+        # Modes the tensor cores take: multiples of 8 up to 128, the first from 64.
+        shape = [8 * rng.randint(8, 16)]
+        side = (_log_between(rng, 1e6, 6e7) / shape[0]) ** (1.0 / (nd - 1))
+        shape += [8 * min(16, max(2, int(side * rng.uniform(0.8, 1.25) / 8))) for _ in range(nd - 1)]
         ranks = [rng.choice([8, 16]) for _ in shape]
         return dict(kind="mixed", shape=_text(shape), ranks=_text(ranks),
                     prec=rng.choice(["xh", "x2"]), sweeps=rng.randint(2, 5), tol=0.0, noise=1e-6,
