@@ -1016,18 +1016,18 @@ __global__ void chol_lower_inv_kernel(const double *Gg, int r, double *Linv, int
 }
 
 // Row Gram on the FP64 tensor cores (mma.sync m8n8k4): A is r x m col-major
-// (factor row k = column k), G = sum_k a_k a_k^T.  With 4 columns per k-step,
-// the fragment A[g][t] = a_{4kk+t}(8h + g) is also the B fragment B[t][g] of
-// tile h, so each lane loads TT values per k-step for TT x TT MMAs.  Warps of
-// a block take interleaved k-steps of the block's column range; tiles are
-// summed over the warps in a fixed order into part[block][r*r].
+// (factor row k = column k), G = sum_k a_k a_k^T, finished to L^{-1} of its
+// Cholesky factor (gram_finish).  With 4 columns per k-step, the fragment
+// A[g][t] = a_{4kk+t}(8h + g) is also the B fragment B[t][g] of tile h, so
+// each lane loads TT values per k-step for TT x TT MMAs.  Warps of a block
+// take interleaved k-steps of the block's column range.
 template <int RT>
-__global__ void __launch_bounds__(256) rows_gram_mma_kernel(const double *__restrict__ A, int r,
-                                                            int64_t m, int64_t cols_per_block,
-                                                            double *__restrict__ part) {
+__global__ void __launch_bounds__(256) rows_gram_kernel(const double *__restrict__ A, int r,
+                                                        int64_t m, int64_t cols_per_block,
+                                                        GramFinish f) {
     constexpr int TT = RT / 8;
-    __shared__ double red[4][RT * RT];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
+    pdl_wait();
     const int64_t k0 = blockIdx.x * cols_per_block;
     const int64_t k1 = min(m, k0 + cols_per_block);
     double acc[TT][TT][2];
@@ -1038,60 +1038,35 @@ __global__ void __launch_bounds__(256) rows_gram_mma_kernel(const double *__rest
 #pragma unroll 4
     for (int64_t c0 = k0 + 4 * w; c0 < k1; c0 += 32) {
         const int64_t col = c0 + t;
-        double f[TT];
+        double v[TT];
 #pragma unroll
         for (int h = 0; h < TT; h++)
-            f[h] = (col < k1 && 8 * h + g < r) ? A[col * r + 8 * h + g] : 0.0;
+            v[h] = (col < k1 && 8 * h + g < r) ? A[col * r + 8 * h + g] : 0.0;
 #pragma unroll
         for (int a = 0; a < TT; a++)
 #pragma unroll
-            for (int b = 0; b < TT; b++) {
-                asm volatile(
-                    "mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
-                    : "+d"(acc[a][b][0]), "+d"(acc[a][b][1])
-                    : "d"(f[a]), "d"(f[b]));
-            }
+            for (int b = 0; b < TT; b++) dmma884(acc[a][b][0], acc[a][b][1], v[a], v[b]);
     }
-    // Warps 0-3 store, warps 4-7 add theirs (fixed order), then 4 slots sum.
-    if (w < 4) {
-#pragma unroll
-        for (int a = 0; a < TT; a++)
-#pragma unroll
-            for (int b = 0; b < TT; b++)
-#pragma unroll
-                for (int q = 0; q < 2; q++)
-                    red[w][(8 * a + g) * RT + 8 * b + 2 * t + q] = acc[a][b][q];
-    }
-    __syncthreads();
-    if (w >= 4) {
-#pragma unroll
-        for (int a = 0; a < TT; a++)
-#pragma unroll
-            for (int b = 0; b < TT; b++)
-#pragma unroll
-                for (int q = 0; q < 2; q++)
-                    red[w - 4][(8 * a + g) * RT + 8 * b + 2 * t + q] += acc[a][b][q];
-    }
-    __syncthreads();
-    for (int e = threadIdx.x; e < r * r; e += blockDim.x) {
-        const int i = e / r, j = e - i * r;
-        double s = 0.0;
-#pragma unroll
-        for (int q = 0; q < 4; q++) s += red[q][i * RT + j];
-        part[(int64_t)blockIdx.x * r * r + i * r + j] = s;
-    }
+    gram_finish<TT>(acc, r, f);
 }
 
-// T = Linv A on the FP64 tensor cores: Linv (r x r lower, col-major) is the A
-// operand (held in registers), 8-column blocks of A (r x m col-major) the B
-// operand; one warp per 8-column block.
-template <int RT>
-__global__ void __launch_bounds__(256) rows_apply_mma_kernel(const double *__restrict__ A, int r,
-                                                             int64_t m,
-                                                             const double *__restrict__ Linv,
-                                                             double *__restrict__ T) {
+// T = Linv A: Linv (r x r lower, col-major) is the A operand (held in
+// registers), 8-column blocks of A (r x m col-major) the B operand; one warp
+// per 8-column block.  Column k goes to column rows[k] of T when `rows` is
+// given.  GRAM: the Gram of T is taken on the way and finished to the next
+// pass's L^{-1}.  A lane's results are T(8 h + g, columns 2 t + q): taking the
+// block's even columns as one k-step and the odd ones as another, these are
+// its Gram fragments as they stand.
+template <int RT, bool GRAM>
+__global__ void __launch_bounds__(256) rows_apply_kernel(const double *__restrict__ A, int r,
+                                                         int64_t m,
+                                                         const double *__restrict__ Linv,
+                                                         double *__restrict__ T,
+                                                         const int32_t *__restrict__ rows,
+                                                         GramFinish f) {
     constexpr int TT = RT / 8, KS = RT / 4;
     const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+    pdl_wait();
     double la[TT][KS];
 #pragma unroll
     for (int h = 0; h < TT; h++)
@@ -1100,6 +1075,11 @@ __global__ void __launch_bounds__(256) rows_apply_mma_kernel(const double *__res
             const int i = 8 * h + g, c = 4 * kk + t;
             la[h][kk] = (i < r && c < r) ? Linv[i + (int64_t)r * c] : 0.0;
         }
+    double gacc[TT][TT][2];
+#pragma unroll
+    for (int a = 0; a < TT; a++)
+#pragma unroll
+        for (int b = 0; b < TT; b++) gacc[a][b][0] = gacc[a][b][1] = 0.0;
     const int64_t warp0 = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
     const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
     const int64_t nblk = (m + 7) / 8;
@@ -1108,53 +1088,36 @@ __global__ void __launch_bounds__(256) rows_apply_mma_kernel(const double *__res
 #pragma unroll
         for (int h = 0; h < TT; h++) acc[h][0] = acc[h][1] = 0.0;
         const int64_t colb = 8 * cb + g;
+        double b[KS];
 #pragma unroll
         for (int kk = 0; kk < KS; kk++) {
             const int c = 4 * kk + t;
-            const double b = (colb < m && c < r) ? A[colb * r + c] : 0.0;
+            b[kk] = (colb < m && c < r) ? A[colb * r + c] : 0.0;
+        }
+#pragma unroll
+        for (int kk = 0; kk < KS; kk++)
+#pragma unroll
+            for (int h = 0; h < TT; h++) dmma884(acc[h][0], acc[h][1], la[h][kk], b[kk]);
+        if (GRAM) {
+#pragma unroll
+            for (int q = 0; q < 2; q++)
+#pragma unroll
+                for (int x = 0; x < TT; x++)
+#pragma unroll
+                    for (int z = 0; z < TT; z++)
+                        dmma884(gacc[x][z][0], gacc[x][z][1], acc[x][q], acc[z][q]);
+        }
+#pragma unroll
+        for (int q = 0; q < 2; q++) {
+            const int64_t col = 8 * cb + 2 * t + q;
+            if (col >= m) continue;
+            double *dst = T + (rows ? (int64_t)rows[col] : col) * r;
 #pragma unroll
             for (int h = 0; h < TT; h++)
-                asm volatile(
-                    "mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
-                    : "+d"(acc[h][0]), "+d"(acc[h][1])
-                    : "d"(la[h][kk]), "d"(b));
+                if (8 * h + g < r) dst[8 * h + g] = acc[h][q];
         }
-#pragma unroll
-        for (int h = 0; h < TT; h++)
-#pragma unroll
-            for (int q = 0; q < 2; q++) {
-                const int64_t col = 8 * cb + 2 * t + q;
-                const int i = 8 * h + g;
-                if (col < m && i < r) T[col * r + i] = acc[h][q];
-            }
     }
-}
-
-// out[e] = sum_b part[b * n + e]: 64 outputs per CTA, 4 threads per output
-// each summing every 4th block into 4 accumulators (16 loads in flight), then
-// a fixed-order add (deterministic).
-__global__ void __launch_bounds__(256) sum_parts_kernel(const double *__restrict__ part, int nblk,
-                                                        int n, double *__restrict__ out) {
-    __shared__ double red[4][64];
-    const int s = threadIdx.x >> 6, o = threadIdx.x & 63;
-    for (int e0 = blockIdx.x * 64; e0 < n; e0 += gridDim.x * 64) {
-        const int e = e0 + o;
-        double a[4] = {0.0, 0.0, 0.0, 0.0};
-        if (e < n) {
-            int b = s;
-            for (; b + 12 < nblk; b += 16) {
-#pragma unroll
-                for (int j = 0; j < 4; j++) a[j] += part[(int64_t)(b + 4 * j) * n + e];
-            }
-#pragma unroll
-            for (int j = 0; j < 3; j++)
-                if (b + 4 * j < nblk) a[j] += part[(int64_t)(b + 4 * j) * n + e];
-        }
-        red[s][o] = (a[0] + a[1]) + (a[2] + a[3]);
-        __syncthreads();
-        if (s == 0 && e < n) out[e] = (red[0][o] + red[1][o]) + (red[2][o] + red[3][o]);
-        __syncthreads();
-    }
+    if (GRAM) gram_finish<TT>(gacc, r, f);
 }
 
 }  // namespace
@@ -1298,54 +1261,96 @@ void lu_inverse(dt_ctx *ctx, const double *A, int64_t n, double *Ainv, double *w
     DT_LAUNCH(ctx, lu_inverse_kernel, 1, LA_NT, n * sizeof(int), A, n, Ainv, work, flag);
 }
 
+size_t orth_scratch_bytes(const dt_ctx *ctx, int r, int64_t m) {
+    const int64_t blocks = orth_max_blocks(ctx), rr = (int64_t)r * r;
+    return (size_t)(r * m + rr * (blocks + (blocks + GRAM_GROUP - 1) / GRAM_GROUP + 2)) *
+           sizeof(double);
+}
+
+int64_t orth_max_blocks(const dt_ctx *ctx) {
+    return std::min<int64_t>(GRAM_MAX_BLOCKS, 4LL * ctx->num_sms);
+}
+
+OrthScratch orth_scratch(const dt_ctx *ctx, void *mem, int r, int64_t m, int *counters,
+                         int *flag) {
+    const int64_t blocks = orth_max_blocks(ctx), rr = (int64_t)r * r;
+    OrthScratch s;
+    double *p = static_cast<double *>(mem);
+    s.T = p;
+    p += r * m;
+    s.f.part = p;
+    p += rr * blocks;
+    s.f.group = p;
+    p += rr * ((blocks + GRAM_GROUP - 1) / GRAM_GROUP);
+    s.f.Linv = p;
+    s.Linv2 = p + rr;
+    s.f.counters = counters;
+    s.f.flag = flag;
+    return s;
+}
+
+void orth_finish(dt_ctx *ctx, const double *A, int r, int64_t m, const OrthScratch &s, double *out,
+                 const int32_t *rows) {
+    DT_CHECK_ARG(r > 0 && r <= 32, "orth_finish: bad row count %d", r);
+    GramFinish f2 = s.f;
+    f2.Linv = s.Linv2;
+    const unsigned gblocks = (unsigned)std::max<int64_t>(
+        1, std::min<int64_t>(((m + 7) / 8 + 7) / 8, orth_max_blocks(ctx)));
+    const unsigned ablocks = (unsigned)std::max<int64_t>(
+        1, std::min<int64_t>(((m + 7) / 8 + 7) / 8, 8LL * ctx->num_sms));
+#define DT_ROWS(R)                                                                          \
+    do {                                                                                    \
+        DT_LAUNCH_PDL(ctx, (rows_apply_kernel<R, true>), gblocks, 256, 0, A, r, m,          \
+                      (const double *)s.f.Linv, s.T, nullptr, f2);                          \
+        DT_LAUNCH_PDL(ctx, (rows_apply_kernel<R, false>), ablocks, 256, 0,                  \
+                      (const double *)s.T, r, m, (const double *)s.Linv2, out, rows, f2);   \
+    } while (0)
+    if (r <= 8) DT_ROWS(8);
+    else if (r <= 16) DT_ROWS(16);
+    else if (r <= 24) DT_ROWS(24);
+    else DT_ROWS(32);
+#undef DT_ROWS
+}
+
+void orth_check(dt_ctx *ctx, const int *flag) {
+    int h = 0;
+    DT_CUDA(cudaMemcpyAsync(&h, flag, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+    DT_CUDA(cudaStreamSynchronize(ctx->stream));
+    if (h) fail(DT_ERR_NUMERIC, "orth2: rows are linearly dependent");
+}
+
 void orth2_rows(dt_ctx *ctx, double *A, int64_t len1, int64_t len2) {
     // Gram-Schmidt over the rows of A (len1 x len2) equals A = L Q with L the
     // Cholesky factor of A A^T; two passes (CholeskyQR2) for FP64 accuracy.
     DT_CHECK_ARG(len1 > 0 && len1 <= 1024 && len2 >= len1, "orth2: bad sizes %lld x %lld",
                  (long long)len1, (long long)len2);
+    if (len1 <= 32) {
+        // Three launches: the Gram of A; T = L^{-1} A with the Gram of T; and
+        // the second pass's product.
+        const int r = (int)len1;
+        DevMem mem(ctx, orth_scratch_bytes(ctx, r, len2));
+        DevMem ints(ctx, (GRAM_COUNTERS + 1) * sizeof(int));
+        DT_CUDA(cudaMemsetAsync(ints.get(), 0, (GRAM_COUNTERS + 1) * sizeof(int), ctx->stream));
+        const OrthScratch s = orth_scratch(ctx, mem.get(), r, len2, ints.as<int>(),
+                                           ints.as<int>() + GRAM_COUNTERS);
+        const int64_t target = orth_max_blocks(ctx);
+        const int64_t cpb = std::max<int64_t>(256, (len2 + target - 1) / target);
+        const unsigned nblk = (unsigned)((len2 + cpb - 1) / cpb);
+        if (r <= 8) DT_LAUNCH_PDL(ctx, rows_gram_kernel<8>, nblk, 256, 0, A, r, len2, cpb, s.f);
+        else if (r <= 16)
+            DT_LAUNCH_PDL(ctx, rows_gram_kernel<16>, nblk, 256, 0, A, r, len2, cpb, s.f);
+        else if (r <= 24)
+            DT_LAUNCH_PDL(ctx, rows_gram_kernel<24>, nblk, 256, 0, A, r, len2, cpb, s.f);
+        else
+            DT_LAUNCH_PDL(ctx, rows_gram_kernel<32>, nblk, 256, 0, A, r, len2, cpb, s.f);
+        orth_finish(ctx, A, r, len2, s, A, nullptr);
+        orth_check(ctx, s.f.flag);
+        return;
+    }
     DevMem G(ctx, len1 * len1 * sizeof(double));
     DevMem Li(ctx, len1 * len1 * sizeof(double));
     DevMem flag(ctx, sizeof(int));
     DT_CUDA(cudaMemsetAsync(flag.get(), 0, sizeof(int), ctx->stream));
-    if (len1 <= 32) {
-        const int r = (int)len1;
-        const int64_t target = 2LL * ctx->num_sms;
-        const int64_t rpb = std::max<int64_t>(256, (len2 + target - 1) / target);
-        const int nblk = (int)((len2 + rpb - 1) / rpb);
-        DevMem part(ctx, (size_t)nblk * r * r * sizeof(double));
-        DevMem T(ctx, (size_t)r * len2 * sizeof(double));
-        const unsigned ablocks = std::max(
-            1u, std::min<unsigned>(ceil_div(len2 * r, 256), 16u * (unsigned)ctx->num_sms));
-        const int RT = r <= 8 ? 8 : (r <= 16 ? 16 : (r <= 24 ? 24 : 32));
-        const unsigned mblocks = (unsigned)std::max<int64_t>(
-            1, std::min<int64_t>(((len2 + 7) / 8 + 7) / 8, 8LL * ctx->num_sms));
-        for (int pass = 0; pass < 2; pass++) {
-            const double *src = pass == 0 ? A : T.as<double>();
-            double *dst = pass == 0 ? T.as<double>() : A;
-#define DT_ROWS(R)                                                                              \
-    do {                                                                                        \
-        DT_LAUNCH(ctx, rows_gram_mma_kernel<R>, nblk, 256, 0, src, r, len2, rpb,                \
-                  part.as<double>());                                                           \
-        DT_LAUNCH(ctx, sum_parts_kernel, ceil_div(r * r, 64), 256, 0, part.as<double>(), nblk,    \
-                  r * r,                                                                     \
-                  G.as<double>());                                                              \
-        DT_LAUNCH(ctx, chol_lower_inv_kernel, 1, 256, 2 * r * r * sizeof(double), G.as<double>(), \
-                  r, Li.as<double>(), flag.as<int>());                                          \
-        DT_LAUNCH(ctx, rows_apply_mma_kernel<R>, mblocks, 256, 0, src, r, len2, Li.as<double>(), \
-                  dst);                                                                         \
-    } while (0)
-            if (RT == 8) DT_ROWS(8);
-            else if (RT == 16) DT_ROWS(16);
-            else if (RT == 24) DT_ROWS(24);
-            else DT_ROWS(32);
-#undef DT_ROWS
-        }
-        int h = 0;
-        DT_CUDA(cudaMemcpyAsync(&h, flag.get(), sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
-        DT_CUDA(cudaStreamSynchronize(ctx->stream));
-        if (h) fail(DT_ERR_NUMERIC, "orth2: rows are linearly dependent");
-        return;
-    }
     DevMem T(ctx, len1 * len2 * sizeof(double));
     for (int pass = 0; pass < 2; pass++) {
         gemm_f64(ctx, 0, 1, len1, len1, len2, A, len1, A, len1, G.as<double>(), len1, 0.0);
@@ -1356,10 +1361,7 @@ void orth2_rows(dt_ctx *ctx, double *A, int64_t len1, int64_t len2) {
         DT_CUDA(cudaMemcpyAsync(A, T.get(), len1 * len2 * sizeof(double),
                                 cudaMemcpyDeviceToDevice, ctx->stream));
     }
-    int h = 0;
-    DT_CUDA(cudaMemcpyAsync(&h, flag.get(), sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
-    DT_CUDA(cudaStreamSynchronize(ctx->stream));
-    if (h) fail(DT_ERR_NUMERIC, "orth2: rows are linearly dependent");
+    orth_check(ctx, flag.as<int>());
 }
 
 }  // namespace dt

@@ -22,6 +22,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <type_traits>
 #include <vector>
 
 #include "dt_kernels.cuh"
@@ -30,7 +31,9 @@
 namespace dt {
 namespace {
 
-constexpr int64_t CHUNK = 512;
+// Chunks of the row layout: at most 512 nonzeros, down to 128 when the tensor
+// has too few for every warp of the GPU (32 per SM) to get one of 512.
+constexpr int64_t CHUNK_MIN = 128, CHUNK_MAX = 512;
 constexpr int FIB_CHUNK = 8;
 constexpr int64_t TASK_PACK_GRP = 128;
 constexpr int64_t TASK_PIECE_BATCHES = 64;
@@ -70,66 +73,6 @@ __global__ void gather_kernel(const T *__restrict__ src, const int32_t *__restri
 }
 
 // ---------------------------------------------------------------------------
-// TTMc row kernel (orders other than 3).  One warp per chunk.  Lane l owns
-// Kronecker entries p = l + 32 q (q < PL); per nonzero it multiplies the
-// value by the other factors' entries at its p.
-// ---------------------------------------------------------------------------
-template <int PL>
-__global__ void __launch_bounds__(256) ttmc_rows_kernel(
-    const int32_t *__restrict__ other, const double *__restrict__ val, int64_t nnz, int nother,
-    const int64_t *__restrict__ rowptr, const int32_t *__restrict__ chunk_row,
-    const int64_t *__restrict__ chunk_beg, const int32_t *__restrict__ chunk_slot,
-    int64_t nchunks, FactorSet f, int P, double *__restrict__ Yc, double *__restrict__ Ypart) {
-    const int lane = threadIdx.x & 31;
-    const int64_t warp0 = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
-    const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    for (int64_t c = warp0; c < nchunks; c += nwarps) {
-        const int32_t k = chunk_row[c];
-        const int64_t beg = chunk_beg[c];
-        const int64_t end = min(rowptr[k + 1], beg + CHUNK);
-        double acc[PL];
-#pragma unroll
-        for (int q = 0; q < PL; q++) acc[q] = 0.0;
-        for (int64_t e0 = beg; e0 < end; e0 += 32) {
-            const int64_t e = e0 + lane;
-            const bool ok = e < end;
-            int32_t myidx[MAXD - 1];
-#pragma unroll
-            for (int d = 0; d < MAXD - 1; d++)
-                myidx[d] = (d < nother && ok) ? other[(int64_t)d * nnz + e] : 0;
-            const double myv = ok ? val[e] : 0.0;
-            const int cnt = (int)(end - e0 < 32 ? end - e0 : 32);
-            for (int j = 0; j < cnt; j++) {
-                const double v = __shfl_sync(0xffffffffu, myv, j);
-                int32_t ix[MAXD - 1];
-#pragma unroll
-                for (int d = 0; d < MAXD - 1; d++) ix[d] = __shfl_sync(0xffffffffu, myidx[d], j);
-#pragma unroll
-                for (int q = 0; q < PL; q++) {
-                    int p = lane + 32 * q;
-                    if (p >= P) break;
-                    double prod = v;
-                    for (int d = 0; d < nother; d++) {
-                        const int r = f.R[d];
-                        const int pd = p % r;
-                        p /= r;
-                        prod *= f.U[d][(int64_t)ix[d] * r + pd];
-                    }
-                    acc[q] += prod;
-                }
-            }
-        }
-        const int32_t slot = chunk_slot[c];
-        double *dst = slot < 0 ? Yc + (int64_t)k * P : Ypart + (int64_t)slot * P;
-#pragma unroll
-        for (int q = 0; q < PL; q++) {
-            const int p = lane + 32 * q;
-            if (p < P) dst[p] = acc[q];
-        }
-    }
-}
-
-// ---------------------------------------------------------------------------
 // FP64 tensor-core fragment helper (mma.sync m8n8k4 .f64).  Fragments: A[g][t]
 // and B[t][g] with g = lane / 4, t = lane % 4; the 8 x 8 result D[g][2t + {0,1}].
 // ---------------------------------------------------------------------------
@@ -137,6 +80,152 @@ __device__ __forceinline__ void sp_dmma(double &d0, double &d1, double a, double
     asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
                  : "+d"(d0), "+d"(d1)
                  : "d"(a), "d"(b));
+}
+
+// ---------------------------------------------------------------------------
+// TTMc row kernel (orders other than 3), on the FP64 tensor cores.  The other
+// modes are cut into a low group (the first nlo, fastest in the Kronecker
+// index) and a high group, so a nonzero's contribution is the outer product
+// of two short Kronecker rows and a chunk's is a matrix product over its
+// nonzeros:
+//     Y(ph, pl) = sum_e hi_e(ph) lo_e(pl),   p = pl + Plo ph,
+//     lo_e = v_e kron of the low factors' rows, hi_e = kron of the high ones'.
+// One warp per chunk takes four nonzeros per mma.sync step: lane (g, t)
+// computes hi of nonzero t at ph = 8 a + g and lo at pl = 8 b + g -- exactly
+// its A and B fragment elements, so nothing is computed twice, and the digits
+// of ph and pl are found once per warp.  STEPS steps are in flight together.
+// Bound by the gather latency of the factor rows (L2).  300,000 nonzeros on
+// 3001 x 2003 x 1009 x 501, ranks 5, 7, 6, 3: 0.95-1.5 ms per mode with a
+// lane per Kronecker entry that split p into digits for every nonzero,
+// 29-34 us here.
+// blockIdx.y: blocks of TA x TB tiles when the row has more.
+// ---------------------------------------------------------------------------
+template <int TA, int TB, int NO, int NLO>
+__global__ void __launch_bounds__(256) ttmc_rows_kernel(
+    const int32_t *__restrict__ other, const double *__restrict__ val, int64_t nnz, int nother_,
+    int nlo_, const int64_t *__restrict__ rowptr, const int32_t *__restrict__ chunk_row,
+    const int64_t *__restrict__ chunk_beg, const int32_t *__restrict__ chunk_slot,
+    int64_t nchunks, int chunk, FactorSet f, int Plo, int Phi, int ablocks,
+    double *__restrict__ Yc, double *__restrict__ Ypart) {
+    constexpr int STEPS = 2;
+    // NLO > 0: exactly NO other modes, NLO of them low, so no branch stands
+    // between one step's gathers; else both counts come at run time.
+    const int nother = NLO ? NO : nother_, nlo = NLO ? NLO : nlo_;
+    // A rank is below 1024 (the product of all is at most 1024): 10 bits per
+    // digit, at most min(NO, 6) digits to a group of several.
+    using Packed = typename std::conditional<NO <= 3, uint32_t, uint64_t>::type;
+    const int lane = threadIdx.x & 31, g = lane >> 2, t4 = lane & 3;
+    const int a0 = (int)(blockIdx.y % ablocks) * 8 * TA, b0 = (int)(blockIdx.y / ablocks) * 8 * TB;
+    const int64_t warp0 = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
+    const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
+    const int64_t P = (int64_t)Plo * Phi;
+    Packed da[TA], db[TB];
+    bool oka[TA], okb[TB];
+#pragma unroll
+    for (int a = 0; a < TA; a++) {
+        int x = a0 + 8 * a + g;
+        oka[a] = x < Phi;
+        if (!oka[a]) x = 0;
+        da[a] = 0;
+        for (int d = nlo; d < nother; d++) {
+            da[a] |= (Packed)(x % f.R[d]) << (10 * (d - nlo));
+            x /= f.R[d];
+        }
+    }
+#pragma unroll
+    for (int b = 0; b < TB; b++) {
+        int x = b0 + 8 * b + g;
+        okb[b] = x < Plo;
+        if (!okb[b]) x = 0;
+        db[b] = 0;
+        for (int d = 0; d < nlo; d++) {
+            db[b] |= (Packed)(x % f.R[d]) << (10 * d);
+            x /= f.R[d];
+        }
+    }
+    for (int64_t c = warp0; c < nchunks; c += nwarps) {
+        const int32_t k = chunk_row[c];
+        const int64_t beg = chunk_beg[c];
+        const int64_t end = min(rowptr[k + 1], beg + chunk);
+        double acc[TA][TB][2];
+#pragma unroll
+        for (int a = 0; a < TA; a++)
+#pragma unroll
+            for (int b = 0; b < TB; b++) acc[a][b][0] = acc[a][b][1] = 0.0;
+        int32_t myidx[NO];
+        double myv;
+        auto load = [&](int64_t e) {
+            const bool ok = e < end;
+#pragma unroll
+            for (int d = 0; d < NO; d++)
+                myidx[d] = (d < nother && ok) ? other[(int64_t)d * nnz + e] : 0;
+            myv = ok ? val[e] : 0.0;
+        };
+        load(beg + lane);
+        for (int64_t e0 = beg; e0 < end; e0 += 32) {
+            int32_t idx[NO];
+            const double v32 = myv;
+#pragma unroll
+            for (int d = 0; d < NO; d++) idx[d] = myidx[d];
+            if (e0 + 32 < end) load(e0 + 32 + lane);  // in flight behind this batch
+            const int cnt = (int)(end - e0 < 32 ? end - e0 : 32);
+            for (int s0 = 0; 4 * s0 < cnt; s0 += STEPS) {
+                double hi[STEPS][TA], lo[STEPS][TB];
+#pragma unroll
+                for (int s = 0; s < STEPS; s++) {
+                    const int j = (4 * (s0 + s) + t4) & 31;
+                    const bool ok = 4 * (s0 + s) + t4 < cnt;
+                    const double v = __shfl_sync(0xffffffffu, v32, j);
+                    // Lanes without a nonzero or an entry gather row 0 or digit
+                    // 0 (no branch around a load) and drop the product.
+#pragma unroll
+                    for (int a = 0; a < TA; a++) hi[s][a] = 1.0;
+#pragma unroll
+                    for (int b = 0; b < TB; b++) lo[s][b] = v;
+#pragma unroll
+                    for (int d = 0; d < NO; d++) {
+                        if (d >= nother) break;
+                        const int32_t i = __shfl_sync(0xffffffffu, idx[d], j);
+                        const double *u = f.U[d] + (int64_t)i * f.R[d];
+                        if (d < nlo) {
+#pragma unroll
+                            for (int b = 0; b < TB; b++)
+                                lo[s][b] *= __ldg(u + ((int)(db[b] >> (10 * d)) & 1023));
+                        } else {
+#pragma unroll
+                            for (int a = 0; a < TA; a++)
+                                hi[s][a] *= __ldg(u + ((int)(da[a] >> (10 * (d - nlo))) & 1023));
+                        }
+                    }
+#pragma unroll
+                    for (int a = 0; a < TA; a++) hi[s][a] = ok && oka[a] ? hi[s][a] : 0.0;
+#pragma unroll
+                    for (int b = 0; b < TB; b++) lo[s][b] = ok && okb[b] ? lo[s][b] : 0.0;
+                }
+#pragma unroll
+                for (int s = 0; s < STEPS; s++)
+#pragma unroll
+                    for (int a = 0; a < TA; a++)
+#pragma unroll
+                        for (int b = 0; b < TB; b++)
+                            sp_dmma(acc[a][b][0], acc[a][b][1], hi[s][a], lo[s][b]);
+            }
+        }
+        // D[row g][cols 2 t, 2 t + 1] of tile (a, b): ph = a0 + 8 a + g,
+        // pl = b0 + 8 b + 2 t + h.
+        const int32_t slot = chunk_slot[c];
+        double *dst = slot < 0 ? Yc + (int64_t)k * P : Ypart + (int64_t)slot * P;
+#pragma unroll
+        for (int a = 0; a < TA; a++)
+#pragma unroll
+            for (int b = 0; b < TB; b++)
+#pragma unroll
+                for (int h = 0; h < 2; h++) {
+                    const int pl = b0 + 8 * b + 2 * t4 + h;
+                    if (oka[a] && pl < Plo)
+                        dst[pl + (int64_t)Plo * (a0 + 8 * a + g)] = acc[a][b][h];
+                }
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -556,15 +645,19 @@ __global__ void __launch_bounds__(1024) combine_partials_kernel(
 // loads hit distinct banks.
 // ---------------------------------------------------------------------------
 
-// out[rows[k] * Rn + r] = sum_p Yc[k, p] L[p + P r].  One warp per 8 compact
-// rows; NTL = ceil(Rn / 8) output tiles.  L staged in shared memory (pitch
-// 8 NTL + 4) when LSM, else read through the read-only cache.
-template <int NTL, bool LSM>
+// W(r, k) = sum_p L[p + P r] Yc[k, p].  One warp per 8 compact rows k;
+// NTL = ceil(Rn / 8) output tiles.  L staged in shared memory (pitch
+// 8 NTL + 4) when LSM, else read through the read-only cache.  ORTH: W goes to
+// out[k Rn + r] (compact) and the kernel finishes its Gram, the first pass of
+// the row orthonormalisation: with L as the A operand a lane holds W(8 j + g,
+// rows 2 t + q), which are the Gram's fragments as they stand (even rows one
+// k-step, odd rows another).  Otherwise row k goes to out[rows[k] Rn + r].
+template <int NTL, bool LSM, bool ORTH>
 __global__ void __launch_bounds__(256) mtl_mma_kernel(const double *__restrict__ Yc,
                                                       const int32_t *__restrict__ rows,
                                                       int64_t nrows, int P,
                                                       const double *__restrict__ L, int Rn,
-                                                      double *__restrict__ out) {
+                                                      double *__restrict__ out, GramFinish f) {
     constexpr int LDL = 8 * NTL + 4;
     extern __shared__ __align__(16) double Ls[];
     const int P4 = (P + 3) & ~3;
@@ -580,6 +673,11 @@ __global__ void __launch_bounds__(256) mtl_mma_kernel(const double *__restrict__
     const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
     const int64_t mtiles = (nrows + 7) / 8;
     const int ksteps = P4 / 4;
+    double gacc[NTL][NTL][2];
+#pragma unroll
+    for (int a = 0; a < NTL; a++)
+#pragma unroll
+        for (int b = 0; b < NTL; b++) gacc[a][b][0] = gacc[a][b][1] = 0.0;
     for (int64_t mt = warp0; mt < mtiles; mt += nwarps) {
         const int64_t k = 8 * mt + g;
         const bool okr = k < nrows;
@@ -605,20 +703,30 @@ __global__ void __launch_bounds__(256) mtl_mma_kernel(const double *__restrict__
                     const double b =
                         LSM ? Ls[p * LDL + r]
                             : ((p < P && r < Rn) ? __ldg(L + p + (int64_t)P * r) : 0.0);
-                    sp_dmma(acc[j][0], acc[j][1], av[u], b);
+                    sp_dmma(acc[j][0], acc[j][1], b, av[u]);
                 }
             }
         }
-        if (okr) {
-            double *o = out + (int64_t)rows[k] * Rn;
+        if (ORTH) {
 #pragma unroll
-            for (int j = 0; j < NTL; j++) {
-                const int r = 8 * j + 2 * t;
-                if (r < Rn) o[r] = acc[j][0];
-                if (r + 1 < Rn) o[r + 1] = acc[j][1];
-            }
+            for (int q = 0; q < 2; q++)
+#pragma unroll
+                for (int a = 0; a < NTL; a++)
+#pragma unroll
+                    for (int b = 0; b < NTL; b++)
+                        sp_dmma(gacc[a][b][0], gacc[a][b][1], acc[a][q], acc[b][q]);
+        }
+#pragma unroll
+        for (int q = 0; q < 2; q++) {
+            const int64_t kr = 8 * mt + 2 * t + q;
+            if (kr >= nrows) continue;
+            double *o = out + (ORTH ? kr : (int64_t)rows[kr]) * Rn;
+#pragma unroll
+            for (int j = 0; j < NTL; j++)
+                if (8 * j + g < Rn) o[8 * j + g] = acc[j][q];
         }
     }
+    if (ORTH) gram_finish<NTL>(gacc, Rn, f);
 }
 
 // mTR partials: part[blk][p + P r] = sum over the block's compact rows k of
@@ -810,9 +918,13 @@ void build_mode_rows(dt_ctx *ctx, dt_sptensor *sp, int n, const std::vector<DevM
     std::vector<int32_t> crow, cslot, mrow, mfirst, mcount;
     std::vector<int64_t> cbeg;
     int64_t slots = 0;
+    const int64_t per_warp = (nnz + 32LL * ctx->num_sms - 1) / (32LL * ctx->num_sms);
+    const int64_t chunk =
+        std::min(CHUNK_MAX, std::max(CHUNK_MIN, (per_warp + 31) / 32 * 32));
+    mc.chunk = (int)chunk;
     for (int64_t k = 0; k < mc.nrows; k++) {
         const int64_t c = rowptr[k + 1] - rowptr[k];
-        const int64_t nch = (c + CHUNK - 1) / CHUNK;
+        const int64_t nch = (c + chunk - 1) / chunk;
         if (nch > 1) {
             mrow.push_back((int32_t)k);
             mfirst.push_back((int32_t)slots);
@@ -820,7 +932,7 @@ void build_mode_rows(dt_ctx *ctx, dt_sptensor *sp, int n, const std::vector<DevM
         }
         for (int64_t j = 0; j < nch; j++) {
             crow.push_back((int32_t)k);
-            cbeg.push_back(rowptr[k] + j * CHUNK);
+            cbeg.push_back(rowptr[k] + j * chunk);
             cslot.push_back(nch > 1 ? (int32_t)(slots + j) : -1);
         }
         if (nch > 1) slots += nch;
@@ -1075,16 +1187,58 @@ void build_mode(dt_ctx *ctx, dt_sptensor *sp, int n, const std::vector<DevMem> &
         build_mode_rows(ctx, sp, n, idx32, vals_dev);
 }
 
-template <int PL>
-void launch_rows(dt_ctx *ctx, const ModeCopy &mc, int nother, int64_t nnz, const FactorSet &f,
-                 int P, double *Yc, double *Ypart) {
-    const int64_t warps = mc.nchunks;
-    const unsigned blocks =
-        std::max(1u, std::min<unsigned>(ceil_div(warps, 8), 32u * (unsigned)ctx->num_sms));
-    DT_LAUNCH(ctx, ttmc_rows_kernel<PL>, blocks, 256, 0, mc.other.as<int32_t>(),
-              mc.val.as<double>(), nnz, nother, mc.rowptr.as<int64_t>(),
+template <int TA, int TB, int NO, int NLO>
+void launch_rows(dt_ctx *ctx, const ModeCopy &mc, int nother, int nlo, int64_t nnz,
+                 const FactorSet &f, int Plo, int Phi, double *Yc, double *Ypart) {
+    const int ab = (int)ceil_div(Phi, 8 * TA), bb = (int)ceil_div(Plo, 8 * TB);
+    const dim3 grid(std::max(1u, std::min<unsigned>(ceil_div(mc.nchunks, 8),
+                                                    32u * (unsigned)ctx->num_sms)),
+                    (unsigned)(ab * bb));
+    DT_LAUNCH(ctx, (ttmc_rows_kernel<TA, TB, NO, NLO>), grid, 256, 0, mc.other.as<int32_t>(),
+              mc.val.as<double>(), nnz, nother, nlo, mc.rowptr.as<int64_t>(),
               mc.chunk_row.as<int32_t>(), mc.chunk_beg.as<int64_t>(),
-              mc.chunk_slot.as<int32_t>(), mc.nchunks, f, P, Yc, Ypart);
+              mc.chunk_slot.as<int32_t>(), mc.nchunks, mc.chunk, f, Plo, Phi, ab, Yc, Ypart);
+}
+
+// Tiles per warp: up to four in each direction, up to six in one when the
+// other has a single one; longer sides go to blockIdx.y (which repeats the
+// other side's gathers).
+template <int TA, int NO, int NLO>
+void rows_dispatch_tb(dt_ctx *ctx, const ModeCopy &mc, int nother, int nlo, int64_t nnz,
+                      const FactorSet &f, int Plo, int Phi, double *Yc, double *Ypart) {
+#define DT_TB(B) launch_rows<TA, B, NO, NLO>(ctx, mc, nother, nlo, nnz, f, Plo, Phi, Yc, Ypart)
+    const int tb = (Plo + 7) / 8;
+    if constexpr (TA > 4) {
+        DT_TB(1);
+    } else {
+        if (tb == 1) DT_TB(1);
+        else if (tb == 2) DT_TB(2);
+        else if (tb == 3) DT_TB(3);
+        else if constexpr (TA == 1) {
+            if (tb == 5) DT_TB(5);
+            else if (tb == 6) DT_TB(6);
+            else DT_TB(4);
+        } else DT_TB(4);
+    }
+#undef DT_TB
+}
+
+template <int NO, int NLO>
+void rows_dispatch(dt_ctx *ctx, const ModeCopy &mc, int nother, int nlo, int64_t nnz,
+                   const FactorSet &f, int Plo, int Phi, double *Yc, double *Ypart) {
+#define DT_TA(A) rows_dispatch_tb<A, NO, NLO>(ctx, mc, nother, nlo, nnz, f, Plo, Phi, Yc, Ypart)
+    const int ta = (Phi + 7) / 8;
+    if constexpr (NO == 1) {
+        DT_TA(1);
+    } else {
+        if (ta == 1) DT_TA(1);
+        else if (ta == 2) DT_TA(2);
+        else if (ta == 3) DT_TA(3);
+        else if (ta == 5 && Plo <= 8) DT_TA(5);
+        else if (ta == 6 && Plo <= 8) DT_TA(6);
+        else DT_TA(4);
+    }
+#undef DT_TA
 }
 
 template <int TF, int TE, bool FLO>
@@ -1216,13 +1370,32 @@ void sp_ttmc_compact(dt_ctx *ctx, const dt_sptensor *sp, const double *const *Ut
     }
     DevMem part(ctx, std::max<int64_t>(mc.nslots, 1) * P * sizeof(double));
     if (timer) timer->begin();
-    const int PL = (P + 31) / 32;
-    if (PL <= 1) launch_rows<1>(ctx, mc, nd - 1, sp->nnz, f, P, Yc, part.as<double>());
-    else if (PL <= 2) launch_rows<2>(ctx, mc, nd - 1, sp->nnz, f, P, Yc, part.as<double>());
-    else if (PL <= 4) launch_rows<4>(ctx, mc, nd - 1, sp->nnz, f, P, Yc, part.as<double>());
-    else if (PL <= 8) launch_rows<8>(ctx, mc, nd - 1, sp->nnz, f, P, Yc, part.as<double>());
-    else if (PL <= 16) launch_rows<16>(ctx, mc, nd - 1, sp->nnz, f, P, Yc, part.as<double>());
-    else launch_rows<32>(ctx, mc, nd - 1, sp->nnz, f, P, Yc, part.as<double>());
+    // The cut between the low and the high group that needs the fewest tiles,
+    // then the fewest gathers (tiles of a side times its modes).
+    const int no = nd - 1;
+    int nlo = 1, Plo = f.R[0];
+    {
+        int64_t best = -1;
+        int lo = 1;
+        for (int c = 1; c <= std::max(1, no - 1); c++) {
+            lo *= f.R[c - 1];
+            const int hi = P / lo;
+            const int64_t ta = (hi + 7) / 8, tb = (lo + 7) / 8;
+            const int64_t cost = ta * tb * 64 + ta * (no - c) + tb * c;
+            if (best < 0 || cost < best) {
+                best = cost;
+                nlo = c;
+                Plo = lo;
+            }
+        }
+    }
+#define DT_ROWS(NO, NLO)                                                                   \
+    rows_dispatch<NO, NLO>(ctx, mc, no, nlo, sp->nnz, f, Plo, P / Plo, Yc, part.as<double>())
+    if (no == 1) DT_ROWS(1, 1);
+    else if (no == 3 && nlo == 1) DT_ROWS(3, 1);
+    else if (no == 3) DT_ROWS(3, 2);
+    else DT_ROWS(MAXD - 1, 0);
+#undef DT_ROWS
     if (mc.nmulti > 0) {
         const unsigned blocks = (unsigned)std::min<int64_t>(mc.nmulti, 65535);
         DT_LAUNCH(ctx, combine_partials_kernel, blocks, 256 * COMB_SPLIT, 0, part.as<double>(),
@@ -1264,38 +1437,44 @@ void sp_mtr(dt_ctx *ctx, const dt_sptensor *sp, const double *Yc, int mode, int 
               256, 0, part.as<double>(), nblk, n, L);
 }
 
+template <int N, bool ORTH>
+void launch_mtl(dt_ctx *ctx, const ModeCopy &mc, const double *Yc, int P, const double *L, int Rn,
+                double *out, const GramFinish &f) {
+    const size_t smem = (size_t)((P + 3) & ~3) * (8 * N + 4) * sizeof(double);
+    const bool lsm = smem <= 160 * 1024;
+    const int64_t most = ORTH ? orth_max_blocks(ctx) : 4LL * ctx->num_sms;
+    const unsigned blocks = std::max(
+        1u, std::min<unsigned>(ceil_div((mc.nrows + 7) / 8, 8), (unsigned)most));
+    if (lsm) {
+        auto kern = mtl_mma_kernel<N, true, ORTH>;
+        smem_limit(ctx, kern, smem);
+        DT_LAUNCH(ctx, kern, blocks, 256, smem, Yc, mc.rows.as<int32_t>(), mc.nrows, P, L, Rn, out,
+                  f);
+    } else {
+        DT_LAUNCH(ctx, (mtl_mma_kernel<N, false, ORTH>), blocks, 256, 0, Yc,
+                  mc.rows.as<int32_t>(), mc.nrows, P, L, Rn, out, f);
+    }
+}
+
+template <bool ORTH>
+void mtl_dispatch(dt_ctx *ctx, const ModeCopy &mc, const double *Yc, int P, const double *L, int Rn,
+                  double *out, const GramFinish &f) {
+    DT_CHECK_ARG(Rn <= 32, "sparse ttmc_mTL: R_n (%d) must be <= 32", Rn);
+    switch ((Rn + 7) / 8) {
+        case 1: launch_mtl<1, ORTH>(ctx, mc, Yc, P, L, Rn, out, f); break;
+        case 2: launch_mtl<2, ORTH>(ctx, mc, Yc, P, L, Rn, out, f); break;
+        case 3: launch_mtl<3, ORTH>(ctx, mc, Yc, P, L, Rn, out, f); break;
+        default: launch_mtl<4, ORTH>(ctx, mc, Yc, P, L, Rn, out, f); break;
+    }
+}
+
 void sp_mtl(dt_ctx *ctx, const dt_sptensor *sp, const double *Yc, int mode, int P,
             const double *L, int Rn, double *out) {
     const ModeCopy &mc = sp->modes[mode];
     SummaryScope sc(ctx, "Function::ttmc_mTL()", 2.0 * mc.nrows * P * Rn,
                     8.0 * mc.nrows * (P + Rn));
-    DT_CHECK_ARG(Rn <= 32, "sparse ttmc_mTL: R_n (%d) must be <= 32", Rn);
     DT_CUDA(cudaMemsetAsync(out, 0, sp->shape[mode] * Rn * sizeof(double), ctx->stream));
-    const int ntl = (Rn + 7) / 8;
-    const size_t smem = (size_t)((P + 3) & ~3) * (8 * ntl + 4) * sizeof(double);
-    const bool lsm = smem <= 160 * 1024;
-    const unsigned blocks = std::max(
-        1u, std::min<unsigned>(ceil_div((mc.nrows + 7) / 8, 8), 4u * (unsigned)ctx->num_sms));
-#define DT_MTL(N, S)                                                                         \
-    do {                                                                                     \
-        auto kern = mtl_mma_kernel<N, S>;                                                    \
-        const size_t sm = S ? smem : 0;                                                      \
-        smem_limit(ctx, kern, sm);                                                           \
-        DT_LAUNCH(ctx, kern, blocks, 256, sm, Yc, mc.rows.as<int32_t>(), mc.nrows, P, L, Rn, \
-                  out);                                                                      \
-    } while (0)
-    if (lsm) {
-        if (ntl == 1) DT_MTL(1, true);
-        else if (ntl == 2) DT_MTL(2, true);
-        else if (ntl == 3) DT_MTL(3, true);
-        else DT_MTL(4, true);
-    } else {
-        if (ntl == 1) DT_MTL(1, false);
-        else if (ntl == 2) DT_MTL(2, false);
-        else if (ntl == 3) DT_MTL(3, false);
-        else DT_MTL(4, false);
-    }
-#undef DT_MTL
+    mtl_dispatch<false>(ctx, mc, Yc, P, L, Rn, out, GramFinish{});
 }
 
 void detach_sptensors(dt_ctx *ctx) {
@@ -1513,24 +1692,49 @@ int dt_sp_hooi(dt_ctx *ctx, const dt_sptensor *sp, const int64_t *R, int max_swe
             maxYc = std::max<int64_t>(maxYc, sp->modes[m].nrows * kron_len(R, nd, m));
         DevMem Yc(ctx, maxYc * sizeof(double));
         DevMem L(ctx, 1024 * 32 * sizeof(double));
+        // W = Y_(n) L over the non-empty rows, and the orthonormalisation's
+        // scratch, for every mode in turn.
+        size_t wbytes = 8, obytes = 8;
+        for (int m = 0; m < nd; m++) {
+            wbytes = std::max(wbytes, (size_t)(sp->modes[m].nrows * R[m]) * sizeof(double));
+            obytes = std::max(obytes, orth_scratch_bytes(ctx, (int)R[m], sp->modes[m].nrows));
+        }
+        const size_t nints = GRAM_COUNTERS + nd;  // arrival counters, a flag per mode
+        DevMem W(ctx, wbytes), oscr(ctx, obytes), oints(ctx, nints * sizeof(int));
+        int *const dep = oints.as<int>() + GRAM_COUNTERS;
+        DT_CUDA(cudaMemsetAsync(oints.get(), 0, nints * sizeof(int), ctx->stream));
         LaunchTimer timer(ctx, true);  // TTMc launches, reported as ttm_x_*
         SummaryScope sc(ctx, "Algorithm::SpTucker::Sp_HOOI_ALS()");
         DT_CUDA(cudaEventRecord(ctx->ev_start, ctx->stream));
         for (int it = 0; it < max_sweeps; it++) {
             for (int n = 0; n < nd; n++) {
-                const int P = (int)kron_len(R, nd, n);
+                const ModeCopy &mc = sp->modes[n];
+                const int P = (int)kron_len(R, nd, n), Rn = (int)R[n];
+                double *Un = const_cast<double *>(ptrs[n]);
                 sp_ttmc_compact(ctx, sp, ptrs, R, n, Yc.as<double>(), &timer);
-                sp_mtr(ctx, sp, Yc.as<double>(), n, P, ptrs[n], (int)R[n], L.as<double>());
-                sp_mtl(ctx, sp, Yc.as<double>(), n, P, L.as<double>(), (int)R[n],
-                       const_cast<double *>(ptrs[n]));
+                sp_mtr(ctx, sp, Yc.as<double>(), n, P, Un, Rn, L.as<double>());
+                const OrthScratch os =
+                    orth_scratch(ctx, oscr.get(), Rn, mc.nrows, oints.as<int>(), dep + n);
+                {
+                    SummaryScope sm(ctx, "Function::ttmc_mTL()", 2.0 * mc.nrows * P * Rn,
+                                    8.0 * mc.nrows * (P + Rn));
+                    mtl_dispatch<true>(ctx, mc, Yc.as<double>(), P, L.as<double>(), Rn,
+                                       W.as<double>(), os.f);
+                }
                 SummaryScope so(ctx, "Operator::orth2()", 2.0 * R[n] * R[n] * sp->shape[n],
                                 8.0 * R[n] * sp->shape[n]);
-                orth2_rows(ctx, const_cast<double *>(ptrs[n]), R[n], sp->shape[n]);
+                // Rows without nonzeros are zero from the first sweep on.
+                if (it == 0)
+                    DT_CUDA(cudaMemsetAsync(Un, 0, sp->shape[n] * Rn * sizeof(double),
+                                            ctx->stream));
+                orth_finish(ctx, W.as<double>(), Rn, mc.nrows, os, Un, mc.rows.as<int32_t>());
             }
         }
+        // The last mode's Y is that of the final factors already: a sweep ends
+        // by updating that mode's own factor.
         const int last = nd - 1;
         const int P = (int)kron_len(R, nd, last);
-        sp_ttmc_compact(ctx, sp, ptrs, R, last, Yc.as<double>());
+        if (max_sweeps == 0) sp_ttmc_compact(ctx, sp, ptrs, R, last, Yc.as<double>());
         sp_mtr(ctx, sp, Yc.as<double>(), last, P, ptrs[last], (int)R[last], L.as<double>());
         DevMem g2(ctx, sizeof(double));
         sumsq(ctx, L.get(), DT_F64, (int64_t)P * R[last], g2.as<double>());
@@ -1538,6 +1742,12 @@ int dt_sp_hooi(dt_ctx *ctx, const dt_sptensor *sp, const int64_t *R, int max_swe
         double hg2 = 0.0;
         DT_CUDA(cudaMemcpyAsync(&hg2, g2.get(), sizeof(double), cudaMemcpyDeviceToHost,
                                 ctx->stream));
+        std::vector<int> dependent((size_t)nd);
+        DT_CUDA(cudaMemcpyAsync(dependent.data(), dep, nd * sizeof(int),
+                                cudaMemcpyDeviceToHost, ctx->stream));
+        DT_CUDA(cudaStreamSynchronize(ctx->stream));
+        for (int d : dependent)
+            if (d) fail(DT_ERR_NUMERIC, "orth2: rows are linearly dependent");
         if (G) {
             DevView g(ctx, G, (size_t)P * R[last] * sizeof(double), false, true);
             DT_CUDA(cudaMemcpyAsync(g.ptr(), L.get(), (size_t)P * R[last] * sizeof(double),

@@ -17,10 +17,11 @@ struct ModeCopy {
     int64_t nrows = 0;  // non-empty rows
     DevMem rows;        // int32 [nrows]: row id of compact row k
     // Row-kernel layout (orders other than 3): nonzeros sorted by this mode's
-    // index, cut into chunks of at most CHUNK nonzeros.
+    // index, cut into chunks of at most `chunk` nonzeros.
     DevMem other;       // int32 [ndim-1][nnz]: the other modes' indices, in mode order
     DevMem val;         // double [nnz]
     DevMem rowptr;      // int64 [nrows+1]
+    int chunk = 0;
     int64_t nchunks = 0;
     DevMem chunk_row;   // int32 [nchunks]: compact row of the chunk
     DevMem chunk_beg;   // int64 [nchunks]

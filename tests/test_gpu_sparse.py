@@ -73,6 +73,32 @@ def test_sparse_four_way_generic_path(ctx, oracle_sparse):
                     oracle_sparse.ttmc_mTR(idx, vals, shape, Ut, R, mode)) < 1e-12
 
 
+@pytest.mark.parametrize("shape,R", [
+    ((700, 90), (8, 31)), ((700, 90), (3, 1)), ((60, 40, 30, 20), (9, 8, 7, 5)),
+    ((60, 40, 30, 20), (1, 16, 4, 16)), ((60, 40, 30, 25), (2, 6, 7, 24)),
+    ((2000, 5, 6, 7), (10, 5, 6, 7)), ((30, 20, 12, 9, 7), (3, 5, 2, 4, 7)),
+    ((9, 8, 7, 6, 5, 4), (2, 3, 4, 2, 3, 4)), ((6, 5, 4, 4, 3, 3, 3, 2), (2, 2, 3, 2, 2, 3, 2, 2))])
+def test_row_kernel_orders_and_tile_edges(ctx, oracle_sparse, shape, R):
+    """The row kernel over two to eight modes: rows of one nonzero and rows of
+    several chunks, sides of the Kronecker cut at, below and above a tile.
+    Sums of up to a few thousand products with factors below 1: 1e-12."""
+    from diana_tucker_b200 import datasets
+    idx, vals, shape = datasets.sparse_zipf(shape, 6000, alpha=1.1, seed=len(shape))
+    Ut = _factors(shape, R, 21)
+    sp = ctx.sptensor(idx, vals, shape)
+    for mode in range(len(shape)):
+        assert _rel(sp.ttmc_rows(Ut, R, mode),
+                    oracle_sparse.ttmc_rows(idx, vals, shape, Ut, R, mode)) < 1e-12
+    Ut0 = _factors(shape, R, 22)
+    if all(R[m] <= np.prod([r for k, r in enumerate(R) if k != m]) for m in range(len(R))):
+        G, U, rep = sp.hooi(R, 2, Ut0)
+        Go, Uo, res = oracle_sparse.hooi(idx, vals, shape, R, 2, Ut0)
+        assert abs(rep["residual"] - res) < 1e-10
+        for n in range(len(shape)):
+            np.testing.assert_allclose(U[n].T @ U[n], np.eye(R[n]), atol=1e-12)
+    sp.close()
+
+
 def test_sparse_hooi_vs_oracle(ctx, oracle_sparse, zipf_small):
     idx, vals, shape = zipf_small
     R = (8, 8, 8)
