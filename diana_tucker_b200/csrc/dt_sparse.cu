@@ -1730,11 +1730,9 @@ int dt_sp_hooi(dt_ctx *ctx, const dt_sptensor *sp, const int64_t *R, int max_swe
                 orth_finish(ctx, W.as<double>(), Rn, mc.nrows, os, Un, mc.rows.as<int32_t>());
             }
         }
-        // The last mode's Y is that of the final factors already: a sweep ends
-        // by updating that mode's own factor.
         const int last = nd - 1;
         const int P = (int)kron_len(R, nd, last);
-        if (max_sweeps == 0) sp_ttmc_compact(ctx, sp, ptrs, R, last, Yc.as<double>());
+        sp_ttmc_compact(ctx, sp, ptrs, R, last, Yc.as<double>());
         sp_mtr(ctx, sp, Yc.as<double>(), last, P, ptrs[last], (int)R[last], L.as<double>());
         DevMem g2(ctx, sizeof(double));
         sumsq(ctx, L.get(), DT_F64, (int64_t)P * R[last], g2.as<double>());
