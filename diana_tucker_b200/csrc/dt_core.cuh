@@ -13,6 +13,7 @@
 #include <functional>
 #include <memory>
 #include <unordered_set>
+#include <utility>
 #include <vector>
 
 #include "dt_cuda.h"
@@ -113,23 +114,39 @@ bool graphs_enabled();
 // Whether the Summary profiler is recording on ctx.
 bool summary_active(dt_ctx *ctx);
 
+// `cluster` > 1: the grid is made of thread-block clusters of that many CTAs.
 template <class... KArgs, class... Args>
-void launch_pdl(dt_ctx *ctx, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,
-                Args &&...args) {
+void launch_pdl_cluster(dt_ctx *ctx, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,
+                        int cluster, Args &&...args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = block;
     cfg.dynamicSmemBytes = smem;
     cfg.stream = ctx->stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
+    cudaLaunchAttribute attr[2];
     const bool plain_stream = ctx->stream != nullptr && ctx->stream != cudaStreamLegacy &&
                               ctx->stream != cudaStreamPerThread;
-    cfg.numAttrs = pdl_enabled() && plain_stream ? 1 : 0;
+    int n = 0;
+    if (pdl_enabled() && plain_stream) {
+        attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[n++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    if (cluster > 1) {
+        attr[n].id = cudaLaunchAttributeClusterDimension;
+        attr[n].val.clusterDim.x = cluster;
+        attr[n].val.clusterDim.y = 1;
+        attr[n++].val.clusterDim.z = 1;
+    }
+    cfg.attrs = attr;
+    cfg.numAttrs = n;
     DT_CUDA(cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...));
     ctx->launches++;
+}
+
+template <class... KArgs, class... Args>
+void launch_pdl(dt_ctx *ctx, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,
+                Args &&...args) {
+    launch_pdl_cluster(ctx, kernel, grid, block, smem, 1, std::forward<Args>(args)...);
 }
 
 #define DT_LAUNCH_PDL(ctx, kernel, grid, block, smem, ...) \

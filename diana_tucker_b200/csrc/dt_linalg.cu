@@ -374,19 +374,25 @@ __global__ void __launch_bounds__(LA_NT) subspace_kernel(const double *Sg, int64
 
 // ---------------------------------------------------------------------------
 // Subspace iteration on the FP64 tensor-core path (mma.sync m8n8k4 .f64) for
-// n <= 256 and r <= RT (8, 16 or 32), one CTA of 8 warps.  Same schedule as
-// subspace_kernel (five products S Z, CholeskyQR after the 2nd and 4th,
-// CholeskyQR2 after the 5th).  Shared-memory layout:
-//  * S col-major with a leading dimension LDS = 4 (mod 16) and Z, Q row-major
-//    n8 x RT with pitch RT + 4: the 8 x 4 and 4 x 8 operand fragments then hit
-//    16 distinct 8-byte bank pairs per half-warp;
+// n <= 256 and r <= RT (8, 16 or 32), one thread-block cluster of C CTAs of 8
+// warps.  One SM's FP64 rate bounds a product S Z (96 x 96 x 16: 2300 cycles
+// at 64 FMA a cycle) and its shared memory holds S up to n = 130 only, so the
+// rows are dealt out: each CTA keeps its rows of S (S is symmetric: its
+// columns, contiguous in memory) in shared memory and computes its rows of
+// every product, reading its own full copy of Z, into the copies of all CTAs.
+// A CTA's rows of Z give its share of the r x r Gram, sent to all CTAs; each
+// adds the shares in the same order, factors the sum with one warp and applies
+// R^{-1} to its rows, so nothing but rows of Z and Gram shares crosses SMs.
+// Same schedule as subspace_kernel: CholeskyQR after every second product,
+// CholeskyQR and a correction after the last.  Cluster barriers: one per plain
+// product, two per CholeskyQR.  Shared-memory layout:
+//  * the CTA's rows of S with a pitch = 4 (mod 16) and Z, Q row-major n8 x RT
+//    with pitch RT + 4: the 8 x 4 and 4 x 8 operand fragments then hit 16
+//    distinct 8-byte bank pairs per half-warp;
 //  * rows n..n8-1 and columns r..RT-1 are zero padding, so every product,
 //    Gram and solve runs on whole 8 x 8 tiles.
-// S Z and Z R^{-1}: each warp owns whole m-tile rows (all RT/8 n-tiles, two
-// m-tiles interleaved).  Z^T Z: whole K split over warps when it has fewer
-// than 8 tiles, partials summed in a fixed order.  Cholesky and R^{-1} in
-// warp 0 (rsqrt per pivot, multiplications by the reciprocal diagonal).  A
-// Cholesky breakdown restarts from the caller's L with Householder steps.
+// A Cholesky breakdown restarts from the caller's L with Householder steps, on
+// the first CTA alone.
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ void la_cp_async16(void *smem, const void *gmem) {
     const unsigned d = (unsigned)__cvta_generic_to_shared(smem);
@@ -411,55 +417,6 @@ struct SmTile {
     static constexpr int LDR = RT + 4;  // R^{-1} pitch
     static constexpr int NT = RT / 8;   // n-tiles
 };
-
-__host__ __device__ inline int sm_lds(int n8) { return ((n8 + 11) / 16) * 16 + 4; }
-
-// dst = S src   (n8 x RT), S from shared (ld lds) or from global (ld n).
-template <int RT, int SMODE>
-__device__ __forceinline__ void sm_product(const double *Ss, int lds, const double *__restrict__ Sg,
-                                           int n, int n8, const double *src, double *dst) {
-    using T = SmTile<RT>;
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const int g = lane >> 2, t = lane & 3;
-    const int mtiles = n8 / 8, ksteps = (n + 3) / 4;
-    for (int mt0 = w; mt0 < mtiles; mt0 += 2 * SM_WARPS) {
-        const int mt1 = mt0 + SM_WARPS;
-        const bool two = mt1 < mtiles;
-        double acc[2][T::NT][2];
-#pragma unroll
-        for (int m = 0; m < 2; m++)
-#pragma unroll
-            for (int j = 0; j < T::NT; j++) acc[m][j][0] = acc[m][j][1] = 0.0;
-        const int i0 = 8 * mt0 + g, i1 = 8 * mt1 + g;
-#pragma unroll 4
-        for (int kk = 0; kk < ksteps; kk++) {
-            const int k = 4 * kk + t;
-            double a0, a1 = 0.0;
-            if (SMODE == S_FULL) {
-                a0 = Ss[i0 + lds * k];
-                if (two) a1 = Ss[i1 + lds * k];
-            } else {
-                a0 = (i0 < n && k < n) ? __ldg(Sg + i0 + (int64_t)n * k) : 0.0;
-                if (two) a1 = (i1 < n && k < n) ? __ldg(Sg + i1 + (int64_t)n * k) : 0.0;
-            }
-#pragma unroll
-            for (int j = 0; j < T::NT; j++) {
-                const double b = src[k * T::LDQ + 8 * j + g];
-                dmma884(acc[0][j][0], acc[0][j][1], a0, b);
-                if (two) dmma884(acc[1][j][0], acc[1][j][1], a1, b);
-            }
-        }
-#pragma unroll
-        for (int m = 0; m < 2; m++) {
-            if (m == 1 && !two) break;
-            const int row = 8 * (m ? mt1 : mt0) + g;
-#pragma unroll
-            for (int j = 0; j < T::NT; j++)
-                *reinterpret_cast<double2 *>(dst + row * T::LDQ + 8 * j + 2 * t) =
-                    make_double2(acc[m][j][0], acc[m][j][1]);
-        }
-    }
-}
 
 // dst = src Ri   (n8 x RT times RT x RT upper).
 template <int RT>
@@ -538,188 +495,213 @@ __device__ __forceinline__ void sm_gram(const double *src, int n, int r, double 
     __syncthreads();
 }
 
-// G = R^T R (R upper, overwriting the upper triangle of G; the strict lower
-// triangle is zeroed), with the whole CTA: per pivot k every thread reads the
-// pivot and row k, then the threads owning entries (i, j), k < i <= j, update
-// them while the owners of row k scale it.  Two barriers per pivot, no
-// divides.  dinv[k] = 1 / R(k, k) (1 for the padding).  Returns false on a
-// non-positive pivot (the same value in every thread).
+// Ri = R^{-1} (row-major, pitch LDR) of G = R^T R, by warp 0 (all threads call
+// it; ends with a barrier).  Returns false on a non-positive pivot.
 template <int RT>
-__device__ __forceinline__ bool sm_chol(double *G, double *dinv, int r) {
-    constexpr int EPT = (RT * RT + SM_NT - 1) / SM_NT;
-    const int t = threadIdx.x;
-    const double g00 = G[0];
-    bool ok = g00 > 0.0;
-    for (int k = 0; k < r; k++) {
-        const double d = G[k * RT + k];
-        ok = ok && (d > 1e-28 * g00);
-        const double ri = rsqrt(fmax(d, 1e-300));
-        double upd[EPT];
-#pragma unroll
-        for (int q = 0; q < EPT; q++) {
-            const int e = t + q * SM_NT, i = e / RT, j = e % RT;
-            upd[q] = (e < RT * RT && i > k && i <= j && j < r)
-                         ? (G[k * RT + i] * ri) * (G[k * RT + j] * ri)
-                         : 0.0;
-        }
-        __syncthreads();
-#pragma unroll
-        for (int q = 0; q < EPT; q++) {
-            const int e = t + q * SM_NT, i = e / RT, j = e % RT;
-            if (e < RT * RT && j < r) {
-                if (i > k && i <= j) G[e] -= upd[q];
-                else if (i == k && j >= k) G[e] *= ri;
-            }
-        }
-        if (t == k) dinv[k] = ri;
-        __syncthreads();
-    }
-    for (int e = t; e < RT * RT; e += SM_NT) {
-        const int i = e / RT, j = e % RT;
-        if (i > j) G[e] = 0.0;
-    }
-    if (t >= r && t < RT) dinv[t] = 1.0;
-    __syncthreads();
-    return ok;
-}
-
-// Warp 0: Ri = R^{-1} (row-major, pitch LDR) from R in the upper triangle of G
-// and dinv.  Lane c solves column c: x_i = (delta_{i,c} - sum_{j>i} R(i,j) x_j) dinv_i.
-template <int RT>
-__device__ __forceinline__ void sm_rinv(const double *G, double *Ri, const double *dinv) {
+__device__ __forceinline__ bool sm_chol_inv(const double *G, double *Ri, int r) {
     constexpr int LDR = SmTile<RT>::LDR;
-    const int lane = threadIdx.x & 31;
-    double x[RT];
+    __shared__ int good;
+    const int lane = threadIdx.x;
+    if (lane < 32) {
+        double y[RT];
+        const bool ok = warp_chol_linv<RT>(G, RT, r, y);
+        // Lane c holds column c of L^{-1} = row c of R^{-1}.
+        if (lane < RT) {
 #pragma unroll
-    for (int i = RT - 1; i >= 0; i--) {
-        double s0 = (i == lane) ? 1.0 : 0.0, s1 = 0.0;
-#pragma unroll
-        for (int j = i + 1; j < RT; j++) {
-            const double rij = G[i * RT + j];
-            if (j & 1)
-                s1 = fma(-rij, x[j], s1);
-            else
-                s0 = fma(-rij, x[j], s0);
+            for (int i = 0; i < RT; i++) Ri[lane * LDR + i] = i >= lane ? y[i] : 0.0;
         }
-        x[i] = (s0 + s1) * dinv[i];
+        if (lane == 0) good = ok;
     }
-    if (lane < RT) {
-#pragma unroll
-        for (int i = 0; i < RT; i++) Ri[i * LDR + lane] = i <= lane ? x[i] : 0.0;
-    }
-}
-
-// Cholesky + R^{-1} (all threads call it; ends with a barrier).
-template <int RT>
-__device__ __forceinline__ bool sm_chol_inv(double *G, double *Ri, double *dinv, int r) {
-    const bool ok = sm_chol<RT>(G, dinv, r);
-    if (threadIdx.x < 32) sm_rinv<RT>(G, Ri, dinv);
     __syncthreads();
-    return ok;
+    return good != 0;
 }
 
-// After one CholeskyQR pass, Q^T Q = I + E with E tiny.  When max |E| <= 1e-8,
-// C = I - E/2 + 3E^2/8 (the series of (I + E)^{-1/2}) makes Q C orthonormal to
-// rounding; C goes to Ri (pitch LDR) for sm_apply.  Returns false when E is too
-// large, and the caller runs a second CholeskyQR pass instead.  All threads.
+// After one CholeskyQR pass, Q^T Q = I + E with E tiny.  When max |E| <= 1e-9,
+// C = I - E/2 makes Q C orthonormal to rounding (the next term of the series of
+// (I + E)^{-1/2} is below 1e-17); C goes to Ri (pitch LDR) for the product.
+// Returns false when E is larger, and the caller runs a second CholeskyQR pass
+// instead.  All threads.
 template <int RT>
-__device__ __forceinline__ bool sm_polar_fix(const double *G, double *Ri, double *red) {
+__device__ __forceinline__ bool sm_polar_fix(const double *G, double *Ri) {
     constexpr int LDR = SmTile<RT>::LDR;
-    const int t = threadIdx.x;
-    double emax = 0.0;
-    for (int e = t; e < RT * RT; e += SM_NT) {
+    bool small = true;
+    for (int e = threadIdx.x; e < RT * RT; e += SM_NT) {
         const int a = e / RT, b = e % RT;
-        emax = fmax(emax, fabs(G[e] - (a == b ? 1.0 : 0.0)));
-    }
-    for (int o = 16; o > 0; o >>= 1) emax = fmax(emax, __shfl_xor_sync(0xffffffffu, emax, o));
-    if ((t & 31) == 0) red[t >> 5] = emax;
-    __syncthreads();
-    double m = 0.0;
-#pragma unroll
-    for (int w = 0; w < SM_WARPS; w++) m = fmax(m, red[w]);
-    if (!(m <= 1e-8)) {
-        __syncthreads();
-        return false;
-    }
-    for (int e = t; e < RT * RT; e += SM_NT) {
-        const int a = e / RT, b = e % RT;
-        double e2 = 0.0;
-#pragma unroll
-        for (int k = 0; k < RT; k++)
-            e2 = fma(G[a * RT + k] - (a == k ? 1.0 : 0.0), G[k * RT + b] - (k == b ? 1.0 : 0.0), e2);
         const double eab = G[e] - (a == b ? 1.0 : 0.0);
-        Ri[a * LDR + b] = (a == b ? 1.0 : 0.0) - 0.5 * eab + 0.375 * e2;
+        small = small && fabs(eab) <= 1e-9;
+        Ri[a * LDR + b] = (a == b ? 1.0 : 0.0) - 0.5 * eab;
     }
-    __syncthreads();
-    return true;
+    return __syncthreads_and(small) != 0;
 }
+
+// The cluster's CTAs: rank, size, barrier, and this CTA's address of shared
+// memory in another one.
+__device__ __forceinline__ unsigned cl_rank() {
+    unsigned v;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(v));
+    return v;
+}
+__device__ __forceinline__ void cl_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::
+                     : "memory");
+}
+__device__ __forceinline__ uint32_t cl_map(const void *p, unsigned rank) {
+    uint32_t a = (uint32_t)__cvta_generic_to_shared(p), out;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(out) : "r"(a), "r"(rank));
+    return out;
+}
+// Sends `bytes` of this CTA's shared memory at p to the same place in the CTAs
+// of the cluster and waits for what all of them send, `bytes_in` in sum (each
+// sends its own part of the same array).  The copies are the hardware's bulk
+// copies between shared memories and complete on the receiver's mbarrier, so an
+// exchange is one way across the SM network: rows stored one 16-byte word per
+// lane into every CTA and a cluster barrier took 1900 cycles more than the
+// product alone for 96 x 16 on four CTAs, 4400 for 200 x 16 on eight.  Steps
+// alternate between two mbarriers: a CTA can be one step ahead of another,
+// never two (its second step needs the other's first).  The sender's rows are
+// read before anybody can answer with the next step's data.  Returns false when
+// the bounded wait ran out (about a second).  All threads; ends like a barrier.
+struct ClExchange {
+    uint64_t *bar;  // two mbarriers, arrival count 1
+    int step;
+    unsigned csize, rank;
+};
+constexpr long long CL_WAIT_CYCLES = 2000000000LL;
+
+__device__ __forceinline__ bool cl_exchange(ClExchange &x, const void *p, uint32_t bytes,
+                                            uint32_t bytes_in) {
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    __syncthreads();
+    if (x.csize == 1) return true;
+    uint64_t *bar = x.bar + (x.step & 1);
+    const uint32_t parity = (x.step >> 1) & 1;
+    x.step++;
+    const uint32_t barl = (uint32_t)__cvta_generic_to_shared(bar);
+    if (threadIdx.x == 0)
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(barl),
+                     "r"(bytes_in)
+                     : "memory");
+    if (threadIdx.x < x.csize && threadIdx.x != x.rank && bytes > 0)
+        asm volatile(
+            "cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, "
+            "[%3];" ::"r"(cl_map(p, threadIdx.x)),
+            "r"((uint32_t)__cvta_generic_to_shared(p)), "r"(bytes), "r"(cl_map(bar, threadIdx.x))
+            : "memory");
+    long long t0 = 0;
+    for (;;) {
+        uint32_t ok;
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}"
+            : "=r"(ok)
+            : "r"(barl), "r"(parity)
+            : "memory");
+        if (ok) return true;
+        if (t0 == 0) t0 = clock64();
+        else if (clock64() - t0 > CL_WAIT_CYCLES) return false;
+    }
+}
+
+// Rows of S a CTA of a cluster of c owns (whole 8-row tiles), and the pitch of
+// a staged row.
+__host__ __device__ inline int sub_rows(int n, int c) { return 8 * (((n + 7) / 8 + c - 1) / c); }
+__host__ __device__ inline int sub_pitch(int n) { return ((n + 11) / 16) * 16 + 4; }
+// Gram shares are received in two alternating sets where they fit.
+template <int RT>
+__host__ __device__ constexpr int sub_sets() { return RT <= 16 ? 2 : 1; }
 
 template <int RT>
-__host__ __device__ inline size_t sm_smem_doubles(int n, bool s_in_smem) {
+__host__ inline size_t sub_smem_bytes(int n, int c, bool s_in_smem) {
     const int n8 = (n + 7) / 8 * 8;
-    size_t d = 2 * (size_t)n8 * SmTile<RT>::LDQ   // Z, Q
-               + (size_t)SM_GP                    // Gram partials
-               + (size_t)RT * RT                  // G / R
-               + (size_t)RT * SmTile<RT>::LDR     // R^{-1}
-               + 32;                              // dinv
-    if (s_in_smem) d += (size_t)sm_lds(n8) * n8;
-    return d;
+    size_t d = 2 * (size_t)n8 * SmTile<RT>::LDQ             // Z, Q
+               + (size_t)sub_sets<RT>() * c * RT * RT       // Gram shares
+               + (size_t)RT * RT                            // G
+               + (size_t)RT * SmTile<RT>::LDR;              // R^{-1}
+    if (s_in_smem) d += (size_t)sub_rows(n, c) * sub_pitch(n);
+    return d * sizeof(double);
 }
 
-template <int RT, int SMODE>
-__global__ void __launch_bounds__(SM_NT, 1) subspace_mma_kernel(const double *Sg, int n,
-                                                             double *Lg, int r, int iters,
-                                                             double *work, int *flag) {
+// One 8 x 8 tile of A B on two interleaved accumulation chains (one chain's 32
+// cycles an MMA would leave the pipe half idle): a(k), b(k) give the lane's
+// fragment elements of k-step k.
+template <class FA, class FB>
+__device__ __forceinline__ void sub_tile(int ksteps, double &d0, double &d1, FA a, FB b) {
+    double x0 = 0.0, x1 = 0.0, y0 = 0.0, y1 = 0.0;
+    int k = 0;
+#pragma unroll 4
+    for (; k + 1 < ksteps; k += 2) {
+        dmma884(x0, x1, a(k), b(k));
+        dmma884(y0, y1, a(k + 1), b(k + 1));
+    }
+    if (k < ksteps) dmma884(x0, x1, a(k), b(k));
+    d0 = x0 + y0;
+    d1 = x1 + y1;
+}
+
+template <int RT, bool SSM>
+__global__ void __launch_bounds__(SM_NT, 1) subspace_cluster_kernel(const double *Sg, int n,
+                                                                    double *Lg, int r, int iters,
+                                                                    double *work, int *flag,
+                                                                    int csize) {
     using T = SmTile<RT>;
+    constexpr int SETS = sub_sets<RT>();
     extern __shared__ __align__(16) double sm[];
     __shared__ double red[33];
-    __shared__ int bad;
-    const int t = threadIdx.x;
-    pdl_wait();
-    const int n8 = (n + 7) / 8 * 8;
-    const int lds = sm_lds(n8);
-    double *A = sm;
-    double *B = A + n8 * T::LDQ;
-    double *Gp = B + n8 * T::LDQ;
-    double *G = Gp + SM_GP;
+    __shared__ __align__(8) uint64_t bars[2];
+    const int t = threadIdx.x, lane = t & 31, w = t >> 5, g = lane >> 2, t4 = lane & 3;
+    const unsigned rank = cl_rank();
+    if (t == 0) {
+        for (int q = 0; q < 2; q++)
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(
+                             (uint32_t)__cvta_generic_to_shared(bars + q))
+                         : "memory");
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    ClExchange ex{bars, 0, (unsigned)csize, rank};
+    const int n8 = (n + 7) / 8 * 8, lds = sub_pitch(n);
+    const int own0 = (int)rank * sub_rows(n, csize);
+    const int own = max(0, min(n8 - own0, sub_rows(n, csize)));  // this CTA's rows
+    const int mt = own / 8, ksteps = (n + 3) / 4;
+    double *cur = sm;
+    double *oth = cur + n8 * T::LDQ;
+    double *shares = oth + n8 * T::LDQ;
+    double *G = shares + SETS * csize * RT * RT;
     double *Ri = G + RT * RT;
-    double *dinv = Ri + RT * T::LDR;
-    double *Ss = dinv + 32;
-    if (SMODE == S_FULL) {
-        // S goes global -> shared with asynchronous 16-byte copies (one
-        // latency for the whole matrix); the padding is zeroed meanwhile.
+    double *Ss = Ri + RT * T::LDR;
+    for (int e = t; e < 2 * n8 * T::LDQ; e += SM_NT) cur[e] = 0.0;  // both buffers
+    if (SSM) {
+        // Padding of the staged rows: k = n .. 4 ksteps - 1, and rows past n.
+        for (int e = t; e < own * (4 * ksteps - n); e += SM_NT) {
+            const int pr = 4 * ksteps - n;
+            Ss[(e / pr) * lds + n + e % pr] = 0.0;
+        }
+        for (int i = max(0, n - own0); i < own; i++)
+            for (int k = t; k < n; k += SM_NT) Ss[i * lds + k] = 0.0;
+    }
+    pdl_wait();
+    const int have = min(own, n - own0);  // rows of S there are (may be <= 0)
+    if (SSM) {
+        const double *src = Sg + (int64_t)n * own0;
         if ((n & 1) == 0) {
             const int hc = n / 2;
-            for (int e = t; e < hc * n; e += SM_NT) {
-                const int k = e / hc, q = e - k * hc;
-                la_cp_async16(Ss + lds * k + 2 * q, Sg + (int64_t)n * k + 2 * q);
+            for (int e = t; e < hc * have; e += SM_NT) {
+                const int i = e / hc, q = e - i * hc;
+                la_cp_async16(Ss + lds * i + 2 * q, src + (int64_t)n * i + 2 * q);
             }
             la_cp_commit();
         } else {
-            for (int e = t; e < n * n; e += SM_NT) {
-                const int k = e / n, i = e - k * n;
-                Ss[i + lds * k] = Sg[e];
+            for (int e = t; e < n * have; e += SM_NT) {
+                const int i = e / n, k = e - i * n;
+                Ss[lds * i + k] = src[e];
             }
         }
-        const int pr = lds - n;
-        for (int e = t; e < pr * n8; e += SM_NT) {
-            const int k = e / pr, i = n + (e - k * pr);
-            Ss[i + lds * k] = 0.0;
-        }
-        for (int e = t; e < (n8 - n) * n; e += SM_NT) {
-            const int k = n + e / n, i = e % n;
-            Ss[i + lds * k] = 0.0;
-        }
     }
-    // L (n x r col-major) -> A (row-major, pitch LDQ, zero padded): all loads
-    // of a thread are issued before its stores.
-    for (int e = t; e < n8 * T::LDQ; e += SM_NT) {
-        A[e] = 0.0;
-        B[e] = 0.0;
-    }
-    __syncthreads();
+    __syncthreads();  // the zeroed buffers
     {
-        constexpr int MAXQ = 32;  // n * r <= 256 * 32 = SM_NT * MAXQ
+        // L (n x r col-major) -> cur (row-major, zero padded): all loads of a
+        // thread are issued before its stores.
+        constexpr int MAXQ = RT;  // n * r <= 256 * RT = SM_NT * MAXQ
         double v[MAXQ];
 #pragma unroll
         for (int q = 0; q < MAXQ; q++) {
@@ -731,52 +713,137 @@ __global__ void __launch_bounds__(SM_NT, 1) subspace_mma_kernel(const double *Sg
             const int e = t + SM_NT * q;
             if (e < n * r) {
                 const int c = e / n, i = e - c * n;
-                A[i * T::LDQ + c] = v[q];
+                cur[i * T::LDQ + c] = v[q];
             }
         }
     }
-    if (SMODE == S_FULL && (n & 1) == 0) la_cp_wait_all();
-    if (t == 0) bad = 0;
-    __syncthreads();
+    if (SSM) la_cp_wait_all();
+    // Every CTA's buffers are ready before any CTA writes into them.
+    if (csize > 1) cl_sync();
+    else __syncthreads();
 
-    double *cur = A, *oth = B;
-    for (int it = 0; it < iters; it++) {
-        sm_product<RT, SMODE>(Ss, lds, Sg, n, n8, cur, oth);
-        __syncthreads();
-        double *tmp = cur;
-        cur = oth;
-        oth = tmp;
-        const bool last = it == iters - 1;
-        if (last || (it & 1)) {
-            const int passes = last ? 2 : 1;
-            for (int p = 0; p < passes; p++) {
-                sm_gram<RT>(cur, n, r, Gp, G);
-                // The second pass is usually a tiny correction (polar fix).
-                if (!(p == 1 && sm_polar_fix<RT>(G, Ri, red))) {
-                    if (!sm_chol_inv<RT>(G, Ri, dinv, r)) {
-                        bad = 1;
-                        break;
-                    }
-                }
-                sm_apply<RT>(cur, Ri, n8, oth);
-                __syncthreads();
-                tmp = cur;
-                cur = oth;
-                oth = tmp;
+    // dst(own rows) = S(own rows, :) src.
+    auto product = [&](const double *src, double *dst) {
+        for (int job = w; job < mt * T::NT; job += SM_WARPS) {
+            const int m = job / T::NT, j = job - m * T::NT;
+            double d0, d1;
+            if (SSM) {
+                const double *as = Ss + (8 * m + g) * lds + t4;
+                const double *bs = src + t4 * T::LDQ + 8 * j + g;
+                sub_tile(ksteps, d0, d1, [&](int k) { return as[4 * k]; },
+                         [&](int k) { return bs[4 * k * T::LDQ]; });
+            } else {
+                const int i = own0 + 8 * m + g;
+                sub_tile(ksteps, d0, d1,
+                         [&](int k) {
+                             const int kk = 4 * k + t4;
+                             return i < n && kk < n ? __ldg(Sg + (int64_t)n * i + kk) : 0.0;
+                         },
+                         [&](int k) { return src[(4 * k + t4) * T::LDQ + 8 * j + g]; });
             }
-            if (bad) break;
+            *reinterpret_cast<double2 *>(dst + (own0 + 8 * m + g) * T::LDQ + 8 * j + 2 * t4) =
+                make_double2(d0, d1);
         }
+    };
+    // Everybody's rows of z to everybody.
+    const uint32_t row_bytes = T::LDQ * sizeof(double);
+    auto exchange_rows = [&](double *z) {
+        return cl_exchange(ex, z + own0 * T::LDQ, own * row_bytes, (n8 - own) * row_bytes);
+    };
+    // This CTA's share of src^T src, to set `set` of all CTAs; then the sum of
+    // all shares in G (rows / columns >= r: the identity).
+    auto gram = [&](const double *src, int set) {
+        double *all = shares + set * csize * RT * RT, *mine = all + rank * RT * RT;
+        for (int job = w; job < T::NT * T::NT; job += SM_WARPS) {
+            const int ta = job % T::NT, tb = job / T::NT;
+            const double *as = src + (own0 + t4) * T::LDQ + 8 * ta + g;
+            const double *bs = src + (own0 + t4) * T::LDQ + 8 * tb + g;
+            double d0, d1;
+            sub_tile(2 * mt, d0, d1, [&](int k) { return as[4 * k * T::LDQ]; },
+                     [&](int k) { return bs[4 * k * T::LDQ]; });
+            *reinterpret_cast<double2 *>(mine + (8 * ta + g) * RT + 8 * tb + 2 * t4) =
+                make_double2(d0, d1);
+        }
+        const uint32_t bytes = RT * RT * sizeof(double);
+        const bool ok = cl_exchange(ex, mine, bytes, (csize - 1) * bytes);
+        for (int e = t; e < RT * RT; e += SM_NT) {
+            const int a = e / RT, b = e % RT;
+            double s = 0.0;
+            for (int q = 0; q < csize; q++) s += all[q * RT * RT + e];
+            G[e] = (a < r && b < r) ? s : (a == b ? 1.0 : 0.0);
+        }
+        __syncthreads();
+        return ok;
+    };
+    // dst(own rows) = src(own rows) Ri.
+    auto apply = [&](const double *src, double *dst) {
+        for (int job = w; job < mt * T::NT; job += SM_WARPS) {
+            const int m = job / T::NT, j = job - m * T::NT;
+            const double *as = src + (own0 + 8 * m + g) * T::LDQ + t4;
+            const double *bs = Ri + t4 * T::LDR + 8 * j + g;
+            double d0, d1;
+            sub_tile(RT / 4, d0, d1, [&](int k) { return as[4 * k]; },
+                     [&](int k) { return bs[4 * k * T::LDR]; });
+            *reinterpret_cast<double2 *>(dst + (own0 + 8 * m + g) * T::LDQ + 8 * j + 2 * t4) =
+                make_double2(d0, d1);
+        }
+    };
+
+    bool bad = false, late = false;
+    int set = 0;
+    for (int it = 0; it < iters && !late; it++) {
+        const bool last = it == iters - 1;
+        product(cur, oth);
+        if (!last && !(it & 1)) {
+            late = !exchange_rows(oth);
+            double *x = cur;
+            cur = oth;
+            oth = x;
+            continue;
+        }
+        __syncthreads();
+        late = !gram(oth, set);
+        if (SETS == 2) set ^= 1;
+        if (!sm_chol_inv<RT>(G, Ri, r)) {  // the same G, so the same answer, in every CTA
+            bad = true;
+            break;
+        }
+        // All CTAs are past their products (their shares came): cur is free.
+        apply(oth, cur);
+        if (!last) {
+            late = late || !exchange_rows(cur);
+            continue;
+        }
+        __syncthreads();
+        // Second pass on the last step, usually a tiny correction.  With one
+        // set of shares the other CTAs have to be done with theirs first.
+        if (SETS == 1 && csize > 1) cl_sync();
+        late = late || !gram(cur, set);
+        if (!sm_polar_fix<RT>(G, Ri) && !sm_chol_inv<RT>(G, Ri, r)) {
+            bad = true;
+            break;
+        }
+        apply(cur, oth);
+        __syncthreads();
+    }
+    // No CTA leaves while another still reads or fills its shared memory.
+    if (csize > 1) cl_sync();
+    if (late) {
+        // An exchange never came: NaN factors, which the driver reports.
+        for (int e = t; e < n * r; e += SM_NT) Lg[e] = __longlong_as_double(0x7ff8000000000000LL);
+        return;
     }
     // Dependents launch once the iteration is done (launched at the start,
     // they took SM slots for the whole kernel; about 1 % of a decomposition).
     pdl_trigger();
     if (!bad) {
-        for (int e = t; e < n * r; e += SM_NT) {
-            const int i = e % n, c = e / n;
-            Lg[e] = cur[i * T::LDQ + c];
+        for (int e = t; e < have * r; e += SM_NT) {
+            const int c = e / have, i = own0 + (e - c * have);
+            Lg[(int64_t)n * c + i] = oth[i * T::LDQ + c];
         }
         return;
     }
+    if (rank != 0) return;
     // Rank-deficient or badly conditioned: restart from the caller's L and run
     // every step with Householder orthonormalisation (col-major, in `work`).
     double *Lw = work, *hw = work + 2 * (int64_t)n * r;
@@ -786,10 +853,8 @@ __global__ void __launch_bounds__(SM_NT, 1) subspace_mma_kernel(const double *Sg
         for (int e = t; e < n * r; e += SM_NT) {
             const int i = e % n, c = e / n;
             double acc = 0.0;
-            for (int k = 0; k < n; k++) {
-                const double sv = SMODE == S_FULL ? Ss[i + lds * k] : __ldg(Sg + i + (int64_t)n * k);
-                acc = fma(sv, Lw[k + n * c], acc);
-            }
+            for (int k = 0; k < n; k++)
+                acc = fma(__ldg(Sg + i + (int64_t)n * k), Lw[k + n * c], acc);
             hw[e] = acc;
         }
         __syncthreads();
@@ -822,7 +887,6 @@ __global__ void __launch_bounds__(SM_NT, 1) cholqr2_batch_kernel(const double *c
     double *Gp = Z1 + M8 * T::LDQ;
     double *G = Gp + SM_GP;
     double *Ri = G + RT * RT;
-    double *dinv = Ri + RT * T::LDR;
     for (int e = t; e < M8 * T::LDQ; e += SM_NT) {
         const int i = e / T::LDQ, c = e % T::LDQ;
         Z0[e] = (i < M && c < r) ? A[b][i + (int64_t)M * c] : 0.0;
@@ -832,7 +896,7 @@ __global__ void __launch_bounds__(SM_NT, 1) cholqr2_batch_kernel(const double *c
     double *cur = Z0, *oth = Z1;
     for (int p = 0; p < 2; p++) {
         sm_gram<RT>(cur, M, r, Gp, G);
-        if (!sm_chol_inv<RT>(G, Ri, dinv, r)) {
+        if (!sm_chol_inv<RT>(G, Ri, r)) {
             bad = 1;
             break;
         }
@@ -855,22 +919,34 @@ __global__ void __launch_bounds__(SM_NT, 1) cholqr2_batch_kernel(const double *c
     hqr_device(W, M, r, W + (int64_t)M * r, Q[b], red);
 }
 
-template <int RT, int SMODE>
-void launch_subspace_mma(dt_ctx *ctx, const double *S, int n, double *L, int r, int iters,
-                         double *work, int *flag) {
-    const size_t smem = sm_smem_doubles<RT>(n, SMODE == S_FULL) * sizeof(double);
-    auto kern = subspace_mma_kernel<RT, SMODE>;
+template <int RT, bool SSM>
+void launch_subspace(dt_ctx *ctx, const double *S, int n, double *L, int r, int iters,
+                     double *work, int *flag, int csize) {
+    const size_t smem = sub_smem_bytes<RT>(n, csize, SSM);
+    auto kern = subspace_cluster_kernel<RT, SSM>;
     smem_limit(ctx, kern, smem);
-    DT_LAUNCH_PDL(ctx, kern, 1, SM_NT, smem, S, n, L, r, iters, work, flag);
+    launch_pdl_cluster(ctx, kern, csize, SM_NT, smem, csize, S, n, L, r, iters, work, flag, csize);
 }
 
 template <int RT>
 void subspace_mma(dt_ctx *ctx, const double *S, int n, double *L, int r, int iters,
                   double *work, int *flag) {
-    if (sm_smem_doubles<RT>(n, true) * sizeof(double) <= 220 * 1024)
-        launch_subspace_mma<RT, S_FULL>(ctx, S, n, L, r, iters, work, flag);
-    else
-        launch_subspace_mma<RT, S_GLOBAL>(ctx, S, n, L, r, iters, work, flag);
+    const size_t cap = 220 * 1024;
+    // Up to 64 rows one CTA: an exchange costs more than the part of a product
+    // it saves (64 x 8, 5 steps: 12.8 us on one CTA, 13.1 on four).  Above, eight:
+    // 96 x 16, 5 steps 28.8 us on one CTA, 25.0 on two, 22.6 on four, 21.9 on
+    // eight; 200 x 10, 30 steps 135 on two or four, 110 on eight.  The single-CTA
+    // kernel before this one took 35 us for 96 x 16 (5 steps), 20 (2 steps), and
+    // 112 us for 256 x 12 with S read from L2.
+    const int c = n <= 64 ? 1 : 8;
+    if (sub_smem_bytes<RT>(n, c, true) <= cap) {
+        launch_subspace<RT, true>(ctx, S, n, L, r, iters, work, flag, c);
+        return;
+    }
+    // r > 16 and n > 200 or so: S stays in L2, fewer CTAs for fewer shares.
+    int few = c;
+    while (few > 1 && sub_smem_bytes<RT>(n, few, false) > cap) few /= 2;
+    launch_subspace<RT, false>(ctx, S, n, L, r, iters, work, flag, few);
 }
 
 // Subspace iteration for ranks above 32: Householder QR every step, S, L and Z

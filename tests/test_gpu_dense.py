@@ -133,6 +133,23 @@ def test_als_subspace_sizes_vs_oracle(ctx, n, r):
     np.testing.assert_allclose(q.T @ q, np.eye(r), atol=1e-13)
 
 
+@pytest.mark.parametrize("n,r,iters", [(64, 8, 1), (65, 9, 2), (72, 16, 3), (121, 3, 4), (129, 17, 6),
+                                       (255, 16, 5), (256, 32, 2), (9, 8, 5)])
+def test_als_cluster_edges(ctx, n, r, iters):
+    """The subspace kernel on one CTA and on a cluster of eight: CTAs with one
+    tile less than others or none, an odd n, S kept or read from L2, and every
+    place the last step can have in the schedule.  Singular values fall by
+    less than 30 in all, so ten powers of S stay far from breakdown."""
+    rng = np.random.default_rng(n + iters)
+    V, _ = np.linalg.qr(rng.standard_normal((n, n)))
+    W, _ = np.linalg.qr(rng.standard_normal((2 * n, n)))
+    Y = np.asfortranarray((V * np.geomspace(30.0, 1.0, n)) @ W.T)
+    L0, _ = np.linalg.qr(rng.standard_normal((n, r)))
+    q = ctx.als(Y, 0, L0, iters)
+    assert dense.principal_angle_max(q, dense.als(Y, 0, L0, iters)) < 1e-10
+    np.testing.assert_allclose(q.T @ q, np.eye(r), atol=1e-13)
+
+
 def _check_hooi(G, U, rep, gn_ref, U_ref, xn):
     assert abs(rep["g_norm"] - gn_ref) <= 1e-10 * gn_ref
     assert abs(np.linalg.norm(G) - gn_ref) <= 1e-10 * gn_ref
