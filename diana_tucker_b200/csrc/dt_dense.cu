@@ -690,47 +690,359 @@ Operand unfolding(const double *p, int64_t L, int64_t I) {
 
 }  // namespace
 
-void ttt_f64(dt_ctx *ctx, const double *A, const double *Bt, int64_t L, int64_t IA,
-             int64_t IB, int64_t B, double *C) {
-    gemm_generic(ctx, unfolding(A, L, IA), unfolding(Bt, L, IB), IA, IB, L * B, C, IA, 0.0);
+// ---------------------------------------------------------------------------
+// Gram of a mode-n unfolding, S(i, j) = sum_q X_(n)(i, q) X_(n)(j, q), on the
+// FP64 tensor cores.  S is symmetric: only the 8 x 8 tiles of its upper block
+// triangle are computed, dealt out evenly over the CTA's warps, and every staged
+// row serves all of them: the CTA stages GR_K columns of all rows of X_(n) (n <=
+// 256) or of the two 128-row blocks of its block pair, GR_ST chunks deep by
+// cp.async, so X is read once up to 200 rows (two CTAs share the tiles up to 256).
+// The list takes row r together with row nt - 1 - r (nt + 1 tiles in all), so a
+// warp's run of tiles lies in at most three rows: it loads three A fragments a
+// k-step and each tile selects one and loads its B fragment, without a branch.
+// K is split over the CTAs; a second launch adds the partial tiles in order and
+// mirrors them.  The column index q = (l, b) is carried along chunk by chunk (no
+// divisions).  Bound by the FP64 tensor rate (64 FMA a cycle and SM): 200 rows, K =
+// 40000: 83 us (20 TFLOP/s, of about 37) against 392 us for the whole square on
+// 64 x 64 tiles with two divisions per loaded element; 203 rows, K = 28417: 78
+// against 276 us.
+// KF: q is contiguous in memory for at least 16 columns (L >= 16); rows are
+// staged with k contiguous, pitch 20.  Else (L < 16, the first modes) k-rows of
+// all i, pitch = 4 (mod 16).  Either way the four k-columns and the rows of a
+// fragment load hit distinct banks.  VEC: 16-byte copies (even L, or L = 1 and
+// an even I, on a 16-byte aligned X), else 8-byte ones.
+// ---------------------------------------------------------------------------
+namespace {
+
+constexpr int GR_K = 16;    // columns per chunk
+constexpr int GR_ST = 3;    // chunks in the ring
+constexpr int GR_KP = GR_K + 4;
+constexpr int GR_BLOCK = 128;  // rows of a block when there are several
+
+struct GramArgs {
+    const double *X;
+    int64_t L, LI, K, kchunk;
+    int n;        // rows
+    int tiles;    // partial tiles per split (stride of the splits)
+    int multi;    // several row blocks, a CTA per pair of them
+    int parts;    // one block: CTAs that share its tiles
+    int pitch;    // !KF: pitch of a staged k-row
+    double *C;    // n x n col-major, written directly when part is null
+    double *part;
+};
+
+// Block pair p of the upper triangle of nb blocks, row by row.
+__host__ __device__ inline void gram_pair(int p, int nb, int &bi, int &bj) {
+    bi = 0;
+    while (p >= nb - bi) {
+        p -= nb - bi;
+        bi++;
+    }
+    bj = bi + p;
+}
+// Tile s of the upper triangle of nt x nt tiles: rows r and nt - 1 - r in turn.
+__host__ __device__ inline void gram_tri(int s, int nt, int &r, int &c) {
+    const int f = s / (nt + 1), o = s - f * (nt + 1);
+    if (o < nt - f) {
+        r = f;
+        c = f + o;
+    } else {
+        r = nt - 1 - f;
+        c = r + o - (nt - f);
+    }
 }
 
-void ttt_f64_scratch(dt_ctx *ctx, const double *A, const double *Bt, int64_t L, int64_t IA,
-                     int64_t IB, int64_t B, double *C, double *scratch, int64_t scratch_doubles) {
-    // Same tiles, split choice and reduction as gemm_generic, with the split-K
-    // partial tiles in the caller's scratch; the split count is lowered when
-    // nsplit * IA * IB doubles would not fit.
-    const int64_t M = IA, N = IB, K = L * B;
-    if (M == 0 || N == 0) return;
-    const int64_t MN = M * N;
-    DT_CHECK_ARG(MN <= scratch_doubles,
-                 "ttt_f64_scratch: %lld x %lld result needs more than %lld scratch doubles",
-                 (long long)M, (long long)N, (long long)scratch_doubles);
-    const Operand a = unfolding(A, L, IA), b = unfolding(Bt, L, IB);
-    const int64_t tiles = (int64_t)ceil_div(M, GM_B) * ceil_div(N, GM_B);
-    const int64_t target = 2LL * ctx->num_sms;
-    int64_t nsplit = 1;
-    if (tiles < target && K > 256) {
-        nsplit = (target + tiles - 1) / tiles;
-        nsplit = std::min<int64_t>(nsplit, (K + 127) / 128);
-        nsplit = std::min<int64_t>(nsplit, scratch_doubles / MN);
-        nsplit = std::max<int64_t>(nsplit, 1);
+template <int W, int NACC, bool KF, bool VEC>
+__global__ void __launch_bounds__(32 * W, W == 8 ? 2 : 1) gram_kernel(GramArgs a) {
+    extern __shared__ __align__(16) double gs[];
+    constexpr int NT = 32 * W;
+    const int t = threadIdx.x, w = t >> 5, lane = t & 31, g = lane >> 2, t4 = lane & 3;
+    int bi = 0, bj = 0;
+    if (a.multi) gram_pair(blockIdx.x, (a.n + GR_BLOCK - 1) / GR_BLOCK, bi, bj);
+    const bool rect = bi != bj;
+    const int i0 = bi * GR_BLOCK, j0 = bj * GR_BLOCK;
+    const int ni = a.multi ? min(GR_BLOCK, a.n - i0) : a.n;   // rows of the first block
+    const int nj = rect ? min(GR_BLOCK, a.n - j0) : 0;        // staged rows of the second
+    const int nti = (ni + 7) / 8, ntj = rect ? (nj + 7) / 8 : nti;
+    const int rows = 8 * (rect ? nti + ntj : nti);            // staged rows
+    const int stage = KF ? rows * GR_KP : GR_K * a.pitch;
+    const int64_t qbeg = (int64_t)blockIdx.y * a.kchunk, qend = min(a.K, qbeg + a.kchunk);
+    const int nch = (int)((qend - qbeg + GR_K - 1) / GR_K);
+    // Staged rows past n are zero in every chunk.
+    for (int q = 0; q < GR_ST; q++) {
+        const int pi = 8 * nti - ni, pj = rect ? 8 * ntj - nj : 0;
+        for (int e = t; e < (pi + pj) * GR_K; e += NT) {
+            const int x = e / GR_K, k = e % GR_K;
+            const int at = x < pi ? ni + x : 8 * nti + nj + (x - pi);
+            gs[q * stage + (KF ? at * GR_KP + k : k * a.pitch + at)] = 0.0;
+        }
     }
-    int64_t kchunk = (K + nsplit - 1) / nsplit;
-    kchunk = ((kchunk + GM_BK - 1) / GM_BK) * GM_BK;
-    if (kchunk == 0) kchunk = GM_BK;
-    nsplit = (K + kchunk - 1) / kchunk;
-    if (nsplit < 1) nsplit = 1;
-    dim3 grid(ceil_div(M, GM_B), ceil_div(N, GM_B), (unsigned)nsplit);
-    if (nsplit == 1) {
-        DT_LAUNCH(ctx, gemm_kernel, grid, GM_NT, 0, a, b, M, N, K, kchunk, C, M, 0.0,
-                  (double *)nullptr);
+
+    // This warp's tiles: [s0, s1) of the list, in at most three rows; tile x
+    // is in the first up to x = x1, in the second up to x2.
+    const int total = rect ? nti * ntj : nti * (nti + 1) / 2;
+    const int wt = W * a.parts, wi = W * (a.multi ? 0 : blockIdx.x) + w;
+    const int s0 = (int)((int64_t)wi * total / wt), s1 = (int)((int64_t)(wi + 1) * total / wt);
+    int row[3], col[3], x1 = NACC, x2 = NACC;  // col: column tile of x = 0 continued
+    if (rect) {  // the first block is whole: one row of ntj tiles per warp
+        row[0] = row[1] = row[2] = w;
+        col[0] = col[1] = col[2] = nti;  // staged after the row tiles
     } else {
-        DT_LAUNCH(ctx, gemm_kernel, grid, GM_NT, 0, a, b, M, N, K, kchunk, C, M, 0.0, scratch);
-        const unsigned blocks = std::min<unsigned>(ceil_div(MN, 256), 4096u);
-        DT_LAUNCH(ctx, splitk_reduce_kernel, blocks, 256, 0, (const double *)scratch, (int)nsplit,
-                  M, N, C, M, 0.0);
+        gram_tri(min(s0, total - 1), nti, row[0], col[0]);
+        x1 = min(nti - col[0], NACC);
+        gram_tri(min(s0 + x1, total - 1), nti, row[1], col[1]);
+        x2 = min(x1 + nti - col[1], NACC);
+        gram_tri(min(s0 + x2, total - 1), nti, row[2], col[2]);
+        col[1] -= x1;
+        col[2] -= x2;
     }
+
+    // Loader: KF: k = (VEC ? 2 : 1) (t % KT), rows t / KT + ...; else warp w
+    // stages k = w, w + W, lanes along i.
+    constexpr int EV = VEC ? 2 : 1;
+    constexpr int KT = GR_K / EV;             // KF: threads along k
+    constexpr int KPW = KF ? 1 : GR_K / W;    // !KF: k-rows per warp
+    const int nq = (int)(qend - qbeg);  // this split's columns
+    const double *src[KPW];             // the next chunk's column, l of it
+    int64_t ql[KPW];
+    for (int x = 0; x < KPW; x++) {
+        const int64_t q = qbeg + (KF ? EV * (t % KT) : w + x * W);
+        const int64_t b = q / a.L;
+        ql[x] = q - b * a.L;
+        src[x] = a.X + ql[x] + a.LI * b + (int64_t)i0 * a.L;
+    }
+    const int64_t jump = rect ? (int64_t)(j0 - i0 - ni) * a.L : 0;  // to the second block's rows
+    auto issue = [&](int c) {
+        double *dst = gs + (c % GR_ST) * stage;
+#pragma unroll
+        for (int x = 0; x < KPW; x++) {
+            const int k = KF ? EV * (t % KT) : w + x * W;
+            const int left = nq - c * GR_K - k;
+            // A pair is cut only where nq is odd.
+            const int bytes = left <= 0 ? 0 : KF && left < EV ? 8 : 8 * EV;
+            for (int i = KF ? t / KT : EV * lane; i < ni + nj; i += KF ? NT / KT : 32 * EV) {
+                const bool second = i >= ni;
+                const int at = second ? 8 * nti + (i - ni) : i;
+                const double *p = bytes ? src[x] + i * a.L + (second ? jump : 0) : a.X;
+                double *o = dst + (KF ? at * GR_KP + k : k * a.pitch + at);
+                if (VEC) cp_async16(o, p, bytes);
+                else cp_async8(o, p, bytes);
+            }
+            ql[x] += GR_K;
+            src[x] += GR_K;
+            while (ql[x] >= a.L) {
+                ql[x] -= a.L;
+                src[x] += a.LI - a.L;
+            }
+        }
+        cp_async_commit();
+    };
+
+    double acc[NACC][2];
+#pragma unroll
+    for (int x = 0; x < NACC; x++) acc[x][0] = acc[x][1] = 0.0;
+    const int RS = KF ? 8 * GR_KP : 8;             // a row tile further
+    const int KS = KF ? 4 : 4 * a.pitch;           // a k-step further
+    const int lane_off = KF ? g * GR_KP + t4 : t4 * a.pitch + g;
+    const int ar0 = lane_off + row[0] * RS, ar1 = lane_off + row[1] * RS,
+              ar2 = lane_off + row[2] * RS;
+    const int bc0 = lane_off + col[0] * RS, bc1 = lane_off + col[1] * RS,
+              bc2 = lane_off + col[2] * RS;
+
+    pdl_wait();
+    for (int c = 0; c < GR_ST - 1; c++) {
+        if (c < nch) issue(c);
+        else cp_async_commit();
+    }
+    for (int c = 0; c < nch; c++) {
+        cp_async_wait<GR_ST - 2>();
+        __syncthreads();
+        if (c + GR_ST - 1 < nch) issue(c + GR_ST - 1);
+        else cp_async_commit();
+        const double *base = gs + (c % GR_ST) * stage;
+#pragma unroll
+        for (int kk = 0; kk < GR_K / 4; kk++) {
+            const double *p = base + kk * KS;
+            const double a0 = p[ar0], a1 = p[ar1], a2 = p[ar2];
+            // Selected anew each k-step: kept, the tiles' addresses cost more
+            // registers than a thread has.
+            asm volatile("" : "+r"(x1), "+r"(x2));
+            // Tiles past s1 read what lies there (within the allocation) and
+            // are not stored.
+#pragma unroll
+            for (int x = 0; x < NACC; x++) {
+                const double av = x < x1 ? a0 : x < x2 ? a1 : a2;
+                const int bc = x < x1 ? bc0 : x < x2 ? bc1 : bc2;
+                gm_dmma884(acc[x][0], acc[x][1], av, p[bc + x * RS]);
+            }
+        }
+    }
+    pdl_trigger();
+    // D[row g][cols 2 t, 2 t + 1] of tile x.
+#pragma unroll
+    for (int x = 0; x < NACC; x++) {
+        if (s0 + x >= s1) continue;
+        if (a.part) {
+            const int64_t tile = (int64_t)blockIdx.y * a.tiles +
+                                 (a.multi ? 256 * (int64_t)blockIdx.x : 0) + s0 + x;
+            *reinterpret_cast<double2 *>(a.part + tile * 64 + g * 8 + 2 * t4) =
+                make_double2(acc[x][0], acc[x][1]);
+        } else {
+            const int r = x < x1 ? row[0] : x < x2 ? row[1] : row[2];
+            const int c = x + (x < x1 ? col[0] : x < x2 ? col[1] : col[2]) - (rect ? nti : 0);
+            const int64_t i = i0 + 8 * r + g;
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                const int64_t j = j0 + 8 * c + 2 * t4 + h;
+                if (i < a.n && j < a.n) {
+                    a.C[i + (int64_t)a.n * j] = acc[x][h];
+                    if (rect || r != c) a.C[j + (int64_t)a.n * i] = acc[x][h];
+                }
+            }
+        }
+    }
+}
+
+// One CTA per tile: four threads an entry, each adding every fourth split (16
+// loads in flight), then the four in order; the tile and its mirror go to C.
+__global__ void __launch_bounds__(256) gram_sum_kernel(const double *__restrict__ part, int nsplit,
+                                                       int tiles, int n, int multi,
+                                                       double *__restrict__ C) {
+    __shared__ double red[4][64];
+    const int t = threadIdx.x, e = t & 63, q = t >> 6;
+    int bi = 0, bj = 0, s = blockIdx.x;
+    if (multi) {
+        gram_pair(s / 256, (n + GR_BLOCK - 1) / GR_BLOCK, bi, bj);
+        s %= 256;
+    }
+    const int ni = multi ? min(GR_BLOCK, n - bi * GR_BLOCK) : n;
+    const int nti = (ni + 7) / 8;
+    const int ntj = bi != bj ? (min(GR_BLOCK, n - bj * GR_BLOCK) + 7) / 8 : nti;
+    if (s >= (bi != bj ? nti * ntj : nti * (nti + 1) / 2)) return;
+    int r, c;
+    if (bi != bj) {
+        r = s / ntj;
+        c = s - r * ntj;
+    } else {
+        gram_tri(s, nti, r, c);
+    }
+    pdl_wait();
+    const double *p = part + (int64_t)blockIdx.x * 64 + e;
+    double sum = 0.0;
+    for (int z = q; z < nsplit; z += 64) {
+        double v[16];
+#pragma unroll
+        for (int x = 0; x < 16; x++)
+            v[x] = z + 4 * x < nsplit ? p[(int64_t)(z + 4 * x) * tiles * 64] : 0.0;
+#pragma unroll
+        for (int x = 0; x < 16; x++) sum += v[x];
+    }
+    red[q][e] = sum;
+    __syncthreads();
+    pdl_trigger();
+    if (q == 0) {
+        const double v = (red[0][e] + red[1][e]) + (red[2][e] + red[3][e]);
+        const int64_t i = bi * GR_BLOCK + 8 * r + (e >> 3), j = bj * GR_BLOCK + 8 * c + (e & 7);
+        if (i < n && j < n) {
+            C[i + (int64_t)n * j] = v;
+            if (bi != bj || r != c) C[j + (int64_t)n * i] = v;
+        }
+    }
+}
+
+template <int W, int NACC>
+void launch_gram(dt_ctx *ctx, const GramArgs &a, dim3 grid, bool kf, bool vec) {
+    // The ring, and room for the tiles a warp computes past its last.
+    const int rows = a.multi ? 2 * GR_BLOCK : (a.n + 7) / 8 * 8;
+    const size_t smem = ((size_t)GR_ST * (kf ? rows * GR_KP : GR_K * a.pitch) +
+                         (size_t)NACC * (kf ? 8 * GR_KP : 8)) * sizeof(double);
+#define DT_GRAM(KF, VEC)                                                   \
+    do {                                                                   \
+        auto kern = gram_kernel<W, NACC, KF, VEC>;                         \
+        smem_limit(ctx, kern, smem);                                       \
+        DT_LAUNCH_PDL(ctx, kern, grid, 32 * W, smem, a);                   \
+    } while (0)
+    if (kf && vec) DT_GRAM(true, true);
+    else if (kf) DT_GRAM(true, false);
+    else if (vec) DT_GRAM(false, true);
+    else DT_GRAM(false, false);
+#undef DT_GRAM
+}
+
+// S = X_(n) X_(n)^T; the partial tiles go to `scratch` (scratch_doubles) or, when
+// it is null, to a stream-ordered allocation.
+void gram_f64(dt_ctx *ctx, const double *X, int64_t L, int64_t I, int64_t B, double *C,
+              double *scratch, int64_t scratch_doubles) {
+    DT_CHECK_ARG(I < (int64_t(1) << 24), "gram: mode size %lld", (long long)I);
+    GramArgs a{};
+    a.X = X;
+    a.L = L;
+    a.LI = L * I;
+    a.K = L * B;
+    a.n = (int)I;
+    a.C = C;
+    const int nt = (a.n + 7) / 8;
+    a.multi = nt > 32;
+    // Above 25 tiles a row (325 in all, 21 per warp of 16) two CTAs share them:
+    // more accumulators do not fit a thread's 128 registers.
+    a.parts = !a.multi && nt > 25 ? 2 : 1;
+    const int nb = (a.n + GR_BLOCK - 1) / GR_BLOCK;
+    const int64_t pairs = a.multi ? (int64_t)nb * (nb + 1) / 2 : a.parts;
+    DT_CHECK_ARG(256 * pairs <= INT32_MAX, "gram: mode size %lld", (long long)I);
+    a.tiles = (int)(a.multi ? 256 * pairs : nt * (nt + 1) / 2);
+    const bool kf = L >= GR_K;
+    const bool vec = reinterpret_cast<uintptr_t>(X) % 16 == 0 &&
+                     (kf ? L % 2 == 0 : L == 1 && I % 2 == 0);
+    const int staged = a.multi ? 2 * GR_BLOCK : 8 * nt;
+    a.pitch = (staged + 11) / 16 * 16 + 4;
+    // Enough splits for the CTAs that fit (two of 8 warps or one of 16 per
+    // SM), of at least two chunks each.
+    const int tiles8 = nt * (nt + 1) / 2;
+    const bool wide = a.multi || nt > 16;
+    const int64_t target = (wide ? 1LL : 2LL) * ctx->num_sms;
+    int64_t nsplit = std::max<int64_t>(1, std::min<int64_t>(target / pairs, (a.K + 2 * GR_K - 1) / (2 * GR_K)));
+    if (scratch) nsplit = std::max<int64_t>(1, std::min<int64_t>(nsplit, scratch_doubles / (64LL * a.tiles)));
+    a.kchunk = std::max<int64_t>(GR_K, ((a.K + nsplit - 1) / nsplit + GR_K - 1) / GR_K * GR_K);
+    nsplit = std::max<int64_t>(1, (a.K + a.kchunk - 1) / a.kchunk);
+    DevMem part;
+    if (nsplit > 1) {
+        if (!scratch) {
+            part.alloc(ctx, (size_t)nsplit * a.tiles * 64 * sizeof(double));
+            scratch = part.as<double>();
+        }
+        a.part = scratch;
+    }
+    const dim3 grid((unsigned)pairs, (unsigned)nsplit);
+    // Tiles per warp, rounded up to the next size there is a kernel for.
+    const int per8 = (tiles8 + 7) / 8, per16 = (tiles8 + 16 * a.parts - 1) / (16 * a.parts);
+    if (a.multi) launch_gram<16, 16>(ctx, a, grid, kf, vec);
+    else if (wide && per16 <= 12) launch_gram<16, 12>(ctx, a, grid, kf, vec);
+    else if (wide && per16 <= 17) launch_gram<16, 17>(ctx, a, grid, kf, vec);
+    else if (wide) launch_gram<16, 21>(ctx, a, grid, kf, vec);
+    else if (per8 <= 2) launch_gram<8, 2>(ctx, a, grid, kf, vec);
+    else if (per8 <= 4) launch_gram<8, 4>(ctx, a, grid, kf, vec);
+    else if (per8 <= 7) launch_gram<8, 7>(ctx, a, grid, kf, vec);
+    else if (per8 <= 10) launch_gram<8, 10>(ctx, a, grid, kf, vec);
+    else if (per8 <= 14) launch_gram<8, 14>(ctx, a, grid, kf, vec);
+    else launch_gram<8, 17>(ctx, a, grid, kf, vec);
+    if (a.part)
+        DT_LAUNCH_PDL(ctx, gram_sum_kernel, (unsigned)a.tiles, 256, 0, (const double *)a.part,
+                      (int)nsplit, a.tiles, a.n, a.multi, C);
+}
+
+}  // namespace
+
+void ttt_f64(dt_ctx *ctx, const double *A, const double *Bt, int64_t L, int64_t IA,
+             int64_t IB, int64_t B, double *C) {
+    if (A == Bt && IA == IB && IA > 0)
+        gram_f64(ctx, A, L, IA, B, C, nullptr, 0);
+    else
+        gemm_generic(ctx, unfolding(A, L, IA), unfolding(Bt, L, IB), IA, IB, L * B, C, IA, 0.0);
+}
+
+void gram_f64_scratch(dt_ctx *ctx, const double *A, int64_t L, int64_t I, int64_t B, double *C,
+                      double *scratch, int64_t scratch_doubles) {
+    gram_f64(ctx, A, L, I, B, C, scratch, scratch_doubles);
 }
 
 void gemm_f64(dt_ctx *ctx, int transA, int transB, int64_t m, int64_t n, int64_t k,

@@ -101,7 +101,7 @@ int dt_gram_f64_noalloc(dt_ctx *ctx, const double *X, int ndim, const int64_t *s
         for (int m = 0; m < mode; m++) L *= shape[m];
         for (int m = mode + 1; m < ndim; m++) B *= shape[m];
         double *scratch = scratch_address(ctx->device);
-        ttt_f64_scratch(ctx, X, X, L, I, I, B, G, scratch, kScratchDoubles);
+        gram_f64_scratch(ctx, X, L, I, B, G, scratch, kScratchDoubles);
     });
 }
 

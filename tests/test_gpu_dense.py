@@ -102,6 +102,24 @@ def test_small_linear_algebra(ctx, oracle_ref):
     assert np.max(np.abs(np.triu(Lm, 1))) < 1e-12 and np.all(np.diag(Lm) > 0)
 
 
+@pytest.mark.parametrize("shape,mode", [
+    ((7, 5, 3), 0), ((8, 33), 0), ((33, 8), 1), ((12, 64, 9), 1), ((15, 65, 7), 1), ((16, 66, 7), 1),
+    ((17, 96, 5), 1), ((97, 31, 3), 0), ((3, 128, 50), 1), ((18, 129, 4), 1), ((200, 40, 21), 0),
+    ((20, 200, 17), 1), ((22, 30, 201), 2), ((41, 256, 3), 1), ((256, 9, 9), 0), ((16, 257, 5), 1),
+    ((300, 20), 0), ((6, 385, 4), 1), ((500, 1000, 24), 2)])
+def test_gram_tiles_and_layouts(ctx, shape, mode):
+    """Rows at, below and above the tile lists' sizes (one CTA, two sharing,
+    block pairs), both staging layouts, 8- and 16-byte copies, one split and
+    many, remainders of the columns.  Sums of up to 5e5 products: 1e-12 of the
+    largest entry."""
+    rng = np.random.default_rng(sum(shape) + mode)
+    X = np.asfortranarray(rng.standard_normal(shape))
+    A = np.moveaxis(X, mode, 0).reshape(shape[mode], -1)
+    G = ctx.gram(X, mode)
+    np.testing.assert_allclose(G, A @ A.T, rtol=0, atol=1e-12 * np.max(np.abs(A @ A.T)))
+    assert np.array_equal(G, G.T)
+
+
 def test_inverse_singular_reports_error(ctx):
     from diana_tucker_b200 import DTError
     with pytest.raises(DTError) as e:
