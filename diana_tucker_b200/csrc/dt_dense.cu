@@ -1,5 +1,6 @@
-// FP64 dense kernels on the CUDA cores: the stride-aware TTM, the unfolding
-// GEMM behind Gram / ttt_except / matmul, and deterministic norms.
+// FP64 dense kernels: the stride-aware TTM, the Gram of an unfolding, the GEMM
+// behind ttt_except / matmul (all on the FP64 tensor cores), and deterministic
+// norms.
 //
 // The reference's Function::ttm (template/function/tensor.tpp:272-335) first
 // permutes A into A_(n)^T with Operator::tenmatt (operator_cpu.tpp:83-103),
@@ -13,390 +14,217 @@
 namespace dt {
 
 // ---------------------------------------------------------------------------
-// TTM: Y[l, j, b] = sum_i M(j, i) X[l, i, b], M(j, i) = M[j*msj + i*msi].  One CTA owns 256 "rows"
-// p = l + L*b of the output and a JT-wide slice of j; X tiles (16 i x 256 p)
-// are staged through shared memory so every global load is coalesced: along
-// l when L > 1, along i when L == 1 (mode 0, where the contracted index is the
-// contiguous one).  Each thread accumulates 2 rows x JT outputs in registers.
+// TTM: Y[l, j, b] = sum_i M(j, i) X[l, i, b], M(j, i) = M[j*msj + i*msi], on the
+// FP64 tensor cores (mma.sync m8n8k4).  One CTA of 8 warps owns 64 MT output
+// rows p = l + L b and 8 NT outputs j; warp w owns rows 8 MT w .. + 8 MT - 1 as
+// MT x NT tiles.  Chunks of 16 i go through a ring of ST stages by cp.async
+// (zero-filled past the end), one barrier per chunk.  Bound by memory for a
+// large X (one read of X and NT >= J / 8, so X is read once for up to 32
+// outputs); the FP64 tensor rate comes next.
+//   KF (L == 1, mode 0): i is contiguous; rows are staged with k contiguous,
+//        pitch 20.
+//   else: rows are contiguous in runs of L; a thread keeps one row (or one
+//        group of EV rows) and its address, found by one division, and walks
+//        along i.  A tile's rows may lie in several b.
+// Either way the four k-columns and eight rows of a fragment load hit distinct
+// banks.  VEC: 16-byte copies, where L (KF: I) is a multiple of the elements
+// in 16 bytes and X is aligned; else one element a copy.
+// 96^4 FP64, 16 outputs: mode 0 243 -> 136 us, mode 1 295 -> 127, mode 3 132 -> 127
+// (6.2 TB/s), FP32 215 -> 100 and 119 -> 105; 181 x 203 x 157, 24 outputs 47 -> 29;
+// 96 x 16 x 96 x 96, 16 outputs 75 -> 44: before, only runs of L % 256 == 0 rows ran on
+// the tensor cores, other layouts on the CUDA cores, ragged ones without a
+// pipeline, and few rows split the contraction over two launches.
 // ---------------------------------------------------------------------------
 namespace {
 
-constexpr int TTM_BP = 256;
-constexpr int TTM_BK = 16;
-constexpr int TTM_NT = 128;
-
-template <class TX, int JT>
-__global__ void __launch_bounds__(TTM_NT) ttm_kernel(const TX *__restrict__ X, int64_t L,
-                                                     int64_t I, int64_t P,
-                                                     const double *__restrict__ M, int64_t msj,
-                                                     int64_t msi, int64_t J,
-                                                     double *__restrict__ Y, int64_t kchunk,
-                                                     int64_t ysize) {
-    __shared__ __align__(16) double Xs[TTM_BK][TTM_BP];
-    __shared__ __align__(16) double Ms[TTM_BK][JT];
-    const int t = threadIdx.x;
-    pdl_wait();
-    const int64_t p0 = (int64_t)blockIdx.x * TTM_BP;
-    const int64_t j0 = (int64_t)blockIdx.y * JT;
-    const int64_t LI = L * I;
-    // Split-K: blockIdx.z owns i in [ibeg, iend) and writes its own partial Y.
-    const int64_t ibeg = (int64_t)blockIdx.z * kchunk;
-    const int64_t iend = min(I, ibeg + kchunk);
-    Y += (int64_t)blockIdx.z * ysize;
-
-    // Loader bookkeeping for L > 1: this thread loads rows t and t + 128.
-    int64_t lbase[2];
-    bool lok[2];
-    if (L > 1) {
-#pragma unroll
-        for (int s = 0; s < 2; s++) {
-            const int64_t p = p0 + t + s * TTM_NT;
-            lok[s] = p < P;
-            const int64_t b = p / L, l = p - b * L;
-            lbase[s] = l + LI * b;
-        }
-    }
-
-    double acc[2][JT];
-#pragma unroll
-    for (int r = 0; r < 2; r++)
-#pragma unroll
-        for (int j = 0; j < JT; j++) acc[r][j] = 0.0;
-
-    for (int64_t i0 = ibeg; i0 < iend; i0 += TTM_BK) {
-        if (L > 1) {
-#pragma unroll
-            for (int s = 0; s < 2; s++) {
-                const int pp = t + s * TTM_NT;
-#pragma unroll 4
-                for (int k = 0; k < TTM_BK; k++) {
-                    const int64_t i = i0 + k;
-                    Xs[k][pp] = (lok[s] && i < iend) ? (double)X[lbase[s] + L * i] : 0.0;
-                }
-            }
-        } else {
-            const int k = t & (TTM_BK - 1);
-            const int g = t >> 4;  // 0..7
-            const int64_t i = i0 + k;
-#pragma unroll 4
-            for (int s = 0; s < TTM_BP / 8; s++) {
-                const int pp = g + 8 * s;
-                const int64_t p = p0 + pp;
-                Xs[k][pp] = (p < P && i < iend) ? (double)X[p * I + i] : 0.0;
-            }
-        }
-        for (int e = t; e < TTM_BK * JT; e += TTM_NT) {
-            const int k = e / JT, j = e - (e / JT) * JT;
-            const int64_t i = i0 + k, jj = j0 + j;
-            Ms[k][j] = (i < iend && jj < J) ? M[jj * msj + i * msi] : 0.0;
-        }
-        __syncthreads();
-#pragma unroll
-        for (int k = 0; k < TTM_BK; k++) {
-            const double2 x = *reinterpret_cast<const double2 *>(&Xs[k][2 * t]);
-#pragma unroll
-            for (int j = 0; j < JT; j += 2) {
-                const double2 m = *reinterpret_cast<const double2 *>(&Ms[k][j]);
-                acc[0][j] = fma(x.x, m.x, acc[0][j]);
-                acc[0][j + 1] = fma(x.x, m.y, acc[0][j + 1]);
-                acc[1][j] = fma(x.y, m.x, acc[1][j]);
-                acc[1][j + 1] = fma(x.y, m.y, acc[1][j + 1]);
-            }
-        }
-        __syncthreads();
-    }
-
-    pdl_trigger();  // dependents may launch while the outputs are stored
-    const int64_t LJ = L * J;
-#pragma unroll
-    for (int r = 0; r < 2; r++) {
-        const int64_t p = p0 + 2 * t + r;
-        if (p >= P) continue;
-        const int64_t b = p / L, l = p - b * L;
-        double *y = Y + l + LJ * b;
-#pragma unroll
-        for (int j = 0; j < JT; j++)
-            if (j0 + j < J) y[L * (j0 + j)] = acc[r][j];
-    }
-}
-
-// ---------------------------------------------------------------------------
-// Pipelined TTM for the two layouts the HOOI dimension tree produces from X:
-//   ROWS (L % 256 == 0): the 256 output rows of a CTA are one contiguous run
-//        of l, so every k of a tile is a 16-byte-aligned contiguous segment;
-//   KFAST (L == 1): the contracted index is contiguous, each row of the tile
-//        is 16 consecutive i.
-// Tiles move with cp.async (16 B, zero-filled past I) into a two-stage ring so
-// the next K-chunk streams while this one is multiplied.
-// ---------------------------------------------------------------------------
 __device__ __forceinline__ void cp_async16(void *smem, const void *gmem, int src_bytes) {
     const uint32_t s = (uint32_t)__cvta_generic_to_shared(smem);
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(s), "l"(gmem),
                  "r"(src_bytes)
                  : "memory");
 }
-__device__ __forceinline__ void cp_async8(void *smem, const void *gmem, int src_bytes) {
+// One element (4 or 8 bytes), through L1: neighbours in a line come later.
+template <int BYTES>
+__device__ __forceinline__ void cp_async_el(void *smem, const void *gmem, int src_bytes) {
     const uint32_t s = (uint32_t)__cvta_generic_to_shared(smem);
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(s), "l"(gmem),
-                 "r"(src_bytes)
+    asm volatile("cp.async.ca.shared.global [%0], [%1], %3, %2;" ::"r"(s), "l"(gmem),
+                 "r"(src_bytes), "n"(BYTES)
                  : "memory");
+}
+__device__ __forceinline__ void cp_async8(void *smem, const void *gmem, int src_bytes) {
+    cp_async_el<8>(smem, gmem, src_bytes);
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N>
 __device__ __forceinline__ void cp_async_wait() {
     asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
-
-template <class TX, int JT, bool KFAST>
-__global__ void __launch_bounds__(TTM_NT) ttm_pipe_kernel(const TX *__restrict__ X, int64_t L,
-                                                          int64_t I, int64_t P,
-                                                          const double *__restrict__ M,
-                                                          int64_t msj, int64_t msi, int64_t J,
-                                                          double *__restrict__ Y, int64_t kchunk,
-                                                          int64_t ysize) {
-    constexpr int EV = 16 / sizeof(TX);              // elements per 16-byte copy
-    constexpr int KROW = 16 + (KFAST ? EV : 0);      // KFAST row stride (elements), padded
-    constexpr int XS_ELEMS = KFAST ? TTM_BP * KROW : TTM_BK * TTM_BP;
-    extern __shared__ __align__(16) uint8_t pipe_smem[];
-    auto Ms = reinterpret_cast<double(*)[TTM_BK][JT]>(pipe_smem);
-    auto Xs = reinterpret_cast<TX(*)[XS_ELEMS]>(pipe_smem + 2 * TTM_BK * JT * sizeof(double));
-    const int t = threadIdx.x;
-    pdl_wait();
-    const int64_t p0 = (int64_t)blockIdx.x * TTM_BP;
-    const int64_t j0 = (int64_t)blockIdx.y * JT;
-    const int64_t ibeg = (int64_t)blockIdx.z * kchunk;
-    const int64_t iend = min(I, ibeg + kchunk);
-    Y += (int64_t)blockIdx.z * ysize;
-    const int64_t nch = (iend - ibeg + TTM_BK - 1) / TTM_BK;
-    // ROWS: the CTA's rows are l0..l0+255 of batch b.
-    const int64_t b0 = KFAST ? 0 : p0 / L;
-    const int64_t l0 = KFAST ? 0 : p0 - b0 * L;
-    const TX *xb = KFAST ? X : X + l0 + L * I * b0;
-
-    auto issue = [&](int64_t c, int st) {
-        const int64_t i0 = ibeg + c * TTM_BK;
-        if (!KFAST) {
-            // 16 k x 256 rows: (256 / EV) copies per k.
-            constexpr int PER_K = TTM_BP / EV;
-            for (int e = t; e < TTM_BK * PER_K; e += TTM_NT) {
-                const int k = e / PER_K, q = e - k * PER_K;
-                const int64_t i = i0 + k;
-                const bool ok = i < iend;
-                cp_async16(&Xs[st][k * TTM_BP + q * EV], ok ? xb + L * i + q * EV : X, ok ? 16 : 0);
-            }
-        } else {
-            // 256 rows x 16 i: (16 / EV) copies per row.
-            constexpr int PER_R = TTM_BK / EV;
-            for (int e = t; e < TTM_BP * PER_R; e += TTM_NT) {
-                const int r = e / PER_R, q = e - r * PER_R;
-                const int64_t p = p0 + r, i = i0 + q * EV;
-                const bool ok = p < P && i < iend;
-                cp_async16(&Xs[st][r * KROW + q * EV], ok ? X + p * I + i : X, ok ? 16 : 0);
-            }
-        }
-        for (int e = t; e < TTM_BK * JT; e += TTM_NT) {
-            const int k = e / JT, j = e - k * JT;
-            const int64_t i = i0 + k, jj = j0 + j;
-            const bool ok = i < iend && jj < J;
-            cp_async8(&Ms[st][k][j], ok ? M + jj * msj + i * msi : M, ok ? 8 : 0);
-        }
-        cp_async_commit();
-    };
-
-    double acc[2][JT];
-#pragma unroll
-    for (int r = 0; r < 2; r++)
-#pragma unroll
-        for (int j = 0; j < JT; j++) acc[r][j] = 0.0;
-
-    if (nch > 0) issue(0, 0);
-    for (int64_t c = 0; c < nch; c++) {
-        const int st = (int)(c & 1);
-        if (c + 1 < nch) {
-            issue(c + 1, st ^ 1);
-            cp_async_wait<1>();
-        } else {
-            cp_async_wait<0>();
-        }
-        __syncthreads();
-        if (!KFAST) {
-#pragma unroll
-            for (int k = 0; k < TTM_BK; k++) {
-                double x0, x1;
-                if (sizeof(TX) == 4) {
-                    const float2 v = *reinterpret_cast<const float2 *>(&Xs[st][k * TTM_BP + 2 * t]);
-                    x0 = v.x;
-                    x1 = v.y;
-                } else {
-                    const double2 v = *reinterpret_cast<const double2 *>(&Xs[st][k * TTM_BP + 2 * t]);
-                    x0 = v.x;
-                    x1 = v.y;
-                }
-#pragma unroll
-                for (int j = 0; j < JT; j += 2) {
-                    const double2 m = *reinterpret_cast<const double2 *>(&Ms[st][k][j]);
-                    acc[0][j] = fma(x0, m.x, acc[0][j]);
-                    acc[0][j + 1] = fma(x0, m.y, acc[0][j + 1]);
-                    acc[1][j] = fma(x1, m.x, acc[1][j]);
-                    acc[1][j + 1] = fma(x1, m.y, acc[1][j + 1]);
-                }
-            }
-        } else {
-            // Rows t and t + 128; EV consecutive k per 16-byte shared load.
-#pragma unroll
-            for (int kq = 0; kq < TTM_BK; kq += EV) {
-                double xv[2][EV];
-#pragma unroll
-                for (int r = 0; r < 2; r++) {
-                    const TX *src = &Xs[st][(t + r * TTM_NT) * KROW + kq];
-                    if (sizeof(TX) == 4) {
-                        const float4 v = *reinterpret_cast<const float4 *>(src);
-                        const float f[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-                        for (int q = 0; q < EV; q++) xv[r][q] = f[q];
-                    } else {
-                        const double2 v = *reinterpret_cast<const double2 *>(src);
-                        const double f[2] = {v.x, v.y};
-#pragma unroll
-                        for (int q = 0; q < EV; q++) xv[r][q] = f[q];
-                    }
-                }
-#pragma unroll
-                for (int q = 0; q < EV; q++) {
-#pragma unroll
-                    for (int j = 0; j < JT; j += 2) {
-                        const double2 m = *reinterpret_cast<const double2 *>(&Ms[st][kq + q][j]);
-                        acc[0][j] = fma(xv[0][q], m.x, acc[0][j]);
-                        acc[0][j + 1] = fma(xv[0][q], m.y, acc[0][j + 1]);
-                        acc[1][j] = fma(xv[1][q], m.x, acc[1][j]);
-                        acc[1][j + 1] = fma(xv[1][q], m.y, acc[1][j + 1]);
-                    }
-                }
-            }
-        }
-        __syncthreads();
-    }
-
-    pdl_trigger();  // dependents may launch while the outputs are stored
-    const int64_t LJ = L * J;
-#pragma unroll
-    for (int r = 0; r < 2; r++) {
-        const int64_t p = KFAST ? p0 + t + r * TTM_NT : p0 + 2 * t + r;
-        if (p >= P) continue;
-        const int64_t b = p / L, l = p - b * L;
-        double *y = Y + l + LJ * b;
-#pragma unroll
-        for (int j = 0; j < JT; j++)
-            if (j0 + j < J) y[L * (j0 + j)] = acc[r][j];
-    }
-}
-
-// The ROWS layout on the FP64 tensor cores (mma.sync m8n8k4 .f64), J tile 16.
-// The CTA's 256 rows and 16 k of X (and the 16 x 16 slice of M) are staged as
-// in ttm_pipe_kernel; warp w owns rows 64 w .. 64 w + 63 as 8 x 2 tiles of 8 x 8
-// accumulators.  Per 4-k step a lane converts its 8 A elements (row g of each
-// tile, k = t) to FP64 and reads its 2 B elements; 16 mma.sync follow.  The
-// staged rows are padded by 32 bytes (X) and the M rows are 20 doubles apart,
-// so the four k-rows of a fragment load fall in different banks (64-bit loads
-// are served per half-warp).
-__device__ __forceinline__ void ttm_dmma884(double &d0, double &d1, double a, double b) {
+__device__ __forceinline__ void gm_dmma884(double &d0, double &d1, double a, double b) {
     asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
                  : "+d"(d0), "+d"(d1)
                  : "d"(a), "d"(b));
 }
+// q / d, in 32 bits where both fit (a 64-bit division takes several times as
+// many instructions).
+__device__ __forceinline__ int64_t div_pos(int64_t q, int64_t d) {
+    if (((q | d) >> 32) == 0) return (uint32_t)q / (uint32_t)d;
+    return q / d;
+}
 
+constexpr int TTM_NT = 256;
+constexpr int TTM_BK = 16;
+constexpr int TTM_KP = TTM_BK + 4;
+// Rows per CTA, ring depth, pitch of a staged k-row and elements of a stage.
+__host__ __device__ constexpr int ttm_rows(int mt) { return 64 * mt; }
+__host__ __device__ constexpr int ttm_stages(int mt) { return mt == 1 ? 6 : mt == 2 ? 3 : 2; }
 template <class TX>
-__host__ __device__ constexpr int ttm_dm_xrow() { return TTM_BP + 32 / (int)sizeof(TX); }  // staged X row pitch
-constexpr int TTM_DM_MROW = 20;                                         // staged M row pitch
+__host__ __device__ constexpr int ttm_pitch(int mt) { return ttm_rows(mt) + (sizeof(TX) == 8 ? 4 : 8); }
+template <class TX>
+__host__ __device__ constexpr int ttm_xstage(int mt, bool kf) {
+    return kf ? ttm_rows(mt) * TTM_KP : TTM_BK * ttm_pitch<TX>(mt);
+}
+template <class TX>
+__host__ __device__ constexpr size_t ttm_smem(int mt, int nt, bool kf) {
+    return (size_t)ttm_stages(mt) *
+           (ttm_xstage<TX>(mt, kf) * sizeof(TX) + TTM_BK * (8 * nt + 4) * sizeof(double));
+}
 
-template <class TX>
-__global__ void __launch_bounds__(TTM_NT) ttm_dmma_kernel(const TX *__restrict__ X, int64_t L,
-                                                          int64_t I, int64_t P,
-                                                          const double *__restrict__ M,
-                                                          int64_t msj, int64_t msi, int64_t J,
-                                                          double *__restrict__ Y, int64_t kchunk,
-                                                          int64_t ysize) {
-    constexpr int EV = 16 / sizeof(TX);
-    constexpr int TTM_DM_XROW = ttm_dm_xrow<TX>();
-    extern __shared__ __align__(16) uint8_t dm_smem[];
-    auto Ms = reinterpret_cast<double(*)[TTM_BK * TTM_DM_MROW]>(dm_smem);
-    auto Xs = reinterpret_cast<TX(*)[TTM_BK * TTM_DM_XROW]>(
-        dm_smem + 2 * TTM_BK * TTM_DM_MROW * sizeof(double));
+template <class TX, int MT, int NT, bool KF, bool VEC>
+__global__ void __launch_bounds__(TTM_NT) ttm_kernel(const TX *__restrict__ X, int64_t L,
+                                                     int64_t I, int64_t P,
+                                                     const double *__restrict__ M, int64_t msj,
+                                                     int64_t msi, int64_t J,
+                                                     double *__restrict__ Y, int64_t kchunk,
+                                                     int64_t ysize) {
+    constexpr int BP = ttm_rows(MT), ST = ttm_stages(MT), MP = 8 * NT + 4;
+    constexpr int PITCH = ttm_pitch<TX>(MT), XSTAGE = ttm_xstage<TX>(MT, KF);
+    constexpr int EV = VEC ? 16 / (int)sizeof(TX) : 1;
+    extern __shared__ __align__(16) uint8_t ttm_sm[];
+    TX *Xs = reinterpret_cast<TX *>(ttm_sm);
+    double *Ms = reinterpret_cast<double *>(ttm_sm + (size_t)ST * XSTAGE * sizeof(TX));
     const int t = threadIdx.x, w = t >> 5, lane = t & 31, g = lane >> 2, t4 = lane & 3;
-    pdl_wait();
-    const int64_t p0 = (int64_t)blockIdx.x * TTM_BP;
-    const int64_t j0 = (int64_t)blockIdx.y * 16;
+    const int64_t p0 = (int64_t)blockIdx.x * BP;
+    const int64_t j0 = (int64_t)blockIdx.y * 8 * NT;
     const int64_t ibeg = (int64_t)blockIdx.z * kchunk;
     const int64_t iend = min(I, ibeg + kchunk);
+    const int nch = (int)((iend - ibeg + TTM_BK - 1) / TTM_BK);
     Y += (int64_t)blockIdx.z * ysize;
-    const int64_t nch = (iend - ibeg + TTM_BK - 1) / TTM_BK;
-    const int64_t b0 = p0 / L;
-    const int64_t l0 = p0 - b0 * L;
-    const TX *xb = X + l0 + L * I * b0;
 
-    auto issue = [&](int64_t c, int st) {
-        const int64_t i0 = ibeg + c * TTM_BK;
-        constexpr int PER_K = TTM_BP / EV;
-        for (int e = t; e < TTM_BK * PER_K; e += TTM_NT) {
-            const int k = e / PER_K, q = e - k * PER_K;
-            const int64_t i = i0 + k;
-            const bool ok = i < iend;
-            cp_async16(&Xs[st][k * TTM_DM_XROW + q * EV], ok ? xb + L * i + q * EV : X, ok ? 16 : 0);
+    // Loader.  !KF: RS row slots of EV rows, KP = 256 / RS k-rows per pass;
+    // KF: KS slots of EV k, RP = 256 / KS rows per pass.
+    constexpr int RS = KF ? TTM_BK / EV : BP / EV;
+    constexpr int PER = TTM_NT / RS;
+    const int slot = t % RS, other = t / RS;
+    const TX *src;
+    bool row_ok = true;
+    if (KF) {
+        src = X + (p0 + other) * I + ibeg + EV * slot;
+    } else {
+        const int64_t p = p0 + EV * slot;
+        row_ok = p < P;
+        const int64_t b = row_ok ? div_pos(p, L) : 0;
+        src = X + (row_ok ? p - b * L + L * I * b : 0) + (ibeg + other) * L;
+    }
+    const int mi = t & 15, mj = t >> 4;  // M: one i, j = mj (+ 16)
+    const double *msrc = M + (ibeg + mi) * msi + (j0 + mj) * msj;
+    auto issue = [&](int c) {
+        TX *xd = Xs + (c % ST) * XSTAGE;
+        const int left = (int)min((int64_t)TTM_BK, iend - ibeg - (int64_t)c * TTM_BK);
+        if (KF) {
+            const bool k_ok = EV * slot < left;
+#pragma unroll
+            for (int q = 0; q < BP / PER; q++) {
+                const int r = other + q * PER;
+                if (p0 + r < P) {
+                    const TX *s = k_ok ? src + (int64_t)q * PER * I : X;
+                    TX *d = xd + r * TTM_KP + EV * slot;
+                    if (VEC) cp_async16(d, s, k_ok ? 16 : 0);
+                    else cp_async_el<sizeof(TX)>(d, s, k_ok ? (int)sizeof(TX) : 0);
+                }
+            }
+            src += TTM_BK;
+        } else {
+            if (row_ok) {
+#pragma unroll
+                for (int q = 0; q < TTM_BK / PER; q++) {
+                    const int k = other + q * PER;
+                    const bool k_ok = k < left;
+                    const TX *s = k_ok ? src + (int64_t)q * PER * L : X;
+                    TX *d = xd + k * PITCH + EV * slot;
+                    if (VEC) cp_async16(d, s, k_ok ? 16 : 0);
+                    else cp_async_el<sizeof(TX)>(d, s, k_ok ? (int)sizeof(TX) : 0);
+                }
+            }
+            src += TTM_BK * L;
         }
-        for (int e = t; e < TTM_BK * 16; e += TTM_NT) {
-            const int k = e >> 4, j = e & 15;
-            const int64_t i = i0 + k, jj = j0 + j;
-            const bool ok = i < iend && jj < J;
-            cp_async8(&Ms[st][k * TTM_DM_MROW + j], ok ? M + jj * msj + i * msi : M, ok ? 8 : 0);
+        double *md = Ms + (c % ST) * TTM_BK * MP + mi * MP;
+#pragma unroll
+        for (int q = 0; q < (NT + 1) / 2; q++) {
+            const int j = mj + 16 * q;
+            if (j < 8 * NT) {
+                const bool ok = mi < left && j0 + j < J;
+                cp_async8(md + j, ok ? msrc + 16 * q * msj : M, ok ? 8 : 0);
+            }
         }
+        msrc += TTM_BK * msi;
         cp_async_commit();
     };
 
-    double acc[8][2][2];
+    double acc[MT][NT][2];
 #pragma unroll
-    for (int m = 0; m < 8; m++)
+    for (int m = 0; m < MT; m++)
 #pragma unroll
-        for (int n = 0; n < 2; n++) acc[m][n][0] = acc[m][n][1] = 0.0;
+        for (int n = 0; n < NT; n++) acc[m][n][0] = acc[m][n][1] = 0.0;
 
-    if (nch > 0) issue(0, 0);
-    for (int64_t c = 0; c < nch; c++) {
-        const int st = (int)(c & 1);
-        if (c + 1 < nch) {
-            issue(c + 1, st ^ 1);
-            cp_async_wait<1>();
-        } else {
-            cp_async_wait<0>();
-        }
+    pdl_wait();
+#pragma unroll
+    for (int c = 0; c < ST - 1; c++) {
+        if (c < nch) issue(c);
+        else cp_async_commit();
+    }
+    const int wrow = 8 * MT * w + g;
+    for (int c = 0; c < nch; c++) {
+        cp_async_wait<ST - 2>();
         __syncthreads();
+        if (c + ST - 1 < nch) issue(c + ST - 1);
+        else cp_async_commit();
+        const TX *xs = Xs + (c % ST) * XSTAGE + (KF ? wrow * TTM_KP + t4 : t4 * PITCH + wrow);
+        const double *ms = Ms + (c % ST) * TTM_BK * MP + t4 * MP + g;
 #pragma unroll
         for (int kk = 0; kk < TTM_BK / 4; kk++) {
-            const int k = 4 * kk + t4;
-            const double b0v = Ms[st][k * TTM_DM_MROW + g];
-            const double b1v = Ms[st][k * TTM_DM_MROW + 8 + g];
-            const TX *xr = &Xs[st][k * TTM_DM_XROW + 64 * w + g];
+            double bv[NT];
 #pragma unroll
-            for (int m = 0; m < 8; m++) {
-                const double a = (double)xr[8 * m];
-                ttm_dmma884(acc[m][0][0], acc[m][0][1], a, b0v);
-                ttm_dmma884(acc[m][1][0], acc[m][1][1], a, b1v);
+            for (int n = 0; n < NT; n++) bv[n] = ms[4 * kk * MP + 8 * n];
+#pragma unroll
+            for (int m = 0; m < MT; m++) {
+                const double av =
+                    (double)(KF ? xs[8 * m * TTM_KP + 4 * kk] : xs[4 * kk * PITCH + 8 * m]);
+#pragma unroll
+                for (int n = 0; n < NT; n++) gm_dmma884(acc[m][n][0], acc[m][n][1], av, bv[n]);
             }
         }
-        __syncthreads();
     }
 
     pdl_trigger();  // dependents may launch while the outputs are stored
-    // D[row g][col 2 t + h] of tile (m, n): row 64 w + 8 m + g, j = 8 n + 2 t + h.
-    double *y = Y + l0 + L * J * b0;
+    // D[row g][col 2 t + h] of tile (m, n).
+    const bool pairs = KF && (J & 1) == 0 && (reinterpret_cast<uintptr_t>(Y) & 15) == 0;
 #pragma unroll
-    for (int m = 0; m < 8; m++) {
-        const int64_t row = 64 * w + 8 * m + g;
+    for (int m = 0; m < MT; m++) {
+        const int64_t p = p0 + wrow + 8 * m;
+        if (p >= P) continue;
+        const int64_t b = KF ? p : div_pos(p, L);
+        double *y = Y + (p - b * L) + L * J * b;
 #pragma unroll
-        for (int n = 0; n < 2; n++)
-#pragma unroll
-            for (int h = 0; h < 2; h++) {
-                const int64_t j = j0 + 8 * n + 2 * t4 + h;
-                if (j < J) y[row + L * j] = acc[m][n][h];
+        for (int n = 0; n < NT; n++) {
+            const int64_t j = j0 + 8 * n + 2 * t4;
+            if (pairs) {
+                if (j < J)
+                    *reinterpret_cast<double2 *>(y + j) = make_double2(acc[m][n][0], acc[m][n][1]);
+            } else {
+                if (j < J) y[L * j] = acc[m][n][0];
+                if (j + 1 < J) y[L * (j + 1)] = acc[m][n][1];
             }
+        }
     }
 }
 
@@ -412,50 +240,61 @@ __global__ void sum_splits_kernel(const double *__restrict__ part, int nsplit, i
     pdl_trigger();
 }
 
-template <class TX, int JT>
-void ttm_launch(dt_ctx *ctx, const TX *X, int64_t L, int64_t I, int64_t B, const double *M,
-                int64_t msj, int64_t msi, int64_t J, double *Y) {
-    const int64_t P = L * B;
-    const int64_t base = (int64_t)ceil_div(P, TTM_BP) * ceil_div(J, JT);
-    // Few output rows: split the contraction so the GPU has enough CTAs, and
-    // sum the partial outputs in a fixed order (deterministic).
-    int64_t nsplit = 1;
-    const int64_t target = 4LL * ctx->num_sms;
-    if (base < target && I >= 64) {
-        nsplit = std::min<int64_t>((target + base - 1) / base, I / 32);
-        nsplit = std::max<int64_t>(nsplit, 1);
+template <class TX, int MT, int NT, bool KF>
+void ttm_launch(dt_ctx *ctx, dim3 grid, bool vec, const TX *X, int64_t L, int64_t I, int64_t P,
+                const double *M, int64_t msj, int64_t msi, int64_t J, double *Y, int64_t kchunk,
+                int64_t ysize) {
+    constexpr size_t smem = ttm_smem<TX>(MT, NT, KF);
+    if (vec) {
+        smem_limit(ctx, ttm_kernel<TX, MT, NT, KF, true>, smem);
+        DT_LAUNCH_PDL(ctx, (ttm_kernel<TX, MT, NT, KF, true>), grid, TTM_NT, smem, X, L, I, P, M,
+                      msj, msi, J, Y, kchunk, ysize);
+    } else {
+        smem_limit(ctx, ttm_kernel<TX, MT, NT, KF, false>, smem);
+        DT_LAUNCH_PDL(ctx, (ttm_kernel<TX, MT, NT, KF, false>), grid, TTM_NT, smem, X, L, I, P, M,
+                      msj, msi, J, Y, kchunk, ysize);
     }
-    int64_t kchunk = ((I + nsplit - 1) / nsplit + TTM_BK - 1) / TTM_BK * TTM_BK;
+}
+
+template <class TX, int NT>
+void ttm_sized(dt_ctx *ctx, const TX *X, int64_t L, int64_t I, int64_t B, const double *M,
+               int64_t msj, int64_t msi, int64_t J, double *Y) {
+    const int64_t P = L * B, jt = ceil_div(J, 8 * NT);
+    // 128 rows a CTA (three of them fit an SM) once these fill the GPU, else
+    // 64: a short contraction over few rows is a matter of latency.  256 rows in
+    // a ring of two for runs of an FP64 X (M is read half as often): 127 against
+    // 148 us for one mode of 96^4 with 16 outputs; no gain for FP32 (105 us both)
+    // or mode 0 (139 against 136).
+    int mt = ceil_div(P, 128) * jt >= 2 * ctx->num_sms ? 2 : 1;
+    const bool four = sizeof(TX) == 8 && NT <= 2 && L > 1 && ceil_div(P, 256) * jt >= 4 * ctx->num_sms;
+    if (four) mt = 4;
+    const int64_t base = ceil_div(P, 64 * mt) * jt;
+    // A long contraction over few rows is split, and the partial outputs are
+    // summed in a fixed order (deterministic).  Up to 512 the chunks' latencies
+    // cost less than the second launch.
+    int64_t nsplit = 1;
+    if (2 * base <= ctx->num_sms && I > 512)
+        nsplit = std::max<int64_t>(1, std::min<int64_t>(ctx->num_sms / base, I / 128));
+    const int64_t kchunk = ((I + nsplit - 1) / nsplit + TTM_BK - 1) / TTM_BK * TTM_BK;
     nsplit = (I + kchunk - 1) / kchunk;
     const int64_t ysize = P * J;
-    dim3 grid(ceil_div(P, TTM_BP), ceil_div(J, JT), (unsigned)nsplit);
-    const uintptr_t xa = reinterpret_cast<uintptr_t>(X);
-    const bool rows_ok = L % TTM_BP == 0 && xa % 16 == 0;
-    const bool kfast_ok = L == 1 && (I * sizeof(TX)) % 16 == 0 && xa % 16 == 0 &&
-                          (kchunk * sizeof(TX)) % 16 == 0;
-    constexpr int EV = 16 / sizeof(TX);
-    const size_t smem_rows = 2 * TTM_BK * JT * sizeof(double) + 2 * TTM_BK * TTM_BP * sizeof(TX);
-    const size_t smem_kfast =
-        2 * TTM_BK * JT * sizeof(double) + 2 * TTM_BP * (TTM_BK + EV) * sizeof(TX);
-    const size_t smem_dmma = 2 * TTM_BK * TTM_DM_MROW * sizeof(double) +
-                             2 * TTM_BK * ttm_dm_xrow<TX>() * sizeof(TX);
+    const dim3 grid(ceil_div(P, 64 * mt), (unsigned)jt, (unsigned)nsplit);
+    const bool kf = L == 1;
+    const bool vec = reinterpret_cast<uintptr_t>(X) % 16 == 0 &&
+                     (kf ? I : L) % (int64_t)(16 / sizeof(TX)) == 0;
     auto launch = [&](double *dst) {
-        if (JT == 16 && rows_ok) {
-            smem_limit(ctx, ttm_dmma_kernel<TX>, smem_dmma);
-            DT_LAUNCH_PDL(ctx, ttm_dmma_kernel<TX>, grid, TTM_NT, smem_dmma, X, L, I, P, M, msj, msi,
-                      J, dst, kchunk, ysize);
-        } else if (rows_ok) {
-            smem_limit(ctx, ttm_pipe_kernel<TX, JT, false>, smem_rows);
-            DT_LAUNCH_PDL(ctx, (ttm_pipe_kernel<TX, JT, false>), grid, TTM_NT, smem_rows, X, L, I, P,
-                      M, msj, msi, J, dst, kchunk, ysize);
-        } else if (kfast_ok) {
-            smem_limit(ctx, ttm_pipe_kernel<TX, JT, true>, smem_kfast);
-            DT_LAUNCH_PDL(ctx, (ttm_pipe_kernel<TX, JT, true>), grid, TTM_NT, smem_kfast, X, L, I, P,
-                      M, msj, msi, J, dst, kchunk, ysize);
-        }
+        if (kf && mt == 1)
+            ttm_launch<TX, 1, NT, true>(ctx, grid, vec, X, L, I, P, M, msj, msi, J, dst, kchunk, ysize);
+        else if (kf)
+            ttm_launch<TX, 2, NT, true>(ctx, grid, vec, X, L, I, P, M, msj, msi, J, dst, kchunk, ysize);
+        else if (four) {
+            if constexpr (sizeof(TX) == 8 && NT <= 2)
+                ttm_launch<TX, 4, NT, false>(ctx, grid, vec, X, L, I, P, M, msj, msi, J, dst, kchunk,
+                                             ysize);
+        } else if (mt == 1)
+            ttm_launch<TX, 1, NT, false>(ctx, grid, vec, X, L, I, P, M, msj, msi, J, dst, kchunk, ysize);
         else
-            DT_LAUNCH_PDL(ctx, (ttm_kernel<TX, JT>), grid, TTM_NT, 0, X, L, I, P, M, msj, msi, J, dst,
-                      kchunk, ysize);
+            ttm_launch<TX, 2, NT, false>(ctx, grid, vec, X, L, I, P, M, msj, msi, J, dst, kchunk, ysize);
     };
     if (nsplit == 1) {
         launch(Y);
@@ -473,12 +312,15 @@ template <class TX>
 void ttm_f64(dt_ctx *ctx, const TX *X, int64_t L, int64_t I, int64_t B, const double *M,
              int64_t msj, int64_t msi, int64_t J, double *Y) {
     if (L * B == 0 || J == 0) return;
-    if (J <= 4)
-        ttm_launch<TX, 4>(ctx, X, L, I, B, M, msj, msi, J, Y);
-    else if (J <= 8)
-        ttm_launch<TX, 8>(ctx, X, L, I, B, M, msj, msi, J, Y);
+    // One pass over X for up to 32 outputs.
+    if (J <= 8)
+        ttm_sized<TX, 1>(ctx, X, L, I, B, M, msj, msi, J, Y);
+    else if (J <= 16)
+        ttm_sized<TX, 2>(ctx, X, L, I, B, M, msj, msi, J, Y);
+    else if (J <= 24)
+        ttm_sized<TX, 3>(ctx, X, L, I, B, M, msj, msi, J, Y);
     else
-        ttm_launch<TX, 16>(ctx, X, L, I, B, M, msj, msi, J, Y);
+        ttm_sized<TX, 4>(ctx, X, L, I, B, M, msj, msi, J, Y);
 }
 template void ttm_f64<double>(dt_ctx *, const double *, int64_t, int64_t, int64_t,
                               const double *, int64_t, int64_t, int64_t, double *);
@@ -561,12 +403,6 @@ __device__ __forceinline__ void store_tile(double (*dst)[GM_P], const TileRegs &
 #pragma unroll
         for (int s = 0; s < 4; s++) dst[(t >> 6) + 4 * s][t & 63] = r.v[s];
     }
-}
-
-__device__ __forceinline__ void gm_dmma884(double &d0, double &d1, double a, double b) {
-    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
-                 : "+d"(d0), "+d"(d1)
-                 : "d"(a), "d"(b));
 }
 
 // 64 x 64 output tile per CTA on the FP64 tensor cores (mma.sync m8n8k4):

@@ -46,13 +46,9 @@ void gemm_f64(dt_ctx *ctx, int transA, int transB, int64_t m, int64_t n, int64_t
 void householder_qr(dt_ctx *ctx, const double *A, int64_t m, int64_t n, double *Q,
                     double *R, double *work);
 
-// Householder QR of `count` matrices in one launch (one CTA each): Q[b] (m[b]
-// x n[b]) from A[b].  Host arrays of device pointers.
-void householder_qr_batch(dt_ctx *ctx, int count, const double *const *A, double *const *Q,
-                          const int64_t *m, const int64_t *n);
-
-// Orthonormal bases Q[b] of span(A[b]) for a batch (CholeskyQR2 on the FP64
-// tensor-core path, Householder on breakdown or for large matrices).
+// Orthonormal bases Q[b] of span(A[b]) for a batch of up to 16 matrices
+// (CholeskyQR2 on the FP64 tensor-core path, Householder on breakdown or for
+// large matrices), one CTA each.
 void orth_batch(dt_ctx *ctx, int count, const double *const *A, double *const *Q,
                 const int64_t *m, const int64_t *n);
 

@@ -401,6 +401,16 @@ __device__ __forceinline__ void la_cp_async16(void *smem, const void *gmem) {
 __device__ __forceinline__ void la_cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 __device__ __forceinline__ void la_cp_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
+// A batch of matrices as a kernel argument (no table to copy to the device
+// and keep until the kernel is done).
+constexpr int ORTH_MAX = 16;
+struct OrthTable {
+    const double *A[ORTH_MAX];
+    double *Q[ORTH_MAX];
+    double *work[ORTH_MAX];  // m n + n doubles each
+    int64_t m[ORTH_MAX], n[ORTH_MAX];
+};
+
 constexpr int SM_WARPS = 8;
 constexpr int SM_NT = SM_WARPS * 32;
 constexpr int SM_GP = 512;  // doubles of Gram partials (K split only below 8 tiles)
@@ -870,17 +880,15 @@ __global__ void __launch_bounds__(SM_NT, 1) subspace_cluster_kernel(const double
 // breakdown falls back to Householder on work[b] (m n + n doubles).  The span
 // is that of A, as with Householder QR; the basis may differ by a rotation.
 template <int RT>
-__global__ void __launch_bounds__(SM_NT, 1) cholqr2_batch_kernel(const double *const *A,
-                                                                double *const *Q,
-                                                                const int64_t *m,
-                                                                const int64_t *n,
-                                                                double *const *work) {
+__global__ void __launch_bounds__(SM_NT, 1) cholqr2_batch_kernel(OrthTable tab) {
     using T = SmTile<RT>;
     extern __shared__ __align__(16) double sm[];
     __shared__ double red[33];
     __shared__ int bad;
     const int b = blockIdx.x, t = threadIdx.x;
-    const int M = (int)m[b], r = (int)n[b];
+    const int M = (int)tab.m[b], r = (int)tab.n[b];
+    const double *Ab = tab.A[b];
+    double *Qb = tab.Q[b];
     const int M8 = (M + 7) / 8 * 8;
     double *Z0 = sm;
     double *Z1 = Z0 + M8 * T::LDQ;
@@ -889,7 +897,7 @@ __global__ void __launch_bounds__(SM_NT, 1) cholqr2_batch_kernel(const double *c
     double *Ri = G + RT * RT;
     for (int e = t; e < M8 * T::LDQ; e += SM_NT) {
         const int i = e / T::LDQ, c = e % T::LDQ;
-        Z0[e] = (i < M && c < r) ? A[b][i + (int64_t)M * c] : 0.0;
+        Z0[e] = (i < M && c < r) ? Ab[i + (int64_t)M * c] : 0.0;
     }
     if (t == 0) bad = 0;
     __syncthreads();
@@ -909,14 +917,14 @@ __global__ void __launch_bounds__(SM_NT, 1) cholqr2_batch_kernel(const double *c
     if (!bad) {
         for (int e = t; e < M * r; e += SM_NT) {
             const int i = e % M, c = e / M;
-            Q[b][e] = cur[i * T::LDQ + c];
+            Qb[e] = cur[i * T::LDQ + c];
         }
         return;
     }
-    double *W = work[b];
-    for (int e = t; e < M * r; e += SM_NT) W[e] = A[b][e];
+    double *W = tab.work[b];
+    for (int e = t; e < M * r; e += SM_NT) W[e] = Ab[e];
     __syncthreads();
-    hqr_device(W, M, r, W + (int64_t)M * r, Q[b], red);
+    hqr_device(W, M, r, W + (int64_t)M * r, Qb, red);
 }
 
 template <int RT, bool SSM>
@@ -1060,16 +1068,14 @@ __global__ void __launch_bounds__(LA_NT) lu_inverse_kernel(const double *A, int6
 
 // Householder QR of several small matrices at once (one CTA each, 128
 // threads so the per-column barriers stay cheap): Q[b] = Q of A[b].
-__global__ void __launch_bounds__(128) hqr_batch_kernel(const double *const *A,
-                                                         double *const *Q, const int64_t *m,
-                                                         const int64_t *n, double *const *work) {
+__global__ void __launch_bounds__(128) hqr_batch_kernel(OrthTable tab) {
     __shared__ double red[33];
     const int b = blockIdx.x;
-    const int64_t mb = m[b], nb = n[b];
-    double *W = work[b];
-    for (int64_t e = threadIdx.x; e < mb * nb; e += blockDim.x) W[e] = A[b][e];
+    const int64_t mb = tab.m[b], nb = tab.n[b];
+    double *W = tab.work[b];
+    for (int64_t e = threadIdx.x; e < mb * nb; e += blockDim.x) W[e] = tab.A[b][e];
     __syncthreads();
-    hqr_device(W, mb, nb, W + mb * nb, Q[b], red);
+    hqr_device(W, mb, nb, W + mb * nb, tab.Q[b], red);
 }
 
 // Cholesky of the r x r SPD G (col-major) and L^{-1} (lower) for the row
@@ -1205,86 +1211,60 @@ void householder_qr(dt_ctx *ctx, const double *A, int64_t m, int64_t n, double *
     DT_LAUNCH(ctx, hqr_kernel, 1, LA_NT, 0, A, m, n, Q, R, work);
 }
 
-void orth_batch(dt_ctx *ctx, int count, const double *const *A, double *const *Q,
-                const int64_t *m, const int64_t *n) {
-    int64_t maxm = 0, maxn = 0;
+namespace {
+
+// The batch's table, its workspaces in one allocation.
+OrthTable orth_table(dt_ctx *ctx, int count, const double *const *A, double *const *Q,
+                     const int64_t *m, const int64_t *n, DevMem &ws) {
+    DT_CHECK_ARG(count >= 1 && count <= ORTH_MAX, "orth_batch: %d matrices", count);
+    OrthTable tab{};
+    int64_t total = 0;
     for (int b = 0; b < count; b++) {
         DT_CHECK_ARG(m[b] >= n[b] && n[b] > 0, "orth_batch: need m >= n > 0");
+        total += m[b] * n[b] + n[b];
+    }
+    ws.alloc(ctx, total * sizeof(double));
+    double *w = ws.as<double>();
+    for (int b = 0; b < count; b++) {
+        tab.A[b] = A[b];
+        tab.Q[b] = Q[b];
+        tab.work[b] = w;
+        tab.m[b] = m[b];
+        tab.n[b] = n[b];
+        w += m[b] * n[b] + n[b];
+    }
+    return tab;
+}
+
+}  // namespace
+
+void orth_batch(dt_ctx *ctx, int count, const double *const *A, double *const *Q,
+                const int64_t *m, const int64_t *n) {
+    DevMem ws;
+    const OrthTable tab = orth_table(ctx, count, A, Q, m, n, ws);
+    int64_t maxm = 0, maxn = 0;
+    for (int b = 0; b < count; b++) {
         maxm = std::max(maxm, m[b]);
         maxn = std::max(maxn, n[b]);
     }
     const int RT = maxn <= 8 ? 8 : (maxn <= 16 ? 16 : 32);
     const int64_t M8 = (maxm + 7) / 8 * 8;
     const size_t smem =
-        (2 * (size_t)M8 * (RT + 4) + SM_GP + RT * RT + RT * (RT + 4) + 32) * sizeof(double);
+        (2 * (size_t)M8 * (RT + 4) + SM_GP + RT * RT + RT * (RT + 4)) * sizeof(double);
     if (maxn > 32 || smem > 220 * 1024) {
-        householder_qr_batch(ctx, count, A, Q, m, n);
+        DT_LAUNCH(ctx, hqr_batch_kernel, count, 128, 0, tab);
         return;
     }
-    std::vector<const double *> hA(A, A + count);
-    std::vector<double *> hQ(Q, Q + count), hW(count);
-    std::vector<int64_t> hm(m, m + count), hn(n, n + count);
-    std::vector<DevMem> ws(count);
-    for (int b = 0; b < count; b++) {
-        ws[b].alloc(ctx, (m[b] * n[b] + n[b]) * sizeof(double));
-        hW[b] = ws[b].as<double>();
-    }
-    DevMem tab(ctx, count * (3 * sizeof(void *) + 2 * sizeof(int64_t)));
-    char *base = static_cast<char *>(tab.get());
-    const size_t pb = count * sizeof(void *);
-    DT_CUDA(cudaMemcpyAsync(base, hA.data(), pb, cudaMemcpyHostToDevice, ctx->stream));
-    DT_CUDA(cudaMemcpyAsync(base + pb, hQ.data(), pb, cudaMemcpyHostToDevice, ctx->stream));
-    DT_CUDA(cudaMemcpyAsync(base + 2 * pb, hW.data(), pb, cudaMemcpyHostToDevice, ctx->stream));
-    DT_CUDA(cudaMemcpyAsync(base + 3 * pb, hm.data(), count * sizeof(int64_t),
-                            cudaMemcpyHostToDevice, ctx->stream));
-    DT_CUDA(cudaMemcpyAsync(base + 3 * pb + count * sizeof(int64_t), hn.data(),
-                            count * sizeof(int64_t), cudaMemcpyHostToDevice, ctx->stream));
-    const auto *tA = reinterpret_cast<const double *const *>(base);
-    auto *tQ = reinterpret_cast<double *const *>(base + pb);
-    auto *tW = reinterpret_cast<double *const *>(base + 2 * pb);
-    const auto *tm = reinterpret_cast<const int64_t *>(base + 3 * pb);
-    const auto *tn = reinterpret_cast<const int64_t *>(base + 3 * pb + count * sizeof(int64_t));
-#define DT_CQR(R)                                                                            \
-    do {                                                                                     \
-        auto kern = cholqr2_batch_kernel<R>;                                                 \
-        smem_limit(ctx, kern, smem);                                                         \
-        DT_LAUNCH(ctx, kern, count, SM_NT, smem, tA, tQ, tm, tn, tW);                        \
+#define DT_CQR(R)                                            \
+    do {                                                     \
+        auto kern = cholqr2_batch_kernel<R>;                 \
+        smem_limit(ctx, kern, smem);                         \
+        DT_LAUNCH(ctx, kern, count, SM_NT, smem, tab);       \
     } while (0)
     if (RT == 8) DT_CQR(8);
     else if (RT == 16) DT_CQR(16);
     else DT_CQR(32);
 #undef DT_CQR
-    DT_CUDA(cudaStreamSynchronize(ctx->stream));  // host tables go out of scope
-}
-
-void householder_qr_batch(dt_ctx *ctx, int count, const double *const *A, double *const *Q,
-                          const int64_t *m, const int64_t *n) {
-    // Pointer and size tables plus per-matrix workspaces, staged to the device.
-    std::vector<const double *> hA(A, A + count);
-    std::vector<double *> hQ(Q, Q + count), hW(count);
-    std::vector<int64_t> hm(m, m + count), hn(n, n + count);
-    std::vector<DevMem> ws(count);
-    for (int b = 0; b < count; b++) {
-        DT_CHECK_ARG(m[b] >= n[b] && n[b] > 0, "householder_qr_batch: need m >= n > 0");
-        ws[b].alloc(ctx, (m[b] * n[b] + n[b]) * sizeof(double));
-        hW[b] = ws[b].as<double>();
-    }
-    DevMem tab(ctx, count * (3 * sizeof(void *) + 2 * sizeof(int64_t)));
-    char *base = static_cast<char *>(tab.get());
-    const size_t pb = count * sizeof(void *);
-    DT_CUDA(cudaMemcpyAsync(base, hA.data(), pb, cudaMemcpyHostToDevice, ctx->stream));
-    DT_CUDA(cudaMemcpyAsync(base + pb, hQ.data(), pb, cudaMemcpyHostToDevice, ctx->stream));
-    DT_CUDA(cudaMemcpyAsync(base + 2 * pb, hW.data(), pb, cudaMemcpyHostToDevice, ctx->stream));
-    DT_CUDA(cudaMemcpyAsync(base + 3 * pb, hm.data(), count * sizeof(int64_t),
-                            cudaMemcpyHostToDevice, ctx->stream));
-    DT_CUDA(cudaMemcpyAsync(base + 3 * pb + count * sizeof(int64_t), hn.data(),
-                            count * sizeof(int64_t), cudaMemcpyHostToDevice, ctx->stream));
-    DT_LAUNCH(ctx, hqr_batch_kernel, count, 128, 0, reinterpret_cast<const double *const *>(base),
-              reinterpret_cast<double *const *>(base + pb),
-              reinterpret_cast<const int64_t *>(base + 3 * pb),
-              reinterpret_cast<const int64_t *>(base + 3 * pb + count * sizeof(int64_t)),
-              reinterpret_cast<double *const *>(base + 2 * pb));
-    DT_CUDA(cudaStreamSynchronize(ctx->stream));  // host tables go out of scope
 }
 
 void subspace_iter(dt_ctx *ctx, const double *S, int64_t n, double *L, int64_t r, int iters,

@@ -102,6 +102,30 @@ def test_small_linear_algebra(ctx, oracle_ref):
     assert np.max(np.abs(np.triu(Lm, 1))) < 1e-12 and np.all(np.diag(Lm) > 0)
 
 
+@pytest.mark.parametrize("shape,mode,J", [
+    ((5, 7), 0, 1), ((16, 64), 0, 8), ((17, 65), 0, 9), ((33, 129, 3), 0, 24), ((48, 900, 50), 0, 16),
+    ((2, 31, 40), 1, 7), ((3, 16, 43), 1, 17), ((63, 15, 9), 1, 16), ((64, 32, 11), 1, 33),
+    ((130, 50, 300), 1, 12), ((131, 49, 300), 1, 25), ((256, 20, 700), 1, 16), ((255, 21, 700), 1, 8),
+    ((300, 700), 1, 40), ((9, 2000), 1, 5), ((1500, 3), 0, 10)])
+def test_ttm_tiles_and_layouts(ctx, shape, mode, J):
+    """Rows and contractions at and past the tiles' edges, runs shorter than a
+    tile and odd ones, one to several output tiles, 64, 128 and 256 rows a CTA,
+    and a split contraction.  Sums of up to 2000 products: 1e-12 of the largest
+    entry; FP32 X through one sweep of the FP64 driver."""
+    rng = np.random.default_rng(sum(shape) + mode)
+    X = np.asfortranarray(rng.standard_normal(shape))
+    M = np.asfortranarray(rng.standard_normal((J, shape[mode])))
+    want = np.moveaxis(np.tensordot(M, X, axes=([1], [mode])), 0, mode)
+    np.testing.assert_allclose(ctx.ttm(X, M, mode), want, rtol=0, atol=1e-12 * np.max(np.abs(want)))
+    ranks = [min(3, s) for s in shape]
+    if len(shape) > 2:
+        X32 = X.astype(np.float32)
+        kw = dict(init="randn", max_sweeps=1)
+        _, _, a = ctx.hooi_dense(X32, ranks, **kw)
+        _, _, b = ctx.hooi_dense(X32.astype(np.float64), ranks, **kw)
+        assert abs(a["g_norm"] - b["g_norm"]) <= 1e-12 * b["g_norm"]
+
+
 @pytest.mark.parametrize("shape,mode", [
     ((7, 5, 3), 0), ((8, 33), 0), ((33, 8), 1), ((12, 64, 9), 1), ((15, 65, 7), 1), ((16, 66, 7), 1),
     ((17, 96, 5), 1), ((97, 31, 3), 0), ((3, 128, 50), 1), ((18, 129, 4), 1), ((200, 40, 21), 0),
