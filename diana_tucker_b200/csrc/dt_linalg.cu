@@ -378,14 +378,16 @@ __global__ void __launch_bounds__(LA_NT) subspace_kernel(const double *Sg, int64
 // warps.  One SM's FP64 rate bounds a product S Z (96 x 96 x 16: 2300 cycles
 // at 64 FMA a cycle) and its shared memory holds S up to n = 130 only, so the
 // rows are dealt out: each CTA keeps its rows of S (S is symmetric: its
-// columns, contiguous in memory) in shared memory and computes its rows of
-// every product, reading its own full copy of Z, into the copies of all CTAs.
-// A CTA's rows of Z give its share of the r x r Gram, sent to all CTAs; each
-// adds the shares in the same order, factors the sum with one warp and applies
-// R^{-1} to its rows, so nothing but rows of Z and Gram shares crosses SMs.
-// Same schedule as subspace_kernel: CholeskyQR after every second product,
-// CholeskyQR and a correction after the last.  Cluster barriers: one per plain
-// product, two per CholeskyQR.  Shared-memory layout:
+// columns, contiguous in memory) in shared memory, computes its rows of every
+// product from its own full copy of Z and sends them to all CTAs.  The r x r
+// Gram, its factorisation by one warp and Z R^{-1} are small and done by every
+// CTA alike, so rows of products are all that crosses SMs.  Each sum is taken
+// in the order that one CTA would take: the results do not depend on the
+// cluster's size.  Same schedule as subspace_kernel: CholeskyQR after every
+// second product, CholeskyQR and a correction after the last.  Z goes through a
+// ring of three buffers, so a CTA may send its rows of the next product while
+// another still applies R^{-1}; with two (a third does not fit) a cluster
+// barrier follows R^{-1}.  Shared-memory layout:
 //  * the CTA's rows of S with a pitch = 4 (mod 16) and Z, Q row-major n8 x RT
 //    with pitch RT + 4: the 8 x 4 and 4 x 8 operand fragments then hit 16
 //    distinct 8-byte bank pairs per half-warp;
@@ -506,19 +508,75 @@ __device__ __forceinline__ void sm_gram(const double *src, int n, int r, double 
 }
 
 // Ri = R^{-1} (row-major, pitch LDR) of G = R^T R, by warp 0 (all threads call
-// it; ends with a barrier).  Returns false on a non-positive pivot.
+// it; ends with a barrier; G is overwritten).  Lane j holds column j in
+// registers.  The next pivot is formed first, from values exchanged before this
+// pivot's root is known, and no branch stands between the rows' updates.  Then
+// lane c solves column c of the inverse by back substitution, R read from
+// shared memory.  Every operation and its rounding is that of the plain
+// elimination (products and differences rounded one by one, two alternating
+// sums in the back substitution): the callers' factors go on to be rounded to
+// BF16 halves, where another rounding of FP64 would show.  Bound by the pivots'
+// chain (a root, a product and a difference each) and the back substitution's;
+// CTA-wide, with two barriers a pivot, it took 7400 cycles for r = 16 (the whole
+// kernel's times are at subspace_mma).  Returns false on a non-positive pivot.
 template <int RT>
-__device__ __forceinline__ bool sm_chol_inv(const double *G, double *Ri, int r) {
+__device__ __forceinline__ bool sm_chol_inv(double *G, double *Ri, int r) {
     constexpr int LDR = SmTile<RT>::LDR;
     __shared__ int good;
     const int lane = threadIdx.x;
     if (lane < 32) {
-        double y[RT];
-        const bool ok = warp_chol_linv<RT>(G, RT, r, y);
-        // Lane c holds column c of L^{-1} = row c of R^{-1}.
+        double g[RT], dinv[RT];
+#pragma unroll
+        for (int i = 0; i < RT; i++) {
+            g[i] = lane < RT ? G[i * RT + lane] : 0.0;
+            dinv[i] = 1.0;
+        }
+        double d = __shfl_sync(0xffffffffu, g[0], 0);
+        const double least = 1e-28 * d;
+        bool ok = d > 0.0;
+#pragma unroll
+        for (int k = 0; k < RT; k++) {
+            if (k >= r) break;
+            double s[RT], next = 0.0;
+#pragma unroll
+            for (int i = k + 1; i < RT; i++) s[i] = __shfl_sync(0xffffffffu, g[k], i);
+            if (k + 1 < RT) next = __shfl_sync(0xffffffffu, g[k + 1], k + 1);
+            ok = ok && d > least;
+            const double ri = rsqrt(fmax(d, 1e-300));
+            dinv[k] = ri;
+            if (k + 1 < RT) {
+                const double l = __dmul_rn(s[k + 1], ri);
+                d = __dsub_rn(next, __dmul_rn(l, l));
+            }
+            const double gk = __dmul_rn(g[k], ri);
+            g[k] = gk;
+#pragma unroll
+            for (int i = k + 1; i < RT; i++)
+                g[i] = __dsub_rn(g[i], __dmul_rn(__dmul_rn(s[i], ri), gk));
+        }
         if (lane < RT) {
 #pragma unroll
-            for (int i = 0; i < RT; i++) Ri[lane * LDR + i] = i >= lane ? y[i] : 0.0;
+            for (int i = 0; i < RT; i++) G[i * RT + lane] = g[i];
+        }
+        __syncwarp();
+        // x_i = (delta_{i,c} - sum_{j>i} R(i, j) x_j) dinv_i
+        double x[RT];
+#pragma unroll
+        for (int i = RT - 1; i >= 0; i--) {
+            double s0 = (i == lane) ? 1.0 : 0.0, s1 = 0.0;
+#pragma unroll
+            for (int j = i + 1; j < RT; j++) {
+                const double rij = G[i * RT + j];
+                if (j & 1)
+                    s1 = fma(-rij, x[j], s1);
+                else
+                    s0 = fma(-rij, x[j], s0);
+            }
+            x[i] = (s0 + s1) * dinv[i];
+        }
+        if (lane < RT) {
+#pragma unroll
+            for (int i = 0; i < RT; i++) Ri[i * LDR + lane] = i <= lane ? x[i] : 0.0;
         }
         if (lane == 0) good = ok;
     }
@@ -526,22 +584,40 @@ __device__ __forceinline__ bool sm_chol_inv(const double *G, double *Ri, int r) 
     return good != 0;
 }
 
-// After one CholeskyQR pass, Q^T Q = I + E with E tiny.  When max |E| <= 1e-9,
-// C = I - E/2 makes Q C orthonormal to rounding (the next term of the series of
-// (I + E)^{-1/2} is below 1e-17); C goes to Ri (pitch LDR) for the product.
-// Returns false when E is larger, and the caller runs a second CholeskyQR pass
-// instead.  All threads.
+// After one CholeskyQR pass, Q^T Q = I + E with E tiny.  When max |E| <= 1e-8,
+// C = I - E/2 + 3E^2/8 (the series of (I + E)^{-1/2}) makes Q C orthonormal to
+// rounding; C goes to Ri (pitch LDR) for sm_apply.  Returns false when E is too
+// large, and the caller runs a second CholeskyQR pass instead.  All threads.
 template <int RT>
-__device__ __forceinline__ bool sm_polar_fix(const double *G, double *Ri) {
+__device__ __forceinline__ bool sm_polar_fix(const double *G, double *Ri, double *red) {
     constexpr int LDR = SmTile<RT>::LDR;
-    bool small = true;
-    for (int e = threadIdx.x; e < RT * RT; e += SM_NT) {
+    const int t = threadIdx.x;
+    double emax = 0.0;
+    for (int e = t; e < RT * RT; e += SM_NT) {
         const int a = e / RT, b = e % RT;
-        const double eab = G[e] - (a == b ? 1.0 : 0.0);
-        small = small && fabs(eab) <= 1e-9;
-        Ri[a * LDR + b] = (a == b ? 1.0 : 0.0) - 0.5 * eab;
+        emax = fmax(emax, fabs(G[e] - (a == b ? 1.0 : 0.0)));
     }
-    return __syncthreads_and(small) != 0;
+    for (int o = 16; o > 0; o >>= 1) emax = fmax(emax, __shfl_xor_sync(0xffffffffu, emax, o));
+    if ((t & 31) == 0) red[t >> 5] = emax;
+    __syncthreads();
+    double m = 0.0;
+#pragma unroll
+    for (int w = 0; w < SM_WARPS; w++) m = fmax(m, red[w]);
+    if (!(m <= 1e-8)) {
+        __syncthreads();
+        return false;
+    }
+    for (int e = t; e < RT * RT; e += SM_NT) {
+        const int a = e / RT, b = e % RT;
+        double e2 = 0.0;
+#pragma unroll
+        for (int k = 0; k < RT; k++)
+            e2 = fma(G[a * RT + k] - (a == k ? 1.0 : 0.0), G[k * RT + b] - (k == b ? 1.0 : 0.0), e2);
+        const double eab = G[e] - (a == b ? 1.0 : 0.0);
+        Ri[a * LDR + b] = (a == b ? 1.0 : 0.0) - 0.5 * eab + 0.375 * e2;
+    }
+    __syncthreads();
+    return true;
 }
 
 // The cluster's CTAs: rank, size, barrier, and this CTA's address of shared
@@ -617,45 +693,23 @@ __device__ __forceinline__ bool cl_exchange(ClExchange &x, const void *p, uint32
 // a staged row.
 __host__ __device__ inline int sub_rows(int n, int c) { return 8 * (((n + 7) / 8 + c - 1) / c); }
 __host__ __device__ inline int sub_pitch(int n) { return ((n + 11) / 16) * 16 + 4; }
-// Gram shares are received in two alternating sets where they fit.
 template <int RT>
-__host__ __device__ constexpr int sub_sets() { return RT <= 16 ? 2 : 1; }
-
-template <int RT>
-__host__ inline size_t sub_smem_bytes(int n, int c, bool s_in_smem) {
+__host__ inline size_t sub_smem_bytes(int n, int c, bool s_in_smem, int bufs) {
     const int n8 = (n + 7) / 8 * 8;
-    size_t d = 2 * (size_t)n8 * SmTile<RT>::LDQ             // Z, Q
-               + (size_t)sub_sets<RT>() * c * RT * RT       // Gram shares
+    size_t d = bufs * (size_t)n8 * SmTile<RT>::LDQ          // Z
+               + (size_t)SM_GP                              // Gram partials
                + (size_t)RT * RT                            // G
                + (size_t)RT * SmTile<RT>::LDR;              // R^{-1}
     if (s_in_smem) d += (size_t)sub_rows(n, c) * sub_pitch(n);
     return d * sizeof(double);
 }
 
-// One 8 x 8 tile of A B on two interleaved accumulation chains (one chain's 32
-// cycles an MMA would leave the pipe half idle): a(k), b(k) give the lane's
-// fragment elements of k-step k.
-template <class FA, class FB>
-__device__ __forceinline__ void sub_tile(int ksteps, double &d0, double &d1, FA a, FB b) {
-    double x0 = 0.0, x1 = 0.0, y0 = 0.0, y1 = 0.0;
-    int k = 0;
-#pragma unroll 4
-    for (; k + 1 < ksteps; k += 2) {
-        dmma884(x0, x1, a(k), b(k));
-        dmma884(y0, y1, a(k + 1), b(k + 1));
-    }
-    if (k < ksteps) dmma884(x0, x1, a(k), b(k));
-    d0 = x0 + y0;
-    d1 = x1 + y1;
-}
-
 template <int RT, bool SSM>
 __global__ void __launch_bounds__(SM_NT, 1) subspace_cluster_kernel(const double *Sg, int n,
                                                                     double *Lg, int r, int iters,
                                                                     double *work, int *flag,
-                                                                    int csize) {
+                                                                    int csize, int bufs) {
     using T = SmTile<RT>;
-    constexpr int SETS = sub_sets<RT>();
     extern __shared__ __align__(16) double sm[];
     __shared__ double red[33];
     __shared__ __align__(8) uint64_t bars[2];
@@ -673,13 +727,12 @@ __global__ void __launch_bounds__(SM_NT, 1) subspace_cluster_kernel(const double
     const int own0 = (int)rank * sub_rows(n, csize);
     const int own = max(0, min(n8 - own0, sub_rows(n, csize)));  // this CTA's rows
     const int mt = own / 8, ksteps = (n + 3) / 4;
-    double *cur = sm;
-    double *oth = cur + n8 * T::LDQ;
-    double *shares = oth + n8 * T::LDQ;
-    double *G = shares + SETS * csize * RT * RT;
+    double *const ring = sm;  // `bufs` copies of Z
+    double *Gp = ring + bufs * n8 * T::LDQ;
+    double *G = Gp + SM_GP;
     double *Ri = G + RT * RT;
     double *Ss = Ri + RT * T::LDR;
-    for (int e = t; e < 2 * n8 * T::LDQ; e += SM_NT) cur[e] = 0.0;  // both buffers
+    for (int e = t; e < bufs * n8 * T::LDQ; e += SM_NT) ring[e] = 0.0;
     if (SSM) {
         // Padding of the staged rows: k = n .. 4 ksteps - 1, and rows past n.
         for (int e = t; e < own * (4 * ksteps - n); e += SM_NT) {
@@ -709,7 +762,7 @@ __global__ void __launch_bounds__(SM_NT, 1) subspace_cluster_kernel(const double
     }
     __syncthreads();  // the zeroed buffers
     {
-        // L (n x r col-major) -> cur (row-major, zero padded): all loads of a
+        // L (n x r col-major) -> the ring's first (row-major, zero padded): all loads of a
         // thread are issued before its stores.
         constexpr int MAXQ = RT;  // n * r <= 256 * RT = SM_NT * MAXQ
         double v[MAXQ];
@@ -723,7 +776,7 @@ __global__ void __launch_bounds__(SM_NT, 1) subspace_cluster_kernel(const double
             const int e = t + SM_NT * q;
             if (e < n * r) {
                 const int c = e / n, i = e - c * n;
-                cur[i * T::LDQ + c] = v[q];
+                ring[i * T::LDQ + c] = v[q];
             }
         }
     }
@@ -732,109 +785,53 @@ __global__ void __launch_bounds__(SM_NT, 1) subspace_cluster_kernel(const double
     if (csize > 1) cl_sync();
     else __syncthreads();
 
-    // dst(own rows) = S(own rows, :) src.
+    // dst(own rows) = S(own rows, :) src, k-steps in order.
     auto product = [&](const double *src, double *dst) {
         for (int job = w; job < mt * T::NT; job += SM_WARPS) {
             const int m = job / T::NT, j = job - m * T::NT;
-            double d0, d1;
+            double d0 = 0.0, d1 = 0.0;
+            const double *bs = src + t4 * T::LDQ + 8 * j + g;
             if (SSM) {
                 const double *as = Ss + (8 * m + g) * lds + t4;
-                const double *bs = src + t4 * T::LDQ + 8 * j + g;
-                sub_tile(ksteps, d0, d1, [&](int k) { return as[4 * k]; },
-                         [&](int k) { return bs[4 * k * T::LDQ]; });
+#pragma unroll 8
+                for (int k = 0; k < ksteps; k++) dmma884(d0, d1, as[4 * k], bs[4 * k * T::LDQ]);
             } else {
                 const int i = own0 + 8 * m + g;
-                sub_tile(ksteps, d0, d1,
-                         [&](int k) {
-                             const int kk = 4 * k + t4;
-                             return i < n && kk < n ? __ldg(Sg + (int64_t)n * i + kk) : 0.0;
-                         },
-                         [&](int k) { return src[(4 * k + t4) * T::LDQ + 8 * j + g]; });
+#pragma unroll 8
+                for (int k = 0; k < ksteps; k++) {
+                    const int kk = 4 * k + t4;
+                    const double av = i < n && kk < n ? __ldg(Sg + (int64_t)n * i + kk) : 0.0;
+                    dmma884(d0, d1, av, bs[4 * k * T::LDQ]);
+                }
             }
             *reinterpret_cast<double2 *>(dst + (own0 + 8 * m + g) * T::LDQ + 8 * j + 2 * t4) =
                 make_double2(d0, d1);
         }
     };
-    // Everybody's rows of z to everybody.
     const uint32_t row_bytes = T::LDQ * sizeof(double);
-    auto exchange_rows = [&](double *z) {
-        return cl_exchange(ex, z + own0 * T::LDQ, own * row_bytes, (n8 - own) * row_bytes);
-    };
-    // This CTA's share of src^T src, to set `set` of all CTAs; then the sum of
-    // all shares in G (rows / columns >= r: the identity).
-    auto gram = [&](const double *src, int set) {
-        double *all = shares + set * csize * RT * RT, *mine = all + rank * RT * RT;
-        for (int job = w; job < T::NT * T::NT; job += SM_WARPS) {
-            const int ta = job % T::NT, tb = job / T::NT;
-            const double *as = src + (own0 + t4) * T::LDQ + 8 * ta + g;
-            const double *bs = src + (own0 + t4) * T::LDQ + 8 * tb + g;
-            double d0, d1;
-            sub_tile(2 * mt, d0, d1, [&](int k) { return as[4 * k * T::LDQ]; },
-                     [&](int k) { return bs[4 * k * T::LDQ]; });
-            *reinterpret_cast<double2 *>(mine + (8 * ta + g) * RT + 8 * tb + 2 * t4) =
-                make_double2(d0, d1);
-        }
-        const uint32_t bytes = RT * RT * sizeof(double);
-        const bool ok = cl_exchange(ex, mine, bytes, (csize - 1) * bytes);
-        for (int e = t; e < RT * RT; e += SM_NT) {
-            const int a = e / RT, b = e % RT;
-            double s = 0.0;
-            for (int q = 0; q < csize; q++) s += all[q * RT * RT + e];
-            G[e] = (a < r && b < r) ? s : (a == b ? 1.0 : 0.0);
-        }
-        __syncthreads();
-        return ok;
-    };
-    // dst(own rows) = src(own rows) Ri.
-    auto apply = [&](const double *src, double *dst) {
-        for (int job = w; job < mt * T::NT; job += SM_WARPS) {
-            const int m = job / T::NT, j = job - m * T::NT;
-            const double *as = src + (own0 + 8 * m + g) * T::LDQ + t4;
-            const double *bs = Ri + t4 * T::LDR + 8 * j + g;
-            double d0, d1;
-            sub_tile(RT / 4, d0, d1, [&](int k) { return as[4 * k]; },
-                     [&](int k) { return bs[4 * k * T::LDR]; });
-            *reinterpret_cast<double2 *>(dst + (own0 + 8 * m + g) * T::LDQ + 8 * j + 2 * t4) =
-                make_double2(d0, d1);
-        }
-    };
+    int at = 0;  // Z's place in the ring
+    auto z = [&](int k) { return ring + ((at + k) % bufs) * n8 * T::LDQ; };
 
     bool bad = false, late = false;
-    int set = 0;
-    for (int it = 0; it < iters && !late; it++) {
+    for (int it = 0; it < iters && !late && !bad; it++) {
         const bool last = it == iters - 1;
-        product(cur, oth);
-        if (!last && !(it & 1)) {
-            late = !exchange_rows(oth);
-            double *x = cur;
-            cur = oth;
-            oth = x;
-            continue;
+        product(z(0), z(1));
+        // Everybody's rows to everybody.
+        late = !cl_exchange(ex, z(1) + own0 * T::LDQ, own * row_bytes, (n8 - own) * row_bytes);
+        at = (at + 1) % bufs;
+        if (!last && !(it & 1)) continue;
+        for (int p = 0; p < (last ? 2 : 1); p++) {
+            sm_gram<RT>(z(0), n, r, Gp, G);
+            // The second pass is usually a tiny correction (polar fix).
+            if (!(p == 1 && sm_polar_fix<RT>(G, Ri, red)) && !sm_chol_inv<RT>(G, Ri, r)) {
+                bad = true;  // the same G, so the same answer, in every CTA
+                break;
+            }
+            sm_apply<RT>(z(0), Ri, n8, z(1));
+            __syncthreads();
+            at = (at + 1) % bufs;
         }
-        __syncthreads();
-        late = !gram(oth, set);
-        if (SETS == 2) set ^= 1;
-        if (!sm_chol_inv<RT>(G, Ri, r)) {  // the same G, so the same answer, in every CTA
-            bad = true;
-            break;
-        }
-        // All CTAs are past their products (their shares came): cur is free.
-        apply(oth, cur);
-        if (!last) {
-            late = late || !exchange_rows(cur);
-            continue;
-        }
-        __syncthreads();
-        // Second pass on the last step, usually a tiny correction.  With one
-        // set of shares the other CTAs have to be done with theirs first.
-        if (SETS == 1 && csize > 1) cl_sync();
-        late = late || !gram(cur, set);
-        if (!sm_polar_fix<RT>(G, Ri) && !sm_chol_inv<RT>(G, Ri, r)) {
-            bad = true;
-            break;
-        }
-        apply(cur, oth);
-        __syncthreads();
+        if (bufs == 2 && csize > 1 && !last && !bad) cl_sync();
     }
     // No CTA leaves while another still reads or fills its shared memory.
     if (csize > 1) cl_sync();
@@ -849,7 +846,7 @@ __global__ void __launch_bounds__(SM_NT, 1) subspace_cluster_kernel(const double
     if (!bad) {
         for (int e = t; e < have * r; e += SM_NT) {
             const int c = e / have, i = own0 + (e - c * have);
-            Lg[(int64_t)n * c + i] = oth[i * T::LDQ + c];
+            Lg[(int64_t)n * c + i] = z(0)[i * T::LDQ + c];
         }
         return;
     }
@@ -929,11 +926,12 @@ __global__ void __launch_bounds__(SM_NT, 1) cholqr2_batch_kernel(OrthTable tab) 
 
 template <int RT, bool SSM>
 void launch_subspace(dt_ctx *ctx, const double *S, int n, double *L, int r, int iters,
-                     double *work, int *flag, int csize) {
-    const size_t smem = sub_smem_bytes<RT>(n, csize, SSM);
+                     double *work, int *flag, int csize, int bufs) {
+    const size_t smem = sub_smem_bytes<RT>(n, csize, SSM, bufs);
     auto kern = subspace_cluster_kernel<RT, SSM>;
     smem_limit(ctx, kern, smem);
-    launch_pdl_cluster(ctx, kern, csize, SM_NT, smem, csize, S, n, L, r, iters, work, flag, csize);
+    launch_pdl_cluster(ctx, kern, csize, SM_NT, smem, csize, S, n, L, r, iters, work, flag, csize,
+                       bufs);
 }
 
 template <int RT>
@@ -941,20 +939,18 @@ void subspace_mma(dt_ctx *ctx, const double *S, int n, double *L, int r, int ite
                   double *work, int *flag) {
     const size_t cap = 220 * 1024;
     // Up to 64 rows one CTA: an exchange costs more than the part of a product
-    // it saves (64 x 8, 5 steps: 12.8 us on one CTA, 13.1 on four).  Above, eight:
-    // 96 x 16, 5 steps 28.8 us on one CTA, 25.0 on two, 22.6 on four, 21.9 on
-    // eight; 200 x 10, 30 steps 135 on two or four, 110 on eight.  The single-CTA
-    // kernel before this one took 35 us for 96 x 16 (5 steps), 20 (2 steps), and
-    // 112 us for 256 x 12 with S read from L2.
+    // it saves (64 x 8, 5 steps: 13.6 us on one CTA, 14.8 on eight).  Above,
+    // eight: 96 x 16, 5 steps 32.0 us on one CTA, 29.7 on two, 26.5 on four, 26.1 on
+    // eight; 200 x 10, 30 steps 154 on four, 128 on eight.  The single-CTA kernel
+    // before this one took 35 us for 96 x 16 in 5 steps and 20 in 2 (15.2 here),
+    // and 112 us for 256 x 12 with S read from L2 (37 here).
     const int c = n <= 64 ? 1 : 8;
-    if (sub_smem_bytes<RT>(n, c, true) <= cap) {
-        launch_subspace<RT, true>(ctx, S, n, L, r, iters, work, flag, c);
-        return;
-    }
-    // r > 16 and n > 200 or so: S stays in L2, fewer CTAs for fewer shares.
-    int few = c;
-    while (few > 1 && sub_smem_bytes<RT>(n, few, false) > cap) few /= 2;
-    launch_subspace<RT, false>(ctx, S, n, L, r, iters, work, flag, few);
+    if (sub_smem_bytes<RT>(n, c, true, 3) <= cap)
+        launch_subspace<RT, true>(ctx, S, n, L, r, iters, work, flag, c, 3);
+    else if (sub_smem_bytes<RT>(n, c, true, 2) <= cap)
+        launch_subspace<RT, true>(ctx, S, n, L, r, iters, work, flag, c, 2);
+    else  // r > 16 and n > 230 or so: S stays in L2
+        launch_subspace<RT, false>(ctx, S, n, L, r, iters, work, flag, c, 2);
 }
 
 // Subspace iteration for ranks above 32: Householder QR every step, S, L and Z
