@@ -20,6 +20,10 @@
 
 struct dt_sptensor;
 
+namespace dt {
+class DevArena;
+}
+
 struct dt_ctx {
     // Sparse tensors created on this context; dt_ctx_destroy frees their device
     // memory and detaches them, so a later dt_sptensor_destroy only frees the
@@ -51,6 +55,10 @@ struct dt_ctx {
     // The batched HOOI's tuned configurations, instantiated graphs and
     // device-resident argument block (dt_hooi_batched).
     std::shared_ptr<void> batched;
+    // While set, DevMem takes its memory from here (a plan's sweep, DevArena);
+    // with `dry` no kernel is launched (the pass that sizes the arena).
+    dt::DevArena *arena = nullptr;
+    bool dry = false;
     // Summary profiler state (dt_summary_*; null until first enabled).
     std::shared_ptr<void> summary;
 };
@@ -90,6 +98,7 @@ void clear_last_error();
 // of this library's kernels a call ran, and launch errors surface at once.
 #define DT_LAUNCH(ctx, kernel, grid, block, smem, ...)                     \
     do {                                                                   \
+        if ((ctx)->dry) break;                                             \
         kernel<<<(grid), (block), (smem), (ctx)->stream>>>(__VA_ARGS__);   \
         (ctx)->launches++;                                                 \
         DT_CUDA(cudaGetLastError());                                       \
@@ -111,6 +120,27 @@ __device__ __forceinline__ void pdl_trigger() {
 bool pdl_enabled();
 // DT_DISABLE_GRAPHS=1 in the environment launches every sweep directly.
 bool graphs_enabled();
+// Whether ctx's stream can be captured and takes programmatic dependent
+// launches: any but the legacy and the per-thread default stream.
+inline bool plain_stream(const dt_ctx *ctx) {
+    return ctx->stream != nullptr && ctx->stream != cudaStreamLegacy &&
+           ctx->stream != cudaStreamPerThread;
+}
+// Captures on the context's own stream when the caller's cannot be captured;
+// the graph is launched into the caller's all the same.
+class CaptureStream {
+   public:
+    explicit CaptureStream(dt_ctx *ctx) : ctx_(ctx), saved_(ctx->stream) {
+        if (!plain_stream(ctx)) ctx->stream = ctx->own_stream;
+    }
+    ~CaptureStream() { ctx_->stream = saved_; }
+    CaptureStream(const CaptureStream &) = delete;
+    CaptureStream &operator=(const CaptureStream &) = delete;
+
+   private:
+    dt_ctx *ctx_;
+    cudaStream_t saved_;
+};
 // Whether the Summary profiler is recording on ctx.
 bool summary_active(dt_ctx *ctx);
 
@@ -118,16 +148,15 @@ bool summary_active(dt_ctx *ctx);
 template <class... KArgs, class... Args>
 void launch_pdl_cluster(dt_ctx *ctx, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,
                         int cluster, Args &&...args) {
+    if (ctx->dry) return;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = block;
     cfg.dynamicSmemBytes = smem;
     cfg.stream = ctx->stream;
     cudaLaunchAttribute attr[2];
-    const bool plain_stream = ctx->stream != nullptr && ctx->stream != cudaStreamLegacy &&
-                              ctx->stream != cudaStreamPerThread;
     int n = 0;
-    if (pdl_enabled() && plain_stream) {
+    if (pdl_enabled() && plain_stream(ctx)) {
         attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
         attr[n++].val.programmaticStreamSerializationAllowed = 1;
     }
@@ -192,8 +221,9 @@ inline void smem_limit(dt_ctx *ctx, K *kernel, size_t bytes) {
 
 // One launch sequence (a HOOI sweep) captured as a CUDA graph and replayed on
 // ctx->stream.  Capture fails over to direct execution: run() then calls fn()
-// itself (the capture executed nothing).  Graphs are not used on the legacy
-// or per-thread default streams, or when DT_DISABLE_GRAPHS=1.
+// itself (the capture executed nothing).  On the legacy and per-thread default
+// streams, which cannot be captured, the capture is taken on the context's own
+// stream (CaptureStream).  Graphs are not used when DT_DISABLE_GRAPHS=1.
 class SweepGraph {
    public:
     SweepGraph() = default;
@@ -234,6 +264,24 @@ void release_plan(dt_ctx *ctx, std::shared_ptr<void> &plan);
 // detaches it (called by dt_ctx_destroy).
 void detach_sptensors(dt_ctx *ctx);
 
+// Device memory that one sequence of kernels takes and gives back in the same
+// order every time it runs (a HOOI sweep): one buffer, handed out first fit
+// from offset 0, so a captured sequence sees the same addresses and holds no
+// allocation nodes.  Blocks are reused as soon as they are given back: their
+// users follow one another on one stream.  Sized by a dry pass (dt_ctx::dry)
+// over the sequence.
+class DevArena {
+   public:
+    size_t need = 0, cap = 0;  // most bytes in use so far; bytes there are
+    char *base = nullptr;
+    void *take(size_t bytes);
+    void give(void *p);
+
+   private:
+    std::vector<std::pair<size_t, size_t>> used_;  // (offset, bytes), by offset
+};
+
+
 // Stream-ordered device allocation owned by one call.
 class DevMem {
    public:
@@ -260,10 +308,12 @@ class DevMem {
         std::swap(p_, o.p_);
         std::swap(bytes_, o.bytes_);
         std::swap(ctx_, o.ctx_);
+        std::swap(arena_, o.arena_);
     }
     void *p_ = nullptr;
     size_t bytes_ = 0;
     dt_ctx *ctx_ = nullptr;
+    DevArena *arena_ = nullptr;  // where it came from (null: the device's pool)
 };
 
 // A host buffer copied to a new device buffer in ctx->kCopyChunks chunks on

@@ -3,6 +3,7 @@
 #include <cstdlib>
 #include <map>
 #include <mutex>
+#include <optional>
 
 #include "dt_core.cuh"
 
@@ -78,13 +79,12 @@ void SweepGraph::reset() {
 }
 
 void SweepGraph::run(dt_ctx *ctx, const std::function<void()> &fn) {
-    const bool plain_stream = ctx->stream != nullptr && ctx->stream != cudaStreamLegacy &&
-                              ctx->stream != cudaStreamPerThread;
     if (!exec_) {
-        if (failed_ || !plain_stream || !graphs_enabled()) {
+        if (failed_ || !graphs_enabled()) {
             fn();
             return;
         }
+        std::optional<CaptureStream> on(ctx);
         const int64_t l0 = ctx->launches;
         auto give_up = [&](cudaGraph_t g) {
             if (g) cudaGraphDestroy(g);
@@ -107,22 +107,26 @@ void SweepGraph::run(dt_ctx *ctx, const std::function<void()> &fn) {
                 throw;
             }
             give_up(g);
+            on.reset();
             fn();
             return;
         } catch (...) {
             cudaStreamEndCapture(ctx->stream, &g);
             give_up(g);
+            on.reset();
             fn();
             return;
         }
         if (cudaStreamEndCapture(ctx->stream, &g) != cudaSuccess || !g) {
             give_up(g);
+            on.reset();
             fn();
             return;
         }
         if (cudaGraphInstantiateWithFlags(&exec_, g, 0) != cudaSuccess) {
             exec_ = nullptr;
             give_up(g);
+            on.reset();
             fn();
             return;
         }
@@ -144,9 +148,36 @@ void raise_smem_limit(dt_ctx *ctx, const void *kernel, size_t bytes) {
     cur = bytes;
 }
 
+void *DevArena::take(size_t bytes) {
+    bytes = (bytes + 255) & ~size_t(255);
+    size_t off = 0;
+    auto at = used_.begin();
+    for (; at != used_.end() && at->first - off < bytes; ++at) off = at->first + at->second;
+    used_.insert(at, {off, bytes});
+    need = std::max(need, off + bytes);
+    if (cap && off + bytes > cap)
+        fail(DT_ERR_CUDA, fmt("internal: sweep arena of %zu bytes exceeded", cap));
+    return base + off;
+}
+
+void DevArena::give(void *p) {
+    const size_t off = (size_t)(static_cast<char *>(p) - base);
+    for (auto it = used_.begin(); it != used_.end(); ++it)
+        if (it->first == off) {
+            used_.erase(it);
+            return;
+        }
+}
+
 void DevMem::alloc(dt_ctx *ctx, size_t bytes) {
     release();
     if (bytes == 0) return;
+    if (ctx->arena) {
+        p_ = ctx->arena->take(bytes);
+        arena_ = ctx->arena;
+        bytes_ = bytes;
+        return;
+    }
     if (ctx->mem_limit && ctx->mem_in_use + bytes > ctx->mem_limit)
         fail(DT_ERR_NOMEM, fmt("device allocation of %zu bytes would exceed the context's "
                                "limit (%llu of %llu bytes in use)",
@@ -168,6 +199,8 @@ void DevMem::alloc(dt_ctx *ctx, size_t bytes) {
 }
 
 void DevMem::release() {
+    if (arena_) arena_->give(p_);
+    arena_ = nullptr;
     if (p_ && ctx_) {
         cudaFreeAsync(p_, ctx_->stream);
         ctx_->mem_in_use -= bytes_;

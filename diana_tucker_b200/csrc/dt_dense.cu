@@ -95,10 +95,11 @@ __global__ void __launch_bounds__(TTM_NT) ttm_kernel(const TX *__restrict__ X, i
                                                      const double *__restrict__ M, int64_t msj,
                                                      int64_t msi, int64_t J,
                                                      double *__restrict__ Y, int64_t kchunk,
-                                                     int64_t ysize) {
+                                                     int64_t ysize, const void *const *slot) {
     constexpr int BP = ttm_rows(MT), ST = ttm_stages(MT), MP = 8 * NT + 4;
     constexpr int PITCH = ttm_pitch<TX>(MT), XSTAGE = ttm_xstage<TX>(MT, KF);
     constexpr int EV = VEC ? 16 / (int)sizeof(TX) : 1;
+    if (slot) X = static_cast<const TX *>(*slot);
     extern __shared__ __align__(16) uint8_t ttm_sm[];
     TX *Xs = reinterpret_cast<TX *>(ttm_sm);
     double *Ms = reinterpret_cast<double *>(ttm_sm + (size_t)ST * XSTAGE * sizeof(TX));
@@ -114,13 +115,13 @@ __global__ void __launch_bounds__(TTM_NT) ttm_kernel(const TX *__restrict__ X, i
     // KF: KS slots of EV k, RP = 256 / KS rows per pass.
     constexpr int RS = KF ? TTM_BK / EV : BP / EV;
     constexpr int PER = TTM_NT / RS;
-    const int slot = t % RS, other = t / RS;
+    const int ls = t % RS, other = t / RS;
     const TX *src;
     bool row_ok = true;
     if (KF) {
-        src = X + (p0 + other) * I + ibeg + EV * slot;
+        src = X + (p0 + other) * I + ibeg + EV * ls;
     } else {
-        const int64_t p = p0 + EV * slot;
+        const int64_t p = p0 + EV * ls;
         row_ok = p < P;
         const int64_t b = row_ok ? div_pos(p, L) : 0;
         src = X + (row_ok ? p - b * L + L * I * b : 0) + (ibeg + other) * L;
@@ -131,13 +132,13 @@ __global__ void __launch_bounds__(TTM_NT) ttm_kernel(const TX *__restrict__ X, i
         TX *xd = Xs + (c % ST) * XSTAGE;
         const int left = (int)min((int64_t)TTM_BK, iend - ibeg - (int64_t)c * TTM_BK);
         if (KF) {
-            const bool k_ok = EV * slot < left;
+            const bool k_ok = EV * ls < left;
 #pragma unroll
             for (int q = 0; q < BP / PER; q++) {
                 const int r = other + q * PER;
                 if (p0 + r < P) {
                     const TX *s = k_ok ? src + (int64_t)q * PER * I : X;
-                    TX *d = xd + r * TTM_KP + EV * slot;
+                    TX *d = xd + r * TTM_KP + EV * ls;
                     if (VEC) cp_async16(d, s, k_ok ? 16 : 0);
                     else cp_async_el<sizeof(TX)>(d, s, k_ok ? (int)sizeof(TX) : 0);
                 }
@@ -150,7 +151,7 @@ __global__ void __launch_bounds__(TTM_NT) ttm_kernel(const TX *__restrict__ X, i
                     const int k = other + q * PER;
                     const bool k_ok = k < left;
                     const TX *s = k_ok ? src + (int64_t)q * PER * L : X;
-                    TX *d = xd + k * PITCH + EV * slot;
+                    TX *d = xd + k * PITCH + EV * ls;
                     if (VEC) cp_async16(d, s, k_ok ? 16 : 0);
                     else cp_async_el<sizeof(TX)>(d, s, k_ok ? (int)sizeof(TX) : 0);
                 }
@@ -243,22 +244,22 @@ __global__ void sum_splits_kernel(const double *__restrict__ part, int nsplit, i
 template <class TX, int MT, int NT, bool KF>
 void ttm_launch(dt_ctx *ctx, dim3 grid, bool vec, const TX *X, int64_t L, int64_t I, int64_t P,
                 const double *M, int64_t msj, int64_t msi, int64_t J, double *Y, int64_t kchunk,
-                int64_t ysize) {
+                int64_t ysize, const void *const *slot) {
     constexpr size_t smem = ttm_smem<TX>(MT, NT, KF);
     if (vec) {
         smem_limit(ctx, ttm_kernel<TX, MT, NT, KF, true>, smem);
         DT_LAUNCH_PDL(ctx, (ttm_kernel<TX, MT, NT, KF, true>), grid, TTM_NT, smem, X, L, I, P, M,
-                      msj, msi, J, Y, kchunk, ysize);
+                      msj, msi, J, Y, kchunk, ysize, slot);
     } else {
         smem_limit(ctx, ttm_kernel<TX, MT, NT, KF, false>, smem);
         DT_LAUNCH_PDL(ctx, (ttm_kernel<TX, MT, NT, KF, false>), grid, TTM_NT, smem, X, L, I, P, M,
-                      msj, msi, J, Y, kchunk, ysize);
+                      msj, msi, J, Y, kchunk, ysize, slot);
     }
 }
 
 template <class TX, int NT>
 void ttm_sized(dt_ctx *ctx, const TX *X, int64_t L, int64_t I, int64_t B, const double *M,
-               int64_t msj, int64_t msi, int64_t J, double *Y) {
+               int64_t msj, int64_t msi, int64_t J, double *Y, const void *const *slot) {
     const int64_t P = L * B, jt = ceil_div(J, 8 * NT);
     // 128 rows a CTA (three of them fit an SM) once these fill the GPU, else
     // 64: a short contraction over few rows is a matter of latency.  256 rows in
@@ -284,17 +285,17 @@ void ttm_sized(dt_ctx *ctx, const TX *X, int64_t L, int64_t I, int64_t B, const 
                      (kf ? I : L) % (int64_t)(16 / sizeof(TX)) == 0;
     auto launch = [&](double *dst) {
         if (kf && mt == 1)
-            ttm_launch<TX, 1, NT, true>(ctx, grid, vec, X, L, I, P, M, msj, msi, J, dst, kchunk, ysize);
+            ttm_launch<TX, 1, NT, true>(ctx, grid, vec, X, L, I, P, M, msj, msi, J, dst, kchunk, ysize, slot);
         else if (kf)
-            ttm_launch<TX, 2, NT, true>(ctx, grid, vec, X, L, I, P, M, msj, msi, J, dst, kchunk, ysize);
+            ttm_launch<TX, 2, NT, true>(ctx, grid, vec, X, L, I, P, M, msj, msi, J, dst, kchunk, ysize, slot);
         else if (four) {
             if constexpr (sizeof(TX) == 8 && NT <= 2)
                 ttm_launch<TX, 4, NT, false>(ctx, grid, vec, X, L, I, P, M, msj, msi, J, dst, kchunk,
-                                             ysize);
+                                             ysize, slot);
         } else if (mt == 1)
-            ttm_launch<TX, 1, NT, false>(ctx, grid, vec, X, L, I, P, M, msj, msi, J, dst, kchunk, ysize);
+            ttm_launch<TX, 1, NT, false>(ctx, grid, vec, X, L, I, P, M, msj, msi, J, dst, kchunk, ysize, slot);
         else
-            ttm_launch<TX, 2, NT, false>(ctx, grid, vec, X, L, I, P, M, msj, msi, J, dst, kchunk, ysize);
+            ttm_launch<TX, 2, NT, false>(ctx, grid, vec, X, L, I, P, M, msj, msi, J, dst, kchunk, ysize, slot);
     };
     if (nsplit == 1) {
         launch(Y);
@@ -310,22 +311,24 @@ void ttm_sized(dt_ctx *ctx, const TX *X, int64_t L, int64_t I, int64_t B, const 
 
 template <class TX>
 void ttm_f64(dt_ctx *ctx, const TX *X, int64_t L, int64_t I, int64_t B, const double *M,
-             int64_t msj, int64_t msi, int64_t J, double *Y) {
+             int64_t msj, int64_t msi, int64_t J, double *Y, const void *const *slot) {
     if (L * B == 0 || J == 0) return;
     // One pass over X for up to 32 outputs.
     if (J <= 8)
-        ttm_sized<TX, 1>(ctx, X, L, I, B, M, msj, msi, J, Y);
+        ttm_sized<TX, 1>(ctx, X, L, I, B, M, msj, msi, J, Y, slot);
     else if (J <= 16)
-        ttm_sized<TX, 2>(ctx, X, L, I, B, M, msj, msi, J, Y);
+        ttm_sized<TX, 2>(ctx, X, L, I, B, M, msj, msi, J, Y, slot);
     else if (J <= 24)
-        ttm_sized<TX, 3>(ctx, X, L, I, B, M, msj, msi, J, Y);
+        ttm_sized<TX, 3>(ctx, X, L, I, B, M, msj, msi, J, Y, slot);
     else
-        ttm_sized<TX, 4>(ctx, X, L, I, B, M, msj, msi, J, Y);
+        ttm_sized<TX, 4>(ctx, X, L, I, B, M, msj, msi, J, Y, slot);
 }
 template void ttm_f64<double>(dt_ctx *, const double *, int64_t, int64_t, int64_t,
-                              const double *, int64_t, int64_t, int64_t, double *);
+                              const double *, int64_t, int64_t, int64_t, double *,
+                              const void *const *);
 template void ttm_f64<float>(dt_ctx *, const float *, int64_t, int64_t, int64_t,
-                             const double *, int64_t, int64_t, int64_t, double *);
+                             const double *, int64_t, int64_t, int64_t, double *,
+                             const void *const *);
 
 // ---------------------------------------------------------------------------
 // Generic FP64 GEMM C(i, j) = sum_q a(i, q) b(j, q) over operands addressed as

@@ -22,7 +22,90 @@ namespace dt {
 
 namespace {
 
+__global__ void loop_begin_kernel(LoopState *st, double thr, int max_sweeps, const void *x) {
+    st->it = 0;
+    st->max_sweeps = max_sweeps;
+    st->prev = -1.0;
+    st->thr = thr;
+    st->x = x;
+}
+
+__global__ void sweep_check_kernel(cudaGraphConditionalHandle h, const double *scal,
+                                   LoopState *st) {
+    pdl_wait();
+    const double x2 = scal[0], g2 = scal[1];
+    const double res = sqrt(fmax(0.0, 1.0 - g2 / x2));
+    const int it = st->it;
+    if (it < DT_MAX_HIST) st->hist[it] = res;
+    const bool stop = it + 1 >= st->max_sweeps ||
+                      (st->thr > 0.0 && it > 0 && fabs(res - st->prev) < st->thr);
+    st->prev = res;
+    st->it = it + 1;
+    cudaGraphSetConditional(h, stop ? 0u : 1u);
+}
+
 }  // namespace
+
+SweepLoop::~SweepLoop() {
+    if (exec_) cudaGraphExecDestroy(exec_);
+}
+
+LoopState *SweepLoop::state(dt_ctx *ctx) {
+    if (!state_.get()) state_.alloc(ctx, sizeof(LoopState));
+    return state_.as<LoopState>();
+}
+
+bool SweepLoop::build(dt_ctx *ctx, const double *scal, const std::function<void()> &sweep) {
+    if (exec_) return true;
+    if (failed_ || !graphs_enabled()) return false;
+    LoopState *st = state(ctx);
+    CaptureStream on(ctx);
+    cudaGraph_t g = nullptr;
+    bool ok = cudaGraphCreate(&g, 0) == cudaSuccess;
+    cudaGraphConditionalHandle h = 0;
+    ok = ok && cudaGraphConditionalHandleCreate(&h, g, 1, cudaGraphCondAssignDefault) == cudaSuccess;
+    cudaGraphNodeParams cp = {};
+    if (ok) {
+        cudaGraphNode_t cond = nullptr;
+        cp.type = cudaGraphNodeTypeConditional;
+        cp.conditional.handle = h;
+        cp.conditional.type = cudaGraphCondTypeWhile;
+        cp.conditional.size = 1;
+        ok = cudaGraphAddNode(&cond, g, nullptr, 0, &cp) == cudaSuccess;
+    }
+    const int64_t l0 = ctx->launches;
+    if (ok) {
+        ok = cudaStreamBeginCaptureToGraph(ctx->stream, cp.conditional.phGraph_out[0], nullptr,
+                                           nullptr, 0, cudaStreamCaptureModeRelaxed) == cudaSuccess;
+        if (ok) {
+            try {
+                sweep();
+                DT_LAUNCH_PDL(ctx, sweep_check_kernel, 1, 1, 0, h, scal, st);
+            } catch (...) {
+                ok = false;
+            }
+            cudaGraph_t out = nullptr;
+            ok = cudaStreamEndCapture(ctx->stream, &out) == cudaSuccess && ok;
+        }
+    }
+    launches_ = ctx->launches - l0;
+    ctx->launches = l0;
+    ok = ok && cudaGraphInstantiate(&exec_, g, 0) == cudaSuccess;
+    if (g) cudaGraphDestroy(g);
+    cudaGetLastError();
+    if (!ok) {
+        if (exec_) cudaGraphExecDestroy(exec_);
+        exec_ = nullptr;
+        failed_ = true;
+    }
+    return ok;
+}
+
+void SweepLoop::launch(dt_ctx *ctx, double thr, int max_sweeps, const void *x) {
+    loop_begin_kernel<<<1, 1, 0, ctx->stream>>>(state(ctx), thr, max_sweeps, x);
+    DT_CUDA(cudaGetLastError());
+    DT_CUDA(cudaGraphLaunch(exec_, ctx->stream));
+}
 
 // The sequence rand() returns after srand(seed) in the GNU C library, which
 // the reference's Util::randn draws from: its additive lagged-Fibonacci
@@ -141,14 +224,15 @@ DevMem DenseHooi::contract(const void *t, int tdtype, int64_t *shape, int m) {
     for (int k = 0; k < m; k++) L *= shape[k];
     for (int k = m + 1; k < N; k++) B *= shape[k];
     DevMem out(ctx, L * R[m] * B * sizeof(double));
-    const bool from_x = xtimer && t == Xdev;
+    const bool is_x = t == Xdev, from_x = xtimer && is_x;
+    const void *const *slot = is_x ? xslot : nullptr;
     if (from_x) xtimer->begin();
     if (tdtype == DT_F32)
         ttm_f64<float>(ctx, static_cast<const float *>(t), L, shape[m], B, U[m].as<double>(),
-                       I[m], 1, R[m], out.as<double>());
+                       I[m], 1, R[m], out.as<double>(), slot);
     else
         ttm_f64<double>(ctx, static_cast<const double *>(t), L, shape[m], B,
-                        U[m].as<double>(), I[m], 1, R[m], out.as<double>());
+                        U[m].as<double>(), I[m], 1, R[m], out.as<double>(), slot);
     if (from_x)
         xtimer->end((double)L * shape[m] * B * (tdtype == DT_F32 ? 4 : 8) +
                     (double)L * R[m] * B * 8 + (double)I[m] * R[m] * 8);
@@ -292,20 +376,30 @@ void DenseHooi::init_factors(double *const *U_user, double *const *dst) {
         f32_to_f64(ctx, static_cast<const float *>(Xdev), xsize, xconv.as<double>());
         X64p = xconv.as<double>();
     }
+    // The Gaussian starts depend on the shape alone: drawn once and kept.
+    if (!hosvd_start.get()) {
+        std::vector<double> all;
+        for (int m = 0; m < N; m++) {
+            const std::vector<double> h = seeded_gaussian((size_t)(I[m] * R[m]), 1000 + m);
+            all.insert(all.end(), h.begin(), h.end());
+        }
+        hosvd_start.alloc(ctx, all.size() * sizeof(double));
+        DT_CUDA(cudaMemcpyAsync(hosvd_start.get(), all.data(), all.size() * sizeof(double),
+                                cudaMemcpyHostToDevice, ctx->stream));
+        DT_CUDA(cudaStreamSynchronize(ctx->stream));  // `all` goes out of scope
+    }
+    int64_t off = 0;
     for (int m = 0; m < N; m++) {
         int64_t L = 1, B = 1;
         for (int k = 0; k < m; k++) L *= I[k];
         for (int k = m + 1; k < N; k++) B *= I[k];
         ttt_f64(ctx, X64p, X64p, L, I[m], I[m], B, S.as<double>());
-        std::vector<double> h = seeded_gaussian((size_t)(I[m] * R[m]), 1000 + m);
-        DT_CUDA(cudaMemcpyAsync(U[m].get(), h.data(), h.size() * sizeof(double),
-                                cudaMemcpyHostToDevice, ctx->stream));
-        subspace_iter(ctx, S.as<double>(), I[m], U[m].as<double>(), R[m], hosvd_iters,
-                      work.as<double>(), flag.as<int>());
-        DT_CUDA(cudaStreamSynchronize(ctx->stream));
-        if (dst)
-            DT_CUDA(cudaMemcpyAsync(dst[m], U[m].get(), I[m] * R[m] * sizeof(double),
-                                    cudaMemcpyDeviceToDevice, ctx->stream));
+        DT_CUDA(cudaMemcpyAsync(out(m), hosvd_start.as<double>() + off,
+                                I[m] * R[m] * sizeof(double), cudaMemcpyDeviceToDevice,
+                                ctx->stream));
+        off += I[m] * R[m];
+        subspace_iter(ctx, S.as<double>(), I[m], out(m), R[m], hosvd_iters, work.as<double>(),
+                      flag.as<int>());
     }
 }
 
@@ -344,8 +438,37 @@ double DenseHooi::read_scalar(int k) {
     return h;
 }
 
+// A dry pass of the sweep sizes the arena; then the loop is captured on it.
+bool DenseHooi::build_loop(SweepLoop &loop) {
+    xslot = &loop.state(ctx)->x;
+    ctx->arena = &arena;
+    bool ok = false;
+    try {
+        if (!arena.cap) {
+            arena.base = reinterpret_cast<char *>(size_t(1) << 20);  // any aligned address
+            ctx->dry = true;
+            sweep();
+            ctx->dry = false;
+            ctx->arena = nullptr;
+            arena_mem.alloc(ctx, arena.need);
+            ctx->arena = &arena;
+            arena.base = static_cast<char *>(arena_mem.get());
+            arena.cap = arena.need;
+        }
+        ok = loop.build(ctx, scal.as<double>(), [&] { sweep(); });
+    } catch (...) {
+        ctx->dry = false;
+        ctx->arena = nullptr;
+        xslot = nullptr;
+        throw;
+    }
+    ctx->arena = nullptr;
+    xslot = nullptr;
+    return ok;
+}
+
 void DenseHooi::run(double *G_user, double *const *U_user, dt_hooi_report *rep,
-                    SweepGraph *graph) {
+                    SweepLoop *loop) {
     const int64_t launches0 = ctx->launches;
     LaunchTimer timer(ctx, opts.profile != 0);
     xtimer = &timer;
@@ -356,15 +479,17 @@ void DenseHooi::run(double *G_user, double *const *U_user, dt_hooi_report *rep,
     double x2 = -1.0;
     double prev = -1.0, res = 0.0;
     int sweeps = 0;
-    for (int it = 0; it < opts.max_sweeps; it++) {
+    // The sweeps and their stop test as one graph launch, unless each sweep is
+    // timed or printed by the host.
+    const bool device_loop = loop && N > 1 && opts.max_sweeps >= 1 && !opts.profile &&
+                             !opts.verbose && !summary_active(ctx) && build_loop(*loop);
+    if (device_loop) loop->launch(ctx, opts.tol, opts.max_sweeps, Xdev);
+    for (int it = 0; it < (device_loop ? 0 : opts.max_sweeps); it++) {
         {
             // Counted work: the sweep's two passes over X (the first
             // contraction of each half of the dimension tree).
             SummaryScope sc(ctx, "HOOI sweep (FP64)", x_pass_flop(), x_pass_bytes());
-            if (graph && !opts.profile)
-                graph->run(ctx, [&] { sweep(); });
-            else
-                sweep();
+            sweep();
         }
         double g2;
         if (x2 < 0.0) {
@@ -384,8 +509,7 @@ void DenseHooi::run(double *G_user, double *const *U_user, dt_hooi_report *rep,
         if (opts.tol > 0 && prev >= 0 && std::fabs(res - prev) < opts.tol) break;
         prev = res;
     }
-    if (x2 < 0.0) x2 = read_scalar(0);
-    if (sweeps == 0) {
+    if (!device_loop && sweeps == 0) {
         // No sweep requested: the core of the initial factors.
         int64_t shape[16];
         std::memcpy(shape, I, N * sizeof(int64_t));
@@ -413,7 +537,28 @@ void DenseHooi::run(double *G_user, double *const *U_user, dt_hooi_report *rep,
         }
         copy_blocks(ctx, 1 + N, dst, src, bytes);
     }
-    const double g2 = read_scalar(1);
+    // ||X||^2, ||G||^2 and the loop's sweep count and residuals.
+    constexpr size_t kLoopAt = 64;
+    static_assert(kLoopAt + sizeof(LoopState) <= dt_ctx::kHostStageBytes, "stage too small");
+    char *st = static_cast<char *>(host_stage(ctx));
+    DT_CUDA(cudaMemcpyAsync(st, scal.as<double>(), 2 * sizeof(double), cudaMemcpyDeviceToHost,
+                            ctx->stream));
+    if (device_loop)
+        DT_CUDA(cudaMemcpyAsync(st + kLoopAt, loop->state(ctx), sizeof(LoopState),
+                                cudaMemcpyDeviceToHost, ctx->stream));
+    DT_CUDA(cudaStreamSynchronize(ctx->stream));
+    double xg[2];
+    std::memcpy(xg, st, sizeof(xg));
+    x2 = xg[0];
+    const double g2 = xg[1];
+    if (device_loop) {
+        LoopState ls;
+        std::memcpy(&ls, st + kLoopAt, sizeof(LoopState));
+        sweeps = ls.it;
+        ctx->launches += (int64_t)sweeps * loop->launches_per_sweep();
+        if (rep)
+            for (int i = 0; i < std::min(sweeps, DT_MAX_HIST); i++) rep->res_hist[i] = ls.hist[i];
+    }
     float ms = 0.f;
     DT_CUDA(cudaEventElapsedTime(&ms, ctx->ev_start, ctx->ev_stop));
     if (!std::isfinite(g2)) fail(DT_ERR_NUMERIC, "HOOI produced a non-finite core");
@@ -432,17 +577,18 @@ void DenseHooi::run(double *G_user, double *const *U_user, dt_hooi_report *rep,
     xtimer = nullptr;
 }
 
-// The FP64 driver's buffers and sweep graph, kept on the context for the next
-// call with the same X, shapes, ranks and inner iterations.
+// The FP64 driver's buffers and captured sweep loop, kept on the context for
+// the next call with the same shapes, ranks and inner iterations (and an X that
+// is 16-byte aligned or not, as before: the captured copies' widths).
 struct Fp64Plan {
-    const void *X;
+    bool aligned;
     int dtype, N, inner;
     int64_t I[16], R[16];
     DenseHooi h;
-    SweepGraph graph;
+    SweepLoop loop;
     Fp64Plan(const void *x, int dt, int n, const int64_t *shape, const int64_t *ranks,
              const dt_hooi_opts &o)
-        : X(x), dtype(dt), N(n), inner(o.inner_iters) {
+        : aligned(reinterpret_cast<uintptr_t>(x) % 16 == 0), dtype(dt), N(n), inner(o.inner_iters) {
         for (int m = 0; m < n; m++) {
             I[m] = shape[m];
             R[m] = ranks[m];
@@ -450,7 +596,9 @@ struct Fp64Plan {
     }
     bool matches(const void *x, int dt, int n, const int64_t *shape, const int64_t *ranks,
                  const dt_hooi_opts &o) const {
-        if (x != X || dt != dtype || n != N || o.inner_iters != inner) return false;
+        if ((reinterpret_cast<uintptr_t>(x) % 16 == 0) != aligned || dt != dtype || n != N ||
+            o.inner_iters != inner)
+            return false;
         for (int m = 0; m < n; m++)
             if (shape[m] != I[m] || ranks[m] != R[m]) return false;
         return true;
@@ -526,7 +674,7 @@ int dt_hooi_dense(dt_ctx *ctx, const void *X, int dtype, int ndim, const int64_t
                 if (keep) ctx->hooi_plan_fp64 = plan;
             }
             plan->h.setup(ctx, x.ptr(), dtype, ndim, shape, ranks, o);
-            plan->h.run(G, U, report, keep ? &plan->graph : nullptr);
+            plan->h.run(G, U, report, keep ? &plan->loop : nullptr);
         } else {
             hooi_dense_lowprec(ctx, x_host ? up.dst.get() : x.ptr(), dtype, ndim, shape, ranks, o,
                                G, U, report, x_host ? &up : nullptr);

@@ -2,6 +2,7 @@
 #pragma once
 
 #include <algorithm>
+#include <functional>
 #include <vector>
 
 #include "dt_core.cuh"
@@ -19,6 +20,42 @@ class LibcRand {
    private:
     int32_t s_[31];
     int f_ = 3, r_ = 0;
+};
+
+// The state of a device-side sweep loop: what the call asked for, the sweeps
+// done, the last residual and the residual of every sweep.
+struct LoopState {
+    int it, max_sweeps;
+    double prev, thr;
+    const void *x;  // this call's X (the captured kernels take it from here)
+    double hist[DT_MAX_HIST];
+};
+
+// A sweep loop as one graph: a WHILE node whose body is one captured sweep
+// followed by a kernel that computes the sweep's residual from scal[0] =
+// ||X||^2 and scal[1] = ||G||^2, applies the stop rule (residual change below
+// thr, or max_sweeps done) and sets the loop's condition.  One graph launch
+// runs every sweep with no host round trip.  The stop rule's numbers and X's
+// address are in the LoopState that launch() writes, so one graph serves every
+// call of a plan.
+class SweepLoop {
+   public:
+    SweepLoop() = default;
+    SweepLoop(const SweepLoop &) = delete;
+    SweepLoop &operator=(const SweepLoop &) = delete;
+    ~SweepLoop();
+    // Captures sweep's launches; false (and no further attempts) when the
+    // runtime refuses any step: the host drives the sweeps then.
+    bool build(dt_ctx *ctx, const double *scal, const std::function<void()> &sweep);
+    void launch(dt_ctx *ctx, double thr, int max_sweeps, const void *x);
+    LoopState *state(dt_ctx *ctx);       // device memory, allocated on first use
+    int64_t launches_per_sweep() const { return launches_; }
+
+   private:
+    cudaGraphExec_t exec_ = nullptr;
+    bool failed_ = false;
+    int64_t launches_ = 0;
+    DevMem state_;
 };
 
 struct DenseHooi {
@@ -39,6 +76,10 @@ struct DenseHooi {
     unsigned init_seed = 0;
     int hosvd_iters = 30;
     LaunchTimer *xtimer = nullptr;  // times the TTM launches that read X
+    DevArena arena;                 // a captured sweep's intermediates
+    DevMem arena_mem;
+    const void *const *xslot = nullptr;  // where a captured sweep finds X
+    DevMem hosvd_start;             // HOSVD's Gaussian starts, mode after mode
 
     // Allocates the buffers on the first call; a later call on the same
     // object (same shapes and ranks) keeps them, so a captured sweep graph
@@ -48,10 +89,10 @@ struct DenseHooi {
     // Writes the initial factors into dst[m] (I_m x R_m col-major device
     // buffers; null: this object's U).
     void init_factors(double *const *U_user, double *const *dst = nullptr);
-    // graph: replays the sweep from a captured CUDA graph (null: launch
-    // directly; never used with opts.profile).
+    // loop: runs the sweeps as one captured device-side loop (null, or where
+    // each sweep needs the host: launches them directly).
     void run(double *G_user, double *const *U_user, dt_hooi_report *rep,
-             SweepGraph *graph = nullptr);
+             SweepLoop *loop = nullptr);
 
    private:
     DevMem contract(const void *t, int tdtype, int64_t *shape, int m);
@@ -63,6 +104,7 @@ struct DenseHooi {
     void read_scalars(int k, int n, double *out);
     double x_pass_flop() const;
     double x_pass_bytes() const;
+    bool build_loop(SweepLoop &loop);
 };
 
 // BF16 / split-BF16 tensor-core HOOI (dt_hooi_tc.cu).

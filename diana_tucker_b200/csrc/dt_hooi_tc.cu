@@ -29,43 +29,6 @@ __global__ void f64_to_f32_kernel(const double *__restrict__ x, int64_t n, float
         y[e] = (float)x[e];
 }
 
-// The device-side sweep loop's state: sweeps done, the last residual, and
-// the residual of every sweep.
-struct LoopState {
-    int it, pad;
-    double prev;
-    double hist[DT_MAX_HIST];
-};
-
-// End of one sweep of the device-side loop: the sweep's residual from its
-// ||G||^2 and ||X||^2, the stop rule of the host loop (residual change below
-// `thr`, or `max_sweeps` done), and the loop's condition for the next pass.
-__global__ void sweep_check_kernel(cudaGraphConditionalHandle h, const double *scal,
-                                   LoopState *st, double thr, int max_sweeps) {
-    pdl_wait();
-    const double x2 = scal[0], g2 = scal[1];
-    const double res = sqrt(fmax(0.0, 1.0 - g2 / x2));
-    const int it = st->it;
-    if (it < DT_MAX_HIST) st->hist[it] = res;
-    const bool stop = it + 1 >= max_sweeps || (thr > 0.0 && it > 0 && fabs(res - st->prev) < thr);
-    st->prev = res;
-    st->it = it + 1;
-    cudaGraphSetConditional(h, stop ? 0u : 1u);
-}
-
-// The whole sweep loop as one graph: a reset of the LoopState, then a WHILE
-// node whose body is one captured sweep followed by sweep_check_kernel.
-struct LoopGraph {
-    cudaGraphExec_t exec = nullptr;
-    bool failed = false;
-    int64_t launches_per_sweep = 0;
-    double thr = -1.0;
-    int max_sweeps = -1;
-    ~LoopGraph() {
-        if (exec) cudaGraphExecDestroy(exec);
-    }
-};
-
 // A BF16 intermediate of the sweep (hi, and lo when split), in the plan's
 // arena.
 struct BfTensor {
@@ -95,78 +58,8 @@ struct MixedHooi {
     DevMem arena;
     size_t arena_cap = 0, arena_off = 0, arena_need = 0;
     bool dry = false;
-    LoopGraph *loop = nullptr;  // the device-side sweep loop (or null)
-    DevMem loopst;              // its LoopState
-
-    // Builds the device-side loop for split sweeps with stop threshold `thr`
-    // and `max_sweeps`; false (and no further attempts) when the runtime
-    // refuses any step, in which case the host drives the sweeps.
-    bool build_loop(double thr, int max_sweeps) {
-        LoopGraph &lg = *loop;
-        if (lg.exec && lg.thr == thr && lg.max_sweeps == max_sweeps) return true;
-        if (lg.failed) return false;
-        if (lg.exec) {
-            cudaGraphExecDestroy(lg.exec);
-            lg.exec = nullptr;
-        }
-        if (!loopst.get()) loopst.alloc(ctx, sizeof(LoopState));
-        cudaGraph_t g = nullptr;
-        bool ok = cudaGraphCreate(&g, 0) == cudaSuccess;
-        cudaGraphConditionalHandle h = 0;
-        ok = ok && cudaGraphConditionalHandleCreate(&h, g, 1, cudaGraphCondAssignDefault) ==
-                       cudaSuccess;
-        cudaGraphNode_t reset = nullptr, cond = nullptr;
-        if (ok) {
-            cudaMemsetParams mp = {};
-            mp.dst = loopst.get();
-            mp.value = 0;
-            mp.elementSize = 4;
-            mp.width = sizeof(LoopState) / 4;
-            mp.height = 1;
-            mp.pitch = 0;
-            ok = cudaGraphAddMemsetNode(&reset, g, nullptr, 0, &mp) == cudaSuccess;
-        }
-        cudaGraphNodeParams cp = {};
-        if (ok) {
-            cp.type = cudaGraphNodeTypeConditional;
-            cp.conditional.handle = h;
-            cp.conditional.type = cudaGraphCondTypeWhile;
-            cp.conditional.size = 1;
-            ok = cudaGraphAddNode(&cond, g, &reset, 1, &cp) == cudaSuccess;
-        }
-        const int64_t l0 = ctx->launches;
-        if (ok) {
-            cudaGraph_t body = cp.conditional.phGraph_out[0];
-            ok = cudaStreamBeginCaptureToGraph(ctx->stream, body, nullptr, nullptr, 0,
-                                               cudaStreamCaptureModeRelaxed) == cudaSuccess;
-            if (ok) {
-                try {
-                    sweep();
-                    DT_LAUNCH_PDL(ctx, sweep_check_kernel, 1, 1, 0, h,
-                              (const double *)scal.as<double>(), loopst.as<LoopState>(), thr,
-                              max_sweeps);
-                } catch (...) {
-                    ok = false;
-                }
-                cudaGraph_t out = nullptr;
-                ok = cudaStreamEndCapture(ctx->stream, &out) == cudaSuccess && ok;
-            }
-        }
-        lg.launches_per_sweep = ctx->launches - l0;
-        ctx->launches = l0;
-        ok = ok && cudaGraphInstantiate(&lg.exec, g, 0) == cudaSuccess;
-        if (g) cudaGraphDestroy(g);
-        cudaGetLastError();
-        if (!ok) {
-            if (lg.exec) cudaGraphExecDestroy(lg.exec);
-            lg.exec = nullptr;
-            lg.failed = true;
-            return false;
-        }
-        lg.thr = thr;
-        lg.max_sweeps = max_sweeps;
-        return true;
-    }
+    SweepLoop *loop = nullptr;  // the device-side sweep loop (or null)
+    DevMem g2hist;              // ||G||^2 of every sweep of a fixed number of them
 
     void *take(size_t bytes) {
         bytes = (bytes + 255) & ~size_t(255);
@@ -446,14 +339,18 @@ struct MixedHooi {
         // device as one graph launch (no synchronisation per sweep), unless
         // per-sweep host work is asked for (profiling, verbose output, the
         // Summary profiler) or the stream cannot be captured.
-        const bool plain_stream = ctx->stream != nullptr && ctx->stream != cudaStreamLegacy &&
-                                  ctx->stream != cudaStreamPerThread;
-        const bool device_loop = split && !refine_mode && loop && plain_stream &&
-                                 graphs_enabled() && !opts.profile && !opts.verbose &&
-                                 !summary_active(ctx) && opts.max_sweeps >= 1 &&
-                                 build_loop(opts.tol > 0 ? std::max(opts.tol, kSplitFloor) : 0.0,
-                                            opts.max_sweeps);
-        if (device_loop) DT_CUDA(cudaGraphLaunch(loop->exec, ctx->stream));
+        const bool device_loop = split && !refine_mode && loop && plain_stream(ctx) &&
+                                 !opts.profile && !opts.verbose && !summary_active(ctx) &&
+                                 opts.max_sweeps >= 1 &&
+                                 loop->build(ctx, scal.as<double>(), [&] { sweep(); });
+        if (device_loop)
+            loop->launch(ctx, opts.tol > 0 ? std::max(opts.tol, kSplitFloor) : 0.0,
+                         opts.max_sweeps, nullptr);
+        // A fixed number of split sweeps needs nothing from the host in between:
+        // their graphs are queued one after the other, each followed by a copy
+        // of its ||G||^2.
+        const bool fixed = !device_loop && split && !refine_mode && opts.tol <= 0 && !opts.verbose;
+        if (fixed && !g2hist.get()) g2hist.alloc(ctx, DT_MAX_HIST * sizeof(double));
         for (int it = 0; it < (device_loop ? 0 : opts.max_sweeps); it++) {
             if (!split && refine_mode && opts.refine_sweeps > 0 &&
                 it >= opts.max_sweeps - opts.refine_sweeps) {
@@ -471,6 +368,13 @@ struct MixedHooi {
                     gr->run(ctx, [&] { sweep(); });
                 else
                     sweep();
+            }
+            if (fixed) {
+                if (it < DT_MAX_HIST)
+                    DT_CUDA(cudaMemcpyAsync(g2hist.as<double>() + it, scal.as<double>() + 1,
+                                            sizeof(double), cudaMemcpyDeviceToDevice, ctx->stream));
+                sweeps = it + 1;
+                continue;
             }
             double g2;
             if (x2 < 0.0) {
@@ -508,7 +412,7 @@ struct MixedHooi {
                 }
             }
         }
-        if (x2 < 0.0 && !device_loop) x2 = read_scalar(0);
+        if (x2 < 0.0 && !device_loop && !fixed) x2 = read_scalar(0);
         // Final core, FP64 projection from the original X (the returned G is
         // X x_1 U_1^T ... x_N U_N^T to FP64 rounding).
         DevMem cur;
@@ -562,6 +466,7 @@ struct MixedHooi {
             copy_blocks(ctx, 1 + N, dst, src, bytes);
         }
         constexpr size_t kErrAt = 32, kLoopAt = 64;
+        const int noted = fixed ? std::min(sweeps, DT_MAX_HIST) : 0;
         static_assert(kLoopAt + sizeof(LoopState) <= dt_ctx::kHostStageBytes, "stage too small");
         char *st = static_cast<char *>(host_stage(ctx));
         DT_CUDA(cudaMemcpyAsync(st, scal.as<double>(), (gslot + 1) * sizeof(double),
@@ -569,7 +474,10 @@ struct MixedHooi {
         DT_CUDA(cudaMemcpyAsync(st + kErrAt, err.get(), sizeof(int), cudaMemcpyDeviceToHost,
                                 ctx->stream));
         if (device_loop)
-            DT_CUDA(cudaMemcpyAsync(st + kLoopAt, loopst.get(), sizeof(LoopState),
+            DT_CUDA(cudaMemcpyAsync(st + kLoopAt, loop->state(ctx), sizeof(LoopState),
+                                    cudaMemcpyDeviceToHost, ctx->stream));
+        if (noted > 0)
+            DT_CUDA(cudaMemcpyAsync(st + kLoopAt, g2hist.get(), noted * sizeof(double),
                                     cudaMemcpyDeviceToHost, ctx->stream));
         DT_CUDA(cudaStreamSynchronize(ctx->stream));
         double sc[gslot + 1];
@@ -582,9 +490,17 @@ struct MixedHooi {
             std::memcpy(&hst, st + kLoopAt, sizeof(LoopState));
             x2 = sc[0];
             sweeps = hst.it;
-            ctx->launches += (int64_t)sweeps * loop->launches_per_sweep;
+            ctx->launches += (int64_t)sweeps * loop->launches_per_sweep();
             if (rep)
                 for (int i = 0; i < std::min(sweeps, DT_MAX_HIST); i++) rep->res_hist[i] = hst.hist[i];
+        }
+        if (fixed) {
+            x2 = sc[0];
+            for (int i = 0; rep && i < noted; i++) {
+                double q;
+                std::memcpy(&q, st + kLoopAt + i * sizeof(double), sizeof(double));
+                rep->res_hist[i] = std::sqrt(std::max(0.0, 1.0 - q / x2));
+            }
         }
         // The FP32 copy of an FP64 X lives for this call only.
         X32own.release();
@@ -615,7 +531,7 @@ struct MixedPlan {
     int64_t I[16], R[16];
     MixedHooi h;
     SweepGraph g_bf16, g_split;
-    LoopGraph loop;  // destroyed before h's buffers
+    SweepLoop loop;  // destroyed before h's buffers
     MixedPlan(int n, const int64_t *shape, const int64_t *ranks, const dt_hooi_opts &o)
         : N(n), inner(o.inner_iters), precision(o.precision) {
         for (int m = 0; m < n; m++) {

@@ -14,10 +14,12 @@ namespace dt {
 
 // Y[l, j, b] = sum_i M(j, i) * X[l, i, b]   (Y is L x J x B), with
 // M(j, i) = M[j*msj + i*msi]: (msj, msi) = (1, J) for a J x I col-major M,
-// (I, 1) for the transpose of an I x J col-major factor U.
+// (I, 1) for the transpose of an I x J col-major factor U.  With `slot` (device
+// memory) the kernel takes X's address from there, and X here only says how it
+// is aligned: a captured launch then serves every X.
 template <class TX>
 void ttm_f64(dt_ctx *ctx, const TX *X, int64_t L, int64_t I, int64_t B, const double *M,
-             int64_t msj, int64_t msi, int64_t J, double *Y);
+             int64_t msj, int64_t msi, int64_t J, double *Y, const void *const *slot = nullptr);
 
 // C[i, j] = sum_{l,b} A[l, i, b] * Bt[l, j, b]   (C is IA x IB col-major).
 void ttt_f64(dt_ctx *ctx, const double *A, const double *Bt, int64_t L, int64_t IA,

@@ -69,3 +69,60 @@ def test_graph_replay_matches_direct_launches(ctx, prec):
         assert _nrel(G, G0) < 1e-12
         for n in range(3):
             assert _nrel(U[n], U0[n]) < 1e-12
+
+
+@pytest.mark.parametrize("stream", ["legacy", "side"])
+@pytest.mark.parametrize("dtype", ["float64", "float32"])
+def test_one_plan_serves_other_tensors(ctx, stream, dtype):
+    """The FP64 sweep loop is captured once per shape and takes X's address and
+    the stop rule from device memory: other buffers (one of them not 16-byte
+    aligned), other sweep counts and stop thresholds, and a return to the first
+    give what a fresh context gives, bit for bit (the same kernels on the same
+    values)."""
+    import torch
+
+    from diana_tucker_b200 import Context
+    shape, ranks = (30, 26, 22), (5, 4, 3)
+    n = int(np.prod(shape))
+    bufs = []
+    for k in range(3):
+        flat = _tensor(shape, ranks, 60 + k).reshape(-1, order="F")
+        room = torch.zeros(n + 8, dtype=getattr(torch, dtype), device="cuda")
+        at = 1 if k == 1 else 0
+        room[at:at + n] = torch.from_numpy(np.ascontiguousarray(flat)).to(room.dtype)
+        bufs.append(room[at:at + n])
+    calls = [(0, 4, 0.0), (1, 4, 0.0), (2, 30, 1e-7), (0, 3, 0.0), (2, 0, 0.0), (0, 4, 0.0)]
+    s = torch.cuda.default_stream() if stream == "legacy" else torch.cuda.Stream()
+    torch.cuda.synchronize()
+    with torch.cuda.stream(s):
+        for k, sweeps, tol in calls:
+            kw = dict(init="randn", seed=3, max_sweeps=sweeps, tol=tol, shape=shape)
+            G, U, rep = ctx.hooi_dense(bufs[k], ranks, **kw)
+            with Context(0) as fresh:
+                Gf, Uf, repf = fresh.hooi_dense(bufs[k].clone() if k != 1 else bufs[k], ranks, **kw)
+            assert rep["sweeps"] == repf["sweeps"] and rep["residual"] == repf["residual"]
+            assert np.array_equal(G, Gf)
+            for a, b in zip(U, Uf):
+                assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("sweeps", [1, 5])
+def test_fixed_sweeps_of_the_tensor_cores_on_the_legacy_stream(ctx, sweeps):
+    """A fixed number of split sweeps queues its graphs without reading back
+    in between: the residuals and factors are those of the device-side loop."""
+    import torch
+
+    from diana_tucker_b200 import DT_PREC_BF16XH
+    shape, ranks = (64, 48, 40), (8, 8, 8)
+    X = torch.from_numpy(np.ascontiguousarray(
+        _tensor(shape, ranks, 43).reshape(-1, order="F"))).cuda()
+    kw = dict(init="randn", seed=3, max_sweeps=sweeps, precision=DT_PREC_BF16XH, inner_iters=2,
+              shape=shape)
+    torch.cuda.synchronize()
+    G0, U0, r0 = ctx.hooi_dense(X, ranks, **kw)
+    with torch.cuda.stream(torch.cuda.Stream()):
+        G1, U1, r1 = ctx.hooi_dense(X, ranks, **kw)
+    assert r0["sweeps"] == r1["sweeps"] == sweeps
+    assert np.array_equal(G0, G1) and all(np.array_equal(a, b) for a, b in zip(U0, U1))
+    for a, b in zip(r0["res_hist"][:sweeps], r1["res_hist"][:sweeps]):
+        assert abs(a - b) <= 1e-15
