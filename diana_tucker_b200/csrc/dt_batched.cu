@@ -12,16 +12,22 @@
 // dimension-tree TTM chain (T = X x_3 U_3^T shared by modes 1 and 2,
 // X x_1 U_1^T x_2 U_2^T for mode 3), the Gram Y_(n) Y_(n)^T, the subspace
 // iteration of ALS_ (hooi_als.tpp:7-34) with CholeskyQR, and finally the FP64
-// core and relative error.  X is read from global memory (mostly from L2 while
-// its group works on it), Y_(n), the Gram and the factors live in shared
-// memory, the one large intermediate (I_1 x I_2 x R_3) in the group's slice of
-// global scratch.  Arithmetic is FP64 throughout; X is FP32.  The reductions
-// keep four independent FMA chains per thread (the FP64 FMA latency is ~23
-// cycles), in a fixed order, so results do not depend on the launch shape.
+// core and relative error.  Arithmetic is FP64 throughout, on the FP64 tensor
+// cores (mma.sync m8n8k4): every product is cut into 8 x 8 tiles, dealt over the
+// group's warps.  X is FP32, read from global memory (from L2 while its group
+// works on it) straight into fragments, 16 loads in flight per lane; the one
+// large intermediate (I_1 x I_2 x R_3) is in the group's slice of global scratch;
+// the factors, Y_(n) and its Gram (which takes Y_(n)'s place) live in shared
+// memory.  In a subspace step each warp keeps its rows of S L in registers, laid
+// out as the next products' fragments, from the product to the new factor.  Sums
+// go in a fixed order for a given number of warps.  4096 tensors (modes 8 to 64,
+// ranks 2 to 8, 10 sweeps): 11.6 ms, of it about half the two passes over X at 0.8
+// of the FP64 tensor rate (ranks padded to 8 columns); 100 tensors 1.15 ms.  With
+// one FMA chain per thread and entry on the CUDA cores 23.3 and 2.4 ms.
 //
 // Autotuning.  The block size (128, 256, 512 threads) and the packing (one
 // tensor per CTA; pairs, and quads, of the tensors small enough to share the
-// CTA's shared memory: largest mode <= 37, <= 21) are chosen by timing every
+// CTA's shared memory: largest mode <= 32, <= 16) are chosen by timing every
 // combination on the batch (a stratified sample of 8192 tensors of larger
 // batches); the choice is cached per batch signature on the context.
 //
@@ -48,25 +54,30 @@ constexpr int BMAX_I = 64;               // largest mode size
 constexpr int BMAX_R = 8;                // largest rank
 constexpr int BMAX_K = BMAX_R * BMAX_R;  // largest product of two ranks
 
-// Shared-memory doubles one tensor of largest mode size m needs:
-// U (3 m R), Y (m K), S (m^2), Z (m R), the R x R Gram, reduction scratch.
+// Shared-memory doubles one tensor of largest mode size m needs: the factors
+// (rows padded to whole tiles, 8 columns), Y_(n) or its Gram (rows of up to 64
+// at a pitch of 4 mod 16), reduction scratch.  Gram shares and factorisation
+// scratch, 128 doubles a warp, come on top for the whole CTA.
+__host__ __device__ constexpr int tile8(int n) { return (n + 7) / 8 * 8; }
+__host__ __device__ constexpr int pitch16(int n) { return (n + 11) / 16 * 16 + 4; }
 __host__ __device__ constexpr int slot_doubles(int m) {
-    return 3 * m * BMAX_R + m * BMAX_K + m * m + m * BMAX_R + BMAX_R * BMAX_R + 40;
+    return 3 * tile8(m) * BMAX_R + tile8(m) * pitch16(BMAX_K) + 40;
 }
 constexpr int SLOT = slot_doubles(BMAX_I);                    // one CTA
-constexpr int64_t SCR = (int64_t)BMAX_I * BMAX_I * BMAX_R;    // global scratch per CTA
-// Largest mode size a tensor may have to share a CTA with 1 / 3 others: its
-// shared-memory needs fit SLOT / g (its scratch then fits SCR / g as well).
-constexpr int pack_limit(int g) {
-    int m = BMAX_I;
-    while (m > 0 && slot_doubles(m) > SLOT / g) m--;
-    return m;
-}
-constexpr int PAIR_MAX_I = pack_limit(2);  // 37
-constexpr int QUAD_MAX_I = pack_limit(4);  // 21
-static_assert(PAIR_MAX_I == 37 && QUAD_MAX_I == 21, "packing limits");
-static_assert((int64_t)PAIR_MAX_I * PAIR_MAX_I * BMAX_R <= SCR / 2, "pair scratch");
-static_assert((int64_t)QUAD_MAX_I * QUAD_MAX_I * BMAX_R <= SCR / 4, "quad scratch");
+// Room for four of the largest tensors that go four to a CTA.
+constexpr int SLOT_ALL = SLOT > 4 * slot_doubles(16) ? SLOT : 4 * slot_doubles(16);
+constexpr int WARP_SCR = 128;
+// Global scratch per CTA: the intermediate and the last Y_(3).
+constexpr int64_t SCR = (int64_t)BMAX_I * BMAX_I * BMAX_R + BMAX_I * BMAX_K;
+// Largest mode size a tensor may have to share a CTA with 1 / 3 others.
+constexpr int PAIR_MAX_I = 32, QUAD_MAX_I = 16;
+static_assert(slot_doubles(PAIR_MAX_I) <= SLOT_ALL / 2 / 2 * 2 &&
+                  slot_doubles(QUAD_MAX_I) <= SLOT_ALL / 4 / 2 * 2,
+              "packing limits");
+static_assert((int64_t)PAIR_MAX_I * PAIR_MAX_I * BMAX_R + PAIR_MAX_I * BMAX_K <= SCR / 2,
+              "pair scratch");
+static_assert((int64_t)QUAD_MAX_I * QUAD_MAX_I * BMAX_R + QUAD_MAX_I * BMAX_K <= SCR / 4,
+              "quad scratch");
 
 struct Item {
     int g;     // tensors worked on side by side (1, 2 or 4)
@@ -90,12 +101,19 @@ struct BatchArgs {
     int *queue;
 };
 
+// Shared memory goes by offsets into this array: the functions that are not
+// inlined (to keep their registers apart) then still address it as such.
+extern __shared__ __align__(16) double bt_sm[];
+
 // A thread group working on one tensor: its threads are a contiguous run of
 // whole warps of the CTA, synchronised by their own named barrier.
 struct Grp {
     int lt;   // thread index in the group
     int gs;   // threads in the group (a multiple of 32)
     int bar;  // named barrier id (1..4; 0 is __syncthreads)
+    int w, W;          // this warp, warps
+    int g, t;          // fragment row / column of the lane
+    int part;          // offset of W x WARP_SCR: the warps' Gram shares and scratch
 };
 
 __device__ __forceinline__ void gsync(const Grp &g) {
@@ -120,275 +138,335 @@ __device__ double gsum(double v, double *red, const Grp &g) {
     return r;
 }
 
-// Cholesky of the r x r Gram in G (row-major, r <= 8) by lane c owning column
-// c; overwrites G with R (upper).  Returns false on a non-positive pivot.
-// Called by one full warp.
-__device__ bool warp_chol8(double *G, int r) {
-    const int lane = threadIdx.x & 31;
-    double g[BMAX_R];
-#pragma unroll
-    for (int i = 0; i < BMAX_R; i++) g[i] = (i < r && lane < r) ? G[i * r + lane] : 0.0;
-    const double g00 = __shfl_sync(0xffffffffu, g[0], 0);
-    bool ok = true;
-#pragma unroll
-    for (int k = 0; k < BMAX_R; k++) {
-        if (k >= r) break;
-        const double d = __shfl_sync(0xffffffffu, g[k], k);
-        if (!(d > 1e-28 * g00)) ok = false;
-        const double rkk = sqrt(fmax(d, 1e-300));
-        const double inv = 1.0 / rkk;
-        if (lane > k) g[k] *= inv;
-        if (lane == k) g[k] = rkk;
-#pragma unroll
-        for (int i = k + 1; i < BMAX_R; i++) {
-            if (i >= r) break;
-            const double rki = __shfl_sync(0xffffffffu, g[k], i);
-            if (lane >= i) g[i] = fma(-rki, g[k], g[i]);
-        }
-    }
-    if (lane < r) {
-#pragma unroll
-        for (int i = 0; i < BMAX_R; i++)
-            if (i < r) G[i * r + lane] = i <= lane ? g[i] : 0.0;
-    }
-    __syncwarp();
-    return ok;
+__device__ __forceinline__ void bt_dmma(double &d0, double &d1, double a, double b) {
+    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
+                 : "+d"(d0), "+d"(d1)
+                 : "d"(a), "d"(b));
 }
 
-// dst (n x r col-major) = orth(src) by CholeskyQR; Gs is r x r scratch.
-// Falls back to modified Gram-Schmidt when the Gram is not positive definite.
-__device__ void gcholqr(const double *src, double *dst, int n, int r, double *Gs, int *bad,
-                        const Grp &g) {
-    // The r x r Gram: four threads per entry, each summing every fourth row,
-    // combined by two shuffles (a fixed order).
-    const int total = 4 * r * r;
-    for (int base = 0; base < total; base += g.gs) {
-        const int idx = base + g.lt;
-        const int e = idx >> 2, part = idx & 3;
-        double s = 0.0;
-        if (idx < total) {
-            const int a = e / r, b = e % r;
-            const double *pa = src + a * n, *pb = src + b * n;
-            for (int k = part; k < n; k += 4) s = fma(pa[k], pb[k], s);
+// Factor entry (i, c): rows of 8, columns 4 apart swapped in every other pair of
+// rows, so the four rows and eight columns of a fragment load hit distinct banks.
+__device__ __forceinline__ int u_at(int i, int c) { return i * BMAX_R + (c ^ ((i & 2) << 1)); }
+
+// dst(i, c, o) = sum_k src(i, o, k) U(k, c) for rows i < ni of no outer indices, K
+// columns k and R <= 8 results c: every contraction of the chain.  Element (i, o,
+// k) is at src[i si + o so + k sk], result (i, c, o) goes to dst[i di + c dc + o dw].
+// A tile is 8 rows of one outer index; a warp takes four at a time, which share
+// the factor's fragments, 16 columns in a block.  The next block's 16 loads per
+// lane (of the same tiles or the next ones) are in flight while a block is
+// multiplied: a block is 64 cycles of an SM's FP64 tensor rate, its loads come
+// from L2.  Past K the last column is read again and meets zeros.
+template <class TX>
+__device__ __noinline__ void contract(const TX *src, int ni, int si, int no, int so, int K, int sk,
+                                      int uo, double *dst, int di, int dc, int dw, int R, Grp g) {
+    const double *U = bt_sm + uo;
+    const int nti = (ni + 7) >> 3, ntile = nti * no, njobs = (ntile + 3) >> 2;
+    auto tile = [&](int tau, int &i, int &o) {  // the lane's row and outer index
+        tau = min(tau, ntile - 1);
+        o = no == 1 ? 0 : tau / nti;
+        i = 8 * (tau - o * nti) + g.g;
+    };
+    const TX *p[4];
+    auto aim = [&](int job) {
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            int i, o;
+            tile(4 * job + j, i, o);
+            p[j] = src + min(i, ni - 1) * si + o * so;
         }
-        s += __shfl_xor_sync(0xffffffffu, s, 1);
-        s += __shfl_xor_sync(0xffffffffu, s, 2);
-        if (idx < total && part == 0) Gs[e] = s;
-    }
-    gsync(g);
-    if (g.lt < 32) {
-        const bool ok = warp_chol8(Gs, r);
-        if (g.lt == 0) *bad = ok ? 0 : 1;
-    }
-    gsync(g);
-    if (!*bad) {
-        for (int i = g.lt; i < n; i += g.gs) {
-            double q[BMAX_R];
+    };
+    TX v[4][4], w[4][4];
+    auto load = [&](TX (&x)[4][4], int k0) {
 #pragma unroll
-            for (int c = 0; c < BMAX_R; c++) {
-                if (c >= r) break;
-                double acc = src[i + c * n];
+        for (int s = 0; s < 4; s++) {
+            const int k = min(k0 + 4 * s + g.t, K - 1) * sk;
 #pragma unroll
-                for (int k = 0; k < BMAX_R; k++) {
-                    if (k >= c) break;
-                    acc = fma(-q[k], Gs[k * r + c], acc);
+            for (int j = 0; j < 4; j++) x[s][j] = p[j][k];
+        }
+    };
+    int job = g.w, lj = g.w, lk = 0;
+    if (job >= njobs) return;
+    aim(job);
+    load(v, 0);
+    double acc[4][2] = {};
+#pragma unroll 1
+    for (int k0 = 0;;) {
+        lk += 16;
+        if (lk >= K) {
+            lk = 0;
+            lj += g.W;
+            if (lj < njobs) aim(lj);
+        }
+        if (lj < njobs) load(w, lk);
+#pragma unroll
+        for (int s = 0; s < 4; s++) {
+            if (k0 + 4 * s >= K) break;
+            const int k = k0 + 4 * s + g.t;
+            const double u = U[u_at(min(k, K - 1), g.g)];
+            const double b = k < K ? u : 0.0;
+#pragma unroll
+            for (int j = 0; j < 4; j++) bt_dmma(acc[j][0], acc[j][1], (double)v[s][j], b);
+        }
+        k0 += 16;
+        if (k0 >= K) {
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                int i, o;
+                tile(4 * job + j, i, o);
+#pragma unroll
+                for (int h = 0; h < 2; h++) {
+                    const int c = 2 * g.t + h;
+                    if (4 * job + j < ntile && i < ni && c < R)
+                        dst[i * di + c * dc + o * dw] = acc[j][h];
+                    acc[j][h] = 0.0;
                 }
-                q[c] = acc / Gs[c * r + c];
-                dst[i + c * n] = q[c];
             }
+            k0 = 0;
+            job += g.W;
+            if (job >= njobs) return;
         }
-        gsync(g);
-        return;
+#pragma unroll
+        for (int s = 0; s < 4; s++)
+#pragma unroll
+            for (int j = 0; j < 4; j++) v[s][j] = w[s][j];
     }
-    // Rank-deficient product: modified Gram-Schmidt with zero columns kept zero.
-    if (g.lt == 0) {
+}
+
+// Zeroes what a Y_(n) of n x K does not fill of its whole tiles.
+__device__ __forceinline__ void zero_pads(double *Y, int n, int K, int pitch, const Grp &g) {
+    const int n8 = tile8(n), K4 = (K + 3) & ~3;
+    for (int e = g.lt; e < n8 * K4; e += g.gs) {
+        const int i = e / K4, k = e - i * K4;
+        if (i >= n || k >= K) Y[i * pitch + k] = 0.0;
+    }
+}
+
+// S (n x n, pitch ps) = Y Y^T in Y's place (pitch py, whole tiles zero padded).
+// The upper triangle's tiles are dealt over the warps, at most 9 each, kept in
+// registers until every warp has read Y.
+__device__ __noinline__ void ggram(int ys, int n, int K, int py, int ps, Grp g) {
+    double *YS = bt_sm + ys;
+    const int nt = tile8(n) / 8, total = nt * (nt + 1) / 2, ks = (K + 3) / 4;
+    double acc[9][2];
+    int at[9];  // tile row | column << 4, -1: none
+#pragma unroll
+    for (int x = 0; x < 9; x++) {
+        int s = g.w + x * g.W;
+        at[x] = -1;
+        if (s < total) {
+            int r = 0;
+            while (s >= nt - r) {
+                s -= nt - r;
+                r++;
+            }
+            at[x] = r | (r + s) << 4;
+        }
+    }
+#pragma unroll
+    for (int b = 0; b < 9; b += 3) {
+        if (at[b] < 0) continue;
+        const double *pr[3], *pc[3];
+#pragma unroll
+        for (int x = 0; x < 3; x++) {
+            const int q = at[b + x] < 0 ? at[b] : at[b + x];
+            pr[x] = YS + (8 * (q & 15) + g.g) * py + g.t;
+            pc[x] = YS + (8 * (q >> 4) + g.g) * py + g.t;
+            acc[b + x][0] = acc[b + x][1] = 0.0;
+        }
+#pragma unroll 2
+        for (int k = 0; k < ks; k++)
+#pragma unroll
+            for (int x = 0; x < 3; x++)
+                bt_dmma(acc[b + x][0], acc[b + x][1], pr[x][4 * k], pc[x][4 * k]);
+    }
+    gsync(g);
+#pragma unroll
+    for (int x = 0; x < 9; x++) {
+        if (at[x] < 0) continue;
+        const int i = 8 * (at[x] & 15) + g.g, j = 8 * (at[x] >> 4) + 2 * g.t;
+        *reinterpret_cast<double2 *>(YS + i * ps + j) = make_double2(acc[x][0], acc[x][1]);
+        if ((at[x] & 15) != (at[x] >> 4)) {
+            YS[j * ps + i] = acc[x][0];
+            YS[(j + 1) * ps + i] = acc[x][1];
+        }
+    }
+    gsync(g);
+}
+
+// Modified Gram-Schmidt of the n x r factor in place, zero columns kept zero: a
+// product whose Gram is not positive definite.
+__device__ __noinline__ void gmgs(int uo, int n, int r, int lt) {
+    double *U = bt_sm + uo;
+    if (lt == 0) {
         for (int c = 0; c < r; c++) {
-            for (int i = 0; i < n; i++) dst[i + c * n] = src[i + c * n];
             for (int p = 0; p < c; p++) {
                 double d = 0.0;
-                for (int i = 0; i < n; i++) d += dst[i + c * n] * dst[i + p * n];
-                for (int i = 0; i < n; i++) dst[i + c * n] -= d * dst[i + p * n];
+                for (int i = 0; i < n; i++) d += U[u_at(i, c)] * U[u_at(i, p)];
+                for (int i = 0; i < n; i++) U[u_at(i, c)] -= d * U[u_at(i, p)];
             }
             double nr = 0.0;
-            for (int i = 0; i < n; i++) nr += dst[i + c * n] * dst[i + c * n];
+            for (int i = 0; i < n; i++) nr += U[u_at(i, c)] * U[u_at(i, c)];
             nr = sqrt(nr);
-            for (int i = 0; i < n; i++) dst[i + c * n] = nr > 0 ? dst[i + c * n] / nr : 0.0;
+            for (int i = 0; i < n; i++) U[u_at(i, c)] = nr > 0 ? U[u_at(i, c)] / nr : 0.0;
         }
     }
-    gsync(g);
 }
 
-// Leading subspace of S (n x n, symmetric) from L (n x r), `iters` steps of
-// L <- orth(S L), in place on L.
-__device__ void gsubspace(const double *S, int n, double *L, int r, int iters, double *Z,
-                          double *Gs, int *bad, const Grp &g) {
+// Leading subspace of S (n x n symmetric, pitch ps, whole tiles zero padded)
+// from the factor U (n x r), `iters` steps of U <- orth(S U), in place.  Warp w
+// owns the 8-row tiles w and w + W (n <= 64 and W >= 4, n <= 32 and W = 2, n <= 16
+// and W = 1: two are enough).  It computes (S U)^T there: with U as the A operand
+// a lane holds column g of Z = S U at rows 2 t, 2 t + 1, which are the fragments
+// of Z^T Z as they stand (even rows one k-step, odd rows another).  Three barriers
+// a step: the Gram shares (then Z takes U's place), the first warp's L^{-1}, the
+// new U.  Bound by latency: a step of 40 x 4 takes about 2700 cycles alone on an SM
+// with 4 warps, 3500 with four tensors on it; shuffles in place of the trip of Z
+// through shared memory, or every warp factoring the sum for itself, were slower.
+__device__ __noinline__ void gsubspace(int ys, int n, int ps, int uo, int r, int iters, Grp g) {
+    const double *S = bt_sm + ys;
+    double *U = bt_sm + uo;
+    const int nt = tile8(n) / 8, m0 = g.w, m1 = g.w + g.W;
+    const bool have0 = m0 < nt, have1 = m1 < nt;
+    const double *s0 = S + (8 * (have0 ? m0 : 0) + g.g) * ps + g.t;
+    const double *s1 = S + (8 * (have1 ? m1 : 0) + g.g) * ps + g.t;
+    const double *u0 = U + u_at(g.t, g.g), *u1 = U + u_at(4 + g.t, g.g);
+    double *const part = bt_sm + g.part, *mine = part + g.w * WARP_SCR + g.g * 8 + 2 * g.t;
+    double *const Li = part + 64;
+#pragma unroll 1
     for (int it = 0; it < iters; it++) {
-        for (int e = g.lt; e < n * r; e += g.gs) {
-            const int i = e % n, c = e / n;
-            const double *lc = L + n * c;
-            double a0 = 0.0, a1 = 0.0, a2 = 0.0, a3 = 0.0;
-            int k = 0;
-            for (; k + 3 < n; k += 4) {
-                a0 = fma(S[i + n * k], lc[k], a0);
-                a1 = fma(S[i + n * (k + 1)], lc[k + 1], a1);
-                a2 = fma(S[i + n * (k + 2)], lc[k + 2], a2);
-                a3 = fma(S[i + n * (k + 3)], lc[k + 3], a3);
+        // Z's tiles, two chains each (even and odd k-steps); what is past n is zero.
+        double z[2][2] = {}, y[2][2] = {};
+        if (have0) {
+#pragma unroll 1
+            for (int k = 0; k < nt; k++) {
+                const double a0 = u0[64 * k], a1 = u1[64 * k], b0 = s0[8 * k], b1 = s0[8 * k + 4];
+                bt_dmma(z[0][0], z[0][1], a0, b0);
+                bt_dmma(y[0][0], y[0][1], a1, b1);
+                if (have1) {
+                    const double c0 = s1[8 * k], c1 = s1[8 * k + 4];
+                    bt_dmma(z[1][0], z[1][1], a0, c0);
+                    bt_dmma(y[1][0], y[1][1], a1, c1);
+                }
             }
-            for (; k < n; k++) a0 = fma(S[i + n * k], lc[k], a0);
-            Z[e] = (a0 + a1) + (a2 + a3);
+        }
+        double d[2][2] = {};
+#pragma unroll
+        for (int m = 0; m < 2; m++)
+#pragma unroll
+            for (int q = 0; q < 2; q++) {
+                z[m][q] += y[m][q];
+                bt_dmma(d[q][0], d[q][1], z[m][q], z[m][q]);
+            }
+        *reinterpret_cast<double2 *>(mine) = make_double2(d[0][0] + d[1][0], d[0][1] + d[1][1]);
+        gsync(g);
+#pragma unroll
+        for (int m = 0; m < 2; m++)
+            if (m ? have1 : have0) {
+                const int i = 8 * (m ? m1 : m0) + 2 * g.t;
+                U[u_at(i, g.g)] = z[m][0];
+                U[u_at(i + 1, g.g)] = z[m][1];
+            }
+        // The first warp adds the shares in order and factors the sum.
+        if (g.w == 0) {
+            double2 a = *reinterpret_cast<const double2 *>(mine);
+            const int shares = min(g.W, nt);
+#pragma unroll 4
+            for (int w = 1; w < shares; w++) {
+                const double2 p = *reinterpret_cast<const double2 *>(mine + w * WARP_SCR);
+                a.x += p.x;
+                a.y += p.y;
+            }
+            *reinterpret_cast<double2 *>(Li + g.g * 8 + 2 * g.t) = a;
+            __syncwarp();
+            double c[BMAX_R];
+            const bool ok = warp_chol_linv<BMAX_R>(Li, BMAX_R, r, c);
+            __syncwarp();
+            // Lane j holds column j of L^{-1}; above the diagonal it holds zeros.
+            const int j = 4 * g.g + g.t;
+            if (j < BMAX_R) {
+#pragma unroll
+                for (int i = 0; i < BMAX_R; i++) Li[i * BMAX_R + j] = c[i];
+            }
+            if (j == 0 && !ok) Li[0] = -1.0;  // (a factor's is positive)
         }
         gsync(g);
-        gcholqr(Z, L, n, r, Gs, bad, g);
+        if (!(Li[0] > 0.0)) {
+            gmgs(uo, n, r, g.lt);
+            gsync(g);
+            continue;
+        }
+        // Q^T = L^{-1} Z^T over the warp's own rows.
+        const double l0 = Li[g.g * 8 + g.t], l1 = Li[g.g * 8 + 4 + g.t];
+#pragma unroll
+        for (int m = 0; m < 2; m++)
+            if (m ? have1 : have0) {
+                const int i0 = 8 * (m ? m1 : m0);
+                const double b0 = U[u_at(i0 + g.g, g.t)], b1 = U[u_at(i0 + g.g, 4 + g.t)];
+                double q0 = 0.0, q1 = 0.0;
+                bt_dmma(q0, q1, l0, b0);
+                bt_dmma(q0, q1, l1, b1);
+                __syncwarp();
+                U[u_at(i0 + 2 * g.t, g.g)] = q0;
+                U[u_at(i0 + 2 * g.t + 1, g.g)] = q1;
+            }
+        gsync(g);
     }
 }
 
-// S (n x n) = Y Y^T for Y n x K col-major (row i at Y[i + n k]): 2 x 2 blocks
-// of S per thread, four independent chains.
-__device__ void ggram(const double *Y, int n, int K, double *S, const Grp &g) {
-    const int nb = (n + 1) >> 1;
-    for (int e = g.lt; e < nb * nb; e += g.gs) {
-        const int bi = e % nb, bj = e / nb;
-        if (bj < bi) continue;  // upper block triangle; mirrored below
-        const int i0 = 2 * bi, j0 = 2 * bj;
-        const int i1 = min(i0 + 1, n - 1), j1 = min(j0 + 1, n - 1);
-        double s00 = 0.0, s01 = 0.0, s10 = 0.0, s11 = 0.0;
-        for (int k = 0; k < K; k++) {
-            const double *y = Y + n * k;
-            const double a0 = y[i0], a1 = y[i1], b0 = y[j0], b1 = y[j1];
-            s00 = fma(a0, b0, s00);
-            s01 = fma(a0, b1, s01);
-            s10 = fma(a1, b0, s10);
-            s11 = fma(a1, b1, s11);
-        }
-        S[i0 + n * j0] = s00;
-        S[j0 + n * i0] = s00;
-        if (j0 + 1 < n) {
-            S[i0 + n * j1] = s01;
-            S[j1 + n * i0] = s01;
-        }
-        if (i0 + 1 < n) {
-            S[i1 + n * j0] = s10;
-            S[j0 + n * i1] = s10;
-        }
-        if (i0 + 1 < n && j0 + 1 < n) {
-            S[i1 + n * j1] = s11;
-            S[j1 + n * i1] = s11;
-        }
-    }
-    gsync(g);
-}
-
-// The whole HOOI of tensor t by one thread group.  `sm` is the group's
-// shared-memory slice (slot_doubles(largest mode) doubles at least), `T` its
-// global scratch slice.
-__device__ void hooi_one(const BatchArgs &a, int t, double *sm, double *T, const Grp &g,
-                         int *bad) {
+// The whole HOOI of tensor t by one thread group.  `slot` is the offset of the
+// group's shared-memory slice (slot_doubles(largest mode) doubles at least), `T`
+// its global scratch slice.
+__device__ __forceinline__ void hooi_one(const BatchArgs &a, int t, int slot, double *T,
+                                         const Grp &g) {
     const int I0 = (int)a.shape[3 * t], I1 = (int)a.shape[3 * t + 1], I2 = (int)a.shape[3 * t + 2];
     const int R0 = (int)a.rank[3 * t], R1 = (int)a.rank[3 * t + 1], R2 = (int)a.rank[3 * t + 2];
-    const int m = max(I0, max(I1, I2));
-    double *U0 = sm, *U1 = U0 + m * BMAX_R, *U2 = U1 + m * BMAX_R;
-    double *Ys = U2 + m * BMAX_R;   // m x K
-    double *Ss = Ys + m * BMAX_K;   // m x m
-    double *Zs = Ss + m * m;        // m x R
-    double *Gs = Zs + m * BMAX_R;   // R x R
-    double *red = Gs + BMAX_R * BMAX_R;
+    const int m = max(I0, max(I1, I2)), m8 = tile8(m);
+    const int uo = slot, us = m8 * BMAX_R, ys = slot + 3 * us;
+    double *U0 = bt_sm + uo, *U1 = U0 + us, *U2 = U1 + us;
+    double *YS = bt_sm + ys;                      // Y_(n), then its Gram
+    double *red = YS + m8 * pitch16(BMAX_K);
+    double *Ylast = T + (int64_t)m * m * BMAX_R;  // the final Y_(3), I2 x K
     const float *X = a.X + a.xoff[t];
     double *ug[3] = {a.U + a.uoff[3 * t], a.U + a.uoff[3 * t + 1], a.U + a.uoff[3 * t + 2]};
-    for (int e = g.lt; e < I0 * R0; e += g.gs) U0[e] = ug[0][e];
-    for (int e = g.lt; e < I1 * R1; e += g.gs) U1[e] = ug[1][e];
-    for (int e = g.lt; e < I2 * R2; e += g.gs) U2[e] = ug[2][e];
-    const int64_t nx = (int64_t)I0 * I1 * I2;
+    for (int e = g.lt; e < 3 * m8 * BMAX_R; e += g.gs) U0[e] = 0.0;
+    gsync(g);
+    for (int e = g.lt; e < I0 * R0; e += g.gs) U0[u_at(e % I0, e / I0)] = ug[0][e];
+    for (int e = g.lt; e < I1 * R1; e += g.gs) U1[u_at(e % I1, e / I1)] = ug[1][e];
+    for (int e = g.lt; e < I2 * R2; e += g.gs) U2[u_at(e % I2, e / I2)] = ug[2][e];
+    const int nx = I0 * I1 * I2;
     double s = 0.0;
-    for (int64_t e = g.lt; e < nx; e += g.gs) s = fma((double)X[e], (double)X[e], s);
+#pragma unroll 8
+    for (int e = g.lt; e < nx; e += g.gs) s = fma((double)X[e], (double)X[e], s);
     const double x2 = gsum(s, red, g);
-    const int I01 = I0 * I1;
+    const int I01 = I0 * I1, I12 = I1 * I2;
     for (int sw = 0; sw < a.sweeps; sw++) {
-        // T = X x_3 U_3^T  (I0 x I1 x R2)
-        for (int p = g.lt; p < I01; p += g.gs) {
-            double acc[BMAX_R] = {};
-#pragma unroll 4
-            for (int i2 = 0; i2 < I2; i2++) {
-                const double x = X[p + (int64_t)I01 * i2];
-#pragma unroll
-                for (int r = 0; r < BMAX_R; r++)
-                    if (r < R2) acc[r] = fma(x, U2[i2 + I2 * r], acc[r]);
-            }
-#pragma unroll
-            for (int r = 0; r < BMAX_R; r++)
-                if (r < R2) T[p + I01 * r] = acc[r];
+        // T = X x_3 U_3^T  (I0 x I1 x R2): rows (i0, i1).
+        contract<float>(X, I01, 1, 1, 0, I2, I01, uo + 2 * us, T, 1, I01, 0, R2, g);
+        // Modes 1 and 2 from T: Y_(1)[i0, r1 + R1 r2], Y_(2)[i1, r0 + R0 r2].
+#pragma unroll 1
+        for (int n = 0; n < 2; n++) {
+            const int I = n ? I1 : I0, R = n ? R0 : R1, K = R * R2, py = pitch16(K);
+            const int ps = pitch16(tile8(I));
+            gsync(g);
+            zero_pads(YS, I, K, py, g);
+            contract<double>(T, I, n ? I0 : 1, R2, I01, n ? I0 : I1, n ? 1 : I0, n ? uo : uo + us, YS,
+                             py, 1, R, R, g);
+            gsync(g);
+            ggram(ys, I, K, py, ps, g);
+            gsubspace(ys, I, ps, n ? uo + us : uo, n ? R1 : R0, a.inner, g);
         }
+        // Mode 3 from X: T2 = X x_1 U0^T (R0 x I1 x I2), rows (i1, i2), then
+        // Y_(3)[i2, r0 + R0 r1] = sum_i1 T2[r0, i1, i2] U1[i1, r1], rows r0.
+        contract<float>(X, I12, I0, 1, 0, I0, 1, uo, T, R0, 1, 0, R0, g);
         gsync(g);
-        // Mode 1: Y_(1)[i0, r1 + R1 r2] = sum_i1 T[i0, i1, r2] U1[i1, r1]
-        for (int q = g.lt; q < I0 * R2; q += g.gs) {
-            const int i0 = q % I0, r2 = q / I0;
-            double acc[BMAX_R] = {};
-#pragma unroll 4
-            for (int i1 = 0; i1 < I1; i1++) {
-                const double v = T[i0 + I0 * i1 + I01 * r2];
-#pragma unroll
-                for (int r = 0; r < BMAX_R; r++)
-                    if (r < R1) acc[r] = fma(v, U1[i1 + I1 * r], acc[r]);
-            }
-#pragma unroll
-            for (int r = 0; r < BMAX_R; r++)
-                if (r < R1) Ys[i0 + I0 * (r + R1 * r2)] = acc[r];
-        }
+        const int K = R0 * R1, py = pitch16(K);
+        zero_pads(YS, I2, K, py, g);
+        contract<double>(T, R0, 1, I2, R0 * I1, I1, R0, uo + us, YS, 1, R0, py, R1, g);
         gsync(g);
-        ggram(Ys, I0, R1 * R2, Ss, g);
-        gsubspace(Ss, I0, U0, R0, a.inner, Zs, Gs, bad, g);
-        // Mode 2: Y_(2)[i1, r0 + R0 r2] = sum_i0 T[i0, i1, r2] U0[i0, r0]
-        for (int q = g.lt; q < I1 * R2; q += g.gs) {
-            const int i1 = q % I1, r2 = q / I1;
-            double acc[BMAX_R] = {};
-#pragma unroll 4
-            for (int i0 = 0; i0 < I0; i0++) {
-                const double v = T[i0 + I0 * i1 + I01 * r2];
-#pragma unroll
-                for (int r = 0; r < BMAX_R; r++)
-                    if (r < R0) acc[r] = fma(v, U0[i0 + I0 * r], acc[r]);
-            }
-#pragma unroll
-            for (int r = 0; r < BMAX_R; r++)
-                if (r < R0) Ys[i1 + I1 * (r + R0 * r2)] = acc[r];
-        }
-        gsync(g);
-        ggram(Ys, I1, R0 * R2, Ss, g);
-        gsubspace(Ss, I1, U1, R1, a.inner, Zs, Gs, bad, g);
-        // Mode 3 from X: T2 = X x_1 U0^T (R0 x I1 x I2), then Y_(3).
-        const int R0I1 = R0 * I1;
-        for (int q = g.lt; q < I1 * I2; q += g.gs) {
-            const int64_t base = (int64_t)I0 * q;
-            double acc[BMAX_R] = {};
-#pragma unroll 4
-            for (int i0 = 0; i0 < I0; i0++) {
-                const double x = X[base + i0];
-#pragma unroll
-                for (int r = 0; r < BMAX_R; r++)
-                    if (r < R0) acc[r] = fma(x, U0[i0 + I0 * r], acc[r]);
-            }
-#pragma unroll
-            for (int r = 0; r < BMAX_R; r++)
-                if (r < R0) T[r + R0 * q] = acc[r];
-        }
-        gsync(g);
-        // Y_(3)[i2, r0 + R0 r1] = sum_i1 T2[r0, i1, i2] U1[i1, r1]
-        for (int q = g.lt; q < R0 * I2; q += g.gs) {
-            const int r0 = q % R0, i2 = q / R0;
-            double acc[BMAX_R] = {};
-#pragma unroll 4
-            for (int i1 = 0; i1 < I1; i1++) {
-                const double v = T[r0 + R0 * i1 + R0I1 * i2];
-#pragma unroll
-                for (int r = 0; r < BMAX_R; r++)
-                    if (r < R1) acc[r] = fma(v, U1[i1 + I1 * r], acc[r]);
-            }
-#pragma unroll
-            for (int r = 0; r < BMAX_R; r++)
-                if (r < R1) Ys[i2 + I2 * (r0 + R0 * r)] = acc[r];
-        }
-        gsync(g);
-        ggram(Ys, I2, R0 * R1, Ss, g);
-        gsubspace(Ss, I2, U2, R2, a.inner, Zs, Gs, bad, g);
+        if (sw == a.sweeps - 1)
+            for (int e = g.lt; e < I2 * K; e += g.gs) Ylast[e] = YS[(e % I2) * py + e / I2];
+        ggram(ys, I2, K, py, pitch16(tile8(I2)), g);
+        gsubspace(ys, I2, pitch16(tile8(I2)), uo + 2 * us, R2, a.inner, g);
     }
     // Core G[k + K r2] = sum_i2 Y_(3)[i2, k] U2[i2, r2] (the last Y_(3) and U2
     // are those of the final sweep), relative error in FP64.
@@ -398,7 +476,7 @@ __device__ void hooi_one(const BatchArgs &a, int t, double *sm, double *T, const
     for (int e = g.lt; e < K * R2; e += g.gs) {
         const int k = e % K, r2 = e / K;
         double acc = 0.0;
-        for (int i2 = 0; i2 < I2; i2++) acc = fma(Ys[i2 + I2 * k], U2[i2 + I2 * r2], acc);
+        for (int i2 = 0; i2 < I2; i2++) acc = fma(Ylast[i2 + I2 * k], U2[u_at(i2, r2)], acc);
         Gout[e] = acc;
         g2 = fma(acc, acc, g2);
     }
@@ -406,16 +484,14 @@ __device__ void hooi_one(const BatchArgs &a, int t, double *sm, double *T, const
     // A non-finite input gives a NaN error (fmax would turn NaN into 0).
     const double q = 1.0 - g2 / x2;
     if (g.lt == 0) a.relerr[t] = isnan(q) ? q : sqrt(fmax(0.0, q));
-    for (int e = g.lt; e < I0 * R0; e += g.gs) ug[0][e] = U0[e];
-    for (int e = g.lt; e < I1 * R1; e += g.gs) ug[1][e] = U1[e];
-    for (int e = g.lt; e < I2 * R2; e += g.gs) ug[2][e] = U2[e];
+    for (int e = g.lt; e < I0 * R0; e += g.gs) ug[0][e] = U0[u_at(e % I0, e / I0)];
+    for (int e = g.lt; e < I1 * R1; e += g.gs) ug[1][e] = U1[u_at(e % I1, e / I1)];
+    for (int e = g.lt; e < I2 * R2; e += g.gs) ug[2][e] = U2[u_at(e % I2, e / I2)];
 }
 
 template <int NT>
-__global__ void __launch_bounds__(NT, (NT <= 256 ? 2 : 1)) batched_hooi_kernel(const BatchArgs *__restrict__ ap) {
-    extern __shared__ __align__(16) double sm[];
+__global__ void __launch_bounds__(NT, 512 / NT) batched_hooi_kernel(const BatchArgs *__restrict__ ap) {
     __shared__ int cur;
-    __shared__ int bad[4];
     const BatchArgs a = *ap;
     double *scr = a.scratch + (int64_t)blockIdx.x * SCR;
     for (;;) {
@@ -427,21 +503,23 @@ __global__ void __launch_bounds__(NT, (NT <= 256 ? 2 : 1)) batched_hooi_kernel(c
         const Item item = a.items[it];
         const int gsz = NT / item.g;
         const int gid = threadIdx.x / gsz;
-        const Grp g{(int)threadIdx.x % gsz, gsz, 1 + gid};
+        const int lt = (int)threadIdx.x % gsz, lane = lt & 31;
+        const Grp g{lt, gsz, 1 + gid, lt >> 5, gsz >> 5, lane >> 2, lane & 3,
+                    SLOT_ALL + gid * (gsz >> 5) * WARP_SCR};
         const int t = item.t[gid];
         if (t >= 0)
-            hooi_one(a, t, sm + (SLOT / item.g) * gid, scr + (SCR / item.g) * gid, g, &bad[gid]);
+            hooi_one(a, t, (SLOT_ALL / item.g / 2 * 2) * gid, scr + (SCR / item.g) * gid, g);
         __syncthreads();
     }
 }
 
-size_t batched_smem() { return (size_t)SLOT * sizeof(double); }
+size_t batched_smem(int nt) { return ((size_t)SLOT_ALL + nt / 32 * WARP_SCR) * sizeof(double); }
 
 template <int NT>
 void kernel_attrs(dt_ctx *ctx, int *per_sm) {
-    smem_limit(ctx, batched_hooi_kernel<NT>, batched_smem());
+    smem_limit(ctx, batched_hooi_kernel<NT>, batched_smem(NT));
     DT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, batched_hooi_kernel<NT>, NT,
-                                                          batched_smem()));
+                                                          batched_smem(NT)));
 }
 
 // Resident CTAs per SM x SMs for a block size.
@@ -458,7 +536,7 @@ unsigned batched_grid(dt_ctx *ctx, int nt) {
 
 void enqueue_kernel(dt_ctx *ctx, int nt, unsigned grid, const BatchArgs *dargs, int *queue) {
     DT_CUDA(cudaMemsetAsync(queue, 0, sizeof(int), ctx->stream));
-    const size_t smem = batched_smem();
+    const size_t smem = batched_smem(nt);
     if (nt == 128)
         DT_LAUNCH(ctx, batched_hooi_kernel<128>, grid, 128, smem, dargs);
     else if (nt == 512)

@@ -263,7 +263,7 @@ typedef struct {
     int grid;             /* persistent CTAs (resident CTAs per SM x SMs) */
     int kernel_launches;
     int pack;             /* 0: one tensor per CTA; 1: tensors with largest mode
-                             <= 37 two to a CTA; 2: also those <= 21 four to a CTA */
+                             <= 32 two to a CTA; 2: also those <= 16 four to a CTA */
     int items;            /* work items (CTA-sized units) of the launch */
     int candidates_timed; /* configurations the autotuner timed (0: cached) */
     double tune_best_ms;  /* the autotuner's fastest and slowest sample times */

@@ -62,6 +62,27 @@ def test_batched_packed_small_tensors_match_oracle(ctx, block):
     _check_vs_numpy_oracle(items, U0, U, G, relerr, sweeps=6)
 
 
+@pytest.mark.parametrize("block", [128, 256, 512])
+def test_batched_tile_edges_match_oracle(ctx, block):
+    """Modes and ranks at and around whole tiles and fragments, alone in a CTA
+    and two and four to one: FP64 against the FP64 oracle, 1e-10 and 1e-8 as
+    above."""
+    from diana_tucker_b200 import datasets
+    cases = [((64, 64, 64), (8, 8, 8)), ((64, 8, 57), (8, 1, 8)), ((33, 40, 41), (5, 8, 7)),
+             ((32, 31, 25), (4, 7, 3)), ((8, 32, 9), (2, 4, 8)), ((16, 15, 9), (3, 3, 1)),
+             ((16, 16, 16), (8, 8, 8)), ((8, 8, 8), (8, 4, 2)), ((5, 4, 3), (2, 2, 1)),
+             ((1, 7, 6), (1, 2, 2)), ((17, 1, 20), (6, 1, 6)), ((63, 20, 12), (7, 6, 5)),
+             ((48, 56, 24), (1, 8, 8)), ((2, 2, 2), (2, 2, 2))]
+    items = [(datasets.tucker_dense(s, r, noise_var=1e-4, seed=70 + k, dtype=np.float32), r)
+             for k, (s, r) in enumerate(cases)]
+    rng = np.random.default_rng(8)
+    U0 = [[np.linalg.qr(rng.standard_normal((X.shape[n], r[n])))[0] for n in range(3)]
+          for X, r in items]
+    U, G, relerr, _ = ctx.hooi_batched([X for X, _ in items], [r for _, r in items], U0, sweeps=6,
+                                       block_threads=block)
+    _check_vs_numpy_oracle(items, U0, U, G, relerr, sweeps=6)
+
+
 def test_batched_autotuner_and_graph_reuse(ctx):
     items, U0 = _batch(600, 5)
     tensors = [X for X, _ in items]
