@@ -676,12 +676,14 @@ class SpTensor:
         return Y
 
     def hooi(self, R, max_sweeps, Ut0):
-        Ut = [np.ascontiguousarray(u, dtype=np.float64).copy() for u in Ut0]
+        start = [np.ascontiguousarray(u, dtype=np.float64) for u in Ut0]
+        Ut = [np.empty_like(u) for u in start]
+        p0 = (ctypes.c_void_p * self.ndim)(*[a.ctypes.data for a in start])
         ptrs = (ctypes.c_void_p * self.ndim)(*[a.ctypes.data for a in Ut])
         r = _shape_arr(R)
         last = self.ndim - 1
         G = np.zeros((self._kron_len(R, last), int(R[last])), order="F")
         rep = HooiReport()
-        _lib.check(self.lib.dt_sp_hooi(self.ctx.h, self.h, _i64p(r), max_sweeps, ptrs,
-                                       G.ctypes.data, ctypes.byref(rep)))
+        _lib.check(self.lib.dt_sp_hooi_from(self.ctx.h, self.h, _i64p(r), max_sweeps, p0, ptrs,
+                                            G.ctypes.data, ctypes.byref(rep)))
         return G, Ut, rep.as_dict()

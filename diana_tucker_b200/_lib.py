@@ -159,6 +159,9 @@ _SIGS = [
                                        _vp]),
     ("dt_sp_hooi", ctypes.c_int, [_vp, _vp, c_i64p, ctypes.c_int, ctypes.POINTER(_vp), _vp,
                                   ctypes.POINTER(HooiReport)]),
+    ("dt_sp_hooi_from", ctypes.c_int, [_vp, _vp, c_i64p, ctypes.c_int, ctypes.POINTER(_vp),
+     ctypes.POINTER(_vp), _vp,
+                                  ctypes.POINTER(HooiReport)]),
     ("dt_sp_ttmc_dense_f64", ctypes.c_int, [_vp, _vp, ctypes.POINTER(_vp), c_i64p,
                                             ctypes.POINTER(ctypes.c_int), ctypes.c_int, _vp]),
     ("dt_sp_mettmc_f64", ctypes.c_int, [_vp, _vp, ctypes.POINTER(_vp), c_i64p,

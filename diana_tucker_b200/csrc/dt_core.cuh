@@ -48,6 +48,11 @@ struct dt_ctx {
     // and synchronises once (allocated on first use).
     static constexpr size_t kHostStageBytes = 4096;
     void *host_stage = nullptr;
+    // Pinned staging for large transfers of pageable host memory (upload_pieces /
+    // download_pieces): as large as the largest so far, at most kBigStageBytes.
+    static constexpr size_t kBigStageBytes = size_t(32) << 20;
+    void *big_stage = nullptr;
+    size_t big_stage_cap = 0;
     // The dense HOOI drivers' last plans (device buffers plus a captured graph
     // of one sweep), reused by the next call with the same shapes, ranks and
     // options; released before the stream at dt_ctx_destroy.
@@ -205,6 +210,21 @@ inline void check_ctx(const dt_ctx *ctx) {
 }
 
 bool is_device_ptr(const void *p);
+
+// Transfers between device memory and a caller's pageable host memory.  From a
+// megabyte on, several host threads copy two-megabyte chunks between the
+// caller's memory and the context's pinned staging while the DMA of other
+// chunks runs (the driver's own staging uses one thread: 36 MB up 3.4 ms, down
+// 2.1 ms); smaller ones are left to the driver.  upload_pieces returns once the
+// host memory has been read, its DMA in order on ctx->stream; download_pieces
+// once it has been written.
+struct HostPiece {
+    void *dev;
+    void *host;
+    size_t bytes;
+};
+void upload_pieces(dt_ctx *ctx, const std::vector<HostPiece> &pieces);
+void download_pieces(dt_ctx *ctx, const std::vector<HostPiece> &pieces);
 
 // Validates a dense shape: 1 <= ndim <= 16, every mode >= 1, and the element
 // count (so every product of modes) below 2^62.  Fails with DT_ERR_ARG naming

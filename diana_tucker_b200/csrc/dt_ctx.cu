@@ -1,9 +1,13 @@
 // Context lifetime, error reporting and host/device staging.
 #include <algorithm>
+#include <atomic>
 #include <cstdlib>
+#include <cstring>
 #include <map>
 #include <mutex>
 #include <optional>
+#include <system_error>
+#include <thread>
 
 #include "dt_core.cuh"
 
@@ -321,6 +325,124 @@ void copy_blocks(dt_ctx *ctx, int n, void *const *dst, const void *const *src,
     DT_LAUNCH(ctx, copy_blocks_kernel, blocks, threads, 0, b);
 }
 
+namespace {
+
+constexpr size_t kChunk = size_t(2) << 20, kStageFrom = size_t(1) << 20;
+
+struct Chunk {
+    char *dev, *host, *stage;
+    size_t bytes;
+};
+
+// fn(0) .. fn(n - 1) over a few threads; the first CUDA error is thrown here.
+void over_threads(dt_ctx *ctx, size_t n, const std::function<cudaError_t(size_t)> &fn) {
+    const size_t most = std::max(1u, std::min(4u, std::thread::hardware_concurrency() / 2));
+    std::atomic<size_t> next{0};
+    std::atomic<int> err{(int)cudaSuccess};
+    auto work = [&] {
+        cudaSetDevice(ctx->device);
+        for (size_t i; (i = next.fetch_add(1)) < n;) {
+            const cudaError_t e = fn(i);
+            if (e != cudaSuccess) err.store((int)e);
+        }
+    };
+    std::vector<std::thread> pool;
+    try {
+        for (size_t k = 1; k < std::min(most, n); k++) pool.emplace_back(work);
+    } catch (const std::system_error &) {  // no more threads: the ones there do it
+    }
+    work();
+    for (auto &t : pool) t.join();
+    DT_CUDA((cudaError_t)err.load());
+}
+
+// The pieces in chunks, in rounds that fit the staging buffer.
+void staged_rounds(dt_ctx *ctx, const std::vector<HostPiece> &pieces, size_t total,
+                   const std::function<void(std::vector<Chunk> &)> &round) {
+    const size_t want = std::min(dt_ctx::kBigStageBytes, (total + kChunk - 1) / kChunk * kChunk);
+    if (ctx->big_stage_cap < want) {
+        if (ctx->big_stage) DT_CUDA(cudaFreeHost(ctx->big_stage));
+        ctx->big_stage = nullptr;
+        ctx->big_stage_cap = 0;
+        DT_CUDA(cudaHostAlloc(&ctx->big_stage, want, cudaHostAllocDefault));
+        ctx->big_stage_cap = want;
+    }
+    std::vector<Chunk> now;
+    size_t used = 0;
+    for (const HostPiece &p : pieces)
+        for (size_t o = 0; o < p.bytes; o += kChunk) {
+            const size_t b = std::min(kChunk, p.bytes - o);
+            if (used + b > ctx->big_stage_cap) {
+                round(now);
+                now.clear();
+                used = 0;
+            }
+            now.push_back({static_cast<char *>(p.dev) + o, static_cast<char *>(p.host) + o,
+                           static_cast<char *>(ctx->big_stage) + used, b});
+            used += b;
+        }
+    if (!now.empty()) round(now);
+}
+
+size_t total_bytes(const std::vector<HostPiece> &pieces) {
+    size_t t = 0;
+    for (const HostPiece &p : pieces) t += p.bytes;
+    return t;
+}
+
+}  // namespace
+
+void upload_pieces(dt_ctx *ctx, const std::vector<HostPiece> &pieces) {
+    const size_t total = total_bytes(pieces);
+    if (total < kStageFrom) {
+        for (const HostPiece &p : pieces)
+            DT_CUDA(cudaMemcpyAsync(p.dev, p.host, p.bytes, cudaMemcpyHostToDevice, ctx->stream));
+        return;
+    }
+    bool reuse = false;
+    // An earlier call's DMA out of the staging is done: every call that uses it
+    // ends with a synchronisation.
+    staged_rounds(ctx, pieces, total, [&](std::vector<Chunk> &cs) {
+        if (reuse) DT_CUDA(cudaStreamSynchronize(ctx->stream));
+        reuse = true;
+        over_threads(ctx, cs.size(), [&](size_t i) {
+            std::memcpy(cs[i].stage, cs[i].host, cs[i].bytes);
+            return cudaMemcpyAsync(cs[i].dev, cs[i].stage, cs[i].bytes, cudaMemcpyHostToDevice,
+                                   ctx->stream);
+        });
+    });
+}
+
+void download_pieces(dt_ctx *ctx, const std::vector<HostPiece> &pieces) {
+    const size_t total = total_bytes(pieces);
+    if (total < kStageFrom) {
+        for (const HostPiece &p : pieces)
+            DT_CUDA(cudaMemcpyAsync(p.host, p.dev, p.bytes, cudaMemcpyDeviceToHost, ctx->stream));
+        DT_CUDA(cudaStreamSynchronize(ctx->stream));
+        return;
+    }
+    staged_rounds(ctx, pieces, total, [&](std::vector<Chunk> &cs) {
+        struct Events {
+            std::vector<cudaEvent_t> e;
+            ~Events() {
+                for (cudaEvent_t x : e) cudaEventDestroy(x);
+            }
+        } done;
+        for (const Chunk &c : cs) {
+            DT_CUDA(cudaMemcpyAsync(c.stage, c.dev, c.bytes, cudaMemcpyDeviceToHost, ctx->stream));
+            cudaEvent_t e;
+            DT_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+            done.e.push_back(e);
+            DT_CUDA(cudaEventRecord(e, ctx->stream));
+        }
+        over_threads(ctx, cs.size(), [&](size_t i) {
+            const cudaError_t e = cudaEventSynchronize(done.e[i]);
+            if (e == cudaSuccess) std::memcpy(cs[i].host, cs[i].stage, cs[i].bytes);
+            return e;
+        });
+    });
+}
+
 void *host_stage(dt_ctx *ctx) {
     if (!ctx->host_stage)
         DT_CUDA(cudaHostAlloc(&ctx->host_stage, dt_ctx::kHostStageBytes, cudaHostAllocDefault));
@@ -395,6 +517,7 @@ int dt_ctx_destroy(dt_ctx *ctx) {
         }
         if (ctx->own_stream) cudaStreamDestroy(ctx->own_stream);
         if (ctx->host_stage) cudaFreeHost(ctx->host_stage);
+        if (ctx->big_stage) cudaFreeHost(ctx->big_stage);
         delete ctx;
     });
 }

@@ -1671,6 +1671,12 @@ int dt_sp_ttmc_mTL(dt_ctx *ctx, const dt_sptensor *sp, const double *const *Ut,
 
 int dt_sp_hooi(dt_ctx *ctx, const dt_sptensor *sp, const int64_t *R, int max_sweeps,
                double *const *Ut, double *G, dt_hooi_report *report) {
+    return dt_sp_hooi_from(ctx, sp, R, max_sweeps, Ut, Ut, G, report);
+}
+
+int dt_sp_hooi_from(dt_ctx *ctx, const dt_sptensor *sp, const int64_t *R, int max_sweeps,
+                    const double *const *Ut0, double *const *Ut, double *G,
+                    dt_hooi_report *report) {
     return guard([&] {
         check_sp(ctx, sp, 0);
         DT_CHECK_ARG(max_sweeps >= 0, "dt_sp_hooi: max_sweeps must be >= 0");
@@ -1678,15 +1684,32 @@ int dt_sp_hooi(dt_ctx *ctx, const dt_sptensor *sp, const int64_t *R, int max_swe
         if (report) std::memset(report, 0, sizeof(*report));
         const int nd = sp->ndim;
         const int64_t launches0 = ctx->launches;
-        std::vector<DevView> views;
-        views.reserve(nd);
+        // The factors on the device: the caller's Ut where that is device
+        // memory, else a copy.
+        std::vector<DevMem> own(nd);
+        std::vector<HostPiece> in, out;
         const double *ptrs[MAXD];
         for (int m = 0; m < nd; m++) {
-            DT_CHECK_ARG(Ut && Ut[m] && R[m] >= 1 && R[m] <= sp->shape[m] && R[m] <= 32,
+            DT_CHECK_ARG(Ut && Ut[m] && Ut0 && Ut0[m] && R[m] >= 1 && R[m] <= sp->shape[m] &&
+                             R[m] <= 32,
                          "dt_sp_hooi: bad factor / rank for mode %d", m);
-            views.emplace_back(ctx, Ut[m], sp->shape[m] * R[m] * sizeof(double), true, true);
-            ptrs[m] = views.back().as<double>();
+            const size_t bytes = sp->shape[m] * R[m] * sizeof(double);
+            double *d = Ut[m];
+            if (!is_device_ptr(d)) {
+                own[m].alloc(ctx, bytes);
+                d = own[m].as<double>();
+                out.push_back({d, Ut[m], bytes});
+            }
+            if (is_device_ptr(Ut0[m])) {
+                if (Ut0[m] != d)
+                    DT_CUDA(cudaMemcpyAsync(d, Ut0[m], bytes, cudaMemcpyDeviceToDevice,
+                                            ctx->stream));
+            } else {
+                in.push_back({d, const_cast<double *>(Ut0[m]), bytes});
+            }
+            ptrs[m] = d;
         }
+        upload_pieces(ctx, in);
         int64_t maxYc = 1;
         for (int m = 0; m < nd; m++)
             maxYc = std::max<int64_t>(maxYc, sp->modes[m].nrows * kron_len(R, nd, m));
@@ -1752,8 +1775,7 @@ int dt_sp_hooi(dt_ctx *ctx, const dt_sptensor *sp, const int64_t *R, int max_swe
                                     cudaMemcpyDeviceToDevice, ctx->stream));
             g.finish();
         }
-        for (auto &v : views) v.finish();
-        DT_CUDA(cudaStreamSynchronize(ctx->stream));
+        download_pieces(ctx, out);
         if (!std::isfinite(hg2)) fail(DT_ERR_NUMERIC, "sparse HOOI produced a non-finite core");
         float ms = 0.f;
         DT_CUDA(cudaEventElapsedTime(&ms, ctx->ev_start, ctx->ev_stop));

@@ -352,6 +352,11 @@ DT_API int dt_sp_mettmc_f64(dt_ctx *ctx, const dt_sptensor *sp, const double *co
  * Algorithm::SpTucker::Sp_HOOI_ALS (sp_hooi_als.tpp:67-118). */
 DT_API int dt_sp_hooi(dt_ctx *ctx, const dt_sptensor *sp, const int64_t *R, int max_sweeps,
                double *const *Ut, double *G, dt_hooi_report *report);
+/* The same from initial factors Ut0 that stay as they are; Ut receives the
+ * result (Ut0[m] and Ut[m] each host or device memory, and may be the same). */
+DT_API int dt_sp_hooi_from(dt_ctx *ctx, const dt_sptensor *sp, const int64_t *R, int max_sweeps,
+                           const double *const *Ut0, double *const *Ut, double *G,
+                           dt_hooi_report *report);
 
 /* ---- Summary profiler ---------------------------------------------------- */
 /* The reference's Summary (include/summary.hpp:27-60, src/summary.cpp):

@@ -147,3 +147,33 @@ def test_sptensor_outlives_its_context(oracle_sparse):
         sp.ttmc_rows(_factors(shape, (2, 2, 2), 6), (2, 2, 2), 0)
     assert e.value.code == 1
     sp.close()
+
+
+@pytest.mark.parametrize("rows", [100, 20_000, 300_011])
+def test_hooi_factor_transfers(ctx, rows):
+    """Factors below the staging threshold, within the staging buffer and
+    larger than it: the start stays as it was, and the in-place entry point
+    (device buffers, no staging) gives the same bits."""
+    import ctypes
+
+    import torch
+
+    from diana_tucker_b200 import _lib, datasets
+    R = (16, 8, 8)
+    idx, vals, shape = datasets.sparse_zipf((rows, 300, 200), 20_000, alpha=1.1, seed=3)
+    Ut0 = _factors(shape, R, 9)
+    kept = [u.copy() for u in Ut0]
+    sp = ctx.sptensor(idx, vals, shape)
+    G, Ut, rep = sp.hooi(R, 2, Ut0)
+    assert all(np.array_equal(a, b) for a, b in zip(Ut0, kept))
+    dev = [torch.from_numpy(u).cuda() for u in Ut0]
+    torch.cuda.synchronize()
+    ptrs = (ctypes.c_void_p * 3)(*[d.data_ptr() for d in dev])
+    r = (ctypes.c_int64 * 3)(*R)
+    Gd = np.zeros_like(G)
+    _lib.check(ctx.lib.dt_sp_hooi(ctx.h, sp.h, r, 2, ptrs, Gd.ctypes.data,
+                                  ctypes.byref(_lib.HooiReport())))
+    assert np.array_equal(G, Gd)
+    for a, b in zip(Ut, dev):
+        assert np.array_equal(a, b.cpu().numpy())
+    sp.close()
