@@ -903,6 +903,7 @@ __global__ void sumsq_partial_kernel(const T *__restrict__ x, int64_t n,
                                      double *__restrict__ part) {
     pdl_wait();
     double s = 0.0;
+#pragma unroll 8
     for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < n;
          e += (int64_t)gridDim.x * blockDim.x) {
         const double v = (double)x[e];
@@ -947,15 +948,23 @@ __global__ void f32_to_f64_kernel(const float *__restrict__ x, int64_t n,
 }  // namespace
 
 void sumsq(dt_ctx *ctx, const void *x, int dtype, int64_t n, double *out) {
-    const int blocks = std::max(1, std::min<int>(4 * ctx->num_sms, (int)ceil_div(n, 256)));
-    DevMem part(ctx, (size_t)blocks * sizeof(double));
+    // One block up to 4096 entries (16 a thread): its partial sum is the result.
+    const int blocks =
+        n <= 4096 ? 1 : std::min<int>(4 * ctx->num_sms, (int)ceil_div(n, 256));
+    DevMem part;
+    double *dst = out;
+    if (blocks > 1) {
+        part.alloc(ctx, (size_t)blocks * sizeof(double));
+        dst = part.as<double>();
+    }
     if (dtype == DT_F64)
         DT_LAUNCH_PDL(ctx, sumsq_partial_kernel<double>, blocks, 256, 0,
-                  static_cast<const double *>(x), n, part.as<double>());
+                      static_cast<const double *>(x), n, dst);
     else
         DT_LAUNCH_PDL(ctx, sumsq_partial_kernel<float>, blocks, 256, 0,
-                  static_cast<const float *>(x), n, part.as<double>());
-    DT_LAUNCH_PDL(ctx, sum_partials_kernel, 1, 1024, 0, part.as<double>(), blocks, out);
+                      static_cast<const float *>(x), n, dst);
+    if (blocks > 1)
+        DT_LAUNCH_PDL(ctx, sum_partials_kernel, 1, 1024, 0, (const double *)dst, blocks, out);
 }
 
 void f32_to_f64(dt_ctx *ctx, const float *x, int64_t n, double *y) {

@@ -45,7 +45,7 @@ struct MixedHooi {
     const float *X32 = nullptr;
     DevMem X32own, Xh, Xl;
     std::vector<DevMem> U;
-    DevMem S, work, flag, err, scal, Gs;
+    DevMem S, work, flag, err, scal, counter;
     bool split = false;   // intermediates, U and the Gram operands as hi + lo
     bool xsplit = false;  // X itself as hi + lo (else X in BF16 hi only)
     DenseHooi helper;  // initial factors (same generators as the FP64 driver)
@@ -221,14 +221,14 @@ struct MixedHooi {
         const __nv_bfloat16 *yh = Y.hi;
         const __nv_bfloat16 *yl = split ? Y.lo : nullptr;
         void *gscr = take(tc_gram_scratch_bytes(I[n], K, split));
-        void *cscr = n == N - 1 ? take(core_rows_scratch_bytes(K)) : nullptr;
+        void *cscr = n == N - 1 ? take(core_norm_scratch_bytes(K)) : nullptr;
         if (dry) return;
         tc_gram(ctx, yh, yl, I[n], K, S.as<double>(), err.as<int>(), gscr);
         subspace_iter(ctx, S.as<double>(), I[n], U[n].as<double>(), R[n], opts.inner_iters,
                       work.as<double>(), flag.as<int>());
         if (n == N - 1)
-            core_rows(ctx, yh, yl, I[n], K, U[n].as<double>(), R[n], Gs.as<double>(),
-                      scal.as<double>() + 1, cscr);
+            core_norm(ctx, yh, yl, I[n], K, U[n].as<double>(), R[n], scal.as<double>() + 1, cscr,
+                      counter.as<int>());
     }
 
     void node(int lo, int hi, const __nv_bfloat16 *Th, const __nv_bfloat16 *Tl,
@@ -597,7 +597,8 @@ void hooi_dense_lowprec(dt_ctx *ctx, const void *X, int dtype, int ndim, const i
         h.flag.alloc(ctx, sizeof(int));
         h.err.alloc(ctx, sizeof(int));
         h.scal.alloc(ctx, 4 * sizeof(double));
-        h.Gs.alloc(ctx, prod(ranks, ndim) * sizeof(double));
+        h.counter.alloc(ctx, sizeof(int));
+        DT_CUDA(cudaMemsetAsync(h.counter.get(), 0, sizeof(int), ctx->stream));
         h.g_bf16 = &plan->g_bf16;
         h.g_split = &plan->g_split;
         h.loop = &plan->loop;

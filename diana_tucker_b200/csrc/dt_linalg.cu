@@ -508,56 +508,65 @@ __device__ __forceinline__ void sm_gram(const double *src, int n, int r, double 
 }
 
 // Ri = R^{-1} (row-major, pitch LDR) of G = R^T R, by warp 0 (all threads call
-// it; ends with a barrier; G is overwritten).  Lane j holds column j in
-// registers.  The next pivot is formed first, from values exchanged before this
-// pivot's root is known, and no branch stands between the rows' updates.  Then
-// lane c solves column c of the inverse by back substitution, R read from
-// shared memory.  Every operation and its rounding is that of the plain
+// it; ends with a barrier; G is overwritten).  32 / RT groups of RT lanes share
+// the rows (row i belongs to group i mod 32 / RT), lane c of a group holds column c
+// of its rows in registers.  The next pivot is formed first, from values exchanged
+// before this pivot's root is known, and no branch stands between the rows'
+// updates.  Then lane c solves column c of the inverse by back substitution, R
+// read from shared memory.  Every operation and its rounding is that of the plain
 // elimination (products and differences rounded one by one, two alternating
 // sums in the back substitution): the callers' factors go on to be rounded to
 // BF16 halves, where another rounding of FP64 would show.  Bound by the pivots'
-// chain (a root, a product and a difference each) and the back substitution's;
-// CTA-wide, with two barriers a pivot, it took 7400 cycles for r = 16 (the whole
-// kernel's times are at subspace_mma).  Returns false on a non-positive pivot.
+// chain (a root, two products, a difference) and by what a warp can issue:
+// r = 16 takes 4800 cycles (860 of them the back substitution), r = 5 1500; CTA-wide,
+// with two barriers a pivot, r = 16 took 7400.  Returns false on a non-positive
+// pivot.
 template <int RT>
 __device__ __forceinline__ bool sm_chol_inv(double *G, double *Ri, int r) {
     constexpr int LDR = SmTile<RT>::LDR;
+    constexpr int GR = 32 / RT, NR = RT / GR;
     __shared__ int good;
     const int lane = threadIdx.x;
     if (lane < 32) {
-        double g[RT], dinv[RT];
+        const int c = lane % RT, h = lane / RT;
+        double g[NR], dinv[RT];
 #pragma unroll
-        for (int i = 0; i < RT; i++) {
-            g[i] = lane < RT ? G[i * RT + lane] : 0.0;
-            dinv[i] = 1.0;
-        }
+        for (int q = 0; q < NR; q++) g[q] = G[(q * GR + h) * RT + c];
+#pragma unroll
+        for (int i = 0; i < RT; i++) dinv[i] = 1.0;
         double d = __shfl_sync(0xffffffffu, g[0], 0);
         const double least = 1e-28 * d;
         bool ok = d > 0.0;
 #pragma unroll
         for (int k = 0; k < RT; k++) {
             if (k >= r) break;
-            double s[RT], next = 0.0;
+            constexpr unsigned ALL = 0xffffffffu;
+            const int qk = k / GR, at = RT * (k % GR);  // row k's lanes: at, at + 1, ...
+            double s[NR], next = 0.0, s1 = 0.0;
+            if (k + 1 < RT) {
+                s1 = __shfl_sync(ALL, g[qk], at + k + 1);
+                next = __shfl_sync(ALL, g[(k + 1) / GR], RT * ((k + 1) % GR) + k + 1);
+            }
+            const double raw = __shfl_sync(ALL, g[qk], at + c);
 #pragma unroll
-            for (int i = k + 1; i < RT; i++) s[i] = __shfl_sync(0xffffffffu, g[k], i);
-            if (k + 1 < RT) next = __shfl_sync(0xffffffffu, g[k + 1], k + 1);
+            for (int q = qk; q < NR; q++) s[q] = __shfl_sync(ALL, g[qk], at + q * GR + h);
             ok = ok && d > least;
             const double ri = rsqrt(fmax(d, 1e-300));
             dinv[k] = ri;
             if (k + 1 < RT) {
-                const double l = __dmul_rn(s[k + 1], ri);
+                const double l = __dmul_rn(s1, ri);
                 d = __dsub_rn(next, __dmul_rn(l, l));
             }
-            const double gk = __dmul_rn(g[k], ri);
-            g[k] = gk;
+            const double gk = __dmul_rn(raw, ri);
 #pragma unroll
-            for (int i = k + 1; i < RT; i++)
-                g[i] = __dsub_rn(g[i], __dmul_rn(__dmul_rn(s[i], ri), gk));
+            for (int q = qk; q < NR; q++) {
+                const double u = __dsub_rn(g[q], __dmul_rn(__dmul_rn(s[q], ri), gk));
+                if (q > qk || h > k % GR) g[q] = u;
+                else if (h == k % GR) g[q] = gk;
+            }
         }
-        if (lane < RT) {
 #pragma unroll
-            for (int i = 0; i < RT; i++) G[i * RT + lane] = g[i];
-        }
+        for (int q = 0; q < NR; q++) G[(q * GR + h) * RT + c] = g[q];
         __syncwarp();
         // x_i = (delta_{i,c} - sum_{j>i} R(i, j) x_j) dinv_i
         double x[RT];

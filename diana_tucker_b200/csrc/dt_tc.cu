@@ -487,62 +487,81 @@ __global__ void split_f32_kernel(const float *__restrict__ x, int64_t n,
     }
 }
 
-// Sweep core from the K-major leaf rows: G[k + K*r] = sum_i Y[i][k] U[i][r]
-// in FP64 (hi + lo converts exactly).  A CTA owns 64 columns k; thread
-// (c, q) = (t % 64, t / 64) sums the rows i = q, q + 4, ... for all R outputs of
-// column k in registers (U staged in shared memory, row-major), and the four
-// partial sums are added in a fixed order.  Per-block partial sum of G^2.
-template <int RMAX>
-__global__ void __launch_bounds__(256) core_rows_kernel(const __nv_bfloat16 *__restrict__ Yh,
-                                                        const __nv_bfloat16 *__restrict__ Yl,
-                                                        int64_t I, int64_t K,
-                                                        const double *__restrict__ U, int R,
-                                                        double *__restrict__ G,
-                                                        double *__restrict__ part) {
-    extern __shared__ double Us[];  // I x RMAX, row i at Us + i * RMAX
-    __shared__ double red[4][64];
-    __shared__ double s2w[8];
-    pdl_wait();
-    for (int64_t e = threadIdx.x; e < I * RMAX; e += blockDim.x) {
-        const int64_t i = e / RMAX;
-        const int r = (int)(e - i * RMAX);
-        Us[e] = r < R ? U[i + I * r] : 0.0;
-    }
-    __syncthreads();
-    const int c = threadIdx.x & 63, q = threadIdx.x >> 6;
-    const int64_t k = (int64_t)blockIdx.x * 64 + c;
+// ||G||^2 of a sweep's core from the K-major leaf rows, G(k, r) = sum_i Y[i][k]
+// U[i][r] in FP64 (hi + lo converts exactly), on the FP64 tensor cores: a warp
+// makes 8 columns k x all r and adds its squares; the last CTA adds the CTAs'
+// sums in order (counter: zero before and after).  The core itself is not
+// kept: the returned one is projected in FP64 from X.  Bound by latency: 32 loads
+// a lane in flight.  K = 4096, I = 96, R = 16: 8.5 us against 20 with one FMA
+// chain per thread and output, a barrier pair per r and a second launch; K = 128: 8
+// against 22.
+constexpr int CORE_WARPS = 4;
+template <int NT>
+__global__ void __launch_bounds__(32 * CORE_WARPS) core_norm_kernel(
+    const __nv_bfloat16 *__restrict__ Yh, const __nv_bfloat16 *__restrict__ Yl, int I, int64_t K,
+    const double *__restrict__ U, int R, double *__restrict__ part, int *__restrict__ counter,
+    double *__restrict__ out) {
+    __shared__ double sums[CORE_WARPS];
+    __shared__ int last;
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+    const int64_t k = ((int64_t)blockIdx.x * CORE_WARPS + w) * 8 + g;
     const bool okk = k < K;
-    double acc[RMAX];
+    const __nv_bfloat16 *yh = Yh + (okk ? k : 0), *yl = Yl ? Yl + (okk ? k : 0) : nullptr;
+    pdl_wait();
+    double acc[NT][2];
 #pragma unroll
-    for (int r = 0; r < RMAX; r++) acc[r] = 0.0;
-    if (okk) {
-        for (int64_t i = q; i < I; i += 4) {
-            double y = (double)__bfloat162float(Yh[i * K + k]);
-            if (Yl) y += (double)__bfloat162float(Yl[i * K + k]);
-            const double *u = Us + i * RMAX;
+    for (int n = 0; n < NT; n++) acc[n][0] = acc[n][1] = 0.0;
+    for (int i0 = 0; i0 < I; i0 += 32) {
+        __nv_bfloat16 h[8], l[8];
+        double u[8][NT];
 #pragma unroll
-            for (int r = 0; r < RMAX; r++) acc[r] = fma(y, u[r], acc[r]);
+        for (int s = 0; s < 8; s++) {
+            const int i = i0 + 4 * s + t, ic = min(i, I - 1);
+            h[s] = yh[ic * K];
+            if (yl) l[s] = yl[ic * K];
+#pragma unroll
+            for (int n = 0; n < NT; n++) {
+                const int r = 8 * n + g;
+                u[s][n] = i < I && r < R ? U[ic + (int64_t)I * r] : 0.0;
+            }
+        }
+#pragma unroll
+        for (int s = 0; s < 8; s++) {
+            double y = (double)__bfloat162float(h[s]);
+            if (yl) y += (double)__bfloat162float(l[s]);
+            if (!okk) y = 0.0;
+#pragma unroll
+            for (int n = 0; n < NT; n++)
+                asm volatile(
+                    "mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
+                    : "+d"(acc[n][0]), "+d"(acc[n][1])
+                    : "d"(y), "d"(u[s][n]));
         }
     }
-    pdl_trigger();  // dependents may launch while the core is stored
+    pdl_trigger();
     double s2 = 0.0;
 #pragma unroll
-    for (int r = 0; r < RMAX; r++) {
-        if (r >= R) break;
-        red[q][c] = acc[r];
-        __syncthreads();
-        if (q == 0 && okk) {
-            const double g = (red[0][c] + red[1][c]) + (red[2][c] + red[3][c]);
-            G[k + K * r] = g;
-            s2 = fma(g, g, s2);
-        }
-        __syncthreads();
-    }
-    // s2 lives in the 64 threads of q == 0 (warps 0 and 1).
-    for (int o = 16; o > 0; o >>= 1) s2 += __shfl_down_sync(0xffffffffu, s2, o);
-    if ((threadIdx.x & 31) == 0) s2w[threadIdx.x >> 5] = s2;
+    for (int n = 0; n < NT; n++) s2 += acc[n][0] * acc[n][0] + acc[n][1] * acc[n][1];
+    for (int o = 16; o > 0; o >>= 1) s2 += __shfl_xor_sync(0xffffffffu, s2, o);
+    if (lane == 0) sums[w] = s2;
     __syncthreads();
-    if (threadIdx.x == 0) part[blockIdx.x] = s2w[0] + s2w[1];
+    if (threadIdx.x == 0) {
+        double s = 0.0;
+        for (int q = 0; q < CORE_WARPS; q++) s += sums[q];
+        part[blockIdx.x] = s;
+        __threadfence();
+        last = atomicAdd(counter, 1) == (int)gridDim.x - 1;
+    }
+    __syncthreads();
+    if (!last || w > 0) return;
+    __threadfence();
+    double s = 0.0;
+    for (int e = lane; e < (int)gridDim.x; e += 32) s += __ldcg(part + e);
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (lane == 0) {
+        *out = s;
+        *counter = 0;
+    }
 }
 
 __global__ void sum_double_kernel(const double *__restrict__ part, int n, double *__restrict__ out) {
@@ -782,32 +801,23 @@ void split_f32_chunks(dt_ctx *ctx, const ChunkedUpload &up, __nv_bfloat16 *hi,
     DT_LAUNCH_PDL(ctx, sum_double_kernel, 1, 1024, 0, part.as<double>(), up.chunks * bpc, sumsq_out);
 }
 
-size_t core_rows_scratch_bytes(int64_t K) {
-    return (size_t)std::max<int64_t>(1, ceil_div(K, 64)) * sizeof(double);
+size_t core_norm_scratch_bytes(int64_t K) {
+    return (size_t)ceil_div(K, 8 * CORE_WARPS) * sizeof(double);
 }
 
-void core_rows(dt_ctx *ctx, const __nv_bfloat16 *Yh, const __nv_bfloat16 *Yl, int64_t I, int64_t K,
-               const double *U, int64_t R, double *G, double *g2_out, void *scratch) {
-    DT_CHECK_ARG(R <= 32, "core_rows: R %lld > 32", (long long)R);
-    const int blocks = (int)std::max<int64_t>(1, ceil_div(K, 64));
-    DevMem own;
-    if (!scratch) own.alloc(ctx, (size_t)blocks * sizeof(double));
-    double *part = scratch ? static_cast<double *>(scratch) : own.as<double>();
-#define DT_CORE_ROWS(RM)                                                                     \
-    do {                                                                                     \
-        const size_t smem = (size_t)I * RM * sizeof(double);                                 \
-        smem_limit(ctx, core_rows_kernel<RM>, smem);                                         \
-        DT_LAUNCH_PDL(ctx, core_rows_kernel<RM>, blocks, 256, smem, Yh, Yl, I, K, U, (int)R, G,  \
-                  part);                                                                     \
-    } while (0)
-    if (R <= 8)
-        DT_CORE_ROWS(8);
-    else if (R <= 16)
-        DT_CORE_ROWS(16);
-    else
-        DT_CORE_ROWS(32);
-#undef DT_CORE_ROWS
-    DT_LAUNCH_PDL(ctx, sum_double_kernel, 1, 1024, 0, part, blocks, g2_out);
+void core_norm(dt_ctx *ctx, const __nv_bfloat16 *Yh, const __nv_bfloat16 *Yl, int64_t I, int64_t K,
+               const double *U, int64_t R, double *g2_out, void *scratch, int *counter) {
+    DT_CHECK_ARG(R <= 32 && I <= INT32_MAX, "core_norm: I %lld R %lld", (long long)I, (long long)R);
+    double *part = static_cast<double *>(scratch);
+    const unsigned blocks = ceil_div(K, 8 * CORE_WARPS);
+#define DT_CORE_NORM(NT)                                                                   \
+    DT_LAUNCH_PDL(ctx, core_norm_kernel<NT>, blocks, 32 * CORE_WARPS, 0, Yh, Yl, (int)I, K, U, \
+                  (int)R, part, counter, g2_out)
+    if (R <= 8) DT_CORE_NORM(1);
+    else if (R <= 16) DT_CORE_NORM(2);
+    else if (R <= 24) DT_CORE_NORM(3);
+    else DT_CORE_NORM(4);
+#undef DT_CORE_NORM
 }
 
 }  // namespace dt

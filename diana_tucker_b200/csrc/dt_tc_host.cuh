@@ -74,11 +74,11 @@ void split_f32_chunks(dt_ctx *ctx, const ChunkedUpload &up, __nv_bfloat16 *hi,
 void split_f32(dt_ctx *ctx, const float *x, int64_t n, __nv_bfloat16 *hi, __nv_bfloat16 *lo,
                double *sumsq_out);
 
-// G[k + K*r] = sum_i Y[i*K + k] U[i + I*r] (FP64 accumulate), ||G||^2 -> g2_out.
-// `scratch` (core_rows_scratch_bytes) holds the per-block partial sums; NULL
-// takes a stream-ordered allocation.
-void core_rows(dt_ctx *ctx, const __nv_bfloat16 *Yh, const __nv_bfloat16 *Yl, int64_t I, int64_t K,
-               const double *U, int64_t R, double *G, double *g2_out, void *scratch = nullptr);
-size_t core_rows_scratch_bytes(int64_t K);
+// ||G||^2 -> g2_out, G[k + K*r] = sum_i Y[i*K + k] U[i + I*r] (FP64 accumulate).
+// `scratch` (core_norm_scratch_bytes) holds the CTAs' sums, `counter` is zero and
+// left so.
+void core_norm(dt_ctx *ctx, const __nv_bfloat16 *Yh, const __nv_bfloat16 *Yl, int64_t I, int64_t K,
+               const double *U, int64_t R, double *g2_out, void *scratch, int *counter);
+size_t core_norm_scratch_bytes(int64_t K);
 
 }  // namespace dt
