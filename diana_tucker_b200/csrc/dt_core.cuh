@@ -53,10 +53,11 @@ struct dt_ctx {
     static constexpr size_t kBigStageBytes = size_t(32) << 20;
     void *big_stage = nullptr;
     size_t big_stage_cap = 0;
-    // The dense HOOI drivers' last plans (device buffers plus a captured graph
-    // of one sweep), reused by the next call with the same shapes, ranks and
-    // options; released before the stream at dt_ctx_destroy.
-    std::shared_ptr<void> hooi_plan_fp64, hooi_plan_mixed;
+    // The dense HOOI drivers' last plans (device buffers plus captured sweeps;
+    // two of the FP64 driver's), reused by the next call with the same shapes,
+    // ranks and options; released before the stream at dt_ctx_destroy.
+    std::vector<std::shared_ptr<void>> hooi_plans_fp64;
+    std::shared_ptr<void> hooi_plan_mixed;
     // The batched HOOI's tuned configurations, instantiated graphs and
     // device-resident argument block (dt_hooi_batched).
     std::shared_ptr<void> batched;

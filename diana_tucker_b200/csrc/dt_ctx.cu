@@ -502,7 +502,7 @@ int dt_ctx_destroy(dt_ctx *ctx) {
         cudaSetDevice(ctx->device);
         detach_sptensors(ctx);
         if (ctx->stream) cudaStreamSynchronize(ctx->stream);
-        ctx->hooi_plan_fp64.reset();
+        ctx->hooi_plans_fp64.clear();
         ctx->hooi_plan_mixed.reset();
         ctx->batched.reset();
         ctx->summary.reset();

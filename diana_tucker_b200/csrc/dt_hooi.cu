@@ -388,19 +388,33 @@ void DenseHooi::init_factors(double *const *U_user, double *const *dst) {
                                 cudaMemcpyHostToDevice, ctx->stream));
         DT_CUDA(cudaStreamSynchronize(ctx->stream));  // `all` goes out of scope
     }
-    int64_t off = 0;
+    // The modes' Grams first, then all subspace iterations in one launch: each is
+    // a chain of small steps on a few SMs.
+    int64_t sn = 0, wn = 0, off = 0, soff = 0, woff = 0;
+    for (int m = 0; m < N; m++) {
+        sn += I[m] * I[m];
+        wn += 3 * I[m] * R[m] + R[m] + 64;
+    }
+    DevMem Sall(ctx, sn * sizeof(double)), wall(ctx, wn * sizeof(double));
+    const double *Sp[16];
+    double *Lp[16], *wp[16];
     for (int m = 0; m < N; m++) {
         int64_t L = 1, B = 1;
         for (int k = 0; k < m; k++) L *= I[k];
         for (int k = m + 1; k < N; k++) B *= I[k];
-        ttt_f64(ctx, X64p, X64p, L, I[m], I[m], B, S.as<double>());
+        double *Sm = Sall.as<double>() + soff;
+        ttt_f64(ctx, X64p, X64p, L, I[m], I[m], B, Sm);
         DT_CUDA(cudaMemcpyAsync(out(m), hosvd_start.as<double>() + off,
                                 I[m] * R[m] * sizeof(double), cudaMemcpyDeviceToDevice,
                                 ctx->stream));
+        Sp[m] = Sm;
+        Lp[m] = out(m);
+        wp[m] = wall.as<double>() + woff;
         off += I[m] * R[m];
-        subspace_iter(ctx, S.as<double>(), I[m], out(m), R[m], hosvd_iters, work.as<double>(),
-                      flag.as<int>());
+        soff += I[m] * I[m];
+        woff += 3 * I[m] * R[m] + R[m] + 64;
     }
+    subspace_iter_batch(ctx, N, Sp, I, Lp, R, hosvd_iters, wp, flag.as<int>());
 }
 
 // The two passes over X of a sweep: each half of the dimension tree first
@@ -665,13 +679,28 @@ int dt_hooi_dense(dt_ctx *ctx, const void *X, int dtype, int ndim, const int64_t
         SummaryScope sc(ctx, "Algorithm::Tucker::HOOI_ALS()");
         if (o.precision == DT_PREC_FP64) {
             // A staged host X lives only for this call: its plan is not kept
-            // and its sweeps are launched directly.
+            // and its sweeps are launched directly.  The two plans used last
+            // are kept, the later one in front (a program often alternates
+            // between a tensor and its sketch).
             const bool keep = x.ptr() == X;
-            auto plan = std::static_pointer_cast<Fp64Plan>(ctx->hooi_plan_fp64);
-            if (!keep || !plan || !plan->matches(x.ptr(), dtype, ndim, shape, ranks, o)) {
-                if (keep) release_plan(ctx, ctx->hooi_plan_fp64);
+            std::shared_ptr<Fp64Plan> plan;
+            auto &kept = ctx->hooi_plans_fp64;
+            for (size_t k = 0; keep && k < kept.size(); k++) {
+                auto p = std::static_pointer_cast<Fp64Plan>(kept[k]);
+                if (!p->matches(x.ptr(), dtype, ndim, shape, ranks, o)) continue;
+                std::rotate(kept.begin(), kept.begin() + k, kept.begin() + k + 1);
+                plan = p;
+                break;
+            }
+            if (!plan) {
                 plan = std::make_shared<Fp64Plan>(x.ptr(), dtype, ndim, shape, ranks, o);
-                if (keep) ctx->hooi_plan_fp64 = plan;
+                if (keep) {
+                    if (kept.size() >= 2) {
+                        release_plan(ctx, kept.back());
+                        kept.pop_back();
+                    }
+                    kept.insert(kept.begin(), plan);
+                }
             }
             plan->h.setup(ctx, x.ptr(), dtype, ndim, shape, ranks, o);
             plan->h.run(G, U, report, keep ? &plan->loop : nullptr);

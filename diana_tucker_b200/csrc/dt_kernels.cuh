@@ -60,6 +60,12 @@ void orth_batch(dt_ctx *ctx, int count, const double *const *A, double *const *Q
 void subspace_iter(dt_ctx *ctx, const double *S, int64_t n, double *L, int64_t r, int iters,
                    double *work, int *flag);
 
+// The same for `count` independent problems, side by side in one launch where
+// the tiled kernel takes them (n <= 256, r <= 32).
+void subspace_iter_batch(dt_ctx *ctx, int count, const double *const *S, const int64_t *n,
+                         double *const *L, const int64_t *r, int iters, double *const *work,
+                         int *flag);
+
 // LU inverse with partial pivoting (one CTA).  *flag = 1 on a zero pivot.
 void lu_inverse(dt_ctx *ctx, const double *A, int64_t n, double *Ainv, double *work,
                 int *flag);

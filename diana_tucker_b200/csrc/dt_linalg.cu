@@ -713,12 +713,22 @@ __host__ inline size_t sub_smem_bytes(int n, int c, bool s_in_smem, int bufs) {
     return d * sizeof(double);
 }
 
+// Independent problems of one launch, a cluster each.
+constexpr int SUB_MAX = 8;
+struct SubBatch {
+    const double *S[SUB_MAX];
+    double *L[SUB_MAX], *work[SUB_MAX];
+    int n[SUB_MAX], r[SUB_MAX];
+};
+
 template <int RT, bool SSM>
-__global__ void __launch_bounds__(SM_NT, 1) subspace_cluster_kernel(const double *Sg, int n,
-                                                                    double *Lg, int r, int iters,
-                                                                    double *work, int *flag,
-                                                                    int csize, int bufs) {
+__global__ void __launch_bounds__(SM_NT, 1) subspace_cluster_kernel(SubBatch batch, int iters,
+                                                                    int *flag, int csize, int bufs) {
     using T = SmTile<RT>;
+    const int prob = blockIdx.x / csize;
+    const double *const Sg = batch.S[prob];
+    double *const Lg = batch.L[prob], *const work = batch.work[prob];
+    const int n = batch.n[prob], r = batch.r[prob];
     extern __shared__ __align__(16) double sm[];
     __shared__ double red[33];
     __shared__ __align__(8) uint64_t bars[2];
@@ -934,18 +944,17 @@ __global__ void __launch_bounds__(SM_NT, 1) cholqr2_batch_kernel(OrthTable tab) 
 }
 
 template <int RT, bool SSM>
-void launch_subspace(dt_ctx *ctx, const double *S, int n, double *L, int r, int iters,
-                     double *work, int *flag, int csize, int bufs) {
+void launch_subspace(dt_ctx *ctx, const SubBatch &batch, int count, int n, int iters, int *flag,
+                     int csize, int bufs) {
     const size_t smem = sub_smem_bytes<RT>(n, csize, SSM, bufs);
     auto kern = subspace_cluster_kernel<RT, SSM>;
     smem_limit(ctx, kern, smem);
-    launch_pdl_cluster(ctx, kern, csize, SM_NT, smem, csize, S, n, L, r, iters, work, flag, csize,
-                       bufs);
+    launch_pdl_cluster(ctx, kern, count * csize, SM_NT, smem, csize, batch, iters, flag, csize, bufs);
 }
 
+// `count` problems of up to n rows.
 template <int RT>
-void subspace_mma(dt_ctx *ctx, const double *S, int n, double *L, int r, int iters,
-                  double *work, int *flag) {
+void subspace_mma(dt_ctx *ctx, const SubBatch &batch, int count, int n, int iters, int *flag) {
     const size_t cap = 220 * 1024;
     // Up to 64 rows one CTA: an exchange costs more than the part of a product
     // it saves (64 x 8, 5 steps: 13.6 us on one CTA, 14.8 on eight).  Above,
@@ -955,11 +964,22 @@ void subspace_mma(dt_ctx *ctx, const double *S, int n, double *L, int r, int ite
     // and 112 us for 256 x 12 with S read from L2 (37 here).
     const int c = n <= 64 ? 1 : 8;
     if (sub_smem_bytes<RT>(n, c, true, 3) <= cap)
-        launch_subspace<RT, true>(ctx, S, n, L, r, iters, work, flag, c, 3);
+        launch_subspace<RT, true>(ctx, batch, count, n, iters, flag, c, 3);
     else if (sub_smem_bytes<RT>(n, c, true, 2) <= cap)
-        launch_subspace<RT, true>(ctx, S, n, L, r, iters, work, flag, c, 2);
+        launch_subspace<RT, true>(ctx, batch, count, n, iters, flag, c, 2);
     else  // r > 16 and n > 230 or so: S stays in L2
-        launch_subspace<RT, false>(ctx, S, n, L, r, iters, work, flag, c, 2);
+        launch_subspace<RT, false>(ctx, batch, count, n, iters, flag, c, 2);
+}
+
+void subspace_mma(dt_ctx *ctx, const SubBatch &batch, int count, int iters, int *flag) {
+    int n = 0, r = 0;
+    for (int b = 0; b < count; b++) {
+        n = std::max(n, batch.n[b]);
+        r = std::max(r, batch.r[b]);
+    }
+    if (r <= 8) subspace_mma<8>(ctx, batch, count, n, iters, flag);
+    else if (r <= 16) subspace_mma<16>(ctx, batch, count, n, iters, flag);
+    else subspace_mma<32>(ctx, batch, count, n, iters, flag);
 }
 
 // Subspace iteration for ranks above 32: Householder QR every step, S, L and Z
@@ -1281,12 +1301,13 @@ void subspace_iter(dt_ctx *ctx, const double *S, int64_t n, double *L, int64_t r
         return;
     }
     if (n <= 256) {
-        if (r <= 8)
-            subspace_mma<8>(ctx, S, (int)n, L, (int)r, iters, work, flag);
-        else if (r <= 16)
-            subspace_mma<16>(ctx, S, (int)n, L, (int)r, iters, work, flag);
-        else
-            subspace_mma<32>(ctx, S, (int)n, L, (int)r, iters, work, flag);
+        SubBatch one{};
+        one.S[0] = S;
+        one.L[0] = L;
+        one.work[0] = work;
+        one.n[0] = (int)n;
+        one.r[0] = (int)r;
+        subspace_mma(ctx, one, 1, iters, flag);
         return;
     }
     const size_t base = 2 * r * r * sizeof(double);
@@ -1314,6 +1335,31 @@ void subspace_iter(dt_ctx *ctx, const double *S, int64_t n, double *L, int64_t r
         DT_LAUNCH(ctx, subspace_kernel<32>, 1, LA_NT, smem, S, n, L, r, iters, work, s_mode,
                   zl_in, flag);
     }
+}
+
+void subspace_iter_batch(dt_ctx *ctx, int count, const double *const *S, const int64_t *n,
+                         double *const *L, const int64_t *r, int iters, double *const *work,
+                         int *flag) {
+    SubBatch batch{};
+    int k = 0;
+    for (int b = 0; b < count; b++) {
+        DT_CHECK_ARG(n[b] >= r[b] && r[b] > 0, "subspace_iter: bad sizes n=%lld r=%lld",
+                     (long long)n[b], (long long)r[b]);
+        if (n[b] > 256 || r[b] > 32) {
+            subspace_iter(ctx, S[b], n[b], L[b], r[b], iters, work[b], flag);
+            continue;
+        }
+        batch.S[k] = S[b];
+        batch.L[k] = L[b];
+        batch.work[k] = work[b];
+        batch.n[k] = (int)n[b];
+        batch.r[k] = (int)r[b];
+        if (++k == SUB_MAX) {
+            subspace_mma(ctx, batch, k, iters, flag);
+            k = 0;
+        }
+    }
+    if (k) subspace_mma(ctx, batch, k, iters, flag);
 }
 
 void lu_inverse(dt_ctx *ctx, const double *A, int64_t n, double *Ainv, double *work,

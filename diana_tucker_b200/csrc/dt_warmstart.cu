@@ -329,25 +329,38 @@ int dt_ws_init(dt_ctx *ctx, const void *X, int dtype, int ndim, const int64_t *s
         sumsq(ctx, a.get(), DT_F64, csize, scal.as<double>() + 1);
         // Leading eigenvectors of each sketch unfolding's Gram, decoded by Q.
         DT_CHECK_ARG(sketch_sweeps >= 0, "dt_ws_init: sketch_sweeps must be >= 0");
-        DevMem S(ctx, (size_t)k * k * sizeof(double));
-        DevMem work(ctx, (3 * (size_t)k * k + k + 64) * sizeof(double)), flag(ctx, sizeof(int));
+        // The modes are independent: their Grams first, one upload of the starts,
+        // then all iterations in one launch.
+        const size_t wlen = 3 * (size_t)k * k + k + 64;
+        DevMem S(ctx, (size_t)ndim * k * k * sizeof(double));
+        DevMem work(ctx, ndim * wlen * sizeof(double)), flag(ctx, sizeof(int));
         DT_CUDA(cudaMemsetAsync(flag.get(), 0, sizeof(int), ctx->stream));
-        std::vector<DevMem> Vm(ndim);
+        std::vector<double> starts;
+        size_t voff[8], vlen = 0;
+        for (int m = 0; m < ndim; m++) {
+            HostGauss g(0x5EED0000ull + (uint64_t)m);
+            voff[m] = vlen;
+            vlen += (size_t)k * ranks[m];
+            while (starts.size() < vlen) starts.push_back(g.normal());
+        }
+        DevMem Vm(ctx, vlen * sizeof(double));
+        DT_CUDA(cudaMemcpyAsync(Vm.get(), starts.data(), vlen * sizeof(double),
+                                cudaMemcpyHostToDevice, ctx->stream));
+        const double *Sp[8];
+        double *vp[8], *wp[8];
+        int64_t ks[8];
         for (int m = 0; m < ndim; m++) {
             int64_t L = 1, B = 1;
             for (int p = 0; p < m; p++) L *= k;
             for (int p = m + 1; p < ndim; p++) B *= k;
-            ttt_f64(ctx, a.as<double>(), a.as<double>(), L, k, k, B, S.as<double>());
-            HostGauss g(0x5EED0000ull + (uint64_t)m);
-            std::vector<double> hv((size_t)k * ranks[m]);
-            for (auto &v : hv) v = g.normal();
-            Vm[m].alloc(ctx, hv.size() * sizeof(double));
-            DT_CUDA(cudaMemcpyAsync(Vm[m].get(), hv.data(), hv.size() * sizeof(double),
-                                    cudaMemcpyHostToDevice, ctx->stream));
-            subspace_iter(ctx, S.as<double>(), k, Vm[m].as<double>(), ranks[m], 60,
-                          work.as<double>(), flag.as<int>());
-            DT_CUDA(cudaStreamSynchronize(ctx->stream));  // the host start is reused
+            double *Sm = S.as<double>() + (size_t)m * k * k;
+            ttt_f64(ctx, a.as<double>(), a.as<double>(), L, k, k, B, Sm);
+            Sp[m] = Sm;
+            vp[m] = Vm.as<double>() + voff[m];
+            wp[m] = work.as<double>() + m * wlen;
+            ks[m] = k;
         }
+        subspace_iter_batch(ctx, ndim, Sp, ks, vp, ranks, 60, wp, flag.as<int>());
         // HOOI on the sketch: the best rank-R Tucker factors inside span(Q).
         if (sketch_sweeps > 0) {
             dt_hooi_opts o;
@@ -355,8 +368,6 @@ int dt_ws_init(dt_ctx *ctx, const void *X, int dtype, int ndim, const int64_t *s
             o.init = DT_INIT_GIVEN;
             o.max_sweeps = sketch_sweeps;
             o.tol = 1e-14;
-            double *vp[8];
-            for (int m = 0; m < ndim; m++) vp[m] = Vm[m].as<double>();
             if (dt_hooi_dense(ctx, a.get(), DT_F64, ndim, cur, ranks, &o, nullptr, vp, nullptr) !=
                 DT_OK)
                 fail(DT_ERR_CUDA, std::string("dt_ws_init: sketch HOOI failed: ") + dt_last_error());
@@ -365,7 +376,7 @@ int dt_ws_init(dt_ctx *ctx, const void *X, int dtype, int ndim, const int64_t *s
         uv.reserve(ndim);
         for (int m = 0; m < ndim; m++) {
             uv.emplace_back(ctx, U[m], (size_t)n * ranks[m] * sizeof(double), false, true);
-            gemm_f64(ctx, 0, 0, n, ranks[m], k, Q.as<double>(), n, Vm[m].as<double>(), k,
+            gemm_f64(ctx, 0, 0, n, ranks[m], k, Q.as<double>(), n, vp[m], k,
                      uv.back().as<double>(), n, 0.0);
         }
         // Fit of the initial factors: |X x_m U_m^T|^2.
