@@ -455,13 +455,13 @@ __device__ __forceinline__ void hooi_one(const BatchArgs &a, int t, int slot, do
             ggram(ys, I, K, py, ps, g);
             gsubspace(ys, I, ps, n ? uo + us : uo, n ? R1 : R0, a.inner, g);
         }
-        // Mode 3 from X: T2 = X x_1 U0^T (R0 x I1 x I2), rows (i1, i2), then
-        // Y_(3)[i2, r0 + R0 r1] = sum_i1 T2[r0, i1, i2] U1[i1, r1], rows r0.
-        contract<float>(X, I12, I0, 1, 0, I0, 1, uo, T, R0, 1, 0, R0, g);
+        // Mode 3 from X: T2[i1, i2, r0] = X x_1 U0^T, rows (i1, i2), then
+        // Y_(3)[i2, r0 + R0 r1] = sum_i1 T2[i1, i2, r0] U1[i1, r1], rows i2.
+        contract<float>(X, I12, I0, 1, 0, I0, 1, uo, T, 1, I12, 0, R0, g);
         gsync(g);
         const int K = R0 * R1, py = pitch16(K);
         zero_pads(YS, I2, K, py, g);
-        contract<double>(T, R0, 1, I2, R0 * I1, I1, R0, uo + us, YS, 1, R0, py, R1, g);
+        contract<double>(T, I2, I1, R0, I12, I1, 1, uo + us, YS, py, R0, 1, R1, g);
         gsync(g);
         if (sw == a.sweeps - 1)
             for (int e = g.lt; e < I2 * K; e += g.gs) Ylast[e] = YS[(e % I2) * py + e / I2];
