@@ -48,6 +48,9 @@ struct dt_ctx {
     // and synchronises once (allocated on first use).
     static constexpr size_t kHostStageBytes = 4096;
     void *host_stage = nullptr;
+    // Pinned staging of a call's host outputs (OutBlocks; on first use).
+    static constexpr size_t kOutStageBytes = size_t(1) << 20;
+    void *out_stage = nullptr;
     // Pinned staging for large transfers of pageable host memory (upload_pieces /
     // download_pieces): as large as the largest so far, at most kBigStageBytes.
     static constexpr size_t kBigStageBytes = size_t(32) << 20;
@@ -356,13 +359,30 @@ struct ChunkedUpload {
 // synchronises once after its last copy.
 void copy_out(dt_ctx *ctx, void *user, const void *src, size_t bytes);
 
-// Queues n block copies on ctx->stream: one kernel launch when every
-// destination is device memory and every address and size is a multiple of
-// 8 bytes, else one copy_out per block.  Null destinations are skipped; at
-// most kMaxCopyBlocks blocks.
-constexpr int kMaxCopyBlocks = 17;
-void copy_blocks(dt_ctx *ctx, int n, void *const *dst, const void *const *src,
-                 const size_t *bytes);
+// A call's block copies out of device memory, in one kernel launch on
+// ctx->stream: destinations are device memory of the context's GPU, the
+// context's pinned block, or host memory, which the kernel reaches by way of
+// pinned staging.  What does not fit that (another GPU's memory, addresses or
+// sizes that are no multiple of 8 bytes, more than kOutStageBytes for the host)
+// is one copy_out per block.  At most kMaxCopyBlocks blocks.
+constexpr int kMaxCopyBlocks = 20;
+class OutBlocks {
+   public:
+    explicit OutBlocks(dt_ctx *ctx) : ctx_(ctx) {}
+    // Null destinations are skipped.
+    void add(void *dst, const void *src, size_t bytes);
+    void queue();
+    // After the stream was synchronised: the host's blocks get their bytes.
+    void finish();
+
+   private:
+    dt_ctx *ctx_;
+    int n_ = 0;
+    void *dst_[kMaxCopyBlocks];
+    const void *src_[kMaxCopyBlocks];
+    size_t bytes_[kMaxCopyBlocks];
+    const void *stage_[kMaxCopyBlocks] = {};  // where a host block waits
+};
 
 // The context's pinned read-back block (dt_ctx::kHostStageBytes bytes).
 void *host_stage(dt_ctx *ctx);

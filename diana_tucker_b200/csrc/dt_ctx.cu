@@ -279,50 +279,80 @@ __global__ void copy_blocks_kernel(BlockList b) {
         for (long long i = t; i < b.words[k]; i += stride) b.dst[k][i] = b.src[k][i];
 }
 
-// Device (or managed) memory of the context's own GPU: a kernel there may
-// store to it without peer access.
-bool is_local_device_ptr(const dt_ctx *ctx, const void *p) {
+// How a kernel on the context's GPU may store to p: directly (device or managed
+// memory of that GPU), by way of the host (host memory), or not at all.
+enum class Reach { Direct, Host, No };
+
+Reach reach(const dt_ctx *ctx, const void *p) {
     cudaPointerAttributes attr;
     if (cudaPointerGetAttributes(&attr, p) != cudaSuccess) {
         cudaGetLastError();
-        return false;
+        return Reach::No;
     }
-    return (attr.type == cudaMemoryTypeDevice || attr.type == cudaMemoryTypeManaged) &&
-           attr.device == ctx->device;
+    if (attr.type == cudaMemoryTypeUnregistered || attr.type == cudaMemoryTypeHost)
+        return Reach::Host;
+    return attr.device == ctx->device ? Reach::Direct : Reach::No;
 }
 
 }  // namespace
 
-void copy_blocks(dt_ctx *ctx, int n, void *const *dst, const void *const *src,
-                 const size_t *bytes) {
-    DT_CHECK_ARG(n >= 0 && n <= kMaxCopyBlocks, "copy_blocks: %d blocks", n);
+void OutBlocks::add(void *dst, const void *src, size_t bytes) {
+    if (!dst || bytes == 0) return;
+    DT_CHECK_ARG(n_ < kMaxCopyBlocks, "OutBlocks: more than %d blocks", kMaxCopyBlocks);
+    dst_[n_] = dst;
+    src_[n_] = src;
+    bytes_[n_++] = bytes;
+}
+
+// A copy into pageable memory holds the calling thread for ~12 us each, and one
+// into pinned memory costs its own slot on the stream; the kernel stores to
+// pinned memory across PCIe, in order with the rest of its blocks.
+void OutBlocks::queue() {
     BlockList b{};
-    bool one_launch = true;
+    size_t staged = 0;
     long long most = 0;
-    for (int k = 0; k < n; k++) {
-        if (!dst[k] || bytes[k] == 0) continue;
-        const bool aligned = (reinterpret_cast<uintptr_t>(dst[k]) | reinterpret_cast<uintptr_t>(src[k]) |
-                              bytes[k]) % 8 == 0;
-        if (!aligned || !is_local_device_ptr(ctx, dst[k])) {
-            one_launch = false;
-            break;
+    bool one_launch = true;
+    for (int k = 0; k < n_ && one_launch; k++) {
+        void *to = dst_[k];
+        one_launch = (reinterpret_cast<uintptr_t>(src_[k]) | bytes_[k]) % 8 == 0;
+        const size_t at = static_cast<char *>(to) - static_cast<char *>(ctx_->host_stage);
+        if (!ctx_->host_stage || at >= dt_ctx::kHostStageBytes) {
+            const Reach r = reach(ctx_, to);
+            if (r == Reach::Host) {
+                if (staged + bytes_[k] > dt_ctx::kOutStageBytes) one_launch = false;
+                if (!one_launch) break;
+                if (!ctx_->out_stage)
+                    DT_CUDA(cudaHostAlloc(&ctx_->out_stage, dt_ctx::kOutStageBytes,
+                                          cudaHostAllocDefault));
+                stage_[k] = to = static_cast<char *>(ctx_->out_stage) + staged;
+                staged += bytes_[k];
+            } else if (r == Reach::No || reinterpret_cast<uintptr_t>(to) % 8 != 0) {
+                one_launch = false;
+            }
         }
-        b.src[b.count] = static_cast<const unsigned long long *>(src[k]);
-        b.dst[b.count] = static_cast<unsigned long long *>(dst[k]);
-        b.words[b.count] = (long long)(bytes[k] / 8);
-        most = std::max(most, b.words[b.count]);
-        b.count++;
+        b.src[k] = static_cast<const unsigned long long *>(src_[k]);
+        b.dst[k] = static_cast<unsigned long long *>(to);
+        b.words[k] = (long long)(bytes_[k] / 8);
+        most = std::max(most, b.words[k]);
     }
     if (!one_launch) {
-        for (int k = 0; k < n; k++)
-            if (dst[k]) copy_out(ctx, dst[k], src[k], bytes[k]);
+        for (int k = 0; k < n_; k++) {
+            stage_[k] = nullptr;
+            copy_out(ctx_, dst_[k], src_[k], bytes_[k]);
+        }
         return;
     }
-    if (b.count == 0) return;
+    if (n_ == 0) return;
+    b.count = n_;
     const int threads = 256;
     const long long want = (most + threads - 1) / threads;
-    const unsigned blocks = (unsigned)std::max(1LL, std::min<long long>(want, 2LL * ctx->num_sms));
-    DT_LAUNCH(ctx, copy_blocks_kernel, blocks, threads, 0, b);
+    const unsigned blocks = (unsigned)std::max(1LL, std::min<long long>(want, 2LL * ctx_->num_sms));
+    DT_LAUNCH(ctx_, copy_blocks_kernel, blocks, threads, 0, b);
+}
+
+void OutBlocks::finish() {
+    for (int k = 0; k < n_; k++)
+        if (stage_[k]) std::memcpy(dst_[k], stage_[k], bytes_[k]);
 }
 
 namespace {
@@ -517,6 +547,7 @@ int dt_ctx_destroy(dt_ctx *ctx) {
         }
         if (ctx->own_stream) cudaStreamDestroy(ctx->own_stream);
         if (ctx->host_stage) cudaFreeHost(ctx->host_stage);
+        if (ctx->out_stage) cudaFreeHost(ctx->out_stage);
         if (ctx->big_stage) cudaFreeHost(ctx->big_stage);
         delete ctx;
     });

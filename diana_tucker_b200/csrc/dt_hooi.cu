@@ -321,17 +321,13 @@ void DenseHooi::init_factors(double *const *U_user, double *const *dst) {
             // The same seed draws the same factors: copy the orthonormal ones
             // kept from the first call (the draws take ~0.1-0.5 ms of host time),
             // all modes in one launch.
-            void *d[16];
-            const void *src[16];
-            size_t bytes[16];
+            OutBlocks blocks(ctx);
             int64_t off = 0;
             for (int m = 0; m < N; m++) {
-                d[m] = out(m);
-                src[m] = init_cache.as<double>() + off;
-                bytes[m] = I[m] * R[m] * sizeof(double);
+                blocks.add(out(m), init_cache.as<double>() + off, I[m] * R[m] * sizeof(double));
                 off += I[m] * R[m];
             }
-            copy_blocks(ctx, N, d, src, bytes);
+            blocks.queue();
             return;
         }
         // Draw every block in mode order (the reference's order), upload once,
@@ -535,32 +531,21 @@ void DenseHooi::run(double *G_user, double *const *U_user, dt_hooi_report *rep,
         sumsq(ctx, G.get(), DT_F64, prod(R, N), scal.as<double>() + 1);
     }
     DT_CUDA(cudaEventRecord(ctx->ev_stop, ctx->stream));
-    // The outputs go straight from the plan's buffers into the caller's (host
-    // or device), queued with the read-back of ||G||^2: one synchronisation.
-    {
-        void *dst[kMaxCopyBlocks];
-        const void *src[kMaxCopyBlocks];
-        size_t bytes[kMaxCopyBlocks];
-        dst[0] = G_user;
-        src[0] = G.get();
-        bytes[0] = prod(R, N) * sizeof(double);
-        for (int m = 0; m < N; m++) {
-            dst[1 + m] = U_user ? U_user[m] : nullptr;
-            src[1 + m] = U[m].get();
-            bytes[1 + m] = I[m] * R[m] * sizeof(double);
-        }
-        copy_blocks(ctx, 1 + N, dst, src, bytes);
-    }
-    // ||X||^2, ||G||^2 and the loop's sweep count and residuals.
+    // The outputs go from the plan's buffers into the caller's (host or device)
+    // with ||X||^2, ||G||^2 and the loop's sweep count and residuals: one launch
+    // and one synchronisation.
     constexpr size_t kLoopAt = 64;
     static_assert(kLoopAt + sizeof(LoopState) <= dt_ctx::kHostStageBytes, "stage too small");
     char *st = static_cast<char *>(host_stage(ctx));
-    DT_CUDA(cudaMemcpyAsync(st, scal.as<double>(), 2 * sizeof(double), cudaMemcpyDeviceToHost,
-                            ctx->stream));
-    if (device_loop)
-        DT_CUDA(cudaMemcpyAsync(st + kLoopAt, loop->state(ctx), sizeof(LoopState),
-                                cudaMemcpyDeviceToHost, ctx->stream));
+    OutBlocks outs(ctx);
+    outs.add(st, scal.get(), 2 * sizeof(double));
+    if (device_loop) outs.add(st + kLoopAt, loop->state(ctx), sizeof(LoopState));
+    outs.add(G_user, G.get(), prod(R, N) * sizeof(double));
+    for (int m = 0; U_user && m < N; m++)
+        outs.add(U_user[m], U[m].get(), I[m] * R[m] * sizeof(double));
+    outs.queue();
     DT_CUDA(cudaStreamSynchronize(ctx->stream));
+    outs.finish();
     double xg[2];
     std::memcpy(xg, st, sizeof(xg));
     x2 = xg[0];

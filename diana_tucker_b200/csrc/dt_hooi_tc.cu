@@ -451,35 +451,21 @@ struct MixedHooi {
         // buffers) before the one synchronisation that reads ||X||^2 and
         // ||G||^2, the kernels' error word and the device loop's sweep count
         // and residuals (all into the context's pinned block).
-        {
-            void *dst[kMaxCopyBlocks];
-            const void *src[kMaxCopyBlocks];
-            size_t bytes[kMaxCopyBlocks];
-            dst[0] = G_user;
-            src[0] = gsrc;
-            bytes[0] = prod(R, N) * sizeof(double);
-            for (int m = 0; m < N; m++) {
-                dst[1 + m] = U_user ? U_user[m] : nullptr;
-                src[1 + m] = U[m].get();
-                bytes[1 + m] = I[m] * R[m] * sizeof(double);
-            }
-            copy_blocks(ctx, 1 + N, dst, src, bytes);
-        }
+        OutBlocks outs(ctx);
+        outs.add(G_user, gsrc, prod(R, N) * sizeof(double));
+        for (int m = 0; U_user && m < N; m++)
+            outs.add(U_user[m], U[m].get(), I[m] * R[m] * sizeof(double));
         constexpr size_t kErrAt = 32, kLoopAt = 64;
         const int noted = fixed ? std::min(sweeps, DT_MAX_HIST) : 0;
         static_assert(kLoopAt + sizeof(LoopState) <= dt_ctx::kHostStageBytes, "stage too small");
         char *st = static_cast<char *>(host_stage(ctx));
-        DT_CUDA(cudaMemcpyAsync(st, scal.as<double>(), (gslot + 1) * sizeof(double),
-                                cudaMemcpyDeviceToHost, ctx->stream));
-        DT_CUDA(cudaMemcpyAsync(st + kErrAt, err.get(), sizeof(int), cudaMemcpyDeviceToHost,
-                                ctx->stream));
-        if (device_loop)
-            DT_CUDA(cudaMemcpyAsync(st + kLoopAt, loop->state(ctx), sizeof(LoopState),
-                                    cudaMemcpyDeviceToHost, ctx->stream));
-        if (noted > 0)
-            DT_CUDA(cudaMemcpyAsync(st + kLoopAt, g2hist.get(), noted * sizeof(double),
-                                    cudaMemcpyDeviceToHost, ctx->stream));
+        outs.add(st, scal.get(), (gslot + 1) * sizeof(double));
+        outs.add(st + kErrAt, err.get(), 2 * sizeof(int));
+        if (device_loop) outs.add(st + kLoopAt, loop->state(ctx), sizeof(LoopState));
+        if (noted > 0) outs.add(st + kLoopAt, g2hist.get(), noted * sizeof(double));
+        outs.queue();
         DT_CUDA(cudaStreamSynchronize(ctx->stream));
+        outs.finish();
         double sc[gslot + 1];
         std::memcpy(sc, st, sizeof(sc));
         const double g2 = sc[gslot];
@@ -595,7 +581,7 @@ void hooi_dense_lowprec(dt_ctx *ctx, const void *X, int dtype, int ndim, const i
         h.S.alloc(ctx, maxI * maxI * sizeof(double));
         h.work.alloc(ctx, (3 * maxI * maxR + maxR + 64) * sizeof(double));
         h.flag.alloc(ctx, sizeof(int));
-        h.err.alloc(ctx, sizeof(int));
+        h.err.alloc(ctx, 2 * sizeof(int));  // read back as one 8-byte word
         h.scal.alloc(ctx, 4 * sizeof(double));
         h.counter.alloc(ctx, sizeof(int));
         DT_CUDA(cudaMemsetAsync(h.counter.get(), 0, sizeof(int), ctx->stream));
@@ -613,7 +599,7 @@ void hooi_dense_lowprec(dt_ctx *ctx, const void *X, int dtype, int ndim, const i
     h.X32 = nullptr;
     h.helper.setup(ctx, X, dtype, ndim, shape, ranks, opts);
     DT_CUDA(cudaMemsetAsync(h.flag.get(), 0, sizeof(int), ctx->stream));
-    DT_CUDA(cudaMemsetAsync(h.err.get(), 0, sizeof(int), ctx->stream));
+    DT_CUDA(cudaMemsetAsync(h.err.get(), 0, 2 * sizeof(int), ctx->stream));
     h.run(X, dtype, G, U, report, upload);
 }
 

@@ -264,3 +264,21 @@ def test_hooi_rejects_bad_ranks(ctx):
     with pytest.raises(DTError) as e:
         ctx.hooi_dense(np.ones((4, 5, 6)), (5, 2, 2))
     assert e.value.code == 1
+
+
+@pytest.mark.parametrize("rows", [7, 6528, 6529])
+def test_hooi_host_outputs_through_the_staging(ctx, rows):
+    """Host outputs are stored by one kernel into 1 MiB of pinned staging and
+    copied from there (6528 rows: 131060 words of 131072), larger ones by one
+    copy each: both are what device outputs hold."""
+    import torch
+    shape, ranks = (rows, 12, 10), (min(rows, 20), 5, 4)
+    X = np.random.default_rng(rows).standard_normal(shape)
+    Xd = torch.from_numpy(X.reshape(-1, order="F").copy()).cuda()
+    kw = dict(init="randn", seed=4, max_sweeps=1, shape=shape)
+    Gd, Ud, repd = ctx.hooi_dense(Xd, ranks, device_out=True, **kw)
+    G, U, rep = ctx.hooi_dense(Xd, ranks, **kw)
+    assert rep["residual"] == repd["residual"]
+    assert np.array_equal(G, Gd.cpu().numpy())
+    for a, b in zip(U, Ud):
+        assert np.array_equal(a, b.cpu().numpy())
