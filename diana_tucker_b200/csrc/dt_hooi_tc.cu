@@ -225,7 +225,7 @@ struct MixedHooi {
         if (dry) return;
         tc_gram(ctx, yh, yl, I[n], K, S.as<double>(), err.as<int>(), gscr);
         subspace_iter(ctx, S.as<double>(), I[n], U[n].as<double>(), R[n], opts.inner_iters,
-                      work.as<double>(), flag.as<int>());
+                      work.as<double>(), flag.as<int>(), true);
         if (n == N - 1)
             core_norm(ctx, yh, yl, I[n], K, U[n].as<double>(), R[n], scal.as<double>() + 1, cscr,
                       counter.as<int>());

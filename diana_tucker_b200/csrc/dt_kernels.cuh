@@ -55,10 +55,11 @@ void orth_batch(dt_ctx *ctx, int count, const double *const *A, double *const *Q
                 const int64_t *m, const int64_t *n);
 
 // Orthonormal basis of span(S^iters L) for the n x n symmetric S and the n x r
-// col-major L (in place), one CTA; CholeskyQR2 per step with a Householder
-// fallback.  work >= 3*n*r + r.  Sets *flag bit 2 when a fallback ran.
+// col-major L (in place); CholeskyQR with a Householder fallback.  work >= 3*n*r
+// + r.  Sets *flag bit 2 when a fallback ran.  plain: round as the plain
+// elimination does (for factors that are rounded to BF16 halves next).
 void subspace_iter(dt_ctx *ctx, const double *S, int64_t n, double *L, int64_t r, int iters,
-                   double *work, int *flag);
+                   double *work, int *flag, bool plain = false);
 
 // The same for `count` independent problems, side by side in one launch where
 // the tiled kernel takes them (n <= 256, r <= 32).

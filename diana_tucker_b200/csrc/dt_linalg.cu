@@ -593,6 +593,30 @@ __device__ __forceinline__ bool sm_chol_inv(double *G, double *Ri, int r) {
     return good != 0;
 }
 
+// The same by warp_chol_linv: the identity is eliminated along with G, with fused
+// products and the hardware's root refined in line.  r = 16: 2200 cycles against
+// 4800, three of them per subspace of 5 steps: 96^4 sweeps 1604 -> 1575 us, 256-cube
+// warm start 1489 -> 1458 us.  For results that stay FP64, where another rounding of
+// the last bit does no harm.
+template <int RT>
+__device__ __forceinline__ bool sm_chol_inv_fused(const double *G, double *Ri, int r) {
+    constexpr int LDR = SmTile<RT>::LDR;
+    __shared__ int good;
+    const int lane = threadIdx.x;
+    if (lane < 32) {
+        double y[RT];
+        const bool ok = warp_chol_linv<RT>(G, RT, r, y);
+        // Lane c holds column c of L^{-1} = row c of R^{-1}.
+        if (lane < RT) {
+#pragma unroll
+            for (int i = 0; i < RT; i++) Ri[lane * LDR + i] = i >= lane ? y[i] : 0.0;
+        }
+        if (lane == 0) good = ok;
+    }
+    __syncthreads();
+    return good != 0;
+}
+
 // After one CholeskyQR pass, Q^T Q = I + E with E tiny.  When max |E| <= 1e-8,
 // C = I - E/2 + 3E^2/8 (the series of (I + E)^{-1/2}) makes Q C orthonormal to
 // rounding; C goes to Ri (pitch LDR) for sm_apply.  Returns false when E is too
@@ -721,7 +745,8 @@ struct SubBatch {
     int n[SUB_MAX], r[SUB_MAX];
 };
 
-template <int RT, bool SSM>
+// PLAIN: the factorisation that rounds as the plain elimination does.
+template <int RT, bool SSM, bool PLAIN>
 __global__ void __launch_bounds__(SM_NT, 1) subspace_cluster_kernel(SubBatch batch, int iters,
                                                                     int *flag, int csize, int bufs) {
     using T = SmTile<RT>;
@@ -842,7 +867,8 @@ __global__ void __launch_bounds__(SM_NT, 1) subspace_cluster_kernel(SubBatch bat
         for (int p = 0; p < (last ? 2 : 1); p++) {
             sm_gram<RT>(z(0), n, r, Gp, G);
             // The second pass is usually a tiny correction (polar fix).
-            if (!(p == 1 && sm_polar_fix<RT>(G, Ri, red)) && !sm_chol_inv<RT>(G, Ri, r)) {
+            if (!(p == 1 && sm_polar_fix<RT>(G, Ri, red)) &&
+                !(PLAIN ? sm_chol_inv<RT>(G, Ri, r) : sm_chol_inv_fused<RT>(G, Ri, r))) {
                 bad = true;  // the same G, so the same answer, in every CTA
                 break;
             }
@@ -945,16 +971,18 @@ __global__ void __launch_bounds__(SM_NT, 1) cholqr2_batch_kernel(OrthTable tab) 
 
 template <int RT, bool SSM>
 void launch_subspace(dt_ctx *ctx, const SubBatch &batch, int count, int n, int iters, int *flag,
-                     int csize, int bufs) {
+                     int csize, int bufs, bool plain) {
     const size_t smem = sub_smem_bytes<RT>(n, csize, SSM, bufs);
-    auto kern = subspace_cluster_kernel<RT, SSM>;
+    auto kern = plain ? subspace_cluster_kernel<RT, SSM, true>
+                      : subspace_cluster_kernel<RT, SSM, false>;
     smem_limit(ctx, kern, smem);
     launch_pdl_cluster(ctx, kern, count * csize, SM_NT, smem, csize, batch, iters, flag, csize, bufs);
 }
 
 // `count` problems of up to n rows.
 template <int RT>
-void subspace_mma(dt_ctx *ctx, const SubBatch &batch, int count, int n, int iters, int *flag) {
+void subspace_mma(dt_ctx *ctx, const SubBatch &batch, int count, int n, int iters, int *flag,
+                  bool plain) {
     const size_t cap = 220 * 1024;
     // Up to 64 rows one CTA: an exchange costs more than the part of a product
     // it saves (64 x 8, 5 steps: 13.6 us on one CTA, 14.8 on eight).  Above,
@@ -964,22 +992,22 @@ void subspace_mma(dt_ctx *ctx, const SubBatch &batch, int count, int n, int iter
     // and 112 us for 256 x 12 with S read from L2 (37 here).
     const int c = n <= 64 ? 1 : 8;
     if (sub_smem_bytes<RT>(n, c, true, 3) <= cap)
-        launch_subspace<RT, true>(ctx, batch, count, n, iters, flag, c, 3);
+        launch_subspace<RT, true>(ctx, batch, count, n, iters, flag, c, 3, plain);
     else if (sub_smem_bytes<RT>(n, c, true, 2) <= cap)
-        launch_subspace<RT, true>(ctx, batch, count, n, iters, flag, c, 2);
+        launch_subspace<RT, true>(ctx, batch, count, n, iters, flag, c, 2, plain);
     else  // r > 16 and n > 230 or so: S stays in L2
-        launch_subspace<RT, false>(ctx, batch, count, n, iters, flag, c, 2);
+        launch_subspace<RT, false>(ctx, batch, count, n, iters, flag, c, 2, plain);
 }
 
-void subspace_mma(dt_ctx *ctx, const SubBatch &batch, int count, int iters, int *flag) {
+void subspace_mma(dt_ctx *ctx, const SubBatch &batch, int count, int iters, int *flag, bool plain) {
     int n = 0, r = 0;
     for (int b = 0; b < count; b++) {
         n = std::max(n, batch.n[b]);
         r = std::max(r, batch.r[b]);
     }
-    if (r <= 8) subspace_mma<8>(ctx, batch, count, n, iters, flag);
-    else if (r <= 16) subspace_mma<16>(ctx, batch, count, n, iters, flag);
-    else subspace_mma<32>(ctx, batch, count, n, iters, flag);
+    if (r <= 8) subspace_mma<8>(ctx, batch, count, n, iters, flag, plain);
+    else if (r <= 16) subspace_mma<16>(ctx, batch, count, n, iters, flag, plain);
+    else subspace_mma<32>(ctx, batch, count, n, iters, flag, plain);
 }
 
 // Subspace iteration for ranks above 32: Householder QR every step, S, L and Z
@@ -1293,7 +1321,7 @@ void orth_batch(dt_ctx *ctx, int count, const double *const *A, double *const *Q
 }
 
 void subspace_iter(dt_ctx *ctx, const double *S, int64_t n, double *L, int64_t r, int iters,
-                   double *work, int *flag) {
+                   double *work, int *flag, bool plain) {
     DT_CHECK_ARG(n >= r && r > 0, "subspace_iter: bad sizes n=%lld r=%lld", (long long)n,
                  (long long)r);
     if (r > 32) {
@@ -1307,7 +1335,7 @@ void subspace_iter(dt_ctx *ctx, const double *S, int64_t n, double *L, int64_t r
         one.work[0] = work;
         one.n[0] = (int)n;
         one.r[0] = (int)r;
-        subspace_mma(ctx, one, 1, iters, flag);
+        subspace_mma(ctx, one, 1, iters, flag, plain);
         return;
     }
     const size_t base = 2 * r * r * sizeof(double);
@@ -1355,11 +1383,11 @@ void subspace_iter_batch(dt_ctx *ctx, int count, const double *const *S, const i
         batch.n[k] = (int)n[b];
         batch.r[k] = (int)r[b];
         if (++k == SUB_MAX) {
-            subspace_mma(ctx, batch, k, iters, flag);
+            subspace_mma(ctx, batch, k, iters, flag, false);
             k = 0;
         }
     }
-    if (k) subspace_mma(ctx, batch, k, iters, flag);
+    if (k) subspace_mma(ctx, batch, k, iters, flag, false);
 }
 
 void lu_inverse(dt_ctx *ctx, const double *A, int64_t n, double *Ainv, double *work,
