@@ -232,13 +232,14 @@ __global__ void __launch_bounds__(256) ttmc_rows_kernel(
 // 3-way fibre TTMc.  The Kronecker index is p = p_lo + R_lo p_hi over the two
 // other modes (lower mode fastest, sp_tensor.tpp:367-417); the warp keeps the
 // current row as TR x TC tiles of 8 x 8 with rows = p_hi and columns = p_lo,
-// so each lane's two accumulators of a tile are adjacent in memory.
+// so each lane's accumulators (two of a tile, or four of two tiles) are adjacent
+// in memory.
 //
 // Layout: every row's (sub-)fibres, longest first, padded to a multiple of 4
 // with empty fibres; four consecutive fibres form a group, the K = 4 slice of
 // one mma.sync step.  Lane (g, t) takes fibre t of the group: it sums
-// w = sum_e v_e U_E(i_E(e), g + 8 j) over its fibre's nonzeros and reads
-// U_F(i_F, g + 8 j) -- exactly its A / B fragment elements -- so the group's
+// w = sum_e v_e U_E(i_E(e), fb_col(g, j)) over its fibre's nonzeros and reads
+// U_F(i_F, fb_col(g, j)) -- exactly its A / B fragment elements -- so the group's
 // four outer products are TF x TE mma.sync steps with no redundant FMAs.
 // FLO: the fibre mode is the lower of the two (columns are p_F), else the
 // higher (rows are p_F).
@@ -253,30 +254,61 @@ __global__ void __launch_bounds__(256) ttmc_rows_kernel(
 //  * batch b: the fibre sums and the mma.sync steps read only shared memory.
 // A row is written when its last group is done (rows of a task are whole,
 // except pieces of long rows, which write a partial row at the task's end).
+//
+// Bound by instruction issue and by the chains between them (16 warps per SM,
+// which is what the stages leave room for): 97 M warp instructions for 4.4 M
+// nonzeros, half of the issue slots used.  250000 x 25000 x 6250, ranks 16, the
+// three modes: 247, 191 and 186 us.  With two 8-byte loads per row, tests of the
+// ranks and of the fibre's length around the loads, and copies in a loop with a
+// branch per four rows it took 282, 215 and 211.
 // ---------------------------------------------------------------------------
 constexpr int FB_NZ = 32;
 constexpr int FB_GRP = 4;
 constexpr int FB_SLOTS = 4 * FB_GRP;
 // One lane per staged nonzero and per fibre slot.
-static_assert(FB_NZ <= 32 && FB_SLOTS <= 32 && 4 * FIB_CHUNK <= FB_NZ, "batch limits");
+static_assert(FB_NZ == 32 && FB_SLOTS <= 32 && 4 * FIB_CHUNK <= FB_NZ, "batch limits");
 constexpr int FB_ROW_END = 1 << 8;  // grp_aux: the group is the last of its row
 
-// A staged factor row of up to 8 T entries has a pitch of 8 T doubles.  Four
-// rows read by one fragment load (8 consecutive doubles each) start in the
-// same bank when the pitch is 16 or 32 doubles, so column c of row j is stored
-// at c ^ fb_swz(j): rows alternate between the two 64-byte halves of a bank
-// cycle (pitch 16) or its four 64-byte quarters (pitch 32).  Pitches 8 and 24
-// alternate by themselves.
+// A staged factor row of up to 8 T entries has a pitch of 8 T doubles.  For an even
+// T, lane group g reads entries 2 g and 2 g + 1 of each 16 in one 16-byte load (the
+// tiles' columns are dealt out that way: tile k's column g is entry fb_col(g, k));
+// for an odd T, entries g + 8 k.  Column c of row j is stored at c ^ fb_swz(j).
+// Even T: the four rows of a load, 8 lanes of it at a time, have to differ in two
+// address bits, for rows 1, 2, 4 or 8 apart (fibres of that length side by side).
+// Odd T: pitches 8 and 24 alternate between the halves of a bank cycle by themselves.
 __host__ __device__ constexpr int fb_pitch(int T) { return 8 * T; }
-__device__ __forceinline__ int fb_swz(int row, int pitch) {
-    return pitch == 16 ? (row & 1) << 3 : pitch == 32 ? (row & 3) << 3 : 0;
+template <int T>
+__device__ __forceinline__ int fb_swz(int row) {
+    return T % 2 == 0 ? ((row ^ (row >> 2) ^ (row >> 4)) & 3) << 2 : 0;
+}
+template <int T>
+__device__ __forceinline__ int fb_col(int g, int k) {
+    return T % 2 == 0 ? 16 * (k / 2) + 2 * g + (k & 1) : 8 * k + g;
+}
+// This lane's T entries of staged row `row`.
+template <int T>
+__device__ __forceinline__ void fb_read(const double *rows, int row, int g, double (&x)[T]) {
+    const double *p = rows + row * fb_pitch(T);
+    const int sw = fb_swz<T>(row);
+    if constexpr (T % 2 == 0) {
+#pragma unroll
+        for (int k = 0; k < T; k += 2) {
+            const double2 v = *reinterpret_cast<const double2 *>(p + (fb_col<T>(g, k) ^ sw));
+            x[k] = v.x;
+            x[k + 1] = v.y;
+        }
+    } else {
+#pragma unroll
+        for (int k = 0; k < T; k++) x[k] = p[fb_col<T>(g, k)];
+    }
 }
 
 template <int TF, int TE>
 struct FbStage {
     static constexpr int PE = fb_pitch(TE), PF = fb_pitch(TF);
     static constexpr int DOUBLES = FB_NZ * PE + FB_SLOTS * PF + FB_NZ;
-    static constexpr int INTS = FB_SLOTS + 1 + 2 * FB_GRP;
+    // The groups' aux words and rows, the slots' words (offset | length << 8).
+    static constexpr int INTS = 2 * FB_GRP + FB_SLOTS;
     static constexpr int BYTES = DOUBLES * 8 + ((INTS * 4 + 15) & ~15);
     static constexpr int WARP_BYTES = 2 * BYTES;
 };
@@ -334,35 +366,37 @@ __host__ __device__ constexpr int fb_pow2(int x) {
     return p;
 }
 
-// Copies n <= 32 rows of the transposed factor U (R <= RMAX doubles each; the
-// index of row j is held by lane j) into dst rows of RMAX doubles, swizzled
+// Copies n <= NMAX <= 32 rows of the transposed factor U (R <= 8 T doubles each;
+// the index of row j is held by lane j) into dst rows of 8 T doubles, swizzled
 // (fb_swz).  Lane l copies piece l % PPR of row l / PPR (+ 32 / PPR per step),
 // PPR a power of two: 16-byte pieces when R is even and U 16-byte aligned,
-// else 8-byte ones.
-template <int RMAX>
+// else 8-byte ones.  The steps are unrolled: the shared addresses differ by
+// constants, and no branch stands between them.
+template <int T, int NMAX>
 __device__ __forceinline__ void fb_stage_rows(double *dst, const double *__restrict__ U, int R,
                                               int n, int ridx, int lane) {
-    constexpr int pitch = RMAX;
+    constexpr int pitch = fb_pitch(T);
     if ((R & 1) == 0 && (reinterpret_cast<uintptr_t>(U) & 15) == 0) {
-        constexpr int PPR = fb_pow2(RMAX / 2), RPI = 32 / PPR;
+        constexpr int PPR = fb_pow2(pitch / 2), RPI = 32 / PPR;
         const int rem = lane % PPR, jl = lane / PPR;
-        const bool okp = 2 * rem < R;
-        for (int j0 = 0; j0 < n; j0 += RPI) {
+        const int left = 2 * rem < R ? n - jl : 0;
+        const double *Up = U + 2 * rem;
+#pragma unroll
+        for (int j0 = 0; j0 < NMAX; j0 += RPI) {
             const int j = j0 + jl;
             const int i = __shfl_sync(0xffffffffu, ridx, j & 31);
-            if (j < n && okp)
-                sp_cp16(dst + j * pitch + ((2 * rem) ^ fb_swz(j, pitch)),
-                        U + (int64_t)i * R + 2 * rem);
+            if (j0 < left)
+                sp_cp16(dst + j * pitch + ((2 * rem) ^ fb_swz<T>(j)), Up + (int64_t)i * R);
         }
     } else {
-        constexpr int PPR = fb_pow2(RMAX), RPI = 32 / PPR;
+        constexpr int PPR = fb_pow2(pitch), RPI = 32 / PPR;
         const int rem = lane % PPR, jl = lane / PPR;
         const bool okp = rem < R;
         for (int j0 = 0; j0 < n; j0 += RPI) {
             const int j = j0 + jl;
             const int i = __shfl_sync(0xffffffffu, ridx, j & 31);
             if (j < n && okp)
-                sp_cp8(dst + j * pitch + (rem ^ fb_swz(j, pitch)), U + (int64_t)i * R + rem);
+                sp_cp8(dst + j * pitch + (rem ^ fb_swz<T>(j)), U + (int64_t)i * R + rem);
         }
     }
 }
@@ -385,20 +419,15 @@ __global__ void __launch_bounds__(256, 2) ttmc3f_kernel(
     const int64_t nw = (int64_t)gridDim.x * nwarp_blk;
     const int P = RF * RE;
     const int Rlo = FLO ? RF : RE, Rhi = FLO ? RE : RF;
-    constexpr int pe = S::PE, pf = S::PF;
-    bool okF[TF], okE[TE];
-#pragma unroll
-    for (int j = 0; j < TF; j++) okF[j] = g + 8 * j < RF;
-#pragma unroll
-    for (int j = 0; j < TE; j++) okE[j] = g + 8 * j < RE;
-    // This lane's two output entries of tile (r, c) in a row: p = pl + Rlo ph
-    // (-1: outside the row).
+    // This lane's output pairs of tile row r in a row of Yc: entries p = pl + Rlo ph,
+    // pl and pl + 1 (-1: outside the row).
     int off[TR][TC];
 #pragma unroll
     for (int r = 0; r < TR; r++)
 #pragma unroll
         for (int c = 0; c < TC; c++) {
-            const int ph = 8 * r + g, pl = 8 * c + 2 * t4;
+            const int ph = fb_col<TR>(g, r);
+            const int pl = TC % 2 == 0 ? 16 * (c / 2) + 4 * t4 + 2 * (c & 1) : 8 * c + 2 * t4;
             off[r][c] = (ph < Rhi && pl < Rlo) ? pl + Rlo * ph : -1;
         }
     const bool pair = (Rlo & 1) == 0;
@@ -406,23 +435,26 @@ __global__ void __launch_bounds__(256, 2) ttmc3f_kernel(
     auto ue_of = [&](int buf) { return reinterpret_cast<double *>(wsm + buf * S::BYTES); };
     auto uf_of = [&](int buf) { return ue_of(buf) + FB_NZ * S::PE; };
     auto vv_of = [&](int buf) { return uf_of(buf) + FB_SLOTS * S::PF; };
-    auto fo_of = [&](int buf) {
+    auto gr_of = [&](int buf) {
         return reinterpret_cast<int *>(wsm + buf * S::BYTES + S::DOUBLES * 8);
     };
+    // Entries beyond the ranks and rows never staged stay zero: the reads need no
+    // test of the ranks.
+    for (int e = lane; e < S::WARP_BYTES / 8; e += 32) reinterpret_cast<double *>(wsm)[e] = 0.0;
+    __syncwarp();
 
     auto stage = [&](const FbMeta &m, int buf) {
-        double *vv = vv_of(buf);
-        int *fo = fo_of(buf);
-        int *gr = fo + FB_SLOTS + 1;
-        if (lane < FB_NZ) vv[lane] = m.v;
-        if (lane < 4 * m.ng) fo[lane] = m.fofs;
-        if (lane == 0) fo[4 * m.ng] = m.nzn;
+        int *gr = gr_of(buf), *fo = gr + 2 * FB_GRP;
+        vv_of(buf)[lane] = m.v;
+        const int nxt = __shfl_down_sync(0xffffffffu, m.fofs, 1);
+        const int end = lane + 1 < 4 * m.ng ? nxt : m.nzn;
+        if (lane < 4 * m.ng) fo[lane] = m.fofs | (end - m.fofs) << 8;
         if (lane < m.ng) {
-            gr[lane] = m.grow;
-            gr[FB_GRP + lane] = m.gaux;
+            gr[lane] = m.gaux;
+            gr[FB_GRP + lane] = m.grow;
         }
-        fb_stage_rows<8 * TE>(ue_of(buf), UE, RE, m.nzn, m.idx, lane);
-        fb_stage_rows<8 * TF>(uf_of(buf), UF, RF, 4 * m.ng, m.fidx, lane);
+        fb_stage_rows<TE, FB_NZ>(ue_of(buf), UE, RE, m.nzn, m.idx, lane);
+        fb_stage_rows<TF, FB_SLOTS>(uf_of(buf), UF, RF, 4 * m.ng, m.fidx, lane);
         sp_cp_commit();
     };
 
@@ -457,57 +489,71 @@ __global__ void __launch_bounds__(256, 2) ttmc3f_kernel(
             }
             __syncwarp();
             const double *ue = ue_of(buf), *uf = uf_of(buf), *vv = vv_of(buf);
-            const int *fo = fo_of(buf);
-            const int *gr = fo + FB_SLOTS + 1;
+            const int *gr = gr_of(buf);
+            const int4 aux4 = *reinterpret_cast<const int4 *>(gr);
+            int fo[FB_GRP];
+#pragma unroll
+            for (int j = 0; j < FB_GRP; j++) fo[j] = gr[2 * FB_GRP + 4 * j + t4];
 #pragma unroll
             for (int j = 0; j < FB_GRP; j++) {
                 if (j >= ng_cur) break;
-                const int s = 4 * j + t4;
-                const int beg = fo[s], len = fo[s + 1] - beg;
-                const int aux = gr[FB_GRP + j];
+                const int beg = fo[j] & 255, len = fo[j] >> 8;
+                const int aux = j == 0 ? aux4.x : j == 1 ? aux4.y : j == 2 ? aux4.z : aux4.w;
                 const int mx = aux & (FB_ROW_END - 1);
-                double w[TE];
+                // The loads stand outside the tests of the fibre's length (a read
+                // past it is of another staged row, not used).
+                double u[TF], w[TE];
+                fb_read<TF>(uf, 4 * j + t4, g, u);
+                {
+                    const int r = min(beg, FB_NZ - 1);
+                    const double v = vv[r];
+                    fb_read<TE>(ue, r, g, w);
 #pragma unroll
-                for (int k = 0; k < TE; k++) w[k] = 0.0;
-                for (int q = 0; q < mx; q++) {
+                    for (int k = 0; k < TE; k++) w[k] = len > 0 ? v * w[k] : 0.0;
+#pragma unroll
+                    for (int k = 0; k < TF; k++) u[k] = len > 0 ? u[k] : 0.0;
+                }
+                for (int q = 1; q < mx; q++) {
+                    const int r = min(beg + q, FB_NZ - 1);
+                    const double v = vv[r];
+                    double x[TE];
+                    fb_read<TE>(ue, r, g, x);
                     if (q < len) {
-                        const int r = beg + q;
-                        const double v = vv[r];
-                        const double *rw = ue + r * pe;
-                        const int sw = fb_swz(r, pe);
 #pragma unroll
-                        for (int k = 0; k < TE; k++)
-                            if (okE[k]) w[k] = fma(v, rw[(g + 8 * k) ^ sw], w[k]);
+                        for (int k = 0; k < TE; k++) w[k] = fma(v, x[k], w[k]);
                     }
                 }
-                double u[TF];
-                const int swf = fb_swz(s, pf);
-#pragma unroll
-                for (int k = 0; k < TF; k++)
-                    u[k] = (okF[k] && len > 0) ? uf[s * pf + ((g + 8 * k) ^ swf)] : 0.0;
 #pragma unroll
                 for (int r = 0; r < TR; r++)
 #pragma unroll
                     for (int c = 0; c < TC; c++)
                         sp_dmma(acc[r][c][0], acc[r][c][1], FLO ? w[r] : u[r], FLO ? u[c] : w[c]);
                 if ((aux & FB_ROW_END) || (b == b1 - 1 && j == ng_cur - 1)) {
-                    double *dst = slot >= 0 ? Ypart + (int64_t)slot * P : Yc + (int64_t)gr[j] * P;
+                    double *dst = slot >= 0 ? Ypart + (int64_t)slot * P
+                                            : Yc + (int64_t)gr[FB_GRP + j] * P;
 #pragma unroll
-                    for (int r = 0; r < TR; r++)
+                    for (int r = 0; r < TR; r++) {
 #pragma unroll
                         for (int c = 0; c < TC; c++) {
+                            // Even TC: entry 4 t4 + 2 h + i of 16 is D's column
+                            // 2 t4 + h of tile i.
                             const int o = off[r][c];
+                            const double2 y =
+                                TC % 2 == 0
+                                    ? make_double2(acc[r][c & ~1][c & 1], acc[r][c | 1][c & 1])
+                                    : make_double2(acc[r][c][0], acc[r][c][1]);
                             if (o >= 0) {
                                 if (pair) {
-                                    *reinterpret_cast<double2 *>(dst + o) =
-                                        make_double2(acc[r][c][0], acc[r][c][1]);
+                                    *reinterpret_cast<double2 *>(dst + o) = y;
                                 } else {
-                                    dst[o] = acc[r][c][0];
-                                    if (8 * c + 2 * t4 + 1 < Rlo) dst[o + 1] = acc[r][c][1];
+                                    dst[o] = y.x;
+                                    if (o - Rlo * fb_col<TR>(g, r) + 1 < Rlo) dst[o + 1] = y.y;
                                 }
                             }
-                            acc[r][c][0] = acc[r][c][1] = 0.0;
                         }
+#pragma unroll
+                        for (int c = 0; c < TC; c++) acc[r][c][0] = acc[r][c][1] = 0.0;
+                    }
                 }
             }
             __syncwarp();

@@ -99,6 +99,25 @@ def test_row_kernel_orders_and_tile_edges(ctx, oracle_sparse, shape, R):
     sp.close()
 
 
+@pytest.mark.parametrize("R", [(16, 9, 16), (31, 17, 1), (25, 32, 32), (24, 15, 10), (7, 8, 23)])
+def test_fibre_kernel_tiles(ctx, oracle_sparse, R):
+    """The fibre kernel over ranks at and around its column tiles (even and odd
+    tile counts lay the columns out differently), with fibres of one nonzero and
+    fibres of several pieces.  Sums of up to a thousand products: 1e-12."""
+    shape = (40, 36, 34)
+    rng = np.random.default_rng(31)
+    keep = np.concatenate([rng.choice(36 * 34 * 20, 9000, replace=False),
+                           36 * 34 * 20 + rng.choice(36 * 34 * 20, 700, replace=False)])
+    idx = [i.astype(np.int64) for i in np.unravel_index(keep, shape)]
+    vals = rng.standard_normal(keep.size)
+    Ut = _factors(shape, R, 32)
+    sp = ctx.sptensor(idx, vals, shape)
+    for mode in range(3):
+        assert _rel(sp.ttmc_rows(Ut, R, mode),
+                    oracle_sparse.ttmc_rows(idx, vals, shape, Ut, R, mode)) < 1e-12
+    sp.close()
+
+
 def test_sparse_hooi_vs_oracle(ctx, oracle_sparse, zipf_small):
     idx, vals, shape = zipf_small
     R = (8, 8, 8)
