@@ -21,8 +21,8 @@
 // memory.  In a subspace step each warp keeps its rows of S L in registers, laid
 // out as the next products' fragments, from the product to the new factor.  Sums
 // go in a fixed order for a given number of warps.  4096 tensors (modes 8 to 64,
-// ranks 2 to 8, 10 sweeps): 11.6 ms, of it about half the two passes over X at 0.8
-// of the FP64 tensor rate (ranks padded to 8 columns); 100 tensors 1.15 ms.  With
+// ranks 2 to 8, 10 sweeps): 11.4 ms, of it about half the two passes over X at 0.8
+// of the FP64 tensor rate (ranks padded to 8 columns); 100 tensors 1.14 ms.  With
 // one FMA chain per thread and entry on the CUDA cores 23.3 and 2.4 ms.
 //
 // Autotuning.  The block size (128, 256, 512 threads) and the packing (one

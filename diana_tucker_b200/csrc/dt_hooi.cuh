@@ -9,7 +9,7 @@
 
 namespace dt {
 
-// The FP64 HOOI: CUDA-core TTM chain over a dimension tree, FP64 Gram and
+// The FP64 HOOI: TTM chain over a dimension tree, FP64 Gram and
 // subspace iteration.  X may be FP64 or FP32 (read as FP32, computed in FP64).
 // The GNU C library's rand() sequence after srand(seed), restated (dt_hooi.cu).
 class LibcRand {

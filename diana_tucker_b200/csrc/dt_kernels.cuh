@@ -7,7 +7,7 @@
 
 namespace dt {
 
-// ---- dense FP64 (CUDA-core) kernels: dt_dense.cu --------------------------
+// ---- dense FP64 kernels: dt_dense.cu --------------------------------------
 // A dense tensor seen around mode n is a 3-way array X[l, i, b] with
 // l < L = prod_{m<n} I_m (unit stride), i < I = I_n (stride L) and
 // b < B = prod_{m>n} I_m (stride L*I).

@@ -2,8 +2,8 @@
 // (src/operator/operator_double.cpp:84-155) and its ALS_ leading-subspace step
 // (template/algorithm/tucker/hooi_als.tpp:7-34), kept on the device so a HOOI
 // sweep never round-trips to the host.  These matrices are tiny (R x R, I_n x R,
-// I_n x I_n): one CTA per problem, latency-bound, so the code minimises block
-// barriers rather than flops.
+// I_n x I_n): one CTA or one cluster per problem, latency-bound, so the code
+// shortens dependency chains and barriers rather than saving flops.
 #include <vector>
 
 #include "dt_kernels.cuh"
