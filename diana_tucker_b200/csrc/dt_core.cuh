@@ -52,10 +52,9 @@ struct dt_ctx {
     static constexpr size_t kOutStageBytes = size_t(1) << 20;
     void *out_stage = nullptr;
     // Pinned staging for large transfers of pageable host memory (upload_pieces /
-    // download_pieces): as large as the largest so far, at most kBigStageBytes.
-    static constexpr size_t kBigStageBytes = size_t(32) << 20;
+    // download_pieces; on first use).
+    static constexpr size_t kBigStageBytes = size_t(8) << 20;
     void *big_stage = nullptr;
-    size_t big_stage_cap = 0;
     // The dense HOOI drivers' last plans (device buffers plus captured sweeps;
     // two of the FP64 driver's), reused by the next call with the same shapes,
     // ranks and options; released before the stream at dt_ctx_destroy.
@@ -216,7 +215,7 @@ inline void check_ctx(const dt_ctx *ctx) {
 bool is_device_ptr(const void *p);
 
 // Transfers between device memory and a caller's pageable host memory.  From a
-// megabyte on, several host threads copy two-megabyte chunks between the
+// megabyte on, several host threads copy one-megabyte chunks between the
 // caller's memory and the context's pinned staging while the DMA of other
 // chunks runs (the driver's own staging uses one thread: 36 MB up 3.4 ms, down
 // 2.1 ms); smaller ones are left to the driver.  upload_pieces returns once the
