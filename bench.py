@@ -704,7 +704,8 @@ def _batched(ctx, steps, cpu):
            "gen_s": round(gen_s, 1),
            "workload": "4096 x 3-way FP32, modes U[8,64], ranks U[2,8], noise var 1e-4, seed 3; "
                        "10 HOOI sweeps x 5 ALS_ steps from seeded orthonormal factors, FP64"}
-    if cpu:
+    from oracle import ref
+    if cpu and ref.available():
         os.environ.setdefault("OMP_NUM_THREADS", "1")
         os.environ.setdefault("OPENBLAS_NUM_THREADS", "1")
         nproc = os.cpu_count() or 1
