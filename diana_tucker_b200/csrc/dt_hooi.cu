@@ -385,11 +385,13 @@ void DenseHooi::init_factors(double *const *U_user, double *const *dst) {
         DT_CUDA(cudaStreamSynchronize(ctx->stream));  // `all` goes out of scope
     }
     // The modes' Grams first, then all subspace iterations in one launch: each is
-    // a chain of small steps on a few SMs.
+    // a chain of small steps on a few SMs.  Each Gram and workspace starts on a
+    // 256-byte boundary, as an allocation of its own would.
+    auto whole = [](int64_t n) { return (n + 31) / 32 * 32; };
     int64_t sn = 0, wn = 0, off = 0, soff = 0, woff = 0;
     for (int m = 0; m < N; m++) {
-        sn += I[m] * I[m];
-        wn += 3 * I[m] * R[m] + R[m] + 64;
+        sn += whole(I[m] * I[m]);
+        wn += whole(3 * I[m] * R[m] + R[m] + 64);
     }
     DevMem Sall(ctx, sn * sizeof(double)), wall(ctx, wn * sizeof(double));
     const double *Sp[16];
@@ -407,8 +409,8 @@ void DenseHooi::init_factors(double *const *U_user, double *const *dst) {
         Lp[m] = out(m);
         wp[m] = wall.as<double>() + woff;
         off += I[m] * R[m];
-        soff += I[m] * I[m];
-        woff += 3 * I[m] * R[m] + R[m] + 64;
+        soff += whole(I[m] * I[m]);
+        woff += whole(3 * I[m] * R[m] + R[m] + 64);
     }
     subspace_iter_batch(ctx, N, Sp, I, Lp, R, hosvd_iters, wp, flag.as<int>());
 }

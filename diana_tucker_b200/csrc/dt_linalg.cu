@@ -790,7 +790,8 @@ __global__ void __launch_bounds__(SM_NT, 1) subspace_cluster_kernel(SubBatch bat
     const int have = min(own, n - own0);  // rows of S there are (may be <= 0)
     if (SSM) {
         const double *src = Sg + (int64_t)n * own0;
-        if ((n & 1) == 0) {
+        // 16-byte copies: an even n on an S that is 16-byte aligned.
+        if ((n & 1) == 0 && (reinterpret_cast<uintptr_t>(Sg) & 15) == 0) {
             const int hc = n / 2;
             for (int e = t; e < hc * have; e += SM_NT) {
                 const int i = e / hc, q = e - i * hc;

@@ -259,6 +259,33 @@ def test_hooi_given_init_and_zero_sweeps(ctx):
     assert abs(rep["g_norm"] - np.linalg.norm(G2)) < 1e-10 * np.linalg.norm(G2)
 
 
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+@pytest.mark.parametrize("shape,ranks", [
+    ((25, 20, 16), (4, 5, 3)),       # an odd mode before even ones
+    ((61, 48, 83), (5, 4, 6)),       # odd, even, odd
+    ((17, 33, 20), (3, 4, 3)),       # odd, odd, even
+    ((9, 70, 7, 24), (3, 5, 2, 4)),  # even modes after one and after two odd ones, one on a cluster
+    ((5, 257, 18), (3, 6, 4)),       # a mode above the batched launch's sizes
+    ((15, 14), (4, 4))])
+def test_hooi_hosvd_start_of_mixed_parity(ctx, shape, ranks, dtype):
+    """The HOSVD start of all modes in one launch, whose Grams lie behind one
+    another: even modes after odd ones, modes of one tile beside modes that a
+    cluster shares.  Zero sweeps give the start itself, whose subspaces are the
+    oracle's leading eigenvectors (well separated by the model: 1e-8)."""
+    from diana_tucker_b200 import datasets
+    X = datasets.tucker_dense(shape, ranks, noise_var=1e-4, seed=11, dtype=dtype)
+    Xd = X.astype(np.float64)
+    want = dense.hosvd_init(Xd, ranks)
+    G, U, rep = ctx.hooi_dense(X, ranks, init="hosvd", max_sweeps=0)
+    for u, w in zip(U, want):
+        assert dense.principal_angle_max(u, w) < 1e-8
+        np.testing.assert_allclose(u.T @ u, np.eye(u.shape[1]), atol=1e-12)
+    assert _rel(G, dense.core(Xd, U)) < 1e-12
+    G, U, rep = ctx.hooi_dense(X, ranks, init="hosvd", max_sweeps=3)
+    Go, Uo, _ = dense.hooi(Xd, ranks, 3, want)
+    _check_hooi(G, U, rep, float(np.linalg.norm(Go)), Uo, float(np.linalg.norm(Xd)))
+
+
 def test_hooi_rejects_bad_ranks(ctx):
     from diana_tucker_b200 import DTError
     with pytest.raises(DTError) as e:
