@@ -389,17 +389,33 @@ void over_threads(dt_ctx *ctx, size_t n, const std::function<cudaError_t(size_t)
     DT_CUDA((cudaError_t)err.load());
 }
 
+// What `later` is given from now on runs after what `earlier` has been given.
+void stream_after(cudaStream_t later, cudaStream_t earlier) {
+    cudaEvent_t ev;
+    DT_CUDA(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
+    cudaError_t e = cudaEventRecord(ev, earlier);
+    if (e == cudaSuccess) e = cudaStreamWaitEvent(later, ev, 0);
+    cudaEventDestroy(ev);  // (its place in the streams stays)
+    DT_CUDA(e);
+}
+
 // The pieces in chunks, dealt to kCopyThreads lanes; lane l has two slots of the
 // pinned staging, so one chunk's DMA runs while the other is copied by the host.
-// run(chunks of the lane, its slots, its events) on a thread of its own where there
-// is one.  281 k rows of 16, 10 sweeps, both ways: 15.0 ms a call and 41 ms for
+// run(stream, chunks of the lane, its slots, its events) on a thread of its own
+// where there is one.  The DMA goes to ctx->stream; cudaStreamPerThread, which names
+// another stream in each thread, is stood in for by the context's own stream, which
+// starts after what the caller's has been given and which that waits for in turn.
+// 281 k rows of 16, 10 sweeps, both ways: 15.0 ms a call and 41 ms for
 // a context's first one with 8 MB of staging; 15.2 and 54 ms with 32 MB filled and
 // drained whole (pinning them is the difference), 18 ms with 8 MB in such rounds.
 void over_lanes(dt_ctx *ctx, const std::vector<HostPiece> &pieces,
-                const std::function<cudaError_t(const std::vector<Chunk> &, char *const *,
-                                                const cudaEvent_t *)> &run) {
+                const std::function<cudaError_t(cudaStream_t, const std::vector<Chunk> &,
+                                                char *const *, const cudaEvent_t *)> &run) {
     if (!ctx->big_stage)
         DT_CUDA(cudaHostAlloc(&ctx->big_stage, dt_ctx::kBigStageBytes, cudaHostAllocDefault));
+    const bool stand_in = ctx->stream == cudaStreamPerThread;
+    const cudaStream_t dma = stand_in ? ctx->own_stream : ctx->stream;
+    if (stand_in) stream_after(dma, ctx->stream);
     std::vector<Chunk> lane[kCopyThreads];
     size_t n = 0;
     for (const HostPiece &p : pieces)
@@ -407,7 +423,7 @@ void over_lanes(dt_ctx *ctx, const std::vector<HostPiece> &pieces,
             lane[n++ % kCopyThreads].push_back({static_cast<char *>(p.dev) + o,
                                                 static_cast<char *>(p.host) + o,
                                                 std::min(kChunk, p.bytes - o)});
-    over_threads(ctx, kCopyThreads, [&](size_t l) {
+    auto one_lane = [&](size_t l) {
         char *slot[2];
         cudaEvent_t ev[2] = {};
         cudaError_t e = cudaSuccess;
@@ -415,11 +431,19 @@ void over_lanes(dt_ctx *ctx, const std::vector<HostPiece> &pieces,
             slot[s] = static_cast<char *>(ctx->big_stage) + (2 * l + s) * kChunk;
             if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ev[s], cudaEventDisableTiming);
         }
-        if (e == cudaSuccess) e = run(lane[l], slot, ev);
+        if (e == cudaSuccess) e = run(dma, lane[l], slot, ev);
         for (cudaEvent_t x : ev)
             if (x) cudaEventDestroy(x);
         return e;
-    });
+    };
+    // (After an error too: the caller's stream then frees what the DMA may still use.)
+    try {
+        over_threads(ctx, kCopyThreads, one_lane);
+    } catch (...) {
+        if (stand_in) stream_after(ctx->stream, dma);
+        throw;
+    }
+    if (stand_in) stream_after(ctx->stream, dma);
 }
 
 size_t total_bytes(const std::vector<HostPiece> &pieces) {
@@ -439,17 +463,16 @@ void upload_pieces(dt_ctx *ctx, const std::vector<HostPiece> &pieces) {
     }
     // An earlier call's DMA out of the staging is done: every call that uses it
     // ends with a synchronisation.
-    over_lanes(ctx, pieces, [&](const std::vector<Chunk> &cs, char *const *slot,
-                                const cudaEvent_t *ev) {
+    over_lanes(ctx, pieces, [&](cudaStream_t dma, const std::vector<Chunk> &cs,
+                                char *const *slot, const cudaEvent_t *ev) {
         cudaError_t e = cudaSuccess;
         for (size_t i = 0; i < cs.size() && e == cudaSuccess; i++) {
             const int s = i & 1;
             if (i >= 2) e = cudaEventSynchronize(ev[s]);  // the slot's last DMA
             if (e != cudaSuccess) break;
             std::memcpy(slot[s], cs[i].host, cs[i].bytes);
-            e = cudaMemcpyAsync(cs[i].dev, slot[s], cs[i].bytes, cudaMemcpyHostToDevice,
-                                ctx->stream);
-            if (e == cudaSuccess) e = cudaEventRecord(ev[s], ctx->stream);
+            e = cudaMemcpyAsync(cs[i].dev, slot[s], cs[i].bytes, cudaMemcpyHostToDevice, dma);
+            if (e == cudaSuccess) e = cudaEventRecord(ev[s], dma);
         }
         return e;
     });
@@ -463,13 +486,13 @@ void download_pieces(dt_ctx *ctx, const std::vector<HostPiece> &pieces) {
         DT_CUDA(cudaStreamSynchronize(ctx->stream));
         return;
     }
-    over_lanes(ctx, pieces, [&](const std::vector<Chunk> &cs, char *const *slot,
-                                const cudaEvent_t *ev) {
+    over_lanes(ctx, pieces, [&](cudaStream_t dma, const std::vector<Chunk> &cs,
+                                char *const *slot, const cudaEvent_t *ev) {
         auto fetch = [&](size_t i) {
             const int s = i & 1;
             const cudaError_t e = cudaMemcpyAsync(slot[s], cs[i].dev, cs[i].bytes,
-                                                  cudaMemcpyDeviceToHost, ctx->stream);
-            return e == cudaSuccess ? cudaEventRecord(ev[s], ctx->stream) : e;
+                                                  cudaMemcpyDeviceToHost, dma);
+            return e == cudaSuccess ? cudaEventRecord(ev[s], dma) : e;
         };
         cudaError_t e = cs.empty() ? cudaSuccess : fetch(0);
         for (size_t i = 0; i < cs.size() && e == cudaSuccess; i++) {

@@ -196,3 +196,38 @@ def test_hooi_factor_transfers(ctx, rows):
     for a, b in zip(Ut, dev):
         assert np.array_equal(a, b.cpu().numpy())
     sp.close()
+
+
+@pytest.mark.parametrize("rows", [20_000, 300_011])
+def test_hooi_factor_transfers_on_the_per_thread_stream(rows):
+    """The handle of the per-thread default stream names another stream in each of
+    the threads that copy the factors: the transfers have to be in order with the
+    calling thread's all the same.  Other starts in turn, so what a call before
+    left in the buffers does not pass for this one's; the in-place entry point
+    (device buffers, no staging) on the context's own stream gives the same bits."""
+    import ctypes
+
+    import torch
+
+    from diana_tucker_b200 import Context, _lib, datasets
+    per_thread = ctypes.c_void_p(2)  # cudaStreamPerThread
+    R = (16, 8, 8)
+    idx, vals, shape = datasets.sparse_zipf((rows, 300, 200), 20_000, alpha=1.1, seed=3)
+    r = (ctypes.c_int64 * 3)(*R)
+    with Context(0) as c:
+        sp = c.sptensor(idx, vals, shape)
+        for seed in range(9, 15):
+            Ut0 = _factors(shape, R, seed)
+            _lib.check(c.lib.dt_ctx_set_stream(c.h, per_thread))
+            G, Ut, _ = sp.hooi(R, 1, Ut0)
+            _lib.check(c.lib.dt_ctx_set_stream(c.h, None))
+            dev = [torch.from_numpy(u).cuda() for u in Ut0]
+            torch.cuda.synchronize()
+            ptrs = (ctypes.c_void_p * 3)(*[d.data_ptr() for d in dev])
+            Gd = np.zeros_like(G)
+            _lib.check(c.lib.dt_sp_hooi(c.h, sp.h, r, 1, ptrs, Gd.ctypes.data,
+                                        ctypes.byref(_lib.HooiReport())))
+            assert np.array_equal(G, Gd)
+            for a, b in zip(Ut, dev):
+                assert np.array_equal(a, b.cpu().numpy())
+        sp.close()
