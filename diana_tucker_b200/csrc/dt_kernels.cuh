@@ -67,6 +67,12 @@ void subspace_iter_batch(dt_ctx *ctx, int count, const double *const *S, const i
                          double *const *L, const int64_t *r, int iters, double *const *work,
                          int *flag);
 
+// The cluster exchange of the subspace iteration, waiting for data that nobody
+// sends: adds the number of threads that give up to *late, out of
+// EXCHANGE_SELFTEST_THREADS.
+constexpr int EXCHANGE_SELFTEST_THREADS = 512;
+void exchange_selftest(dt_ctx *ctx, int *late, long long limit_cycles);
+
 // LU inverse with partial pivoting (one CTA).  *flag = 1 on a zero pivot.
 void lu_inverse(dt_ctx *ctx, const double *A, int64_t n, double *Ainv, double *work,
                 int *flag);

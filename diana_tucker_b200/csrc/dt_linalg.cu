@@ -679,13 +679,15 @@ __device__ __forceinline__ uint32_t cl_map(const void *p, unsigned rank) {
 // alternate between two mbarriers: a CTA can be one step ahead of another,
 // never two (its second step needs the other's first).  The sender's rows are
 // read before anybody can answer with the next step's data.  Returns false when
-// the bounded wait ran out (about a second).  All threads; ends like a barrier.
+// the bounded wait ran out (about a second) for any thread of the CTA.  All
+// threads; the verdict is the CTA's, so the threads go on or leave together, and
+// taking it is a barrier.
 struct ClExchange {
     uint64_t *bar;  // two mbarriers, arrival count 1
     int step;
     unsigned csize, rank;
+    long long limit = 2000000000LL;  // cycles
 };
-constexpr long long CL_WAIT_CYCLES = 2000000000LL;
 
 __device__ __forceinline__ bool cl_exchange(ClExchange &x, const void *p, uint32_t bytes,
                                             uint32_t bytes_in) {
@@ -707,8 +709,8 @@ __device__ __forceinline__ bool cl_exchange(ClExchange &x, const void *p, uint32
             "r"((uint32_t)__cvta_generic_to_shared(p)), "r"(bytes), "r"(cl_map(bar, threadIdx.x))
             : "memory");
     long long t0 = 0;
+    uint32_t ok;
     for (;;) {
-        uint32_t ok;
         asm volatile(
             "{\n\t.reg .pred p;\n\t"
             "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
@@ -716,10 +718,29 @@ __device__ __forceinline__ bool cl_exchange(ClExchange &x, const void *p, uint32
             : "=r"(ok)
             : "r"(barl), "r"(parity)
             : "memory");
-        if (ok) return true;
+        if (ok) break;
         if (t0 == 0) t0 = clock64();
-        else if (clock64() - t0 > CL_WAIT_CYCLES) return false;
+        else if (clock64() - t0 > x.limit) break;
     }
+    return !__syncthreads_or(!ok);
+}
+
+// A cluster of two CTAs that each wait for data nobody sends: adds up the threads
+// that take the exchange for late.
+__global__ void __launch_bounds__(SM_NT) exchange_selftest_kernel(int *late, long long limit) {
+    __shared__ __align__(16) double data[2];
+    __shared__ __align__(8) uint64_t bars[2];
+    if (threadIdx.x == 0) {
+        for (int q = 0; q < 2; q++)
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(
+                             (uint32_t)__cvta_generic_to_shared(bars + q))
+                         : "memory");
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    cl_sync();
+    ClExchange ex{bars, 0, 2u, cl_rank(), limit};
+    if (!cl_exchange(ex, data, 0, sizeof(data))) atomicAdd(late, 1);
+    cl_sync();
 }
 
 // Rows of S a CTA of a cluster of c owns (whole 8-row tiles), and the pitch of
@@ -858,11 +879,13 @@ __global__ void __launch_bounds__(SM_NT, 1) subspace_cluster_kernel(SubBatch bat
     auto z = [&](int k) { return ring + ((at + k) % bufs) * n8 * T::LDQ; };
 
     bool bad = false, late = false;
-    for (int it = 0; it < iters && !late && !bad; it++) {
+    int it = 0;
+    for (; it < iters && !bad; it++) {
         const bool last = it == iters - 1;
         product(z(0), z(1));
         // Everybody's rows to everybody.
         late = !cl_exchange(ex, z(1) + own0 * T::LDQ, own * row_bytes, (n8 - own) * row_bytes);
+        if (late) break;
         at = (at + 1) % bufs;
         if (!last && !(it & 1)) continue;
         for (int p = 0; p < (last ? 2 : 1); p++) {
@@ -879,7 +902,11 @@ __global__ void __launch_bounds__(SM_NT, 1) subspace_cluster_kernel(SubBatch bat
         }
         if (bufs == 2 && csize > 1 && !last && !bad) cl_sync();
     }
-    // No CTA leaves while another still reads or fills its shared memory.
+    // No CTA leaves while another still reads or fills its shared memory: a late one
+    // takes part in the barriers of the steps it leaves out.
+    if (late && bufs == 2)
+        for (int k = it; k < iters - 1; k++)
+            if (k & 1) cl_sync();
     if (csize > 1) cl_sync();
     if (late) {
         // An exchange never came: NaN factors, which the driver reports.
@@ -1389,6 +1416,10 @@ void subspace_iter_batch(dt_ctx *ctx, int count, const double *const *S, const i
         }
     }
     if (k) subspace_mma(ctx, batch, k, iters, flag, false);
+}
+
+void exchange_selftest(dt_ctx *ctx, int *late, long long limit_cycles) {
+    launch_pdl_cluster(ctx, exchange_selftest_kernel, 2, SM_NT, 0, 2, late, limit_cycles);
 }
 
 void lu_inverse(dt_ctx *ctx, const double *A, int64_t n, double *Ainv, double *work,

@@ -32,12 +32,17 @@ int dt_selftest_wait_timeout(dt_ctx *ctx, int64_t limit_cycles) {
                      "dt_selftest_wait_timeout: limit %lld outside [0, %lld]",
                      (long long)limit_cycles, (long long)tc::kWaitCycles);
         DT_CUDA(cudaSetDevice(ctx->device));
-        DevMem err(ctx, sizeof(int));
-        DT_CUDA(cudaMemsetAsync(err.get(), 0, sizeof(int), ctx->stream));
+        DevMem err(ctx, 2 * sizeof(int));
+        DT_CUDA(cudaMemsetAsync(err.get(), 0, 2 * sizeof(int), ctx->stream));
         DT_LAUNCH(ctx, wait_selftest_kernel, 1, 32, 0, err.as<int>(), (long long)limit_cycles);
-        int h = 0;
-        DT_CUDA(cudaMemcpyAsync(&h, err.get(), sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+        exchange_selftest(ctx, err.as<int>() + 1, limit_cycles);
+        int hs[2] = {};
+        DT_CUDA(cudaMemcpyAsync(hs, err.get(), sizeof(hs), cudaMemcpyDeviceToHost, ctx->stream));
         DT_CUDA(cudaStreamSynchronize(ctx->stream));
+        const int h = hs[0];
+        if (hs[1] != EXCHANGE_SELFTEST_THREADS)
+            fail(DT_ERR_CUDA, fmt("self-test: %d of %d threads found the cluster exchange late",
+                                  hs[1], EXCHANGE_SELFTEST_THREADS));
         if (h) fail(DT_ERR_TIMEOUT, fmt("self-test: the bounded wait ran out after %lld cycles "
                                         "(error word %d)", (long long)limit_cycles, h));
     });

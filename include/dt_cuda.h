@@ -125,8 +125,10 @@ DT_API int dt_ctx_set_mem_limit(dt_ctx *ctx, uint64_t bytes);
  * since creation. */
 DT_API int dt_ctx_mem_usage(dt_ctx *ctx, uint64_t *in_use, uint64_t *peak);
 /* Self-test of the bounded device waits: one kernel waits on an mbarrier that
- * nothing arrives on, for limit_cycles SM clock cycles (<= the 2e9 budget of
- * every wait in the library), records the timeout and returns.  Returns
+ * nothing arrives on, another in the subspace iteration's exchange between CTAs
+ * for data that nobody sends, for limit_cycles SM clock cycles each (<= the 2e9
+ * budget of every wait in the library); they record the timeout (every thread of
+ * the exchange has to take it) and return.  Returns
  * DT_ERR_TIMEOUT, as a real wait that ran out does; the context stays usable. */
 DT_API int dt_selftest_wait_timeout(dt_ctx *ctx, int64_t limit_cycles);
 

@@ -46,6 +46,26 @@ def test_bounded_wait_runs_out_and_context_survives(ctx):
         assert np.array_equal(a, b)
 
 
+@pytest.mark.parametrize("limit", [0, 20_000, 2_000_000])
+def test_cluster_exchange_that_runs_out_is_late_for_all_threads(ctx, limit):
+    """The self-test's second kernel waits in the exchange of the subspace
+    iteration for data that nobody sends: whatever the limit, all threads of both
+    CTAs leave with the same verdict (the call reports the timeout, not a
+    disagreement), and the iteration on a cluster runs as before."""
+    from diana_tucker_b200 import DTError
+    L = _codes()
+    rng = np.random.default_rng(8)
+    Y = np.asfortranarray(rng.standard_normal((96, 12, 20)))
+    L0, _ = np.linalg.qr(rng.standard_normal((96, 16)))
+    q = ctx.als(Y, 0, L0, 5)
+    n0 = ctx.kernel_launches()
+    with pytest.raises(DTError) as e:
+        ctx.selftest_wait_timeout(limit)
+    assert e.value.code == L.DT_ERR_TIMEOUT
+    assert ctx.kernel_launches() - n0 == 2
+    assert np.array_equal(ctx.als(Y, 0, L0, 5), q)
+
+
 XBYTES = 40 * 36 * 32 * 8
 
 
