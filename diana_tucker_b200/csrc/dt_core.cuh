@@ -305,6 +305,11 @@ class DevArena {
 };
 
 
+// Gives back one thing that ctx keeps for later calls and no running call uses:
+// a dense HOOI plan (the one used longest ago first).  False when there is none,
+// or when the stream is being captured.
+bool release_idle(dt_ctx *ctx);
+
 // Stream-ordered device allocation owned by one call.
 class DevMem {
    public:
@@ -319,7 +324,11 @@ class DevMem {
         return *this;
     }
     ~DevMem() { release(); }
+    // Fails with DT_ERR_NOMEM where there is no room, also without what the
+    // context keeps for later calls (release_idle).
     void alloc(dt_ctx *ctx, size_t bytes);
+    // The same, false where there is no room: for a caller with a smaller way.
+    bool try_alloc(dt_ctx *ctx, size_t bytes);
     void release();
     template <class T>
     T *as() const { return static_cast<T *>(p_); }

@@ -173,33 +173,59 @@ void DevArena::give(void *p) {
         }
 }
 
-void DevMem::alloc(dt_ctx *ctx, size_t bytes) {
+bool release_idle(dt_ctx *ctx) {
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(ctx->stream, &st) != cudaSuccess) cudaGetLastError();
+    if (st != cudaStreamCaptureStatusNone) return false;
+    // A running call holds a reference of its own to the plan it uses.
+    auto &kept = ctx->hooi_plans_fp64;
+    for (size_t k = kept.size(); k-- > 0;)
+        if (kept[k].use_count() == 1) {
+            release_plan(ctx, kept[k]);
+            kept.erase(kept.begin() + k);
+            return true;
+        }
+    if (ctx->hooi_plan_mixed.use_count() == 1) {
+        release_plan(ctx, ctx->hooi_plan_mixed);
+        return true;
+    }
+    return false;
+}
+
+bool DevMem::try_alloc(dt_ctx *ctx, size_t bytes) {
     release();
-    if (bytes == 0) return;
+    if (bytes == 0) return true;
     if (ctx->arena) {
         p_ = ctx->arena->take(bytes);
         arena_ = ctx->arena;
         bytes_ = bytes;
-        return;
+        return true;
     }
-    if (ctx->mem_limit && ctx->mem_in_use + bytes > ctx->mem_limit)
-        fail(DT_ERR_NOMEM, fmt("device allocation of %zu bytes would exceed the context's "
-                               "limit (%llu of %llu bytes in use)",
-                               bytes, (unsigned long long)ctx->mem_in_use,
-                               (unsigned long long)ctx->mem_limit));
-    const cudaError_t e = cudaMallocAsync(&p_, bytes, ctx->stream);
-    if (e != cudaSuccess) {
-        p_ = nullptr;
-        if (e == cudaErrorMemoryAllocation) {
+    for (;;) {
+        if (!ctx->mem_limit || ctx->mem_in_use + bytes <= ctx->mem_limit) {
+            const cudaError_t e = cudaMallocAsync(&p_, bytes, ctx->stream);
+            if (e == cudaSuccess) break;
+            p_ = nullptr;
+            if (e != cudaErrorMemoryAllocation) DT_CUDA(e);
             cudaGetLastError();
-            fail(DT_ERR_NOMEM, fmt("device allocation of %zu bytes failed", bytes));
         }
-        DT_CUDA(e);
+        if (!release_idle(ctx)) return false;
     }
     ctx_ = ctx;
     bytes_ = bytes;
     ctx->mem_in_use += bytes;
     ctx->mem_peak = std::max(ctx->mem_peak, ctx->mem_in_use);
+    return true;
+}
+
+void DevMem::alloc(dt_ctx *ctx, size_t bytes) {
+    if (try_alloc(ctx, bytes)) return;
+    if (ctx->mem_limit && ctx->mem_in_use + bytes > ctx->mem_limit)
+        fail(DT_ERR_NOMEM, fmt("device allocation of %zu bytes would exceed the context's "
+                               "limit (%llu of %llu bytes in use)",
+                               bytes, (unsigned long long)ctx->mem_in_use,
+                               (unsigned long long)ctx->mem_limit));
+    fail(DT_ERR_NOMEM, fmt("device allocation of %zu bytes failed", bytes));
 }
 
 void DevMem::release() {

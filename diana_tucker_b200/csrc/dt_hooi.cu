@@ -335,8 +335,11 @@ void DenseHooi::init_factors(double *const *U_user, double *const *dst) {
         // orthonormal basis of span(U_rand) gives the same sweeps: the TTM
         // chain's Gram matrices only see U U^T).
         LibcRand gen(seeded ? opts.seed : 1u);
-        std::vector<double> h((size_t)total);
-        for (auto &v : h) v = libc_polar_randn(seeded ? &gen : nullptr);
+        std::vector<double> own, &h = drawn ? *drawn : own;
+        if (h.empty()) {
+            h.resize((size_t)total);
+            for (auto &v : h) v = libc_polar_randn(seeded ? &gen : nullptr);
+        }
         DevMem a(ctx, total * sizeof(double));
         DT_CUDA(cudaMemcpyAsync(a.get(), h.data(), total * sizeof(double), cudaMemcpyHostToDevice,
                                 ctx->stream));
@@ -669,28 +672,52 @@ int dt_hooi_dense(dt_ctx *ctx, const void *X, int dtype, int ndim, const int64_t
             // and its sweeps are launched directly.  The two plans used last
             // are kept, the later one in front (a program often alternates
             // between a tensor and its sketch).
-            const bool keep = x.ptr() == X;
-            std::shared_ptr<Fp64Plan> plan;
-            auto &kept = ctx->hooi_plans_fp64;
-            for (size_t k = 0; keep && k < kept.size(); k++) {
-                auto p = std::static_pointer_cast<Fp64Plan>(kept[k]);
-                if (!p->matches(x.ptr(), dtype, ndim, shape, ranks, o)) continue;
-                std::rotate(kept.begin(), kept.begin() + k, kept.begin() + k + 1);
-                plan = p;
-                break;
-            }
-            if (!plan) {
-                plan = std::make_shared<Fp64Plan>(x.ptr(), dtype, ndim, shape, ranks, o);
-                if (keep) {
-                    if (kept.size() >= 2) {
-                        release_plan(ctx, kept.back());
-                        kept.pop_back();
+            std::vector<double> draws;
+            auto call = [&](bool keep) {
+                std::shared_ptr<Fp64Plan> plan;
+                auto &kept = ctx->hooi_plans_fp64;
+                for (size_t k = 0; keep && k < kept.size(); k++) {
+                    auto p = std::static_pointer_cast<Fp64Plan>(kept[k]);
+                    if (!p->matches(x.ptr(), dtype, ndim, shape, ranks, o)) continue;
+                    std::rotate(kept.begin(), kept.begin() + k, kept.begin() + k + 1);
+                    plan = p;
+                    break;
+                }
+                if (!plan) {
+                    plan = std::make_shared<Fp64Plan>(x.ptr(), dtype, ndim, shape, ranks, o);
+                    if (keep) {
+                        if (kept.size() >= 2) {
+                            release_plan(ctx, kept.back());
+                            kept.pop_back();
+                        }
+                        kept.insert(kept.begin(), plan);
                     }
-                    kept.insert(kept.begin(), plan);
+                }
+                plan->h.drawn = &draws;
+                plan->h.setup(ctx, x.ptr(), dtype, ndim, shape, ranks, o);
+                plan->h.run(G, U, report, keep ? &plan->loop : nullptr);
+                plan->h.drawn = nullptr;
+            };
+            const int64_t launches0 = ctx->launches;
+            bool keep = x.ptr() == X;
+            if (keep) {
+                // A plan holds all its sweep's intermediates at once, besides
+                // what the start takes.  Where that does not fit, the call
+                // starts over without one: nothing has been handed out yet.
+                try {
+                    call(true);
+                } catch (const Error &e) {
+                    if (e.code != DT_ERR_NOMEM) throw;
+                    keep = false;
+                }
+                if (!keep) {
+                    while (release_idle(ctx)) {
+                    }
+                    ctx->launches = launches0;
+                    if (report) std::memset(report, 0, sizeof(*report));
                 }
             }
-            plan->h.setup(ctx, x.ptr(), dtype, ndim, shape, ranks, o);
-            plan->h.run(G, U, report, keep ? &plan->loop : nullptr);
+            if (!keep) call(false);
         } else {
             hooi_dense_lowprec(ctx, x_host ? up.dst.get() : x.ptr(), dtype, ndim, shape, ranks, o,
                                G, U, report, x_host ? &up : nullptr);

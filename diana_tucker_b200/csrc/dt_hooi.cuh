@@ -80,6 +80,9 @@ struct DenseHooi {
     DevMem arena_mem;
     const void *const *xslot = nullptr;  // where a captured sweep finds X
     DevMem hosvd_start;             // HOSVD's Gaussian starts, mode after mode
+    // Where a call keeps its random draws, so that starting over draws no more
+    // (null: not kept).
+    std::vector<double> *drawn = nullptr;
 
     // Allocates the buffers on the first call; a later call on the same
     // object (same shapes and ranks) keeps them, so a captured sweep graph

@@ -177,3 +177,102 @@ def test_nan_tensor_in_a_batch_stays_in_its_slot(ctx):
     assert np.array_equal(e1[keep], e2[keep])
     for t in keep:
         assert np.array_equal(G1[t], G2[t])
+
+
+def _device(shape, seed, dtype="float64"):
+    import torch
+    X = np.random.default_rng(seed).standard_normal(shape)
+    return torch.from_numpy(X.reshape(-1, order="F").copy()).cuda().to(getattr(torch, dtype))
+
+
+def _peak(shape, ranks, **kw):
+    """Bytes that one call takes in a context that keeps nothing yet."""
+    from diana_tucker_b200 import Context
+    with Context(0) as c:
+        c.hooi_dense(_device(shape, 1), ranks, shape=shape, **kw)
+        return c.mem_usage()[1]
+
+
+@pytest.mark.parametrize("then", ["fp64", "bf16xh", "sparse", "batched"])
+def test_kept_plans_make_room(ctx, then):
+    """Two FP64 shapes, whose plans the context keeps, then a call of a third kind
+    under a cap that it fits by itself: the plans go, the call gives what it gives
+    in a fresh context, and the first shape builds its plan again."""
+    from diana_tucker_b200 import DT_PREC_BF16XH, Context, datasets
+    kw = dict(max_sweeps=3, seed=2)
+    shapes, ranks = [(60, 52, 44), (52, 60, 44)], (6, 5, 4)
+    Xs = [_device(s, k) for k, s in enumerate(shapes)]
+    rng = np.random.default_rng(4)
+
+    def third(c):
+        if then == "fp64":
+            return c.hooi_dense(_device((44, 52, 60), 7), ranks, shape=(44, 52, 60), **kw)[:2]
+        if then == "bf16xh":
+            return c.hooi_dense(_device((64, 48, 40), 7, "float32"), (8, 8, 8), shape=(64, 48, 40),
+                                precision=DT_PREC_BF16XH, inner_iters=2, **kw)[:2]
+        if then == "sparse":
+            shape, R = (3000, 500, 200), (8, 8, 8)
+            idx, vals, _ = datasets.sparse_zipf(shape, 20000, alpha=1.1, seed=12)
+            sp = c.sptensor(idx, vals, shape)
+            out = sp.hooi(R, 2, datasets.random_orthonormal_transposed(shape, R, 3))[:2]
+            sp.close()
+            return out
+        X = [np.asfortranarray(np.random.default_rng(k).standard_normal((12, 11, 10)), dtype=np.float32)
+             for k in range(4)]
+        r = np.random.default_rng(6)
+        U0 = [[np.linalg.qr(r.standard_normal((s, 3)))[0] for s in x.shape] for x in X]
+        return c.hooi_batched(X, [(3, 3, 3)] * 4, U0, sweeps=2, block_threads=128)[:2]
+
+    def flat(out):
+        for v in out:
+            if isinstance(v, (list, tuple)):
+                yield from flat(v)
+            else:
+                yield np.asarray(v)
+
+    with Context(0) as c:
+        want = list(flat(third(c)))
+        cap = c.mem_usage()[1]
+    with Context(0) as c:
+        first = [c.hooi_dense(X, ranks, shape=s, **kw) for X, s in zip(Xs, shapes)]
+        assert c.mem_usage()[0] > 0
+        c.set_mem_limit(cap)
+        for a, b in zip(flat(third(c)), want, strict=True):
+            assert np.array_equal(a, b)
+        c.set_mem_limit(0)
+        G, U, _ = c.hooi_dense(Xs[0], ranks, shape=shapes[0], **kw)
+        assert np.array_equal(G, first[0][0])
+        assert all(np.array_equal(a, b) for a, b in zip(U, first[0][1]))
+
+
+@pytest.mark.parametrize("shape,ranks,cap", [((40, 36, 32, 28), (5, 5, 5, 5), 1934868),
+                                             ((8, 8, 8), (2, 2, 2), 3580)])
+@pytest.mark.parametrize("stream", ["legacy", "side"])
+def test_cap_without_room_for_a_plan(ctx, shape, ranks, cap, stream):
+    """A cap that holds a call's own buffers and the largest intermediates that
+    live at one time, but no plan beside them (the driver's state, all
+    intermediates): the call runs without one, the second time too.  The process's
+    rand() is drawn from once."""
+    import ctypes
+
+    import torch
+
+    from diana_tucker_b200 import Context
+    libc = ctypes.CDLL(None)
+    assert _peak(shape, ranks, max_sweeps=3) > cap
+    X = _device(shape, 3)
+    s = torch.cuda.default_stream() if stream == "legacy" else torch.cuda.Stream()
+    torch.cuda.synchronize()
+    with Context(0) as c, torch.cuda.stream(s):
+        outs = []
+        for limit in (0, cap, cap):
+            c.set_mem_limit(limit)
+            libc.srand(5)
+            G, U, rep = c.hooi_dense(X, ranks, shape=shape, seed=0xFFFFFFFF, max_sweeps=3)
+            outs.append((G, U, rep["residual"], libc.rand()))
+            assert rep["sweeps"] == 3
+        for G, U, res, after in outs[1:]:
+            assert after == outs[0][3] and abs(res - outs[0][2]) <= 1e-12
+            assert np.linalg.norm(G - outs[0][0]) <= 1e-12 * np.linalg.norm(G)
+            for a, b in zip(U, outs[0][1]):
+                assert np.linalg.norm(a - b) <= 1e-12
