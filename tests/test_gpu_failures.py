@@ -245,6 +245,26 @@ def test_kept_plans_make_room(ctx, then):
         assert all(np.array_equal(a, b) for a, b in zip(U, first[0][1]))
 
 
+@pytest.mark.parametrize("shape,mode,spare", [((200, 40, 21), 0, 1 << 20), ((181, 203, 157), 1, 0),
+                                              ((500, 100, 24), 0, 1 << 21), ((40, 50), 0, 0),
+                                              ((300, 200, 5), 1, 1 << 22)])
+def test_gram_in_any_room(shape, mode, spare):
+    """The Gram takes fewer splits, at last one, under a cap that leaves its partial
+    tiles little room beside X and the result, or none.  Sums of up to 28417
+    products: 1e-12 of the largest entry."""
+    from diana_tucker_b200 import Context
+    X = np.asfortranarray(np.random.default_rng(sum(shape)).standard_normal(shape))
+    A = np.moveaxis(X, mode, 0).reshape(shape[mode], -1)
+    with Context(0) as c:
+        c.gram(X, mode)
+        cap = 8 * (X.size + shape[mode] ** 2) + spare
+        assert c.mem_usage()[1] > cap
+        c.set_mem_limit(cap)
+        G = c.gram(X, mode)
+        assert np.array_equal(G, G.T)
+        np.testing.assert_allclose(G, A @ A.T, rtol=0, atol=1e-12 * np.max(np.abs(A @ A.T)))
+
+
 @pytest.mark.parametrize("shape,ranks,cap", [((40, 36, 32, 28), (5, 5, 5, 5), 1934868),
                                              ((8, 8, 8), (2, 2, 2), 3580)])
 @pytest.mark.parametrize("stream", ["legacy", "side"])
