@@ -375,17 +375,27 @@ void DenseHooi::init_factors(double *const *U_user, double *const *dst) {
         f32_to_f64(ctx, static_cast<const float *>(Xdev), xsize, xconv.as<double>());
         X64p = xconv.as<double>();
     }
+    auto start = [&](int m) { return seeded_gaussian((size_t)(I[m] * R[m]), 1000 + m); };
+    auto mode_gram = [&](int m, double *Sm) {
+        int64_t L = 1, B = 1;
+        for (int k = 0; k < m; k++) L *= I[k];
+        for (int k = m + 1; k < N; k++) B *= I[k];
+        ttt_f64(ctx, X64p, X64p, L, I[m], I[m], B, Sm);
+    };
     // The Gaussian starts depend on the shape alone: drawn once and kept.
+    bool room = true;
     if (!hosvd_start.get()) {
         std::vector<double> all;
         for (int m = 0; m < N; m++) {
-            const std::vector<double> h = seeded_gaussian((size_t)(I[m] * R[m]), 1000 + m);
+            const std::vector<double> h = start(m);
             all.insert(all.end(), h.begin(), h.end());
         }
-        hosvd_start.alloc(ctx, all.size() * sizeof(double));
-        DT_CUDA(cudaMemcpyAsync(hosvd_start.get(), all.data(), all.size() * sizeof(double),
-                                cudaMemcpyHostToDevice, ctx->stream));
-        DT_CUDA(cudaStreamSynchronize(ctx->stream));  // `all` goes out of scope
+        room = hosvd_start.try_alloc(ctx, all.size() * sizeof(double));
+        if (room) {
+            DT_CUDA(cudaMemcpyAsync(hosvd_start.get(), all.data(), all.size() * sizeof(double),
+                                    cudaMemcpyHostToDevice, ctx->stream));
+            DT_CUDA(cudaStreamSynchronize(ctx->stream));  // `all` goes out of scope
+        }
     }
     // The modes' Grams first, then all subspace iterations in one launch: each is
     // a chain of small steps on a few SMs.  Each Gram and workspace starts on a
@@ -396,15 +406,28 @@ void DenseHooi::init_factors(double *const *U_user, double *const *dst) {
         sn += whole(I[m] * I[m]);
         wn += whole(3 * I[m] * R[m] + R[m] + 64);
     }
-    DevMem Sall(ctx, sn * sizeof(double)), wall(ctx, wn * sizeof(double));
+    DevMem Sall, wall;
+    room = room && Sall.try_alloc(ctx, sn * sizeof(double)) &&
+           wall.try_alloc(ctx, wn * sizeof(double));
+    if (!room) {
+        // Without room for all modes at once: one after another in the plan's S.
+        Sall.release();
+        for (int m = 0; m < N; m++) {
+            mode_gram(m, S.as<double>());
+            const std::vector<double> h = start(m);
+            DT_CUDA(cudaMemcpyAsync(out(m), h.data(), h.size() * sizeof(double),
+                                    cudaMemcpyHostToDevice, ctx->stream));
+            subspace_iter(ctx, S.as<double>(), I[m], out(m), R[m], hosvd_iters, work.as<double>(),
+                          flag.as<int>());
+            DT_CUDA(cudaStreamSynchronize(ctx->stream));  // `h` goes out of scope
+        }
+        return;
+    }
     const double *Sp[16];
     double *Lp[16], *wp[16];
     for (int m = 0; m < N; m++) {
-        int64_t L = 1, B = 1;
-        for (int k = 0; k < m; k++) L *= I[k];
-        for (int k = m + 1; k < N; k++) B *= I[k];
         double *Sm = Sall.as<double>() + soff;
-        ttt_f64(ctx, X64p, X64p, L, I[m], I[m], B, Sm);
+        mode_gram(m, Sm);
         DT_CUDA(cudaMemcpyAsync(out(m), hosvd_start.as<double>() + off,
                                 I[m] * R[m] * sizeof(double), cudaMemcpyDeviceToDevice,
                                 ctx->stream));

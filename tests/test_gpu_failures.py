@@ -245,6 +245,33 @@ def test_kept_plans_make_room(ctx, then):
         assert all(np.array_equal(a, b) for a, b in zip(U, first[0][1]))
 
 
+@pytest.mark.parametrize("shape,ranks,dtype,cap", [
+    ((60, 50, 40), (6, 5, 4), "float64", 505956), ((60, 50, 40), (6, 5, 4), "float32", 1465956),
+    ((300, 280, 20), (6, 5, 4), "float64", 9430996), ((300, 280, 20), (6, 5, 4), "float64", 1800000),
+    ((40, 36, 32, 28), (5, 5, 5, 5), "float64", 1934868)])
+def test_hosvd_start_one_mode_at_a_time(shape, ranks, dtype, cap):
+    """A cap that holds the largest mode's Gram, or that and an FP64 copy of X, but
+    not all modes' Grams side by side: the HOSVD start takes one mode after
+    another.  Other splits and another order of the modes' work: 1e-12 of the
+    core's norm, 1e-10 of the subspaces."""
+    import torch
+
+    from diana_tucker_b200 import Context, datasets
+    from oracle import dense
+    X = datasets.tucker_dense(shape, ranks, noise_var=1e-4, seed=5, dtype=np.float64)
+    Xd = torch.from_numpy(X.reshape(-1, order="F").copy()).cuda().to(getattr(torch, dtype))
+    kw = dict(init="hosvd", max_sweeps=2, shape=shape)
+    with Context(0) as c:
+        G0, U0, r0 = c.hooi_dense(Xd, ranks, **kw)
+        assert c.mem_usage()[1] > cap
+        for _ in range(2):
+            c.set_mem_limit(cap)
+            G, U, r = c.hooi_dense(Xd, ranks, **kw)
+            assert abs(r["g_norm"] - r0["g_norm"]) <= 1e-12 * r0["g_norm"]
+            for a, b in zip(U, U0):
+                assert dense.principal_angle_max(a, b) <= 1e-10
+
+
 @pytest.mark.parametrize("shape,mode,spare", [((200, 40, 21), 0, 1 << 20), ((181, 203, 157), 1, 0),
                                               ((500, 100, 24), 0, 1 << 21), ((40, 50), 0, 0),
                                               ((300, 200, 5), 1, 1 << 22)])
