@@ -81,19 +81,23 @@ void lu_inverse(dt_ctx *ctx, const double *A, int64_t n, double *Ainv, double *w
 void orth2_rows(dt_ctx *ctx, double *A, int64_t len1, int64_t len2);
 
 // The same in pieces, for r <= 32 and a caller that keeps the scratch (at
-// least orth_scratch_bytes; GRAM_COUNTERS counters and a flag, zeroed once)
-// over many calls: orth_scratch lays it out; the kernel that produces the
-// r x m col-major A ends in gram_finish(s.f) (at most orth_max_blocks CTAs of
-// 256 threads), and orth_finish makes the two products that follow, out(:, k)
+// least what orth_alloc takes, T of r x m and a flag, zeroed once) over many
+// calls: orth_scratch lays it out for rows up to that r; the kernel that produces
+// the r x m col-major A ends in gram_finish(s.f) (at most s.blocks CTAs of 256
+// threads), and orth_finish makes the two products that follow, out(:, k)
 // or, given `rows`, out(:, rows[k]); orth_check reads the flag back (one
 // synchronisation) and fails on dependent rows.
 struct OrthScratch {
     GramFinish f;
     double *T, *Linv2;
+    int64_t blocks;
 };
-int64_t orth_max_blocks(const dt_ctx *ctx);
-size_t orth_scratch_bytes(const dt_ctx *ctx, int r, int64_t m);
-OrthScratch orth_scratch(const dt_ctx *ctx, void *mem, int r, int64_t m, int *counters, int *flag);
+// The CTAs that a Gram over m columns keeps busy; any smaller number does too.
+int64_t orth_blocks(const dt_ctx *ctx, int64_t m);
+// Scratch for `blocks` CTAs, or as many as there is room for; returns how many
+// (no room for one: fails with DT_ERR_NOMEM, or returns 0 when `may_fail`).
+int64_t orth_alloc(dt_ctx *ctx, DevMem &mem, int r, int64_t blocks, bool may_fail = false);
+OrthScratch orth_scratch(void *mem, double *T, int r, int64_t blocks, int *flag);
 void orth_finish(dt_ctx *ctx, const double *A, int r, int64_t m, const OrthScratch &s, double *out,
                  const int32_t *rows);
 void orth_check(dt_ctx *ctx, const int *flag);

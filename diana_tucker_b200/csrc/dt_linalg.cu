@@ -1428,30 +1428,50 @@ void lu_inverse(dt_ctx *ctx, const double *A, int64_t n, double *Ainv, double *w
     DT_LAUNCH(ctx, lu_inverse_kernel, 1, LA_NT, n * sizeof(int), A, n, Ainv, work, flag);
 }
 
-size_t orth_scratch_bytes(const dt_ctx *ctx, int r, int64_t m) {
-    const int64_t blocks = orth_max_blocks(ctx), rr = (int64_t)r * r;
-    return (size_t)(r * m + rr * (blocks + (blocks + GRAM_GROUP - 1) / GRAM_GROUP + 2)) *
+namespace {
+
+int64_t gram_groups(int64_t blocks) { return (blocks + GRAM_GROUP - 1) / GRAM_GROUP; }
+// The arrival counters, in front, in doubles.
+int64_t gram_counters(int64_t blocks) { return (gram_groups(blocks) + 2) / 2; }
+
+size_t orth_scratch_bytes(int r, int64_t blocks) {
+    const int64_t rr = (int64_t)r * r, groups = gram_groups(blocks);
+    return (size_t)(gram_counters(blocks) + rr * (blocks + (groups > 1 ? groups : 0) + 2)) *
            sizeof(double);
 }
 
-int64_t orth_max_blocks(const dt_ctx *ctx) {
-    return std::min<int64_t>(GRAM_MAX_BLOCKS, 4LL * ctx->num_sms);
+}  // namespace
+
+int64_t orth_blocks(const dt_ctx *ctx, int64_t m) {
+    return std::max<int64_t>(
+        1, std::min<int64_t>({((m + 7) / 8 + 7) / 8, GRAM_MAX_BLOCKS, 4LL * ctx->num_sms}));
 }
 
-OrthScratch orth_scratch(const dt_ctx *ctx, void *mem, int r, int64_t m, int *counters,
-                         int *flag) {
-    const int64_t blocks = orth_max_blocks(ctx), rr = (int64_t)r * r;
+int64_t orth_alloc(dt_ctx *ctx, DevMem &mem, int r, int64_t blocks, bool may_fail) {
+    while (!mem.try_alloc(ctx, orth_scratch_bytes(r, blocks))) {
+        if (blocks == 1 && may_fail) return 0;
+        if (blocks == 1) mem.alloc(ctx, orth_scratch_bytes(r, 1));  // (fails)
+        blocks = (blocks + 3) / 4;
+    }
+    DT_CUDA(cudaMemsetAsync(mem.get(), 0, gram_counters(blocks) * sizeof(double), ctx->stream));
+    return blocks;
+}
+
+OrthScratch orth_scratch(void *mem, double *T, int r, int64_t blocks, int *flag) {
+    const int64_t rr = (int64_t)r * r, groups = gram_groups(blocks);
     OrthScratch s;
-    double *p = static_cast<double *>(mem);
-    s.T = p;
-    p += r * m;
-    s.f.part = p;
+    s.f.counters = static_cast<int *>(mem);
+    double *p = static_cast<double *>(mem) + gram_counters(blocks);
+    s.T = T;
+    s.blocks = blocks;
+    s.f.part = s.f.group = p;
     p += rr * blocks;
-    s.f.group = p;
-    p += rr * ((blocks + GRAM_GROUP - 1) / GRAM_GROUP);
+    if (groups > 1) {
+        s.f.group = p;
+        p += rr * groups;
+    }
     s.f.Linv = p;
     s.Linv2 = p + rr;
-    s.f.counters = counters;
     s.f.flag = flag;
     return s;
 }
@@ -1462,7 +1482,7 @@ void orth_finish(dt_ctx *ctx, const double *A, int r, int64_t m, const OrthScrat
     GramFinish f2 = s.f;
     f2.Linv = s.Linv2;
     const unsigned gblocks = (unsigned)std::max<int64_t>(
-        1, std::min<int64_t>(((m + 7) / 8 + 7) / 8, orth_max_blocks(ctx)));
+        1, std::min<int64_t>(((m + 7) / 8 + 7) / 8, s.blocks));
     const unsigned ablocks = (unsigned)std::max<int64_t>(
         1, std::min<int64_t>(((m + 7) / 8 + 7) / 8, 8LL * ctx->num_sms));
 #define DT_ROWS(R)                                                                          \
@@ -1495,13 +1515,12 @@ void orth2_rows(dt_ctx *ctx, double *A, int64_t len1, int64_t len2) {
         // Three launches: the Gram of A; T = L^{-1} A with the Gram of T; and
         // the second pass's product.
         const int r = (int)len1;
-        DevMem mem(ctx, orth_scratch_bytes(ctx, r, len2));
-        DevMem ints(ctx, (GRAM_COUNTERS + 1) * sizeof(int));
-        DT_CUDA(cudaMemsetAsync(ints.get(), 0, (GRAM_COUNTERS + 1) * sizeof(int), ctx->stream));
-        const OrthScratch s = orth_scratch(ctx, mem.get(), r, len2, ints.as<int>(),
-                                           ints.as<int>() + GRAM_COUNTERS);
-        const int64_t target = orth_max_blocks(ctx);
-        const int64_t cpb = std::max<int64_t>(256, (len2 + target - 1) / target);
+        DevMem T(ctx, (size_t)r * len2 * sizeof(double)), mem;
+        const int64_t blocks = orth_alloc(ctx, mem, r, orth_blocks(ctx, len2));
+        DevMem flag(ctx, sizeof(int));
+        DT_CUDA(cudaMemsetAsync(flag.get(), 0, sizeof(int), ctx->stream));
+        const OrthScratch s = orth_scratch(mem.get(), T.as<double>(), r, blocks, flag.as<int>());
+        const int64_t cpb = std::max<int64_t>(256, (len2 + blocks - 1) / blocks);
         const unsigned nblk = (unsigned)((len2 + cpb - 1) / cpb);
         if (r <= 8) DT_LAUNCH_PDL(ctx, rows_gram_kernel<8>, nblk, 256, 0, A, r, len2, cpb, s.f);
         else if (r <= 16)

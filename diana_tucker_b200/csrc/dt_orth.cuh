@@ -79,11 +79,10 @@ __device__ __forceinline__ bool warp_chol_linv(const double *G, int ldg, int r, 
 // first use; the last CTA leaves them zero).
 constexpr int GRAM_GROUP = 16;
 constexpr int GRAM_MAX_BLOCKS = 1024;
-constexpr int GRAM_COUNTERS = 1 + GRAM_MAX_BLOCKS / GRAM_GROUP;
 struct GramFinish {
     double *part;       // gridDim.x x r x r
-    double *group;      // ceil(gridDim.x / GRAM_GROUP) x r x r
-    int *counters;      // GRAM_COUNTERS
+    double *group;      // ceil(gridDim.x / GRAM_GROUP) x r x r (one group: may be `part`)
+    int *counters;      // one and one for each group
     double *Linv;       // r x r, col-major
     int *flag;          // bit 0: the rows are linearly dependent
 };

@@ -1356,21 +1356,45 @@ void fib_dispatch(dt_ctx *ctx, const ModeCopy &mc, const double *UF, int RF, con
 
 }  // namespace
 
+namespace {
+
+// Doubles of partial rows that sp_ttmc_compact takes for a mode with P entries a
+// row: what its tasks or chunks write, and (3-way) the segments' sums behind that.
+int64_t ttmc_scratch(const ModeCopy &mc, int nd, int64_t P) {
+    if (nd != 3) return std::max<int64_t>(mc.nslots, 1) * P;
+    return (std::max<int64_t>(mc.tslots, 1) + (mc.tmulti > 0 ? mc.nseg : 0)) * P;
+}
+
+// Rows of a block of mtr_mma_kernel, and the blocks, at most `most`.
+int64_t mtr_rows(int64_t nrows, int64_t most) {
+    return std::max<int64_t>(64, (nrows + most - 1) / most);
+}
+int mtr_blocks(int64_t nrows, int64_t most) {
+    const int64_t rpb = mtr_rows(nrows, most);
+    return (int)std::max<int64_t>(1, (nrows + rpb - 1) / rpb);
+}
+
+}  // namespace
+
 // Compact Y_(n): Yc is nrows x P row-major (row k = mode-n row mc.rows[k]).
+// `scratch`: ttmc_scratch doubles (null: allocated here).
 void sp_ttmc_compact(dt_ctx *ctx, const dt_sptensor *sp, const double *const *Ut_dev,
-                     const int64_t *R, int mode, double *Yc, LaunchTimer *timer = nullptr) {
+                     const int64_t *R, int mode, double *Yc, LaunchTimer *timer = nullptr,
+                     double *scratch = nullptr) {
     const ModeCopy &mc = sp->modes[mode];
     const int nd = sp->ndim;
     const int64_t P64 = kron_len(R, nd, mode);
     DT_CHECK_ARG(P64 <= 1024, "sparse TTMc: prod of the other ranks (%lld) exceeds 1024",
                  (long long)P64);
     const int P = (int)P64;
+    DevMem own;
+    if (!scratch) own.alloc(ctx, ttmc_scratch(mc, nd, P) * sizeof(double));
+    double *const part = scratch ? scratch : own.as<double>();
     if (nd == 3) {
         const int F = mc.fmode;
         int E = 0;
         for (int m = 0; m < 3; m++)
             if (m != mode && m != F) E = m;
-        DevMem tpart(ctx, std::max<int64_t>(mc.tslots, 1) * P * sizeof(double));
         SummaryScope sc(ctx, "Function::ttmc()",
                         2.0 * ((double)sp->nnz * R[E] + (double)mc.nfib * R[F] * R[E]),
                         (double)sp->nnz * 12.0 + (double)mc.nfib * 8.0 +
@@ -1378,19 +1402,18 @@ void sp_ttmc_compact(dt_ctx *ctx, const dt_sptensor *sp, const double *const *Ut
         if (timer) timer->begin();
         if (F < E)
             fib_dispatch<true>(ctx, mc, Ut_dev[F], (int)R[F], Ut_dev[E], (int)R[E], Yc,
-                               tpart.as<double>());
+                               part);
         else
             fib_dispatch<false>(ctx, mc, Ut_dev[F], (int)R[F], Ut_dev[E], (int)R[E], Yc,
-                                tpart.as<double>());
+                                part);
         if (mc.tmulti > 0) {
-            DevMem segs(ctx, (size_t)mc.nseg * P * sizeof(double));
+            double *const segs = part + std::max<int64_t>(mc.tslots, 1) * P;
             DT_LAUNCH(ctx, sum_segments_kernel,
-                      (unsigned)std::min<int64_t>(mc.nseg, 65535), 256, 0, tpart.as<double>(),
-                      mc.tseg_first.as<int32_t>(), mc.tseg_count.as<int32_t>(), mc.nseg, P,
-                      segs.as<double>());
+                      (unsigned)std::min<int64_t>(mc.nseg, 65535), 256, 0, (const double *)part,
+                      mc.tseg_first.as<int32_t>(), mc.tseg_count.as<int32_t>(), mc.nseg, P, segs);
             const unsigned blocks = (unsigned)std::min<int64_t>(mc.tmulti, 65535);
             DT_LAUNCH(ctx, combine_partials_kernel, blocks, 256 * COMB_SPLIT, 0,
-                      segs.as<double>(), mc.tmulti_row.as<int32_t>(),
+                      (const double *)segs, mc.tmulti_row.as<int32_t>(),
                       mc.tmulti_first.as<int32_t>(), mc.tmulti_count.as<int32_t>(), mc.tmulti, P,
                       Yc);
         }
@@ -1414,7 +1437,6 @@ void sp_ttmc_compact(dt_ctx *ctx, const dt_sptensor *sp, const double *const *Ut
         f.R[d] = (int)R[m];
         d++;
     }
-    DevMem part(ctx, std::max<int64_t>(mc.nslots, 1) * P * sizeof(double));
     if (timer) timer->begin();
     // The cut between the low and the high group that needs the fewest tiles,
     // then the fewest gathers (tiles of a side times its modes).
@@ -1436,7 +1458,7 @@ void sp_ttmc_compact(dt_ctx *ctx, const dt_sptensor *sp, const double *const *Ut
         }
     }
 #define DT_ROWS(NO, NLO)                                                                   \
-    rows_dispatch<NO, NLO>(ctx, mc, no, nlo, sp->nnz, f, Plo, P / Plo, Yc, part.as<double>())
+    rows_dispatch<NO, NLO>(ctx, mc, no, nlo, sp->nnz, f, Plo, P / Plo, Yc, part)
     if (no == 1) DT_ROWS(1, 1);
     else if (no == 3 && nlo == 1) DT_ROWS(3, 1);
     else if (no == 3) DT_ROWS(3, 2);
@@ -1444,7 +1466,7 @@ void sp_ttmc_compact(dt_ctx *ctx, const dt_sptensor *sp, const double *const *Ut
 #undef DT_ROWS
     if (mc.nmulti > 0) {
         const unsigned blocks = (unsigned)std::min<int64_t>(mc.nmulti, 65535);
-        DT_LAUNCH(ctx, combine_partials_kernel, blocks, 256 * COMB_SPLIT, 0, part.as<double>(),
+        DT_LAUNCH(ctx, combine_partials_kernel, blocks, 256 * COMB_SPLIT, 0, (const double *)part,
                   mc.multi_row.as<int32_t>(), mc.multi_first.as<int32_t>(),
                   mc.multi_count.as<int32_t>(), mc.nmulti, P, Yc);
     }
@@ -1459,20 +1481,24 @@ void sp_ttmc_compact(dt_ctx *ctx, const dt_sptensor *sp, const double *const *Ut
     }
 }
 
+// `scratch`: mtr_blocks(nrows, most) x P x Rn doubles (null: allocated here, for
+// two blocks an SM).
 void sp_mtr(dt_ctx *ctx, const dt_sptensor *sp, const double *Yc, int mode, int P,
-            const double *Un, int Rn, double *L) {
+            const double *Un, int Rn, double *L, double *scratch = nullptr, int64_t most = 0) {
     const ModeCopy &mc = sp->modes[mode];
     SummaryScope sc(ctx, "Function::ttmc_mTR()", 2.0 * mc.nrows * P * Rn,
                     8.0 * mc.nrows * (P + Rn));
     DT_CHECK_ARG(Rn <= 32, "sparse ttmc_mTR: R_n (%d) must be <= 32", Rn);
-    const int64_t target = 2LL * ctx->num_sms;
-    const int64_t rpb = std::max<int64_t>(64, (mc.nrows + target - 1) / target);
-    const int nblk = (int)std::max<int64_t>(1, (mc.nrows + rpb - 1) / rpb);
-    DevMem part(ctx, (size_t)nblk * P * Rn * sizeof(double));
+    if (!scratch) most = 2LL * ctx->num_sms;
+    const int64_t rpb = mtr_rows(mc.nrows, most);
+    const int nblk = mtr_blocks(mc.nrows, most);
+    DevMem own;
+    if (!scratch) own.alloc(ctx, (size_t)nblk * P * Rn * sizeof(double));
+    double *const part = scratch ? scratch : own.as<double>();
     const int ntl = (Rn + 7) / 8;
 #define DT_MTR(N)                                                                          \
     DT_LAUNCH(ctx, mtr_mma_kernel<N>, nblk, 256, 0, Yc, mc.rows.as<int32_t>(), mc.nrows, P, \
-              Un, Rn, rpb, part.as<double>())
+              Un, Rn, rpb, part)
     if (ntl == 1) DT_MTR(1);
     else if (ntl == 2) DT_MTR(2);
     else if (ntl == 3) DT_MTR(3);
@@ -1480,15 +1506,15 @@ void sp_mtr(dt_ctx *ctx, const dt_sptensor *sp, const double *Yc, int mode, int 
 #undef DT_MTR
     const int64_t n = (int64_t)P * Rn;
     DT_LAUNCH(ctx, sum_blocks_kernel, std::max(1u, std::min<unsigned>(ceil_div(n, 64), 65535)),
-              256, 0, part.as<double>(), nblk, n, L);
+              256, 0, (const double *)part, nblk, n, L);
 }
 
+// At most `most` CTAs.
 template <int N, bool ORTH>
 void launch_mtl(dt_ctx *ctx, const ModeCopy &mc, const double *Yc, int P, const double *L, int Rn,
-                double *out, const GramFinish &f) {
+                double *out, const GramFinish &f, int64_t most) {
     const size_t smem = (size_t)((P + 3) & ~3) * (8 * N + 4) * sizeof(double);
     const bool lsm = smem <= 160 * 1024;
-    const int64_t most = ORTH ? orth_max_blocks(ctx) : 4LL * ctx->num_sms;
     const unsigned blocks = std::max(
         1u, std::min<unsigned>(ceil_div((mc.nrows + 7) / 8, 8), (unsigned)most));
     if (lsm) {
@@ -1504,13 +1530,13 @@ void launch_mtl(dt_ctx *ctx, const ModeCopy &mc, const double *Yc, int P, const 
 
 template <bool ORTH>
 void mtl_dispatch(dt_ctx *ctx, const ModeCopy &mc, const double *Yc, int P, const double *L, int Rn,
-                  double *out, const GramFinish &f) {
+                  double *out, const GramFinish &f, int64_t most) {
     DT_CHECK_ARG(Rn <= 32, "sparse ttmc_mTL: R_n (%d) must be <= 32", Rn);
     switch ((Rn + 7) / 8) {
-        case 1: launch_mtl<1, ORTH>(ctx, mc, Yc, P, L, Rn, out, f); break;
-        case 2: launch_mtl<2, ORTH>(ctx, mc, Yc, P, L, Rn, out, f); break;
-        case 3: launch_mtl<3, ORTH>(ctx, mc, Yc, P, L, Rn, out, f); break;
-        default: launch_mtl<4, ORTH>(ctx, mc, Yc, P, L, Rn, out, f); break;
+        case 1: launch_mtl<1, ORTH>(ctx, mc, Yc, P, L, Rn, out, f, most); break;
+        case 2: launch_mtl<2, ORTH>(ctx, mc, Yc, P, L, Rn, out, f, most); break;
+        case 3: launch_mtl<3, ORTH>(ctx, mc, Yc, P, L, Rn, out, f, most); break;
+        default: launch_mtl<4, ORTH>(ctx, mc, Yc, P, L, Rn, out, f, most); break;
     }
 }
 
@@ -1520,7 +1546,7 @@ void sp_mtl(dt_ctx *ctx, const dt_sptensor *sp, const double *Yc, int mode, int 
     SummaryScope sc(ctx, "Function::ttmc_mTL()", 2.0 * mc.nrows * P * Rn,
                     8.0 * mc.nrows * (P + Rn));
     DT_CUDA(cudaMemsetAsync(out, 0, sp->shape[mode] * Rn * sizeof(double), ctx->stream));
-    mtl_dispatch<false>(ctx, mc, Yc, P, L, Rn, out, GramFinish{});
+    mtl_dispatch<false>(ctx, mc, Yc, P, L, Rn, out, GramFinish{}, 4LL * ctx->num_sms);
 }
 
 void detach_sptensors(dt_ctx *ctx) {
@@ -1756,22 +1782,42 @@ int dt_sp_hooi_from(dt_ctx *ctx, const dt_sptensor *sp, const int64_t *R, int ma
             ptrs[m] = d;
         }
         upload_pieces(ctx, in);
-        int64_t maxYc = 1;
-        for (int m = 0; m < nd; m++)
-            maxYc = std::max<int64_t>(maxYc, sp->modes[m].nrows * kron_len(R, nd, m));
-        DevMem Yc(ctx, maxYc * sizeof(double));
-        DevMem L(ctx, 1024 * 32 * sizeof(double));
-        // W = Y_(n) L over the non-empty rows, and the orthonormalisation's
-        // scratch, for every mode in turn.
-        size_t wbytes = 8, obytes = 8;
+        // All memory of the sweeps, for every mode in turn: Y_(n), in whose place
+        // the orthonormalisation's first product comes (Y_(n) is read for the last
+        // time when W = Y_(n) L over the non-empty rows is made); the TTMc's
+        // partial rows, in whose place come L and the partial sums of L, then W.
+        int64_t maxYc = 1, maxL = 0, maxW = 1, parts = 1, maxR = 1, blocks = 1;
         for (int m = 0; m < nd; m++) {
-            wbytes = std::max(wbytes, (size_t)(sp->modes[m].nrows * R[m]) * sizeof(double));
-            obytes = std::max(obytes, orth_scratch_bytes(ctx, (int)R[m], sp->modes[m].nrows));
+            const ModeCopy &mc = sp->modes[m];
+            const int64_t P = kron_len(R, nd, m);
+            maxYc = std::max(maxYc, mc.nrows * std::max(P, R[m]));
+            maxL = std::max(maxL, (P * R[m] + 31) / 32 * 32);  // (W on a boundary of lines)
+            maxW = std::max(maxW, mc.nrows * R[m]);
+            parts = std::max(parts, ttmc_scratch(mc, nd, P));
+            maxR = std::max(maxR, R[m]);
+            blocks = std::max(blocks, orth_blocks(ctx, mc.nrows));
         }
-        const size_t nints = GRAM_COUNTERS + nd;  // arrival counters, a flag per mode
-        DevMem W(ctx, wbytes), oscr(ctx, obytes), oints(ctx, nints * sizeof(int));
-        int *const dep = oints.as<int>() + GRAM_COUNTERS;
-        DT_CUDA(cudaMemsetAsync(oints.get(), 0, nints * sizeof(int), ctx->stream));
+        DevMem Yc(ctx, maxYc * sizeof(double));
+        DevMem scratch, flags(ctx, nd * sizeof(int)), oscr;  // a flag per mode
+        // Fewer blocks for L's partial sums, down to one, where there is no room
+        // for those and the orthonormalisation (on one CTA at the least).
+        int64_t mtr_most = 2LL * ctx->num_sms;
+        for (;; mtr_most /= 2) {
+            int64_t behindL = maxW;
+            for (int m = 0; m < nd; m++)
+                behindL = std::max(behindL, mtr_blocks(sp->modes[m].nrows, mtr_most) *
+                                                kron_len(R, nd, m) * R[m]);
+            const size_t bytes = std::max(parts, maxL + behindL) * sizeof(double);
+            if (mtr_most == 1) scratch.alloc(ctx, bytes);
+            else if (!scratch.try_alloc(ctx, bytes)) continue;
+            const int64_t got = orth_alloc(ctx, oscr, (int)maxR, blocks, mtr_most > 1);
+            if (got == 0) continue;
+            blocks = got;
+            break;
+        }
+        double *const L = scratch.as<double>(), *const W = L + maxL;
+        int *const dep = flags.as<int>();
+        DT_CUDA(cudaMemsetAsync(dep, 0, nd * sizeof(int), ctx->stream));
         LaunchTimer timer(ctx, true);  // TTMc launches, reported as ttm_x_*
         SummaryScope sc(ctx, "Algorithm::SpTucker::Sp_HOOI_ALS()");
         DT_CUDA(cudaEventRecord(ctx->ev_start, ctx->stream));
@@ -1780,15 +1826,14 @@ int dt_sp_hooi_from(dt_ctx *ctx, const dt_sptensor *sp, const int64_t *R, int ma
                 const ModeCopy &mc = sp->modes[n];
                 const int P = (int)kron_len(R, nd, n), Rn = (int)R[n];
                 double *Un = const_cast<double *>(ptrs[n]);
-                sp_ttmc_compact(ctx, sp, ptrs, R, n, Yc.as<double>(), &timer);
-                sp_mtr(ctx, sp, Yc.as<double>(), n, P, Un, Rn, L.as<double>());
+                sp_ttmc_compact(ctx, sp, ptrs, R, n, Yc.as<double>(), &timer, L);
+                sp_mtr(ctx, sp, Yc.as<double>(), n, P, Un, Rn, L, W, mtr_most);
                 const OrthScratch os =
-                    orth_scratch(ctx, oscr.get(), Rn, mc.nrows, oints.as<int>(), dep + n);
+                    orth_scratch(oscr.get(), Yc.as<double>(), Rn, blocks, dep + n);
                 {
                     SummaryScope sm(ctx, "Function::ttmc_mTL()", 2.0 * mc.nrows * P * Rn,
                                     8.0 * mc.nrows * (P + Rn));
-                    mtl_dispatch<true>(ctx, mc, Yc.as<double>(), P, L.as<double>(), Rn,
-                                       W.as<double>(), os.f);
+                    mtl_dispatch<true>(ctx, mc, Yc.as<double>(), P, L, Rn, W, os.f, os.blocks);
                 }
                 SummaryScope so(ctx, "Operator::orth2()", 2.0 * R[n] * R[n] * sp->shape[n],
                                 8.0 * R[n] * sp->shape[n]);
@@ -1796,15 +1841,16 @@ int dt_sp_hooi_from(dt_ctx *ctx, const dt_sptensor *sp, const int64_t *R, int ma
                 if (it == 0)
                     DT_CUDA(cudaMemsetAsync(Un, 0, sp->shape[n] * Rn * sizeof(double),
                                             ctx->stream));
-                orth_finish(ctx, W.as<double>(), Rn, mc.nrows, os, Un, mc.rows.as<int32_t>());
+                orth_finish(ctx, W, Rn, mc.nrows, os, Un, mc.rows.as<int32_t>());
             }
         }
+        oscr.release();
         const int last = nd - 1;
         const int P = (int)kron_len(R, nd, last);
-        sp_ttmc_compact(ctx, sp, ptrs, R, last, Yc.as<double>());
-        sp_mtr(ctx, sp, Yc.as<double>(), last, P, ptrs[last], (int)R[last], L.as<double>());
+        sp_ttmc_compact(ctx, sp, ptrs, R, last, Yc.as<double>(), nullptr, L);
+        sp_mtr(ctx, sp, Yc.as<double>(), last, P, ptrs[last], (int)R[last], L, W, mtr_most);
         DevMem g2(ctx, sizeof(double));
-        sumsq(ctx, L.get(), DT_F64, (int64_t)P * R[last], g2.as<double>());
+        sumsq(ctx, L, DT_F64, (int64_t)P * R[last], g2.as<double>());
         DT_CUDA(cudaEventRecord(ctx->ev_stop, ctx->stream));
         double hg2 = 0.0;
         DT_CUDA(cudaMemcpyAsync(&hg2, g2.get(), sizeof(double), cudaMemcpyDeviceToHost,
@@ -1817,7 +1863,7 @@ int dt_sp_hooi_from(dt_ctx *ctx, const dt_sptensor *sp, const int64_t *R, int ma
             if (d) fail(DT_ERR_NUMERIC, "orth2: rows are linearly dependent");
         if (G) {
             DevView g(ctx, G, (size_t)P * R[last] * sizeof(double), false, true);
-            DT_CUDA(cudaMemcpyAsync(g.ptr(), L.get(), (size_t)P * R[last] * sizeof(double),
+            DT_CUDA(cudaMemcpyAsync(g.ptr(), L, (size_t)P * R[last] * sizeof(double),
                                     cudaMemcpyDeviceToDevice, ctx->stream));
             g.finish();
         }

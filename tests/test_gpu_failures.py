@@ -272,6 +272,42 @@ def test_hosvd_start_one_mode_at_a_time(shape, ranks, dtype, cap):
                 assert dense.principal_angle_max(a, b) <= 1e-10
 
 
+@pytest.mark.parametrize("r,n,cap", [(5, 300, 24804), (16, 100_000, 26_210_308), (32, 50_000, 27_222_020)])
+def test_row_orthonormalisation_in_little_room(r, n, cap):
+    """A cap that holds the matrix and its copy and little else: the Gram's partial
+    sums of fewer CTAs, at last of one.  Orthonormal to 1e-13 as without a cap."""
+    from diana_tucker_b200 import Context
+    W = np.random.default_rng(r).standard_normal((r, n))
+    with Context(0) as c:
+        c.set_mem_limit(cap)
+        out = c.orth2(W)
+        np.testing.assert_allclose(out @ out.T, np.eye(r), atol=1e-13)
+        Lm = W @ out.T
+        assert np.max(np.abs(np.triu(Lm, 1))) < 1e-12 * np.sqrt(n) and np.all(np.diag(Lm) > 0)
+
+
+@pytest.mark.parametrize("shape,R,nnz,cap", [
+    ((20000, 3000, 200), (16, 8, 8), 60000, 13664764), ((3001, 2003, 1009, 501), (5, 7, 6, 3), 30000, 6345860),
+    ((3000, 2000), (5, 5), 20000, 1223136), ((20000, 300, 200), (32, 32, 32), 60000, 106931420)])
+def test_sparse_hooi_in_little_room(shape, R, nnz, cap):
+    """A cap that holds the tensor, the factors, Y_(n) and one product of a factor's
+    size: the sweep fits, with the residual and subspaces of the uncapped call
+    (other partial sums: 1e-12, 1e-10)."""
+    from diana_tucker_b200 import Context, datasets
+    from oracle import dense
+    idx, vals, shape = datasets.sparse_zipf(shape, nnz, alpha=1.1, seed=3)
+    Ut0 = datasets.random_orthonormal_transposed(shape, R, 1)
+    with Context(0) as c:
+        sp = c.sptensor(idx, vals, shape)
+        G0, U0, r0 = sp.hooi(R, 2, Ut0)
+        c.set_mem_limit(cap)
+        G, U, r = sp.hooi(R, 2, Ut0)
+        sp.close()
+    assert abs(r["residual"] - r0["residual"]) <= 1e-12
+    for a, b in zip(U, U0):
+        assert dense.principal_angle_max(a, b) <= 1e-10
+
+
 @pytest.mark.parametrize("shape,mode,spare", [((200, 40, 21), 0, 1 << 20), ((181, 203, 157), 1, 0),
                                               ((500, 100, 24), 0, 1 << 21), ((40, 50), 0, 0),
                                               ((300, 200, 5), 1, 1 << 22)])
