@@ -613,6 +613,16 @@ struct BatchedState {
     }
 };
 
+bool release_batched_scratch(dt_ctx *ctx) {
+    if (ctx->batched.use_count() != 1) return false;  // none, or a running call's
+    BatchedState &st = *std::static_pointer_cast<BatchedState>(ctx->batched);
+    if (!st.scratch.get()) return false;
+    DT_CUDA(cudaStreamSynchronize(ctx->stream));
+    st.scratch.release();
+    st.scratch_grid = 0;
+    return true;
+}
+
 }  // namespace dt
 
 using namespace dt;
@@ -668,15 +678,14 @@ int dt_hooi_batched(dt_ctx *ctx, int count, const int64_t *shapes, const int64_t
         const std::vector<int64_t> sig = {count, maxI, maxR, sweeps, inner_iters, n_pair, n_quad};
         DT_CUDA(cudaSetDevice(ctx->device));
         if (!ctx->batched) ctx->batched = std::make_shared<BatchedState>();
-        BatchedState &st = *std::static_pointer_cast<BatchedState>(ctx->batched);
+        const auto state = std::static_pointer_cast<BatchedState>(ctx->batched);
+        BatchedState &st = *state;
         DevView xv(ctx, X, xn * sizeof(float), true, false);
         DevView uv(ctx, U, un * sizeof(double), true, true);
         DevView gv(ctx, G, gn * sizeof(double), false, true);
         DevView ev(ctx, relerr, count * sizeof(double), false, true);
-        if (!st.args.get()) {
-            st.args.alloc(ctx, sizeof(BatchArgs));
-            st.queue.alloc(ctx, sizeof(int));
-        }
+        if (!st.args.get()) st.args.alloc(ctx, sizeof(BatchArgs));
+        if (!st.queue.get()) st.queue.alloc(ctx, sizeof(int));
         const int64_t launches0 = ctx->launches;
 
         // Descriptor tables (shapes, ranks, offsets, items) in one device
@@ -694,6 +703,7 @@ int dt_hooi_batched(dt_ctx *ctx, int count, const int64_t *shapes, const int64_t
             std::memcpy(p + 3 * n3 + count, g_offsets, count * sizeof(int64_t));
             std::memcpy(p + 3 * n3 + 2 * count, items.data(), items.size() * sizeof(Item));
             if (st.tables_bytes < bytes) {
+                st.tables_bytes = 0;  // (also when the allocation fails)
                 st.tables.alloc(ctx, bytes);
                 st.tables_bytes = bytes;
             }
@@ -712,11 +722,16 @@ int dt_hooi_batched(dt_ctx *ctx, int count, const int64_t *shapes, const int64_t
             // memory only until the call returns; the runtime stages it.
             DT_CUDA(cudaStreamSynchronize(ctx->stream));
         };
-        auto ensure_scratch = [&](unsigned grid) {
-            if (st.scratch_grid < grid) {
-                st.scratch.alloc(ctx, (size_t)grid * SCR * sizeof(double));
-                st.scratch_grid = grid;
+        // Scratch for `grid` CTAs, or for as many as there is room for; how many.
+        auto with_scratch = [&](unsigned grid) {
+            if (st.scratch_grid >= grid) return grid;
+            st.scratch_grid = 0;
+            while (!st.scratch.try_alloc(ctx, (size_t)grid * SCR * sizeof(double))) {
+                if (grid == 1) st.scratch.alloc(ctx, SCR * sizeof(double));  // (fails)
+                grid = std::max(1u, grid * 3 / 4);
             }
+            st.scratch_grid = grid;
+            return grid;
         };
         BatchArgs base{};
         base.X = xv.as<float>();
@@ -756,8 +771,7 @@ int dt_hooi_batched(dt_ctx *ctx, int count, const int64_t *shapes, const int64_t
                         BatchArgs b = base;
                         upload(make_items(sord, cost, tmaxI, pk), b);
                         b.U = ucopy.as<double>();
-                        const unsigned grid = batched_grid(ctx, cand_nt[c]);
-                        ensure_scratch(grid);
+                        const unsigned grid = with_scratch(batched_grid(ctx, cand_nt[c]));
                         b.scratch = st.scratch.as<double>();
                         DT_CUDA(cudaMemcpyAsync(st.args.get(), &b, sizeof(b),
                                                 cudaMemcpyHostToDevice, ctx->stream));
@@ -786,8 +800,7 @@ int dt_hooi_batched(dt_ctx *ctx, int count, const int64_t *shapes, const int64_t
                 st.tuned[sig] = {nt, pack};
             }
         }
-        const unsigned grid = batched_grid(ctx, nt);
-        ensure_scratch(grid);
+        const unsigned grid = with_scratch(batched_grid(ctx, nt));
         const std::vector<Item> items = make_items(order, cost, tmaxI, pack);
         BatchArgs a = base;
         upload(items, a);

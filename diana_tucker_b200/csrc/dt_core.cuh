@@ -306,9 +306,10 @@ class DevArena {
 
 
 // Gives back one thing that ctx keeps for later calls and no running call uses:
-// a dense HOOI plan (the one used longest ago first).  False when there is none,
-// or when the stream is being captured.
+// a dense HOOI plan (the one used longest ago first), then the batched HOOI's
+// scratch.  False when there is none, or when the stream is being captured.
 bool release_idle(dt_ctx *ctx);
+bool release_batched_scratch(dt_ctx *ctx);
 
 // Stream-ordered device allocation owned by one call.
 class DevMem {

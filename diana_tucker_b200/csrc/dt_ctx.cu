@@ -189,7 +189,7 @@ bool release_idle(dt_ctx *ctx) {
         release_plan(ctx, ctx->hooi_plan_mixed);
         return true;
     }
-    return false;
+    return release_batched_scratch(ctx);
 }
 
 bool DevMem::try_alloc(dt_ctx *ctx, size_t bytes) {

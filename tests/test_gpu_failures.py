@@ -272,6 +272,64 @@ def test_hosvd_start_one_mode_at_a_time(shape, ranks, dtype, cap):
                 assert dense.principal_angle_max(a, b) <= 1e-10
 
 
+def _small_batch(count):
+    from diana_tucker_b200 import datasets
+    items = datasets.batched_small(count=count, seed=9)
+    rng = np.random.default_rng(1)
+    U0 = [[np.linalg.qr(rng.standard_normal((x.shape[n], r[n])))[0] for n in range(3)]
+          for x, r in items]
+    return [x for x, _ in items], [r for _, r in items], U0
+
+
+@pytest.mark.parametrize("block", [0, 128, 256, 512])
+def test_batch_in_little_room(block):
+    """A cap below the scratch of every CTA that fits the GPU: fewer CTAs, the same
+    results (block 0 may choose another shape: 1e-10)."""
+    from diana_tucker_b200 import Context
+    args = _small_batch(100)
+    with Context(0) as c:
+        want = c.hooi_batched(*args, sweeps=3, block_threads=block)
+    with Context(0) as c:
+        c.set_mem_limit(60_000_000)
+        got = c.hooi_batched(*args, sweeps=3, block_threads=block)
+        assert c.mem_usage()[1] <= 60_000_000
+        assert got[3]["grid"] < want[3]["grid"] or block == 0
+    if block:
+        assert np.array_equal(got[2], want[2])
+        assert all(np.array_equal(a, b) for a, b in zip(got[1], want[1]))
+    np.testing.assert_allclose(got[2], want[2], atol=1e-10)
+
+
+def test_batch_after_one_that_found_no_room(ctx):
+    """A batch whose scratch cannot grow fails; what it gave up on the way is not
+    taken for there by the next."""
+    import torch
+
+    from diana_tucker_b200 import Context, DTError
+    L = _codes()
+    tensors, ranks, U0 = _small_batch(24)
+    with Context(0) as c:
+        pk = c.pack_batched(tensors, ranks, U0)
+        Xd, U0d = torch.from_numpy(pk["X"]).cuda(), torch.from_numpy(pk["U"]).cuda()
+        Gd = torch.zeros(pk["g_size"], dtype=torch.float64, device="cuda")
+        Ed = torch.zeros(pk["count"], dtype=torch.float64, device="cuda")
+
+        def call(block):
+            Ud = U0d.clone()
+            torch.cuda.synchronize()
+            c.hooi_batched_packed(pk, Ud, Gd, Ed, X=Xd, sweeps=2, block_threads=block)
+            return Ed.cpu().numpy()
+
+        want = call(512)
+        c.set_mem_limit(1)
+        for _ in range(2):
+            with pytest.raises(DTError) as e:
+                call(128)
+            assert e.value.code == L.DT_ERR_NOMEM
+        c.set_mem_limit(0)
+        assert np.array_equal(call(512), want)
+
+
 @pytest.mark.parametrize("r,n,cap", [(5, 300, 24804), (16, 100_000, 26_210_308), (32, 50_000, 27_222_020)])
 def test_row_orthonormalisation_in_little_room(r, n, cap):
     """A cap that holds the matrix and its copy and little else: the Gram's partial
