@@ -218,9 +218,9 @@ bool is_device_ptr(const void *p);
 // megabyte on, several host threads copy one-megabyte chunks between the
 // caller's memory and the context's pinned staging while the DMA of other
 // chunks runs (the driver's own staging uses one thread: 36 MB up 3.4 ms, down
-// 2.1 ms); smaller ones are left to the driver.  upload_pieces returns once the
-// host memory has been read, its DMA in order on ctx->stream; download_pieces
-// once it has been written.
+// 2.1 ms); smaller ones, and all where the staging cannot be pinned, are left to
+// the driver.  upload_pieces returns once the host memory has been read, its DMA
+// in order on ctx->stream; download_pieces once it has been written.
 struct HostPiece {
     void *dev;
     void *host;

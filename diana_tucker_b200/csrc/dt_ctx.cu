@@ -6,7 +6,6 @@
 #include <map>
 #include <mutex>
 #include <optional>
-#include <system_error>
 #include <thread>
 
 #include "dt_core.cuh"
@@ -406,9 +405,10 @@ void over_threads(dt_ctx *ctx, size_t n, const std::function<cudaError_t(size_t)
         }
     };
     std::vector<std::thread> pool;
+    pool.reserve(kCopyThreads);
     try {
         for (size_t k = 1; k < std::min(most, n); k++) pool.emplace_back(work);
-    } catch (const std::system_error &) {  // no more threads: the ones there do it
+    } catch (...) {  // no more threads or memory for one: the ones there do it
     }
     work();
     for (auto &t : pool) t.join();
@@ -437,8 +437,6 @@ void stream_after(cudaStream_t later, cudaStream_t earlier) {
 void over_lanes(dt_ctx *ctx, const std::vector<HostPiece> &pieces,
                 const std::function<cudaError_t(cudaStream_t, const std::vector<Chunk> &,
                                                 char *const *, const cudaEvent_t *)> &run) {
-    if (!ctx->big_stage)
-        DT_CUDA(cudaHostAlloc(&ctx->big_stage, dt_ctx::kBigStageBytes, cudaHostAllocDefault));
     const bool stand_in = ctx->stream == cudaStreamPerThread;
     const cudaStream_t dma = stand_in ? ctx->own_stream : ctx->stream;
     if (stand_in) stream_after(dma, ctx->stream);
@@ -472,17 +470,23 @@ void over_lanes(dt_ctx *ctx, const std::vector<HostPiece> &pieces,
     if (stand_in) stream_after(ctx->stream, dma);
 }
 
-size_t total_bytes(const std::vector<HostPiece> &pieces) {
-    size_t t = 0;
-    for (const HostPiece &p : pieces) t += p.bytes;
-    return t;
+// Whether the pieces go through the staging: enough bytes, and memory to pin.
+bool staged(dt_ctx *ctx, const std::vector<HostPiece> &pieces) {
+    size_t total = 0;
+    for (const HostPiece &p : pieces) total += p.bytes;
+    if (total < kStageFrom) return false;
+    if (!ctx->big_stage &&
+        cudaHostAlloc(&ctx->big_stage, dt_ctx::kBigStageBytes, cudaHostAllocDefault) != cudaSuccess) {
+        cudaGetLastError();
+        ctx->big_stage = nullptr;
+    }
+    return ctx->big_stage != nullptr;
 }
 
 }  // namespace
 
 void upload_pieces(dt_ctx *ctx, const std::vector<HostPiece> &pieces) {
-    const size_t total = total_bytes(pieces);
-    if (total < kStageFrom) {
+    if (!staged(ctx, pieces)) {
         for (const HostPiece &p : pieces)
             DT_CUDA(cudaMemcpyAsync(p.dev, p.host, p.bytes, cudaMemcpyHostToDevice, ctx->stream));
         return;
@@ -505,8 +509,7 @@ void upload_pieces(dt_ctx *ctx, const std::vector<HostPiece> &pieces) {
 }
 
 void download_pieces(dt_ctx *ctx, const std::vector<HostPiece> &pieces) {
-    const size_t total = total_bytes(pieces);
-    if (total < kStageFrom) {
+    if (!staged(ctx, pieces)) {
         for (const HostPiece &p : pieces)
             DT_CUDA(cudaMemcpyAsync(p.host, p.dev, p.bytes, cudaMemcpyDeviceToHost, ctx->stream));
         DT_CUDA(cudaStreamSynchronize(ctx->stream));
