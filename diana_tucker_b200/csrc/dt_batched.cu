@@ -19,8 +19,10 @@
 // large intermediate (I_1 x I_2 x R_3) is in the group's slice of global scratch;
 // the factors, Y_(n) and its Gram (which takes Y_(n)'s place) live in shared
 // memory.  In a subspace step each warp keeps its rows of S L in registers, laid
-// out as the next products' fragments, from the product to the new factor.  Sums
-// go in a fixed order for a given number of warps.  4096 tensors (modes 8 to 64,
+// out as the next products' fragments, from the product to the new factor.  Every
+// sum goes in an order of the tensor's own (over its 8 x 8 tiles; over 512 classes
+// of entries, as many as the largest block has threads): the results are the same
+// bit for bit for every block size and packing, whatever the tuner takes.  4096 tensors (modes 8 to 64,
 // ranks 2 to 8, 10 sweeps): 11.4 ms, of it about half the two passes over X at 0.8
 // of the FP64 tensor rate (ranks padded to 8 columns); 100 tensors 1.14 ms.  With
 // one FMA chain per thread and entry on the CUDA cores 23.3 and 2.4 ms.
@@ -56,12 +58,13 @@ constexpr int BMAX_K = BMAX_R * BMAX_R;  // largest product of two ranks
 
 // Shared-memory doubles one tensor of largest mode size m needs: the factors
 // (rows padded to whole tiles, 8 columns), Y_(n) or its Gram (rows of up to 64
-// at a pitch of 4 mod 16), reduction scratch.  Gram shares and factorisation
-// scratch, 128 doubles a warp, come on top for the whole CTA.
+// at a pitch of 4 mod 16; before and after the sweeps the classes of a sum).  The
+// Gram shares of a subspace step, two tiles of 64 doubles a warp, come on top for
+// the whole CTA.
 __host__ __device__ constexpr int tile8(int n) { return (n + 7) / 8 * 8; }
 __host__ __device__ constexpr int pitch16(int n) { return (n + 11) / 16 * 16 + 4; }
 __host__ __device__ constexpr int slot_doubles(int m) {
-    return 3 * tile8(m) * BMAX_R + tile8(m) * pitch16(BMAX_K) + 40;
+    return 3 * tile8(m) * BMAX_R + tile8(m) * pitch16(BMAX_K);
 }
 constexpr int SLOT = slot_doubles(BMAX_I);                    // one CTA
 // Room for four of the largest tensors that go four to a CTA.
@@ -113,27 +116,27 @@ struct Grp {
     int bar;  // named barrier id (1..4; 0 is __syncthreads)
     int w, W;          // this warp, warps
     int g, t;          // fragment row / column of the lane
-    int part;          // offset of W x WARP_SCR: the warps' Gram shares and scratch
+    int part;          // offset of W x WARP_SCR: the tiles' Gram shares
 };
 
 __device__ __forceinline__ void gsync(const Grp &g) {
     asm volatile("bar.sync %0, %1;" ::"r"(g.bar), "r"(g.gs) : "memory");
 }
 
-// Sum over the group, fixed order (warp tree, then warps in order).
-__device__ double gsum(double v, double *red, const Grp &g) {
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-    const int w = g.lt >> 5, l = g.lt & 31;
+// Sum of the group's 512 classes in `cls` (shared memory), an order that does not
+// depend on the group's size.
+constexpr int CLASSES = 512;
+static_assert(tile8(1) * pitch16(BMAX_K) >= CLASSES, "the classes take Y_(n)'s place");
+__device__ double gsum(double *cls, const Grp &g) {
     gsync(g);
-    if (l == 0) red[w] = v;
-    gsync(g);
-    if (g.lt == 0) {
+    if (g.w == 0) {
         double s = 0.0;
-        for (int i = 0; i < (g.gs >> 5); i++) s += red[i];
-        red[32] = s;
+        for (int i = g.lt; i < CLASSES; i += 32) s += cls[i];
+        for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+        if (g.lt == 0) cls[0] = s;
     }
     gsync(g);
-    const double r = red[32];
+    const double r = cls[0];
     gsync(g);
     return r;
 }
@@ -318,8 +321,8 @@ __device__ __noinline__ void gmgs(int uo, int n, int r, int lt) {
 // and W = 1: two are enough).  It computes (S U)^T there: with U as the A operand
 // a lane holds column g of Z = S U at rows 2 t, 2 t + 1, which are the fragments
 // of Z^T Z as they stand (even rows one k-step, odd rows another).  Three barriers
-// a step: the Gram shares (then Z takes U's place), the first warp's L^{-1}, the
-// new U.  Bound by latency: a step of 40 x 4 takes about 2700 cycles alone on an SM
+// a step: each tile's share of the Gram (then Z takes U's place), the first warp's
+// L^{-1}, the new U.  Bound by latency: a step of 40 x 4 takes about 2700 cycles alone on an SM
 // with 4 warps, 3500 with four tensors on it; shuffles in place of the trip of Z
 // through shared memory, or every warp factoring the sum for itself, were slower.
 __device__ __noinline__ void gsubspace(int ys, int n, int ps, int uo, int r, int iters, Grp g) {
@@ -330,8 +333,7 @@ __device__ __noinline__ void gsubspace(int ys, int n, int ps, int uo, int r, int
     const double *s0 = S + (8 * (have0 ? m0 : 0) + g.g) * ps + g.t;
     const double *s1 = S + (8 * (have1 ? m1 : 0) + g.g) * ps + g.t;
     const double *u0 = U + u_at(g.t, g.g), *u1 = U + u_at(4 + g.t, g.g);
-    double *const part = bt_sm + g.part, *mine = part + g.w * WARP_SCR + g.g * 8 + 2 * g.t;
-    double *const Li = part + 64;
+    double *const Li = bt_sm + g.part, *const mine = Li + g.g * 8 + 2 * g.t;
 #pragma unroll 1
     for (int it = 0; it < iters; it++) {
         // Z's tiles, two chains each (even and odd k-steps); what is past n is zero.
@@ -349,15 +351,18 @@ __device__ __noinline__ void gsubspace(int ys, int n, int ps, int uo, int r, int
                 }
             }
         }
-        double d[2][2] = {};
+        double d[2][2][2] = {};
 #pragma unroll
-        for (int m = 0; m < 2; m++)
+        for (int m = 0; m < 2; m++) {
 #pragma unroll
             for (int q = 0; q < 2; q++) {
                 z[m][q] += y[m][q];
-                bt_dmma(d[q][0], d[q][1], z[m][q], z[m][q]);
+                bt_dmma(d[m][q][0], d[m][q][1], z[m][q], z[m][q]);
             }
-        *reinterpret_cast<double2 *>(mine) = make_double2(d[0][0] + d[1][0], d[0][1] + d[1][1]);
+            if (m ? have1 : have0)
+                *reinterpret_cast<double2 *>(mine + 64 * (m ? m1 : m0)) =
+                    make_double2(d[m][0][0] + d[m][1][0], d[m][0][1] + d[m][1][1]);
+        }
         gsync(g);
 #pragma unroll
         for (int m = 0; m < 2; m++)
@@ -366,17 +371,17 @@ __device__ __noinline__ void gsubspace(int ys, int n, int ps, int uo, int r, int
                 U[u_at(i, g.g)] = z[m][0];
                 U[u_at(i + 1, g.g)] = z[m][1];
             }
-        // The first warp adds the shares in order and factors the sum.
+        // The first warp adds the tiles' shares in order and factors the sum, in the
+        // first share's place.
         if (g.w == 0) {
             double2 a = *reinterpret_cast<const double2 *>(mine);
-            const int shares = min(g.W, nt);
 #pragma unroll 4
-            for (int w = 1; w < shares; w++) {
-                const double2 p = *reinterpret_cast<const double2 *>(mine + w * WARP_SCR);
+            for (int k = 1; k < nt; k++) {
+                const double2 p = *reinterpret_cast<const double2 *>(mine + 64 * k);
                 a.x += p.x;
                 a.y += p.y;
             }
-            *reinterpret_cast<double2 *>(Li + g.g * 8 + 2 * g.t) = a;
+            *reinterpret_cast<double2 *>(mine) = a;
             __syncwarp();
             double c[BMAX_R];
             const bool ok = warp_chol_linv<BMAX_R>(Li, BMAX_R, r, c);
@@ -424,7 +429,6 @@ __device__ __forceinline__ void hooi_one(const BatchArgs &a, int t, int slot, do
     const int uo = slot, us = m8 * BMAX_R, ys = slot + 3 * us;
     double *U0 = bt_sm + uo, *U1 = U0 + us, *U2 = U1 + us;
     double *YS = bt_sm + ys;                      // Y_(n), then its Gram
-    double *red = YS + m8 * pitch16(BMAX_K);
     double *Ylast = T + (int64_t)m * m * BMAX_R;  // the final Y_(3), I2 x K
     const float *X = a.X + a.xoff[t];
     double *ug[3] = {a.U + a.uoff[3 * t], a.U + a.uoff[3 * t + 1], a.U + a.uoff[3 * t + 2]};
@@ -434,10 +438,13 @@ __device__ __forceinline__ void hooi_one(const BatchArgs &a, int t, int slot, do
     for (int e = g.lt; e < I1 * R1; e += g.gs) U1[u_at(e % I1, e / I1)] = ug[1][e];
     for (int e = g.lt; e < I2 * R2; e += g.gs) U2[u_at(e % I2, e / I2)] = ug[2][e];
     const int nx = I0 * I1 * I2;
-    double s = 0.0;
+    for (int c = g.lt; c < CLASSES; c += g.gs) {
+        double s = 0.0;
 #pragma unroll 8
-    for (int e = g.lt; e < nx; e += g.gs) s = fma((double)X[e], (double)X[e], s);
-    const double x2 = gsum(s, red, g);
+        for (int e = c; e < nx; e += CLASSES) s = fma((double)X[e], (double)X[e], s);
+        YS[c] = s;
+    }
+    const double x2 = gsum(YS, g);
     const int I01 = I0 * I1, I12 = I1 * I2;
     for (int sw = 0; sw < a.sweeps; sw++) {
         // T = X x_3 U_3^T  (I0 x I1 x R2): rows (i0, i1).
@@ -472,15 +479,15 @@ __device__ __forceinline__ void hooi_one(const BatchArgs &a, int t, int slot, do
     // are those of the final sweep), relative error in FP64.
     const int K = R0 * R1;
     double *Gout = a.G + a.goff[t];
-    double g2 = 0.0;
     for (int e = g.lt; e < K * R2; e += g.gs) {
         const int k = e % K, r2 = e / K;
         double acc = 0.0;
         for (int i2 = 0; i2 < I2; i2++) acc = fma(Ylast[i2 + I2 * k], U2[u_at(i2, r2)], acc);
         Gout[e] = acc;
-        g2 = fma(acc, acc, g2);
+        YS[e] = acc * acc;  // at most 512 entries
     }
-    g2 = gsum(g2, red, g);
+    for (int e = K * R2 + g.lt; e < CLASSES; e += g.gs) YS[e] = 0.0;
+    const double g2 = gsum(YS, g);
     // A non-finite input gives a NaN error (fmax would turn NaN into 0).
     const double q = 1.0 - g2 / x2;
     if (g.lt == 0) a.relerr[t] = isnan(q) ? q : sqrt(fmax(0.0, q));

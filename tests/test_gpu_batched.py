@@ -163,3 +163,22 @@ def test_batched_on_the_legacy_default_stream(ctx):
         torch.cuda.synchronize()
     assert rep["graph_reused"] == 0
     np.testing.assert_array_equal(Ed.cpu().numpy(), e1)
+
+
+@pytest.mark.parametrize("lo,hi", [(8, 64), (5, 16), (12, 32)])
+def test_batched_results_do_not_depend_on_the_launch_shape(ctx, lo, hi):
+    """Factors, cores and relative errors bit for bit equal for every block size
+    (groups of 1 to 16 warps with two and four tensors to a CTA), for the tuner's
+    choice of block and packing, and for a tensor alone."""
+    items, U0 = _batch(60, 21, lo=lo, hi=hi)
+    tensors, ranks = [X for X, _ in items], [r for _, r in items]
+    outs = [ctx.hooi_batched(tensors, ranks, U0, sweeps=4, block_threads=b)[:3]
+            for b in (128, 256, 512, 0)]
+    for U, G, e in outs[1:]:
+        assert np.array_equal(e, outs[0][2])
+        for t in range(len(items)):
+            assert np.array_equal(G[t], outs[0][1][t])
+            assert all(np.array_equal(a, b) for a, b in zip(U[t], outs[0][0][t]))
+    for t in (0, 17, 59):
+        U, G, e, _ = ctx.hooi_batched([tensors[t]], [ranks[t]], [U0[t]], sweeps=4)
+        assert e[0] == outs[0][2][t] and np.array_equal(G[0], outs[0][1][t])
