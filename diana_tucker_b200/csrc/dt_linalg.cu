@@ -1159,22 +1159,38 @@ __global__ void __launch_bounds__(128) hqr_batch_kernel(OrthTable tab) {
     hqr_device(W, mb, nb, W + mb * nb, tab.Q[b], red);
 }
 
-// Cholesky of the r x r SPD G (col-major) and L^{-1} (lower) for the row
-// orthonormalisation; one CTA, r small.  Output Linv col-major.
-__global__ void chol_lower_inv_kernel(const double *Gg, int r, double *Linv, int *flag) {
-    extern __shared__ double sm[];
-    double *G = sm, *Ri = sm + r * r;
-    for (int e = threadIdx.x; e < r * r; e += blockDim.x) G[e] = Gg[e];  // symmetric
+// Cholesky of the r x r SPD G (col-major, its lower triangle overwritten) and L^{-1}
+// (lower, col-major) for the orthonormalisation of more than 32 rows; one CTA of 1024
+// threads, r <= 1024, both matrices in global memory (L2).  The row operations that
+// eliminate G are applied to the identity as well.  Not on a measured path: bound
+// by one SM's traffic with L2.
+__global__ void __launch_bounds__(1024) chol_lower_inv_kernel(double *G, int r, double *Linv,
+                                                              int *flag) {
+    __shared__ double l[1024], y[1024];  // column k of L below k, row k of L^{-1}
+    const int t = threadIdx.x, w = t >> 5, lane = t & 31;
+    const double least = fmax(1e-28 * G[0], 2.3e-308);
+    for (int c = w; c < r; c += 32)
+        for (int i = lane; i < r; i += 32) Linv[i + (int64_t)r * c] = i == c ? 1.0 : 0.0;
     __syncthreads();
-    if (threadIdx.x < 32) {
-        const bool ok = warp_chol_inv<32>(G, Ri, r);
-        if (!ok && threadIdx.x == 0) atomicOr(flag, 1);
-    }
-    __syncthreads();
-    // G = R^T R with R upper; L = R^T, so L^{-1} = (R^{-1})^T.
-    for (int e = threadIdx.x; e < r * r; e += blockDim.x) {
-        const int i = e % r, c = e / r;  // Linv(i, c) = Rinv(c, i)
-        Linv[e] = Ri[c * r + i];
+    for (int k = 0; k < r; k++) {
+        const double d = G[k + (int64_t)r * k];
+        if (t == 0 && !(d > least)) atomicOr(flag, 1);
+        const double ri = 1.0 / sqrt(d);
+        for (int i = t; i < r; i += 1024) {
+            if (i > k) {
+                l[i] = G[i + (int64_t)r * k] * ri;
+            } else {
+                y[i] = Linv[k + (int64_t)r * i] * ri;
+                Linv[k + (int64_t)r * i] = y[i];
+            }
+        }
+        __syncthreads();
+        for (int c = w; c < r; c += 32) {
+            double *col = c > k ? G + (int64_t)r * c : Linv + (int64_t)r * c;
+            const double f = c > k ? l[c] : y[c];
+            for (int i = (c > k ? c : k + 1) + lane; i < r; i += 32) col[i] = fma(-l[i], f, col[i]);
+        }
+        __syncthreads();
     }
 }
 
@@ -1540,8 +1556,8 @@ void orth2_rows(dt_ctx *ctx, double *A, int64_t len1, int64_t len2) {
     DevMem T(ctx, len1 * len2 * sizeof(double));
     for (int pass = 0; pass < 2; pass++) {
         gemm_f64(ctx, 0, 1, len1, len1, len2, A, len1, A, len1, G.as<double>(), len1, 0.0);
-        DT_LAUNCH(ctx, chol_lower_inv_kernel, 1, 256, 2 * len1 * len1 * sizeof(double),
-                  G.as<double>(), (int)len1, Li.as<double>(), flag.as<int>());
+        DT_LAUNCH(ctx, chol_lower_inv_kernel, 1, 1024, 0, G.as<double>(), (int)len1,
+                  Li.as<double>(), flag.as<int>());
         gemm_f64(ctx, 0, 0, len1, len2, len1, Li.as<double>(), len1, A, len1, T.as<double>(),
                  len1, 0.0);
         DT_CUDA(cudaMemcpyAsync(A, T.get(), len1 * len2 * sizeof(double),

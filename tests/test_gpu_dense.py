@@ -102,6 +102,30 @@ def test_small_linear_algebra(ctx, oracle_ref):
     assert np.max(np.abs(np.triu(Lm, 1))) < 1e-12 and np.all(np.diag(Lm) > 0)
 
 
+@pytest.mark.parametrize("r,n", [(1, 1), (8, 40), (31, 200), (32, 128), (33, 140), (40, 160), (64, 256),
+                                 (97, 400), (257, 1100)])
+def test_orth2_row_counts(ctx, r, n):
+    """Row orthonormalisation on the tensor cores (up to 32 rows) and above: the
+    rows of Gram-Schmidt, which are those of the triangular factorisation with a
+    positive diagonal.  Gaussian rows four times as long as there are rows have a
+    condition below 10: 1e-12."""
+    W = np.random.default_rng(r).standard_normal((r, n))
+    Q, R = np.linalg.qr(W.T)
+    O = ctx.orth2(W)
+    np.testing.assert_allclose(O, (Q * np.sign(np.diag(R))).T, rtol=0, atol=1e-12)
+    np.testing.assert_allclose(O @ O.T, np.eye(r), atol=1e-13)
+
+
+def test_orth2_zero_row(ctx):
+    from diana_tucker_b200 import DTError
+    for r in (20, 50):
+        W = np.random.default_rng(r).standard_normal((r, 300))
+        W[-1] = 0.0
+        with pytest.raises(DTError) as e:
+            ctx.orth2(W)
+        assert e.value.code == 4
+
+
 @pytest.mark.parametrize("shape,mode,J", [
     ((5, 7), 0, 1), ((16, 64), 0, 8), ((17, 65), 0, 9), ((33, 129, 3), 0, 24), ((48, 900, 50), 0, 16),
     ((2, 31, 40), 1, 7), ((3, 16, 43), 1, 17), ((63, 15, 9), 1, 16), ((64, 32, 11), 1, 33),
