@@ -58,9 +58,6 @@ bool pdl_enabled() {
     return on;
 }
 
-namespace {
-}  // namespace
-
 bool graphs_enabled() {
     static const bool on = [] {
         const char *e = std::getenv("DT_DISABLE_GRAPHS");

@@ -119,15 +119,15 @@ __global__ void __launch_bounds__(LA_NT) hqr_kernel(const double *A, int64_t m, 
     }
 }
 
-// Cholesky G = R^T R of the r x r SPD matrix in smem (row-major G[i*r+c]) by
-// one warp, then Rinv = R^{-1} (upper, row-major).  Lane c keeps column c in
-// registers and rows are exchanged with shuffles, so the r pivots form one
-// short dependency chain (one sqrt and one reciprocal per pivot).  Returns
-// false on a non-positive pivot.  Runs in warp 0 only; r <= 32.
-template <int RMAX, bool INV = true>
-__device__ bool warp_chol_inv(double *G, double *Rinv, int r) {
+// Cholesky G = R^T R of the r x r SPD matrix in smem (row-major G[i*r+c]), R in
+// G's place, by one warp.  Lane c keeps column c in registers and rows are
+// exchanged with shuffles, so the r pivots form one short dependency chain (one
+// sqrt and one reciprocal per pivot).  Returns false on a non-positive pivot.
+// Runs in warp 0 only; r <= 32.
+template <int RMAX>
+__device__ bool warp_chol(double *G, int r) {
     const int lane = threadIdx.x & 31;
-    double g[RMAX], x[RMAX], invd[RMAX];
+    double g[RMAX];
 #pragma unroll
     for (int i = 0; i < RMAX; i++) g[i] = (i < r && lane < r) ? G[i * r + lane] : 0.0;
     const double g00 = __shfl_sync(0xffffffffu, g[0], 0);
@@ -139,7 +139,6 @@ __device__ bool warp_chol_inv(double *G, double *Rinv, int r) {
         if (!(d > 1e-28 * g00)) ok = false;
         const double rkk = sqrt(fmax(d, 1e-300));
         const double inv = 1.0 / rkk;
-        invd[k] = inv;
         if (lane > k) g[k] *= inv;
         if (lane == k) g[k] = rkk;
 #pragma unroll
@@ -149,60 +148,23 @@ __device__ bool warp_chol_inv(double *G, double *Rinv, int r) {
             if (lane >= i) g[i] = fma(-rki, g[k], g[i]);
         }
     }
-    if constexpr (!INV) {
-        if (lane < r) {
+    if (lane < r) {
 #pragma unroll
-            for (int i = 0; i < RMAX; i++)
-                if (i < r) G[i * r + lane] = i <= lane ? g[i] : 0.0;
-        }
-        __syncwarp();
-        return ok;
-    } else {
-        // Column `lane` of R^{-1} by back substitution; x[j] = 0 for j > lane.
-#pragma unroll
-        for (int i = 0; i < RMAX; i++) x[i] = (i == lane) ? invd[i] : 0.0;
-#pragma unroll
-        for (int i = RMAX - 2; i >= 0; i--) {
-            if (i >= r - 1) continue;
-            double sacc = 0.0;
-#pragma unroll
-            for (int j = i + 1; j < RMAX; j++) {
-                if (j >= r) break;
-                const double rij = __shfl_sync(0xffffffffu, g[i], j);
-                sacc = fma(rij, x[j], sacc);
-            }
-            if (i < lane) x[i] = -sacc * invd[i];
-        }
-        if (lane < r) {
-#pragma unroll
-            for (int i = 0; i < RMAX; i++)
-                if (i < r) {
-                    Rinv[i * r + lane] = x[i];
-                    G[i * r + lane] = i <= lane ? g[i] : 0.0;
-                }
-        }
-        __syncwarp();
-        return ok;
+        for (int i = 0; i < RMAX; i++)
+            if (i < r) G[i * r + lane] = i <= lane ? g[i] : 0.0;
     }
+    __syncwarp();
+    return ok;
 }
 
-// Subspace iteration L <- orth(S L), `iters` times, one CTA.  S (n x n,
-// symmetric) is staged in shared memory -- whole when it fits, as its packed
-// upper triangle for n up to ~220, else read from L2.  L and Z (n x r) live in
-// shared memory when they fit.  Intermediate steps orthonormalise with one
-// CholeskyQR pass (only conditioning matters there), the last step with two
-// (CholeskyQR2, orthonormal to FP64 rounding); a Cholesky breakdown
-// (rank-deficient S L) switches that step to Householder.
-enum { S_GLOBAL = 0, S_FULL = 1, S_PACKED = 2 };
-
-__device__ __forceinline__ double s_at(const double *S, int64_t n, int mode, int64_t i,
-                                       int64_t k) {
-    if (mode == S_PACKED) {
-        const int64_t a = i < k ? i : k, b = i < k ? k : i;
-        return S[a + b * (b + 1) / 2];
-    }
-    return S[i + n * k];
-}
+// Subspace iteration L <- orth(S L), `iters` times, one CTA: more than 256 rows (fewer
+// go to subspace_cluster_kernel), up to 32 columns.  S (n x n, symmetric) is read
+// from L2 for every product, which bounds it (n = 256, before the cluster kernel took
+// that size: 112 us for 12 columns and 5 steps); L and Z (n x r) live in shared memory
+// when they fit.  Intermediate steps orthonormalise with one CholeskyQR pass (only
+// conditioning matters there), the last step with two (CholeskyQR2, orthonormal to
+// FP64 rounding); a Cholesky breakdown (rank-deficient S L) switches that step to
+// Householder.
 
 // Forward substitution Q[i, :] = Z[i, :] R^{-1} for every row i (R upper,
 // row-major r x r in smem, Rinv_diag its reciprocal diagonal), one thread per
@@ -227,37 +189,19 @@ __device__ __forceinline__ void rows_trsm(const double *Z, double *Q, int64_t n,
 }
 
 template <int RMAX>
-__global__ void __launch_bounds__(LA_NT) subspace_kernel(const double *Sg, int64_t n,
+__global__ void __launch_bounds__(LA_NT) subspace_kernel(const double *S, int64_t n,
                                                          double *Lg, int64_t r, int iters,
-                                                         double *work, int s_mode,
-                                                         int zl_in_smem, int *flag) {
+                                                         double *work, int zl_in_smem,
+                                                         int *flag) {
     extern __shared__ __align__(16) double sm[];
     __shared__ double red[33];
     __shared__ int bad;
     const int t = threadIdx.x;
-    double *G = sm;                // r*r
-    double *Ri = sm + r * r;       // r*r (unused scratch for the Cholesky helper)
-    double *cur = sm + 2 * r * r;  // after the two r x r blocks
-    const double *S = Sg;
-    if (s_mode == S_FULL) {
-        double *Ss = cur;
-        for (int64_t e = t; e < n * n; e += blockDim.x) Ss[e] = Sg[e];
-        S = Ss;
-        cur += n * n;
-    } else if (s_mode == S_PACKED) {
-        double *Ss = cur;
-        const int64_t np = n * (n + 1) / 2;
-        for (int64_t e = t; e < n * n; e += blockDim.x) {
-            const int64_t i = e % n, k = e / n;
-            if (i <= k) Ss[i + k * (k + 1) / 2] = Sg[e];
-        }
-        S = Ss;
-        cur += (np + 1) & ~int64_t(1);
-    }
+    double *G = sm;  // r*r
     double *L, *Z;
     if (zl_in_smem) {
-        L = cur;
-        Z = cur + n * r;
+        L = sm + r * r;
+        Z = L + n * r;
     } else {
         L = work;
         Z = work + n * r;
@@ -293,7 +237,7 @@ __global__ void __launch_bounds__(LA_NT) subspace_kernel(const double *Sg, int64
         }
         __syncthreads();
         if (t < 32) {
-            const bool ok = warp_chol_inv<RMAX, false>(G, Ri, (int)r);
+            const bool ok = warp_chol<RMAX>(G, (int)r);
             if (t == 0) bad = ok ? 0 : 1;
         }
         __syncthreads();
@@ -315,7 +259,7 @@ __global__ void __launch_bounds__(LA_NT) subspace_kernel(const double *Sg, int64
             const bool h1 = c0 + 1 < r, h2 = c0 + 2 < r, h3 = c0 + 3 < r;
 #pragma unroll 4
             for (int64_t k = 0; k < n; k++) {
-                const double sv = s_at(S, n, s_mode, i, k);
+                const double sv = S[i + n * k];
                 a0 = fma(sv, l0[k], a0);
                 if (h1) a1 = fma(sv, l0[k + n], a1);
                 if (h2) a2 = fma(sv, l0[k + 2 * n], a2);
@@ -358,7 +302,7 @@ __global__ void __launch_bounds__(LA_NT) subspace_kernel(const double *Sg, int64
             for (int64_t e = t; e < n * r; e += blockDim.x) {
                 const int64_t i = e % n, c = e / n;
                 double acc = 0.0;
-                for (int64_t k = 0; k < n; k++) acc = fma(s_at(S, n, s_mode, i, k), L[k + c * n], acc);
+                for (int64_t k = 0; k < n; k++) acc = fma(S[i + n * k], L[k + c * n], acc);
                 hwork[e] = acc;
             }
             __syncthreads();
@@ -1382,30 +1326,17 @@ void subspace_iter(dt_ctx *ctx, const double *S, int64_t n, double *L, int64_t r
         subspace_mma(ctx, one, 1, iters, flag, plain);
         return;
     }
-    const size_t base = 2 * r * r * sizeof(double);
-    const size_t full_bytes = n * n * sizeof(double);
-    const size_t packed_bytes = ((n * (n + 1) / 2 + 1) & ~int64_t(1)) * sizeof(double);
-    const size_t zl_bytes = 2 * n * r * sizeof(double);
-    const size_t cap = 220 * 1024;
-    int s_mode = S_GLOBAL;
-    size_t s_bytes = 0;
-    if (base + full_bytes + zl_bytes <= cap) {
-        s_mode = S_FULL;
-        s_bytes = full_bytes;
-    } else if (base + packed_bytes + zl_bytes <= cap) {
-        s_mode = S_PACKED;
-        s_bytes = packed_bytes;
-    }
-    const int zl_in = base + s_bytes + zl_bytes <= cap;
-    const size_t smem = base + s_bytes + (zl_in ? zl_bytes : 0);
+    const size_t zl_bytes = 2 * n * r * sizeof(double), base = r * r * sizeof(double);
+    const int zl_in = base + zl_bytes <= 220 * 1024;
+    const size_t smem = base + (zl_in ? zl_bytes : 0);
     if (r <= 16) {
         smem_limit(ctx, subspace_kernel<16>, smem);
-        DT_LAUNCH(ctx, subspace_kernel<16>, 1, LA_NT, smem, S, n, L, r, iters, work, s_mode,
-                  zl_in, flag);
+        DT_LAUNCH(ctx, subspace_kernel<16>, 1, LA_NT, smem, S, n, L, r, iters, work, zl_in,
+                  flag);
     } else {
         smem_limit(ctx, subspace_kernel<32>, smem);
-        DT_LAUNCH(ctx, subspace_kernel<32>, 1, LA_NT, smem, S, n, L, r, iters, work, s_mode,
-                  zl_in, flag);
+        DT_LAUNCH(ctx, subspace_kernel<32>, 1, LA_NT, smem, S, n, L, r, iters, work, zl_in,
+                  flag);
     }
 }
 
