@@ -182,3 +182,24 @@ def test_batched_results_do_not_depend_on_the_launch_shape(ctx, lo, hi):
     for t in (0, 17, 59):
         U, G, e, _ = ctx.hooi_batched([tensors[t]], [ranks[t]], [U0[t]], sweeps=4)
         assert e[0] == outs[0][2][t] and np.array_equal(G[0], outs[0][1][t])
+
+
+def test_inverse_root_over_all_exponents(ctx):
+    """The factorisation's 1 / sqrt(d), an approximation refined by a series, seen from
+    outside: a rank-1 factor is Z / sqrt(Z^T Z) by one such root, so its length is 1 up
+    to the rounding of a sum of at most 7 squares, of the root and of the product:
+    below 9 half units in the last place, 1e-15.  X scaled by 2^-120 to 2^120 takes d
+    = |X|^4 or so over 2^-480 to 2^480, with other mantissas each time."""
+    rng = np.random.default_rng(12)
+    shape = (7, 5, 6)
+    tensors, U0 = [], []
+    for k in range(-120, 121):
+        X = np.asfortranarray(rng.standard_normal(shape) * 2.0 ** k, dtype=np.float32)
+        tensors.append(X)
+        U0.append([np.linalg.qr(rng.standard_normal((s, 1)))[0] for s in shape])
+    U, G, relerr, _ = ctx.hooi_batched(tensors, [(1, 1, 1)] * len(tensors), U0, sweeps=2)
+    assert np.all(np.isfinite(relerr))
+    for t in range(len(tensors)):
+        for u in U[t]:
+            norm = np.sqrt(np.sum(u.astype(np.longdouble) ** 2))
+            assert abs(norm - 1) <= 1e-15, (t - 120, norm - 1)
