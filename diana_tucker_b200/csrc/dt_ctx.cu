@@ -170,8 +170,11 @@ void DevArena::give(void *p) {
 }
 
 bool release_idle(dt_ctx *ctx) {
-    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(ctx->stream, &st) != cudaSuccess) cudaGetLastError();
+    cudaStreamCaptureStatus st;
+    if (cudaStreamIsCapturing(ctx->stream, &st) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
     if (st != cudaStreamCaptureStatusNone) return false;
     // A running call holds a reference of its own to the plan it uses.
     auto &kept = ctx->hooi_plans_fp64;

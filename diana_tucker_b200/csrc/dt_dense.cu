@@ -841,14 +841,17 @@ void gram_f64(dt_ctx *ctx, const double *X, int64_t L, int64_t I, int64_t B, dou
     const int64_t target = (wide ? 1LL : 2LL) * ctx->num_sms;
     int64_t nsplit = std::max<int64_t>(1, std::min<int64_t>(target / pairs, (a.K + 2 * GR_K - 1) / (2 * GR_K)));
     if (scratch) nsplit = std::max<int64_t>(1, std::min<int64_t>(nsplit, scratch_doubles / (64LL * a.tiles)));
+    // A split's columns are counted in 32 bits.
+    const int64_t least = std::max<int64_t>(1, (a.K + (int64_t(1) << 30) - 1) >> 30);
+    nsplit = std::max(nsplit, least);
     DevMem part;
-    for (;; nsplit /= 2) {
+    for (;; nsplit = std::max(least, nsplit / 2)) {
         a.kchunk = std::max<int64_t>(GR_K, ((a.K + nsplit - 1) / nsplit + GR_K - 1) / GR_K * GR_K);
         nsplit = std::max<int64_t>(1, (a.K + a.kchunk - 1) / a.kchunk);
         // Fewer splits where there is no room for their tiles; one needs none.
-        if (nsplit == 1 || scratch ||
-            part.try_alloc(ctx, (size_t)nsplit * a.tiles * 64 * sizeof(double)))
-            break;
+        const size_t bytes = (size_t)nsplit * a.tiles * 64 * sizeof(double);
+        if (nsplit == 1 || scratch || part.try_alloc(ctx, bytes)) break;
+        if (nsplit <= least) part.alloc(ctx, bytes);  // (fails)
     }
     if (nsplit > 1) a.part = scratch ? scratch : part.as<double>();
     const dim3 grid((unsigned)pairs, (unsigned)nsplit);
