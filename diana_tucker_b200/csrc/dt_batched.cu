@@ -22,10 +22,11 @@
 // out as the next products' fragments, from the product to the new factor.  Every
 // sum goes in an order of the tensor's own (over its 8 x 8 tiles; over 512 classes
 // of entries, as many as the largest block has threads): the results are the same
-// bit for bit for every block size and packing, whatever the tuner takes.  4096 tensors (modes 8 to 64,
-// ranks 2 to 8, 10 sweeps): 11.4 ms, of it about half the two passes over X at 0.8
-// of the FP64 tensor rate (ranks padded to 8 columns); 100 tensors 1.14 ms.  With
-// one FMA chain per thread and entry on the CUDA cores 23.3 and 2.4 ms.
+// bit for bit for every block size and packing, whatever the tuner takes.  4096
+// tensors (modes 8 to 64, ranks 2 to 8, 10 sweeps): 11.5 ms, of it about half the
+// two passes over X at 0.8 of the FP64 tensor rate (ranks padded to 8 columns); 100
+// tensors 1.14 ms.  With one FMA chain per thread and entry on the CUDA cores 23.3
+// and 2.4 ms.
 //
 // Autotuning.  The block size (128, 256, 512 threads) and the packing (one
 // tensor per CTA; pairs, and quads, of the tensors small enough to share the
